@@ -531,7 +531,7 @@ extern "C" int dftcuda_kctx_destroy(dftcuda_kctx* c) {
   void* ptrs[] = {c->d_plane_off, c->d_pw_idx, c->d_pw_spos, c->d_slot_xpos, c->d_kinetic, c->d_gcart, c->d_vt,
                   c->d_vt32, c->d_box, c->d_coef, c->d_coef2, c->d_gemm_ws, c->d_x, c->d_y, c->d_rho, c->d_w,
                   c->d_pwmap, c->d_stick_off, c->d_stick_y, c->d_slot_of_x, c->d_tw4x64, c->d_tw4x32,
-                  c->d_tw4p64, c->d_tw4p32, c->d_err, c->d_mlp, c->d_vstage, c->d_st_sy, c->d_st_map, c->d_st_sox,
+                  c->d_tw4p64, c->d_tw4p32, c->d_err, c->d_mlp, c->d_vstage, c->d_st_of, c->d_st_map, c->d_st_sox,
                   c->d_twz64, c->d_twz32, c->d_twx64, c->d_twx32, c->d_vn, c->d_vn32};
   for (void* p : ptrs)
     if (p) cudaFree(p);

@@ -133,7 +133,7 @@ struct dftcuda_kctx {
   // Stick-layout passes (local_sticks.cu), used when sticks64 / sticks32 is set for the precision.
   bool sticks64 = false, sticks32 = false;
   int n_st = 0;                // sticks: (x, y) pairs holding plane waves, in slot order
-  int* d_st_sy = nullptr;      // [n_st] slot << 16 | y
+  int* d_st_of = nullptr;      // [ny][n_act] stick of (y, slot) or -1
   int* d_st_map = nullptr;     // [n_st][nz] plane-wave index of (stick, z) or -1
   int* d_st_sox = nullptr;     // [nx] slot of each x frequency or -1
   void* d_twz64 = nullptr;     // twiddles of the z length

@@ -9,12 +9,11 @@
 //  k_stick_inv   32 sticks per CTA: gather the plane waves (zero elsewhere) and run the inverse z
 //                transform of each stick in shared memory; rows r of S in the four-step's
 //                digit-permuted z order (r = (z mod N1) N2 + z / N1).
-//  k_zplane      one z-plane per CTA (a few columns in turn): scatter the plane's stick values into
-//                Q[slot][y], inverse y transform of every slot row, then per y line the inverse x
+//  k_zplane      one z-plane per CTA (a few columns in turn): inverse y transform of every slot row,
+//                reading the plane's sticks, into Q[slot][y]; then per y line the inverse x
 //                transform over the active slots, x V(r), the forward x transform back to the active
 //                slots (one warp handles a few lines, exchanges through a per-warp buffer), then the
-//                forward y transform and the gather of the stick values.  Everything between the
-//                stick row load and store stays in shared memory.
+//                forward y transform, writing the sticks.  Everything between stays in shared memory.
 //  k_stick_fwd   forward z transform of each stick, then per plane wave y = kinetic x + (1/N) psi(G).
 //
 // Each transform is the four-step register DFT of fft_reg.cuh.  The inverse runs with the split
@@ -37,9 +36,9 @@ namespace {
 constexpr int kStickTile = 32;    // sticks per CTA of the stick passes
 constexpr int kStickPad = kStickTile + 1;
 constexpr int kStickThreads = 256;
-// warps of a z-plane CTA: FP64 lines need more registers per lane (launch bound 384 threads = 170
-// registers), FP32 ones fit 512 threads
-template <typename T> constexpr int plane_max_warps() { return sizeof(T) == 8 ? 12 : 16; }
+// warps of a z-plane CTA (128 registers per lane)
+template <typename T> constexpr int plane_max_warps() { return 16; }
+template <typename T> constexpr int kDensityWarps() { return 16; }
 
 template <typename T> __device__ __forceinline__ cplx<T> twl(const cplx<T>* tw, int e, T sg) {
   cplx<T> w = tw[e];
@@ -179,109 +178,94 @@ __global__ void __launch_bounds__(kStickThreads) k_stick_fwd(const cplx<T>* __re
 // ------------------------------------------------------------------------------------------
 // Pass 2: one z-plane per CTA.
 // ------------------------------------------------------------------------------------------
-// Exchange layout of the H|psi> z-plane pass's x lines.  The inverse half keeps the [N1][N2] layout
-// (stride N2); the forward half stores its [N2][N1] intermediate with row stride R and each line's
-// buffer spans SF entries, chosen per length so that the 16-byte accesses of a quarter warp fall on
-// distinct bank groups (for 108: 222 wavefronts per line group against 330 with R = N1, S = 113; the
-// forward read with stride N1 = 12 was 3.25-way conflicted).
-struct XStrides {
-  int R, SF;
-};
-constexpr XStrides xline_strides(int n) {
-  switch (n) {
-    case 20: return {5, 20};
-    case 24: return {6, 27};
-    case 27: return {9, 27};
-    case 30: return {9, 45};
-    case 32: return {9, 36};
-    case 36: return {9, 54};
-    case 40: return {9, 45};
-    case 45: return {9, 45};
-    case 48: return {9, 54};
-    case 60: return {17, 85};
-    case 64: return {9, 72};
-    case 72: return {9, 72};
-    case 75: return {17, 85};
-    case 80: return {11, 88};
-    case 90: return {17, 153};
-    case 96: return {13, 104};
-    case 100: return {13, 130};
-    case 108: return {17, 153};
-    case 120: return {13, 130};
-    case 128: return {17, 136};
-    default: return {0, 0};
-  }
-}
-
+// Exchange buffer of one x line: N1 rows of N2 entries, row stride RP odd, so that a quarter warp's
+// 16-byte accesses fall on distinct bank groups both along a row (lanes over t) and down a column of rows
+// (lanes over k1); line stride S = N2 modulo 8 entries, which continues the pattern across a warp's lines.
 template <int NX> struct PlaneXGeom {
   static constexpr int N1 = Split<NX>::N1, N2 = Split<NX>::N2;
   static constexpr int LW = 32 / N2;                                 // lines per warp
   static constexpr int Q = (N1 + N2 - 1) / N2;                       // phase-2 rows per lane
-  static constexpr int S = NX + ((N2 - NX) % 8 + 8) % 8;             // exchange stride per line
-  static constexpr int R = xline_strides(NX).R;    // forward row stride (H|psi> pass)
-  static constexpr int SF = xline_strides(NX).SF;  // per-line exchange entries (H|psi> pass)
-  static_assert(R >= N1 && SF >= N2 * R && SF >= NX, "x-line exchange strides");
+  static constexpr int RP = N2 | 1;
+  static constexpr int S = N1 * RP + ((N2 - N1 * RP) % 8 + 8) % 8;
 };
 
+// The inverse y transform of a plane's active slots, the plane's sticks read from Srow (st_of[y][slot]: the
+// stick at (slot, y) or -1) by step A itself; position k1 + N1 k2 ends at Q[slot][k1 N2 + k2].
 template <typename T, int N>
-__global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>* __restrict__ S, int n_st, const int* __restrict__ st_sy,
+__device__ __forceinline__ void plane_y_inverse(const cplx<T>* Srow, const int* __restrict__ st_of, int n_act, cplx<T>* Q, const cplx<T>* twa) {
+  using C = cplx<T>;
+  constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2, QS = N + 1;
+  for (int w = threadIdx.x; w < N2 * n_act; w += blockDim.x) {  // step A: task (t, slot), lanes over slots
+    const int sl = w % n_act, tt = w / n_act;
+    C* q = Q + sl * QS;
+    C v[N1];
+#pragma unroll
+    for (int j = 0; j < N1; ++j) {
+      const int g = __ldg(st_of + (j * N2 + tt) * n_act + sl);
+      v[j] = g >= 0 ? Srow[g] : mk<C>(0.0, 0.0);
+    }
+    RegDft<T, N1>::run(v, (T)1);
+    q[tt] = v[0];
+#pragma unroll
+    for (int k1 = 1; k1 < N1; ++k1) q[k1 * N2 + tt] = cmul(v[k1], twa[k1 * N2 + tt]);
+  }
+  __syncthreads();
+  for (int w = threadIdx.x; w < N1 * n_act; w += blockDim.x) {  // step B
+    const int sl = w % n_act, k1 = w / n_act;
+    C* q = Q + sl * QS + k1 * N2;
+    C u[N2];
+#pragma unroll
+    for (int j = 0; j < N2; ++j) u[j] = q[j];
+    RegDft<T, N2>::run(u, (T)1);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) q[k2] = u[k2];
+  }
+  __syncthreads();
+}
+
+// Per (z plane, column): inverse y, then per y line inverse x, x V(r), forward x, then forward y.  The
+// plane's sticks are read by the first step and written by the last one; the x lines exchange through a
+// per-warp buffer in which a lane's rows stay its own from the inverse step B to the forward step A, so one
+// row at a time is in registers and 16 FP64 warps fit an SM (128 registers; the two rows that a transposed
+// layout held at once allowed 12).  The four-step twiddles sit in shared memory in the order the lanes
+// read them.  Bound by shared memory / L1 wavefronts and the FP64 pipe, about equally.
+template <typename T, int N>
+__global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>* __restrict__ S, int n_st, const int* __restrict__ st_of,
                                                                      int n_act, const int* __restrict__ slot_of_x,
                                                                      const T* __restrict__ Vn, int n1z, int n2z, int ncols,
                                                                      int cols_per_cta, const cplx<T>* __restrict__ tw) {
   using C = cplx<T>;
   using G = PlaneXGeom<N>;
-  constexpr int N1 = G::N1, N2 = G::N2, LW = G::LW, QR = G::Q, SX = G::SF, RF = G::R;
+  constexpr int N1 = G::N1, N2 = G::N2, LW = G::LW, QR = G::Q, RP = G::RP;
   constexpr int QS = N + 1;  // Q row stride: odd, so lanes over slots hit distinct banks
   extern __shared__ __align__(16) unsigned char smraw[];
-  C* Q = reinterpret_cast<C*>(smraw);  // [n_act][QS]
+  C* twa = reinterpret_cast<C*>(smraw);  // [k1][t] = w^(t k1)
+  C* twb = twa + N;                      // [k2][k1] = w^-(k1 k2)
+  C* Q = twb + N;                        // [n_act][QS]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  C* Bw = Q + (size_t)n_act * QS + (size_t)warp * LW * SX;  // this warp's exchange buffer [LW][SX]
+  C* Bw = Q + (size_t)n_act * QS + (size_t)warp * LW * G::S;  // this warp's exchange buffer
   const int z = blockIdx.x;
   const int r = (z % n1z) * n2z + z / n1z;  // storage row of z in S
   const int c0 = blockIdx.y * cols_per_cta;
   const int c1 = min(ncols, c0 + cols_per_cta);
-  const int nq = n_act * QS;
   const T* Vz = Vn + (long)z * N * N;
   const int L = lane / N2, t = lane - L * N2;
   const bool lane_ok = L < LW;
-  C* B = Bw + (lane_ok ? L : 0) * SX;
+  C* B = Bw + (lane_ok ? L : 0) * G::S;
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    twa[i] = twl<T>(tw, ((i / N2) * (i % N2)) % N, (T)1);
+    twb[i] = twl<T>(tw, ((i / N1) * (i % N1)) % N, (T)-1);
+  }
+  int so[N1];  // Q offsets of this lane's slots along x, or -1
+#pragma unroll
+  for (int m = 0; m < N1; ++m) {
+    const int sm = lane_ok ? __ldg(slot_of_x + t + N2 * m) : -1;
+    so[m] = sm >= 0 ? sm * QS : -1;
+  }
   for (int c = c0; c < c1; ++c) {
     C* Srow = S + ((long)c * gridDim.x + r) * n_st;
-    __syncthreads();  // the previous column's gather has read Q
-    for (int i = threadIdx.x; i < nq; i += blockDim.x) Q[i] = mk<C>(0.0, 0.0);
-    __syncthreads();
-    for (int g = threadIdx.x; g < n_st; g += blockDim.x) {
-      const int sy = __ldg(st_sy + g);
-      Q[(sy >> 16) * QS + (sy & 0xffff)] = Srow[g];
-    }
-    __syncthreads();
-    // inverse y, step A: task (t, slot), lanes over slots
-    for (int w = threadIdx.x; w < N2 * n_act; w += blockDim.x) {
-      const int sl = w % n_act, tt = w / n_act;
-      C* q = Q + sl * QS;
-      C v[N1];
-#pragma unroll
-      for (int j = 0; j < N1; ++j) v[j] = q[j * N2 + tt];
-      RegDft<T, N1>::run(v, (T)1);
-#pragma unroll
-      for (int k1 = 1; k1 < N1; ++k1)
-        if (tt) v[k1] = cmul(v[k1], twl<T>(tw, (tt * k1) % N, (T)1));
-#pragma unroll
-      for (int k1 = 0; k1 < N1; ++k1) q[k1 * N2 + tt] = v[k1];
-    }
-    __syncthreads();
-    // inverse y, step B: position k1 + N1 k2 lands at column k1 N2 + k2
-    for (int w = threadIdx.x; w < N1 * n_act; w += blockDim.x) {
-      const int sl = w % n_act, k1 = w / n_act;
-      C* q = Q + sl * QS + k1 * N2;
-      C u[N2];
-#pragma unroll
-      for (int j = 0; j < N2; ++j) u[j] = q[j];
-      RegDft<T, N2>::run(u, (T)1);
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) q[k2] = u[k2];
-    }
-    __syncthreads();
+    __syncthreads();  // the previous column's last step has read Q
+    plane_y_inverse<T, N>(Srow, st_of, n_act, Q, twa);
     // x lines: LW lines per warp; line y sits in column col(y) of every active slot
     for (int lt = warp; lt * LW < N; lt += nwarp) {
       const int yl = lt * LW + L;
@@ -290,56 +274,42 @@ __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>
       {  // inverse step A over x = t + N2 m
         C v[N1];
 #pragma unroll
-        for (int m = 0; m < N1; ++m) {
-          const int sm = lv ? __ldg(slot_of_x + t + N2 * m) : -1;
-          v[m] = sm >= 0 ? Q[sm * QS + col] : mk<C>(0.0, 0.0);
-        }
+        for (int m = 0; m < N1; ++m) v[m] = so[m] >= 0 ? Q[so[m] + col] : mk<C>(0.0, 0.0);
         RegDft<T, N1>::run(v, (T)1);
-#pragma unroll
-        for (int k1 = 1; k1 < N1; ++k1)
-          if (t) v[k1] = cmul(v[k1], twl<T>(tw, (t * k1) % N, (T)1));
         if (lane_ok) {
+          B[t] = v[0];
 #pragma unroll
-          for (int k1 = 0; k1 < N1; ++k1) B[k1 * N2 + t] = v[k1];
-        }
-      }
-      __syncwarp();
-      C u[QR][N2];
-#pragma unroll
-      for (int q = 0; q < QR; ++q) {
-        const int k1 = t + N2 * q;
-        if (lane_ok && k1 < N1) {
-#pragma unroll
-          for (int j = 0; j < N2; ++j) u[q][j] = B[k1 * N2 + j];
+          for (int k1 = 1; k1 < N1; ++k1) B[k1 * RP + t] = cmul(v[k1], twa[k1 * N2 + t]);
         }
       }
       __syncwarp();
 #pragma unroll
-      for (int q = 0; q < QR; ++q) {  // inverse step B, x V(r), forward step A (split swapped)
+      for (int q = 0; q < QR; ++q) {  // inverse step B, x V(r), forward step A (split swapped), row k1 in place
         const int k1 = t + N2 * q;
-        if (lane_ok && k1 < N1) {
-          RegDft<T, N2>::run(u[q], (T)1);
+        if (lv && k1 < N1) {
+          C* row = B + k1 * RP;
+          C u[N2];
 #pragma unroll
-          for (int k2 = 0; k2 < N2; ++k2) u[q][k2] = cscale(u[q][k2], lv ? __ldg(Vz + (long)yl * N + k1 + N1 * k2) : (T)0);
-          RegDft<T, N2>::run(u[q], (T)-1);
+          for (int j = 0; j < N2; ++j) u[j] = row[j];
+          RegDft<T, N2>::run(u, (T)1);
+          const T* Vy = Vz + (long)yl * N + k1;
 #pragma unroll
-          for (int kf = 1; kf < N2; ++kf)
-            if (k1) u[q][kf] = cmul(u[q][kf], twl<T>(tw, (k1 * kf) % N, (T)-1));
+          for (int k2 = 0; k2 < N2; ++k2) u[k2] = cscale(u[k2], __ldg(Vy + N1 * k2));
+          RegDft<T, N2>::run(u, (T)-1);
+          row[0] = u[0];
 #pragma unroll
-          for (int kf = 0; kf < N2; ++kf) B[kf * RF + k1] = u[q][kf];
+          for (int kf = 1; kf < N2; ++kf) row[kf] = cmul(u[kf], twb[kf * N1 + k1]);
         }
       }
       __syncwarp();
       {  // forward step B for frequency index t: outputs x = t + N2 m
         C v[N1];
 #pragma unroll
-        for (int tf = 0; tf < N1; ++tf) v[tf] = lane_ok ? B[t * RF + tf] : mk<C>(0.0, 0.0);
+        for (int tf = 0; tf < N1; ++tf) v[tf] = lane_ok ? B[tf * RP + t] : mk<C>(0.0, 0.0);
         RegDft<T, N1>::run(v, (T)-1);
 #pragma unroll
-        for (int m = 0; m < N1; ++m) {
-          const int sm = lv ? __ldg(slot_of_x + t + N2 * m) : -1;
-          if (sm >= 0) Q[sm * QS + col] = v[m];
-        }
+        for (int m = 0; m < N1; ++m)
+          if (lv && so[m] >= 0) Q[so[m] + col] = v[m];
       }
       __syncwarp();
     }
@@ -352,28 +322,24 @@ __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>
 #pragma unroll
       for (int j = 0; j < N2; ++j) v[j] = q[j];
       RegDft<T, N2>::run(v, (T)-1);
+      q[0] = v[0];
 #pragma unroll
-      for (int k = 1; k < N2; ++k)
-        if (tt) v[k] = cmul(v[k], twl<T>(tw, (tt * k) % N, (T)-1));
-#pragma unroll
-      for (int k = 0; k < N2; ++k) q[k] = v[k];
+      for (int k = 1; k < N2; ++k) q[k] = cmul(v[k], twb[k * N1 + tt]);
     }
     __syncthreads();
-    // forward y, step B: task (k < N2, slot), frequency k + N2 m lands at column k + N2 m
+    // forward y, step B: task (k < N2, slot), frequencies k + N2 m to their sticks
     for (int w = threadIdx.x; w < N2 * n_act; w += blockDim.x) {
       const int sl = w % n_act, k = w / n_act;
-      C* q = Q + sl * QS;
+      const C* q = Q + sl * QS;
       C u[N1];
 #pragma unroll
       for (int tt = 0; tt < N1; ++tt) u[tt] = q[tt * N2 + k];
       RegDft<T, N1>::run(u, (T)-1);
 #pragma unroll
-      for (int m = 0; m < N1; ++m) q[m * N2 + k] = u[m];
-    }
-    __syncthreads();
-    for (int g = threadIdx.x; g < n_st; g += blockDim.x) {
-      const int sy = __ldg(st_sy + g);
-      Srow[g] = Q[(sy >> 16) * QS + (sy & 0xffff)];
+      for (int m = 0; m < N1; ++m) {
+        const int g = __ldg(st_of + (k + N2 * m) * n_act + sl);
+        if (g >= 0) Srow[g] = u[m];
+      }
     }
   }
 }
@@ -388,100 +354,80 @@ template <int N> __host__ __device__ constexpr int density_plane_words() { retur
 // added to the global density once at the end (several CTAs share a plane: atomics).
 // ------------------------------------------------------------------------------------------
 template <typename T, int N>
-__global__ void __launch_bounds__(256, 1) k_zplane_density(const cplx<T>* __restrict__ S, int n_st, const int* __restrict__ st_sy,
+__global__ void __launch_bounds__(kDensityWarps<T>() * 32, 1) k_zplane_density(const cplx<T>* __restrict__ S, int n_st, const int* __restrict__ st_of,
                                                            int n_act, const int* __restrict__ slot_of_x, int n1z, int n2z, int ncols,
                                                            int cols_per_cta, const cplx<T>* __restrict__ tw,
                                                            const double* __restrict__ wgt, double inv_vol, double* __restrict__ rho) {
   using C = cplx<T>;
   using G = PlaneXGeom<N>;
-  constexpr int N1 = G::N1, N2 = G::N2, LW = G::LW, QR = G::Q, SX = G::S;
+  constexpr int N1 = G::N1, N2 = G::N2, LW = G::LW, QR = G::Q, RP = G::RP;
   constexpr int QS = N + 1;
   extern __shared__ __align__(16) unsigned char smraw[];
-  double* R = reinterpret_cast<double*>(smraw);               // [N][N] density plane, x fastest
-  C* Q = reinterpret_cast<C*>(R + density_plane_words<N>());  // [n_act][QS], 16-byte aligned
+  double* R = reinterpret_cast<double*>(smraw);                 // [N][N] density plane, x fastest
+  C* twa = reinterpret_cast<C*>(R + density_plane_words<N>());  // [k1][t] = w^(t k1), 16-byte aligned
+  C* Q = twa + N;                                               // [n_act][QS]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  C* Bw = Q + (size_t)n_act * QS + (size_t)warp * LW * SX;
+  T* Bw = reinterpret_cast<T*>(Q + (size_t)n_act * QS) + (size_t)warp * LW * G::S;  // one part at a time
   const int z = blockIdx.x;
   const int r = (z % n1z) * n2z + z / n1z;
   const int c0 = blockIdx.y * cols_per_cta;
   const int c1 = min(ncols, c0 + cols_per_cta);
-  const int nq = n_act * QS;
   const int L = lane / N2, t = lane - L * N2;
   const bool lane_ok = L < LW;
-  C* B = Bw + (lane_ok ? L : 0) * SX;
+  T* B = Bw + (lane_ok ? L : 0) * G::S;
+  for (int i = threadIdx.x; i < N; i += blockDim.x) twa[i] = twl<T>(tw, ((i / N2) * (i % N2)) % N, (T)1);
   for (int i = threadIdx.x; i < N * N; i += blockDim.x) R[i] = 0.0;
+  int so[N1];
+#pragma unroll
+  for (int m = 0; m < N1; ++m) {
+    const int sm = lane_ok ? __ldg(slot_of_x + t + N2 * m) : -1;
+    so[m] = sm >= 0 ? sm * QS : -1;
+  }
   for (int c = c0; c < c1; ++c) {
     const C* Srow = S + ((long)c * gridDim.x + r) * n_st;
     const double wc = __ldg(wgt + c) * inv_vol;
     __syncthreads();
-    for (int i = threadIdx.x; i < nq; i += blockDim.x) Q[i] = mk<C>(0.0, 0.0);
-    __syncthreads();
-    for (int g = threadIdx.x; g < n_st; g += blockDim.x) {
-      const int sy = __ldg(st_sy + g);
-      Q[(sy >> 16) * QS + (sy & 0xffff)] = Srow[g];
-    }
-    __syncthreads();
-    for (int w = threadIdx.x; w < N2 * n_act; w += blockDim.x) {
-      const int sl = w % n_act, tt = w / n_act;
-      C* q = Q + sl * QS;
-      C v[N1];
-#pragma unroll
-      for (int j = 0; j < N1; ++j) v[j] = q[j * N2 + tt];
-      RegDft<T, N1>::run(v, (T)1);
-#pragma unroll
-      for (int k1 = 1; k1 < N1; ++k1)
-        if (tt) v[k1] = cmul(v[k1], twl<T>(tw, (tt * k1) % N, (T)1));
-#pragma unroll
-      for (int k1 = 0; k1 < N1; ++k1) q[k1 * N2 + tt] = v[k1];
-    }
-    __syncthreads();
-    for (int w = threadIdx.x; w < N1 * n_act; w += blockDim.x) {
-      const int sl = w % n_act, k1 = w / n_act;
-      C* q = Q + sl * QS + k1 * N2;
-      C u[N2];
-#pragma unroll
-      for (int j = 0; j < N2; ++j) u[j] = q[j];
-      RegDft<T, N2>::run(u, (T)1);
-#pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) q[k2] = u[k2];
-    }
-    __syncthreads();
+    plane_y_inverse<T, N>(Srow, st_of, n_act, Q, twa);
     for (int lt = warp; lt * LW < N; lt += nwarp) {
       const int yl = lt * LW + L;
       const bool lv = lane_ok && yl < N;
       const int col = lv ? (yl % N1) * N2 + yl / N1 : 0;
-      {
-        C v[N1];
+      C v[N1];
 #pragma unroll
-        for (int m = 0; m < N1; ++m) {
-          const int sm = lv ? __ldg(slot_of_x + t + N2 * m) : -1;
-          v[m] = sm >= 0 ? Q[sm * QS + col] : mk<C>(0.0, 0.0);
-        }
-        RegDft<T, N1>::run(v, (T)1);
+      for (int m = 0; m < N1; ++m) v[m] = so[m] >= 0 ? Q[so[m] + col] : mk<C>(0.0, 0.0);
+      RegDft<T, N1>::run(v, (T)1);
 #pragma unroll
-        for (int k1 = 1; k1 < N1; ++k1)
-          if (t) v[k1] = cmul(v[k1], twl<T>(tw, (t * k1) % N, (T)1));
+      for (int k1 = 1; k1 < N1; ++k1) v[k1] = cmul(v[k1], twa[k1 * N2 + (lane_ok ? t : 0)]);
+      // the line's exchange, real parts then imaginary parts
+      C u[QR][N2];
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
         if (lane_ok) {
 #pragma unroll
-          for (int k1 = 0; k1 < N1; ++k1) B[k1 * N2 + t] = v[k1];
+          for (int k1 = 0; k1 < N1; ++k1) B[k1 * RP + t] = part ? v[k1].y : v[k1].x;
         }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < QR; ++q) {
+          const int k1 = t + N2 * q;
+          if (lane_ok && k1 < N1) {
+#pragma unroll
+            for (int j = 0; j < N2; ++j) (part ? u[q][j].y : u[q][j].x) = B[k1 * RP + j];
+          }
+        }
+        __syncwarp();
       }
-      __syncwarp();
 #pragma unroll
       for (int q = 0; q < QR; ++q) {  // inverse step B: x = k1 + N1 k2, then the density
         const int k1 = t + N2 * q;
         if (lv && k1 < N1) {
-          C u[N2];
-#pragma unroll
-          for (int j = 0; j < N2; ++j) u[j] = B[k1 * N2 + j];
-          RegDft<T, N2>::run(u, (T)1);
+          RegDft<T, N2>::run(u[q], (T)1);
           double* Ry = R + (size_t)yl * N;
 #pragma unroll
           for (int k2 = 0; k2 < N2; ++k2)
-            Ry[k1 + N1 * k2] += wc * ((double)u[k2].x * (double)u[k2].x + (double)u[k2].y * (double)u[k2].y);
+            Ry[k1 + N1 * k2] += wc * ((double)u[q][k2].x * (double)u[q][k2].x + (double)u[q][k2].y * (double)u[q][k2].y);
         }
       }
-      __syncwarp();
     }
   }
   __syncthreads();
@@ -502,10 +448,13 @@ static constexpr int kSmemSticks = 227 * 1024;
 
 static size_t stick_smem(size_t cs, int nz) { return cs * (size_t)nz * kStickPad; }
 
+// Warps of a z-plane CTA: eight where two such CTAs share an SM (one's barriers under the other's work, and
+// fewer idle warps in the short y steps of small planes), else as many as fit one.
 template <int N> static int plane_warps(size_t cs, int n_act) {
   using G = PlaneXGeom<N>;
-  const size_t q = cs * (size_t)n_act * (N + 1);
-  const size_t per_warp = cs * (size_t)G::LW * G::SF;
+  const size_t q = cs * ((size_t)n_act * (N + 1) + 2 * N);
+  const size_t per_warp = cs * (size_t)G::LW * G::S;
+  if (2 * (q + 8 * per_warp + 1024) <= (size_t)kSmemSticks) return 8;
   const int maxw = cs == sizeof(double2) ? plane_max_warps<double>() : plane_max_warps<float>();
   if (q + per_warp > (size_t)kSmemSticks) return 0;
   return (int)std::min<size_t>(maxw, ((size_t)kSmemSticks - q) / per_warp);
@@ -571,12 +520,13 @@ static int launch_zplane(dftcuda_kctx* c, cplx<T>* S, size_t ncols, cudaStream_t
   const size_t cs = sizeof(cplx<T>);
   const int nw = plane_warps<N>(cs, c->n_act);
   if (nw < 1) return fail(DFTCUDA_ERR_UNSUPPORTED, "z-plane pass does not fit shared memory");
-  const size_t smem = cs * ((size_t)c->n_act * (N + 1) + (size_t)nw * G::LW * G::SF);
+  const size_t smem = cs * ((size_t)c->n_act * (N + 1) + 2 * N + (size_t)nw * G::LW * G::S);
   DFT_TRY(ensure_max_dynamic_smem((const void*)k_zplane<T, N>, (int)smem));
   const T* vn = std::is_same<T, double>::value ? (const T*)c->d_vn : (const T*)c->d_vn32;
   const cplx<T>* tw = std::is_same<T, double>::value ? (const cplx<T>*)c->d_twx64 : (const cplx<T>*)c->d_twx32;
-  // a few columns per CTA: enough CTAs for two waves of one CTA per SM
-  const int cpc = std::max(1, (int)std::min<size_t>(8, ncols * c->nz / 296));
+  // a few columns per CTA: enough CTAs for two waves
+  const int per_sm = nw == 8 && 2 * (smem + 1024) <= (size_t)kSmemSticks ? 2 : 1;
+  const int cpc = std::max(1, (int)std::min<size_t>(8, ncols * c->nz / (296 * per_sm)));
   dim3 g((unsigned)c->nz, ceil_div(ncols, cpc));
   int n1z = 0, n2z = 0;
   switch (c->nz) {
@@ -589,26 +539,34 @@ static int launch_zplane(dftcuda_kctx* c, cplx<T>* S, size_t ncols, cudaStream_t
 #undef X
     default: return fail(DFTCUDA_ERR_UNSUPPORTED, "z length without a four-step split");
   }
-  k_zplane<T, N><<<g, nw * 32, smem, s>>>(S, c->n_st, c->d_st_sy, c->n_act, c->d_st_sox, vn, n1z, n2z, (int)ncols, cpc, tw);
+  k_zplane<T, N><<<g, nw * 32, smem, s>>>(S, c->n_st, c->d_st_of, c->n_act, c->d_st_sox, vn, n1z, n2z, (int)ncols, cpc, tw);
   count_launch();
   return DFTCUDA_OK;
 }
 
-static constexpr int kDensityWarps = 8;
-
-template <int N> static size_t density_plane_smem(size_t cs, int n_act) {
+template <typename T, int N> static size_t density_plane_smem(int n_act, int warps) {
   using G = PlaneXGeom<N>;
-  return sizeof(double) * (size_t)density_plane_words<N>() + cs * ((size_t)n_act * (N + 1) + (size_t)kDensityWarps * G::LW * G::S);
+  return sizeof(double) * (size_t)density_plane_words<N>() + sizeof(cplx<T>) * ((size_t)n_act * (N + 1) + N) +
+         sizeof(T) * (size_t)warps * G::LW * G::S;
+}
+// Warps of the density pass, likewise; eight at least, or the pass is not used.
+template <typename T, int N> static int density_warps(int n_act) {
+  if (2 * (density_plane_smem<T, N>(n_act, 8) + 1024) <= (size_t)kSmemSticks) return 8;
+  for (int w = kDensityWarps<T>(); w >= 8; --w)
+    if (density_plane_smem<T, N>(n_act, w) <= (size_t)kSmemSticks) return w;
+  return 0;
 }
 
 template <typename T, int N>
 static int launch_zplane_density(dftcuda_kctx* c, const cplx<T>* S, size_t ncols, const double* w, double* rho, cudaStream_t s) {
-  const size_t smem = density_plane_smem<N>(sizeof(cplx<T>), c->n_act);
-  if (smem > (size_t)kSmemSticks) return fail(DFTCUDA_ERR_UNSUPPORTED, "z-plane density pass does not fit shared memory");
+  const int nw = density_warps<T, N>(c->n_act);
+  const size_t smem = density_plane_smem<T, N>(c->n_act, nw);
+  if (nw == 0) return fail(DFTCUDA_ERR_UNSUPPORTED, "z-plane density pass does not fit shared memory");
   DFT_TRY(ensure_max_dynamic_smem((const void*)k_zplane_density<T, N>, (int)smem));
   const cplx<T>* tw = std::is_same<T, double>::value ? (const cplx<T>*)c->d_twx64 : (const cplx<T>*)c->d_twx32;
   // columns per CTA: every CTA sums its columns in shared memory before one atomic pass over its plane
-  const int cpc = std::max(1, (int)((ncols * c->nz + 295) / 296));
+  const int slots = nw == 8 && 2 * (smem + 1024) <= (size_t)kSmemSticks ? 592 : 296;
+  const int cpc = std::max(1, (int)((ncols * c->nz + slots - 1) / slots));
   dim3 g((unsigned)c->nz, ceil_div(ncols, cpc));
   int n1z = 0, n2z = 0;
   switch (c->nz) {
@@ -621,7 +579,7 @@ static int launch_zplane_density(dftcuda_kctx* c, const cplx<T>* S, size_t ncols
 #undef X
     default: return fail(DFTCUDA_ERR_UNSUPPORTED, "z length without a four-step split");
   }
-  k_zplane_density<T, N><<<g, kDensityWarps * 32, smem, s>>>(S, c->n_st, c->d_st_sy, c->n_act, c->d_st_sox, n1z, n2z, (int)ncols, cpc, tw,
+  k_zplane_density<T, N><<<g, nw * 32, smem, s>>>(S, c->n_st, c->d_st_of, c->n_act, c->d_st_sox, n1z, n2z, (int)ncols, cpc, tw,
                                                               w, 1.0 / c->volume, rho);
   count_launch();
   return DFTCUDA_OK;
@@ -640,10 +598,10 @@ static int dispatch_zplane_density(dftcuda_kctx* c, const cplx<T>* S, size_t nco
 
 bool kctx_sticks_density_ok(const dftcuda_kctx* c, int precision) {
   if (!(precision == DFTCUDA_PRECISION_FP64 ? c->sticks64 : c->sticks32)) return false;
-  const size_t cs = precision == DFTCUDA_PRECISION_FP64 ? sizeof(double2) : sizeof(float2);
+  const bool f64 = precision == DFTCUDA_PRECISION_FP64;
   switch (c->nx) {
 #define X(N) \
-  case N: return density_plane_smem<N>(cs, c->n_act) <= (size_t)kSmemSticks;
+  case N: return (f64 ? density_warps<double, N>(c->n_act) : density_warps<float, N>(c->n_act)) > 0;
     DFTCUDA_FOUR_STEP_LENGTHS(X)
 #undef X
     default: return false;
@@ -715,7 +673,7 @@ int density_block_sticks(dftcuda_kctx* c, const double2* x, size_t ncols, const 
 template int density_block_sticks<double>(dftcuda_kctx*, const double2*, size_t, const double*, double*, cudaStream_t);
 template int density_block_sticks<float>(dftcuda_kctx*, const double2*, size_t, const double*, double*, cudaStream_t);
 
-// Stick tables: sticks in slot order (y ascending within a slot), the packed (slot, y) of each, the
+// Stick tables: sticks in slot order (y ascending within a slot), the stick of every (y, slot) (or -1), the
 // plane-wave index of every (stick, z) (or -1), and the z and x/y twiddle tables.
 int kctx_setup_sticks(dftcuda_kctx* c, const std::vector<int>& slot_of_x, const std::vector<int>& xpos, const int32_t* hkl) {
   c->sticks64 = kctx_sticks_ok(c, DFTCUDA_PRECISION_FP64);
@@ -736,13 +694,13 @@ int kctx_setup_sticks(dftcuda_kctx* c, const std::vector<int>& slot_of_x, const 
   }
   std::vector<int> first(n_act + 1, 0);
   std::vector<std::vector<int>> gidx(n_act, std::vector<int>(ny, -1));
-  std::vector<int> sy;
+  std::vector<int> of((size_t)ny * n_act, -1);
   for (int sl = 0; sl < n_act; ++sl) {
     std::sort(ys[sl].begin(), ys[sl].end());
     first[sl + 1] = first[sl] + (int)ys[sl].size();
     for (size_t k = 0; k < ys[sl].size(); ++k) {
       gidx[sl][ys[sl][k]] = first[sl] + (int)k;
-      sy.push_back((sl << 16) | ys[sl][k]);
+      of[(size_t)ys[sl][k] * n_act + sl] = gidx[sl][ys[sl][k]];
     }
   }
   c->n_st = first[n_act];
@@ -766,7 +724,7 @@ int kctx_setup_sticks(dftcuda_kctx* c, const std::vector<int>& slot_of_x, const 
   roots(nz, tz64, tz32);
   roots(c->nx, tx64, tx32);
   std::vector<int> sox(slot_of_x.begin(), slot_of_x.end());
-  bool ok = dev_malloc(&c->d_st_sy, sizeof(int) * std::max<size_t>(sy.size(), 1)) == cudaSuccess &&
+  bool ok = dev_malloc(&c->d_st_of, sizeof(int) * std::max<size_t>(of.size(), 1)) == cudaSuccess &&
             dev_malloc(&c->d_st_map, sizeof(int) * std::max<size_t>(map.size(), 1)) == cudaSuccess &&
             dev_malloc(&c->d_st_sox, sizeof(int) * c->nx) == cudaSuccess &&
             dev_malloc(&c->d_twz64, sizeof(double2) * nz) == cudaSuccess &&
@@ -777,7 +735,7 @@ int kctx_setup_sticks(dftcuda_kctx* c, const std::vector<int>& slot_of_x, const 
             dev_malloc(&c->d_vn32, sizeof(float) * c->N) == cudaSuccess;
   if (!ok) return fail(DFTCUDA_ERR_OUT_OF_MEMORY, "stick tables");
   cudaStream_t st = c->stream;
-  if (!sy.empty()) DFT_CUDA_TRY(cudaMemcpyAsync(c->d_st_sy, sy.data(), sizeof(int) * sy.size(), cudaMemcpyHostToDevice, st));
+  if (!of.empty()) DFT_CUDA_TRY(cudaMemcpyAsync(c->d_st_of, of.data(), sizeof(int) * of.size(), cudaMemcpyHostToDevice, st));
   if (!map.empty()) DFT_CUDA_TRY(cudaMemcpyAsync(c->d_st_map, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice, st));
   DFT_CUDA_TRY(cudaMemcpyAsync(c->d_st_sox, sox.data(), sizeof(int) * c->nx, cudaMemcpyHostToDevice, st));
   DFT_CUDA_TRY(cudaMemcpyAsync(c->d_twz64, tz64.data(), sizeof(double2) * nz, cudaMemcpyHostToDevice, st));
