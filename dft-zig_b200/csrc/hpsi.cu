@@ -1201,12 +1201,23 @@ extern "C" int dftcuda_accumulate_density(dftcuda_kctx* c, const double* vectors
     if (hw[b] > 0.0) keep.push_back(b);
   if (keep.empty()) return DFTCUDA_OK;
   const bool dv = is_device_pointer(vectors), dr = is_device_pointer(rho);
-  DFT_TRY(kctx_stage(c, keep.size()));
-  // Pack the kept bands contiguously into the staging buffer.
-  const size_t colb = sizeof(double2) * n;
-  for (size_t i = 0; i < keep.size(); ++i)
-    DFT_CUDA_TRY(cudaMemcpyAsync(c->d_x + i * n, vectors + 2 * keep[i] * n, colb,
-                                 dv ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->stream));
+  // Aligned vectors on this device whose kept bands are consecutive (the occupied bands usually are) are
+  // read where they are; otherwise the kept bands are packed into the staging buffer, one copy per run of consecutive
+  // bands (448 bands of 1 MB: the packing took 1.6 of 10.4 ms, one copy per band, a third of it the issue).
+  const double2* vecs = (const double2*)vectors + keep[0] * n;
+  cudaPointerAttributes at{};
+  const bool here = dv && ((uintptr_t)vectors & 15) == 0 && cudaPointerGetAttributes(&at, vectors) == cudaSuccess && at.device == c->device;
+  if (!here || keep.back() - keep[0] + 1 != keep.size()) {
+    DFT_TRY(kctx_stage(c, keep.size()));
+    for (size_t i = 0; i < keep.size();) {
+      size_t j = i + 1;
+      while (j < keep.size() && keep[j] == keep[j - 1] + 1) ++j;
+      DFT_CUDA_TRY(cudaMemcpyAsync(c->d_x + i * n, vectors + 2 * keep[i] * n, sizeof(double2) * n * (j - i),
+                                   dv ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->stream));
+      i = j;
+    }
+    vecs = c->d_x;
+  }
   std::vector<double> kw(keep.size());
   for (size_t i = 0; i < keep.size(); ++i) kw[i] = hw[keep[i]];
   if (keep.size() > c->w_cap) {
@@ -1222,7 +1233,7 @@ extern "C" int dftcuda_accumulate_density(dftcuda_kctx* c, const double* vectors
     DFT_CUDA_TRY(cudaMemcpyAsync(c->d_rho, rho, sizeof(double) * c->N, cudaMemcpyHostToDevice, c->stream));
     rd = c->d_rho;
   }
-  DFT_TRY(kctx_density_dev(c, c->d_x, keep.size(), c->d_w, rd, c->stream));
+  DFT_TRY(kctx_density_dev(c, vecs, keep.size(), c->d_w, rd, c->stream));
   if (!dr) DFT_CUDA_TRY(cudaMemcpyAsync(rho, rd, sizeof(double) * c->N, cudaMemcpyDeviceToHost, c->stream));
   DFT_CUDA_TRY(cudaStreamSynchronize(c->stream));
   return DFTCUDA_OK;
