@@ -32,6 +32,7 @@ struct Fft1d {
   const double2* tw64;
   const float2* tw32;
   const int* pinv;  // natural index -> digit-reversed position
+  const double2* root64;  // exp(+2 pi i e / n), e < n
 };
 
 // Host-owned plan with its device tables.
