@@ -571,7 +571,9 @@ static int eig_alloc(dftcuda_kctx* c, size_t n, size_t max_sub, size_t nb) {
 // orthonormalisation's projections and block overlaps) runs on the tensor cores in the split-TF32
 // form (FP32-class accuracy); the Cholesky factorisations, the subspace eigensolver and the residual
 // norms stay FP64.  FP64 and FP32 contexts use the FP64 GEMM throughout.
-static int gemm_dispatch(KCtxImpl* e, const GemmArgs& g, bool /*rr*/, cudaStream_t s) {
+static int gemm_dispatch(KCtxImpl* e, GemmArgs& g, bool /*rr*/, cudaStream_t s) {
+  g.i8 = e->tcs;
+  g.err = e->err;
   if (e->rr_tc && tc_worthwhile(g.M, g.N, g.K, e->tc_min_flops)) return cgemm_tf32(g, s, e->ws, e->ws_elems, e->err, true, e->tcs);
   return zgemm(g, s, e->ws, e->ws_elems);
 }
@@ -581,7 +583,10 @@ static int gram(KCtxImpl* e, const double2* X, int mx, const double2* Y, int my,
   GemmArgs g{};
   g.M = mx; g.N = my; g.K = (int)e->n;
   g.A = X; g.lda = (long)e->n; g.a_kc = true; g.conj_a = true;
-  if (e->v_cache && X == e->V) g.a_cache = &e->vt_gram;
+  if (e->v_cache && X == e->V) {
+    g.a_cache = &e->vt_gram;
+    g.a_share = 1.0 / 3.0;  // read by three products of an iteration
+  }
   g.B = Y; g.ldb = (long)e->n; g.b_kc = true; g.conj_b = false;
   g.O = out; g.ldo_r = 1; g.ldo_c = ldo;
   g.alpha = 1.0; g.beta = 0.0;
@@ -595,7 +600,10 @@ static int combine(KCtxImpl* e, const double2* X, int mx, const double2* C, int 
   g.M = ncols; g.N = (int)e->n; g.K = mx;
   g.A = C; g.lda = ldc; g.a_kc = true; g.conj_a = false;
   g.B = X; g.ldb = (long)e->n; g.b_kc = false; g.conj_b = false;
-  if (e->v_cache && X == e->V) g.b_cache = &e->vt_comb;
+  if (e->v_cache && X == e->V) {
+    g.b_cache = &e->vt_comb;
+    g.b_share = 1.0 / 3.0;
+  }
   g.O = out; g.ldo_r = (long)e->n; g.ldo_c = 1;
   g.alpha = alpha; g.beta = beta;
   return gemm_dispatch(e, g, rr, s);
@@ -801,16 +809,22 @@ static int run_init(EigRun& r, const double* diag, const double* init_vecs, size
   DFT_TRY(eig_alloc(c, n, r.max_sub, r.nbands));
   KCtxImpl* e = r.e = c->eig;
   e->rr_tc = precision_uses_tc(c->precision);
-  if (e->rr_tc && !c->d_err) {
-    DFT_CUDA_TRY(dev_malloc(&c->d_err, sizeof(int)));
-    DFT_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, sizeof(int), s));
-  }
+  if (e->rr_tc || zgemm_i8_worthwhile((int)r.max_sub, (int)r.max_sub, (int)n, 1.0 / 3.0, 1.0 / 3.0)) DFT_TRY(kctx_ensure_err(c));
   e->err = c->d_err;
   e->tcs = &c->tc_scratch;
   v_changed(e);
-  if (e->rr_tc && !e->v_cache) {
-    const size_t bg = tc4_operand_bytes((int)e->max_sub, (int)n, true), bc = tc4_operand_bytes((int)n, (int)e->max_sub, true);
-    if (bg + bc <= kVTileCacheBytes && e->vt_gram.ensure(bg) == DFTCUDA_OK && e->vt_comb.ensure(bc) == DFTCUDA_OK) {
+  const bool i8 = !e->rr_tc && zgemm_i8_worthwhile((int)r.max_sub, (int)r.nbands, (int)n, 1.0 / 3.0, 1.0);
+  if ((e->rr_tc || i8) && !e->v_cache) {
+    size_t bg = e->rr_tc ? tc4_operand_bytes((int)e->max_sub, (int)n, true) : 0;
+    size_t bc = e->rr_tc ? tc4_operand_bytes((int)n, (int)e->max_sub, true) : 0;
+    if (i8) {
+      bg = std::max(bg, zgemm_i8_cache_bytes((int)e->max_sub, (int)n));
+      bc = std::max(bc, zgemm_i8_cache_bytes((int)n, (int)e->max_sub));
+    }
+    // kept tiles only save conversions: they leave the memory to workspaces where it is scarce
+    size_t free_b = 0, total_b = 0;
+    const bool room = !i8 || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && 4 * (bg + bc) <= free_b);
+    if (room && bg + bc <= kVTileCacheBytes && e->vt_gram.ensure(bg) == DFTCUDA_OK && e->vt_comb.ensure(bc) == DFTCUDA_OK) {
       e->v_cache = true;
     } else {
       e->vt_gram.release();
@@ -848,6 +862,7 @@ static int run_init(EigRun& r, const double* diag, const double* init_vecs, size
                                  is_device_pointer(init_vecs) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
   }
   DFT_TRY(orthonormalize_all(c, (int)m, r.seed, s));
+      cudaGetLastError();
   DFT_TRY(kctx_apply_h_dev(c, e->V, e->W, m, s));
   r.applies = m;
   r.m = m;

@@ -312,6 +312,14 @@ static int local_block(dftcuda_kctx* c, const double2* x, double2* y, size_t nco
   return DFTCUDA_OK;
 }
 
+int kctx_ensure_err(dftcuda_kctx* c) {
+  if (c->d_err) return DFTCUDA_OK;
+  if (dev_malloc(&c->d_err, sizeof(int)) != cudaSuccess) return fail(DFTCUDA_ERR_OUT_OF_MEMORY, "error flag");
+  DFT_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
+  DFT_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  return DFTCUDA_OK;
+}
+
 int kctx_ensure_coef(dftcuda_kctx* c, size_t cols) {
   if (c->nl.nproj == 0) return DFTCUDA_OK;
   if (cols > c->coef_cols) {
@@ -329,12 +337,10 @@ int kctx_ensure_coef(dftcuda_kctx* c, size_t cols) {
   if (precision_uses_tc(c->precision)) {
     need = std::max(need, cgemm_tf32_workspace_elems(c->nl.nproj, (int)cols, (int)c->npw));
     need = std::max(need, cgemm_tf32_workspace_elems((int)cols, (int)c->npw, c->nl.nproj));
-    if (!c->d_err) {
-      if (dev_malloc(&c->d_err, sizeof(int)) != cudaSuccess) return fail(DFTCUDA_ERR_OUT_OF_MEMORY, "error flag");
-      DFT_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-      DFT_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    }
   }
+  if (precision_uses_tc(c->precision) || zgemm_i8_worthwhile(c->nl.nproj, (int)cols, (int)c->npw, 0.0, 1.0) ||
+      zgemm_i8_worthwhile((int)cols, (int)c->npw, c->nl.nproj, 1.0, 0.0))
+    DFT_TRY(kctx_ensure_err(c));
   // forced split counts (autotuner) need their partial sums
   need = std::max(need, (size_t)std::max(c->split_proj, 0) * c->nl.nproj * cols);
   need = std::max(need, (size_t)std::min(std::max(c->split_back, 0), std::max(1, c->nl.nproj / 32)) * cols * c->npw);
@@ -348,6 +354,13 @@ int kctx_ensure_coef(dftcuda_kctx* c, size_t cols) {
   return DFTCUDA_OK;
 }
 
+// TF32 contexts take the TF32 form for the projector products, TF32X3 contexts its split form below the
+// size where the exact residue form is the faster one.
+static bool projectors_on_tf32(const dftcuda_kctx* c, const GemmArgs& g) {
+  if (!precision_uses_tc(c->precision) || !tc_worthwhile(g.M, g.N, g.K, c->tc_min_flops)) return false;
+  return c->precision == DFTCUDA_PRECISION_TF32 || !zgemm_i8_beats_split_tf32(g.M, g.N, g.K, g.a_share, g.b_share);
+}
+
 // d_coef[p][c] = sum_g P[p][g] x[c][g]   (batch_project_coeffs, apply.zig:1143-1183)
 int kctx_project(dftcuda_kctx* c, const double2* x, size_t ncols, cudaStream_t s) {
   GemmArgs g{};
@@ -358,7 +371,9 @@ int kctx_project(dftcuda_kctx* c, const double2* x, size_t ncols, cudaStream_t s
   g.alpha = 1.0; g.beta = 0.0;
   g.splits = c->split_proj;
   g.a_cache = &c->tc_ptiles_proj;
-  if (precision_uses_tc(c->precision) && tc_worthwhile(g.M, g.N, g.K, c->tc_min_flops))
+  g.a_share = 0.0;
+  g.i8 = &c->tc_scratch; g.err = c->d_err;
+  if (projectors_on_tf32(c, g))
     return cgemm_tf32(g, s, c->d_gemm_ws, c->gemm_ws_elems, c->d_err, c->precision == DFTCUDA_PRECISION_TF32X3, &c->tc_scratch);
   return zgemm(g, s, c->d_gemm_ws, c->gemm_ws_elems);
 }
@@ -384,7 +399,9 @@ static int nonlocal_block(dftcuda_kctx* c, const double2* x, double2* y, size_t 
   g.alpha = 1.0 / c->volume; g.beta = 1.0;
   g.splits = c->split_back;
   g.b_cache = &c->tc_ptiles_back;
-  if (precision_uses_tc(c->precision) && tc_worthwhile(g.M, g.N, g.K, c->tc_min_flops))
+  g.b_share = 0.0;
+  g.i8 = &c->tc_scratch; g.err = c->d_err;
+  if (projectors_on_tf32(c, g))
     return cgemm_tf32(g, s, c->d_gemm_ws, c->gemm_ws_elems, c->d_err, c->precision == DFTCUDA_PRECISION_TF32X3, &c->tc_scratch);
   return zgemm(g, s, c->d_gemm_ws, c->gemm_ws_elems);
 }
@@ -422,7 +439,7 @@ int kctx_apply_h_dev(dftcuda_kctx* c, const double2* x, double2* y, size_t ncols
     }
   }
   if (c->nl.nproj > 0) {
-    const size_t nch = std::min<size_t>(ncols, 256);
+    const size_t nch = std::min<size_t>(ncols, zgemm_i8_worthwhile(c->nl.nproj, (int)std::min<size_t>(ncols, 512), (int)c->npw, 0.0, 1.0) ? 512 : 256);
     DFT_TRY(kctx_ensure_coef(c, nch));
     for (size_t c0 = 0; c0 < ncols; c0 += nch) {
       const size_t nc = std::min(nch, ncols - c0);
@@ -912,7 +929,7 @@ extern "C" int dftcuda_nonlocal_energies(dftcuda_kctx* c, const double* psi, siz
   }
   if (!de) DFT_CUDA_TRY(cudaMemcpyAsync(e_out, ed, sizeof(double) * nbands, cudaMemcpyDeviceToHost, c->stream));
   DFT_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return DFTCUDA_OK;
+  return kctx_check_error(c);
 }
 
 // y[c][g] = (k + G)_d x[c][g]: the band times one Cartesian component of k + G.
@@ -1013,6 +1030,7 @@ extern "C" int dftcuda_nonlocal_forces(dftcuda_kctx* c, const double* vectors, s
     }
     DFT_CUDA_TRY(cudaMemcpyAsync(hf.data(), d_F, sizeof(double) * 3 * natoms, cudaMemcpyDeviceToHost, s));
     DFT_CUDA_TRY(cudaStreamSynchronize(s));
+    DFT_TRY(kctx_check_error(c));
     if (is_device_pointer(forces)) DFT_CUDA_TRY(cudaMemcpy(forces, hf.data(), sizeof(double) * 3 * natoms, cudaMemcpyHostToDevice));
     else std::memcpy(forces, hf.data(), sizeof(double) * 3 * natoms);
     return DFTCUDA_OK;
@@ -1157,6 +1175,7 @@ extern "C" int dftcuda_nonlocal_stress(dftcuda_kctx* c, const double* kpg, size_
           g.B = c->d_y; g.ldb = (long)n; g.b_kc = true; g.conj_b = false;
           g.O = d_u; g.ldo_r = (long)nc; g.ldo_c = 1;
           g.alpha = 1.0; g.beta = 0.0;
+          g.i8 = &c->tc_scratch; g.err = c->d_err;
           DFT_TRY(zgemm(g, s, c->d_gemm_ws, c->gemm_ws_elems));
           k_stress_reduce<<<rb, 256, 0, s>>>(c->d_coef2, d_u, nullptr, d_w + c0, nproj, (long)nc,
                                              -2.0 / (c->volume * c->volume), d_acc + packed(a, b), nullptr);
@@ -1167,6 +1186,7 @@ extern "C" int dftcuda_nonlocal_stress(dftcuda_kctx* c, const double* kpg, size_
     double acc[7];
     DFT_CUDA_TRY(cudaMemcpyAsync(acc, d_acc, sizeof(acc), cudaMemcpyDeviceToHost, s));
     DFT_CUDA_TRY(cudaStreamSynchronize(s));
+    DFT_TRY(kctx_check_error(c));
     // sigma_ab (a <= b, as the reference fills it) and the diagonal -sum_n f_n E_nl,n / Omega
     const double enl = acc[6] / c->volume;
     for (int a = 0; a < 3; ++a)

@@ -33,9 +33,20 @@ struct GemmArgs {
   // Constant operands whose TF32 split the tensor-core GEMM may keep between calls (null: split per call).
   TcScratch* a_cache = nullptr;
   TcScratch* b_cache = nullptr;
+  // FP64 products large enough for the int8 residue form (zgemm_i8.cu) run there when the caller gives
+  // room for its tiles and an error flag for its bounded waits.
+  TcScratch* i8 = nullptr;
+  int* err = nullptr;
+  double a_share = 1.0, b_share = 1.0;  // the part of an operand's conversion this product pays for
 };
 int zgemm(const GemmArgs& g, cudaStream_t s, double2* workspace, size_t workspace_elems);
 size_t zgemm_workspace_elems(int M, int N, int K);
+// The FP64 product by residues on the int8 tensor cores (zgemm_i8.cu).  *done = false, with status OK, when
+// its buffers could not be allocated: nothing was launched on the output.
+bool zgemm_i8_worthwhile(int M, int N, int K, double share_m = 1.0, double share_n = 1.0);
+bool zgemm_i8_beats_split_tf32(int M, int N, int K, double share_m, double share_n);
+size_t zgemm_i8_cache_bytes(int R, int K);  // one operand's kept tiles (a_cache, b_cache)
+int zgemm_i8(const GemmArgs& g, cudaStream_t s, TcScratch* scratch, int* err, bool* done);
 // The same contraction on the tensor cores (tc_gemm.cu): TF32 inputs, FP32 accumulation.  err_dev
 // receives 1 if a bounded wait gave up.
 // split = true: 3xTF32 (hi + lo operand parts), FP32-class accuracy.  scratch (may be null): where the
@@ -187,6 +198,7 @@ namespace dftcuda {
 int kctx_apply_h_dev(dftcuda_kctx* c, const double2* x, double2* y, size_t ncols, cudaStream_t s);
 int kctx_project(dftcuda_kctx* c, const double2* x, size_t ncols, cudaStream_t s);  // d_coef = P x
 int kctx_ensure_coef(dftcuda_kctx* c, size_t cols);
+int kctx_ensure_err(dftcuda_kctx* c);  // d_err, the bounded waits' error flag
 int kctx_stage(dftcuda_kctx* c, size_t cols);
 int kctx_check_error(dftcuda_kctx* c);
 int kctx_density_dev(dftcuda_kctx* c, const double2* vecs, size_t nbands, const double* w_dev, double* rho_dev,

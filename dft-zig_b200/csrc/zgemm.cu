@@ -1,6 +1,7 @@
 // FP64 complex GEMM over strided operands, used for the Kleinman-Bylander projections
 // (apply.zig:1143-1183, 1278-1336) and the Rayleigh-Ritz contractions V^H W and V C
-// (lobpcg/common.zig:113-143, 231-259).  B200 has no FP64 tcgen05 kind, so the FP64 path runs on
+// (lobpcg/common.zig:113-143, 231-259).  B200 has no FP64 tcgen05 kind: large products run as exact
+// integer products on the int8 tensor cores (zgemm_i8.cu; the line is zgemm_i8_worthwhile), the others on
 // the FP64 tensor cores through mma.sync m8n8k4 .f64 with three real products per complex one
 // (k_zgemm_dmma3m, the default: the FP64 MMA pipe is the bound, and it does a quarter less work),
 // with the plain four products (k_zgemm_dmma, DFTCUDA_ZGEMM=dmma8) or on the m16n8k8 shape
@@ -442,8 +443,8 @@ size_t zgemm_workspace_elems(int M, int N, int K) {
   return s > 1 ? (size_t)s * M * N : 0;
 }
 
-// DFTCUDA_ZGEMM=fma / dmma8 / dmma16 select the other kernels (A/B measurements); the
-// three-product m8n8k4 kernel is the default.
+// DFTCUDA_ZGEMM=fma / dmma8 / dmma16 select the other kernels, dmma3m the three-product m8n8k4 kernel at
+// every size (A/B measurements); unset, that kernel below the residue form's sizes.
 static int zgemm_kind() {
   static const int v = [] {
     const char* e = std::getenv("DFTCUDA_ZGEMM");
@@ -500,6 +501,11 @@ int zgemm(const GemmArgs& g, cudaStream_t s, double2* ws, size_t ws_elems) {
   switch (key) {
     case 0: launch<false, false, false, false>(g, grid, kps, part, s); break;
     case 1: launch<false, false, false, true>(g, grid, kps, part, s); break;
+  if (g.i8 && g.err && zgemm_i8_worthwhile(g.M, g.N, g.K, g.a_share, g.b_share)) {
+    bool done = false;
+    DFT_TRY(zgemm_i8(g, s, g.i8, g.err, &done));
+    if (done) return DFTCUDA_OK;
+  }
     case 2: launch<false, false, true, false>(g, grid, kps, part, s); break;
     case 3: launch<false, false, true, true>(g, grid, kps, part, s); break;
     case 4: launch<false, true, false, false>(g, grid, kps, part, s); break;

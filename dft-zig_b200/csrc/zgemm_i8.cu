@@ -1,0 +1,931 @@
+// FP64 complex GEMM by exact integer arithmetic on the int8 tensor cores (tcgen05 kind::i8): the
+// residue-number form of the Ozaki splitting (Ozaki scheme II: K. Ozaki, Y. Uchino, T. Imamura,
+// 2025).  Same contraction and operand conventions as zgemm.cu:
+//
+//   out(r, c) = alpha * sum_k opA(A(r, k)) * opB(B(c, k)) + beta * out(r, c)
+//
+// Each row of either operand is scaled by a power of two, so that its 2-norm is at most 2^58, and
+// rounded to (Gaussian) integers a' and b'.  By Cauchy-Schwarz |sum a' b'| <= 2^116 < P / 2 for the
+// product P = 2^117.7 of 16 pairwise coprime moduli below 256, so the integer result is determined by
+// its residues.  The only rounding is that of the entries, half a unit of 2^-58 times the row's norm: an
+// error of about 2^-59 |a||b| per output whatever K is, against 2^-55 |a||b| for a 64-bit accumulation of
+// the same products.
+//
+// Every prime factor of the moduli is 1 mod 4, so -1 has a square root w modulo each, and
+// x + iy -> (x + wy, x - wy) maps complex products modulo p onto two independent real ones: a complex
+// GEMM is two real int8 GEMMs per modulus (four, or three with 25 % more planes, for other moduli).
+//
+// Four steps per product:
+//   k_i8_norm, k_i8_scale   the rows' scale exponents (one read of the operand);
+//   k_i8_tiles              both residues of the scaled entries as int8 core-matrix tiles, 32 bytes per
+//                           entry (one read; the projector matrix keeps its tiles between calls);
+//   k_i8_gemm               the residue products, 32 real GEMMs in one persistent launch;
+//   k_i8_out                the sum from its residues (Chinese remainder theorem), scaled.
+//
+// A row that holds an infinity or a NaN gives NaN in its whole output row (or column), and in no other.
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <cstdlib>
+#include <type_traits>
+#include <vector>
+
+#include "kctx.cuh"
+
+namespace dftcuda {
+
+constexpr int I8_MODS = 16;
+constexpr int kI8P[I8_MODS] = {241, 233, 229, 221, 205, 197, 193, 181, 173, 157, 149, 137, 113, 109, 101, 97};
+constexpr int I8_NORM_EXP = 58;   // log2 of the scaled rows' norm bound
+constexpr int I8_BAD = INT_MIN;   // scale exponent of a row with a non-finite entry
+constexpr long long I8_OFFSET = 1LL << 60;  // makes every scaled entry non-negative
+
+__host__ __device__ constexpr int i8_balance(long v, int p) {  // v mod p in (-p/2, p/2)
+  v %= p;
+  if (v < 0) v += p;
+  return (int)(v > p / 2 ? v - p : v);
+}
+__host__ __device__ constexpr int i8_pow2(int e, int p) {
+  long v = 1;
+  for (int i = 0; i < e; ++i) v = v * 2 % p;
+  return (int)v;
+}
+__host__ __device__ constexpr int i8_root(int p) {  // w with w^2 = -1 mod p
+  for (int w = 1; w < p; ++w)
+    if ((w * w + 1) % p == 0) return w;
+  return 0;
+}
+// factor * 256^j mod p for the four low (h = 0) or high (h = 1) bytes of a 64-bit integer, packed as int8.
+__host__ __device__ constexpr unsigned i8_coef(int h, int factor, int p) {
+  unsigned w = 0;
+  for (int j = 0; j < 4; ++j) w |= ((unsigned)i8_balance((long)factor * i8_pow2(8 * (4 * h + j), p), p) & 255u) << (8 * j);
+  return w;
+}
+__host__ __device__ constexpr int i8_off(int factor, int p) { return i8_balance(-(long)factor * i8_pow2(60, p), p); }
+
+// ---- scale exponents ----------------------------------------------------------------------------
+
+// Partial (largest magnitude, sum of squares) of row r over one K chunk: part[chunk * R + r].
+// KC: K contiguous, one block per (row, chunk); else rows contiguous, one thread per row.
+template <bool KC>
+__global__ void __launch_bounds__(256) k_i8_norm(const double2* __restrict__ X, long ld, int R, int K, int kchunk,
+                                                 double2* __restrict__ part) {
+  const int k0 = blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
+  double mx = 0.0, ss = 0.0;
+  // fmax ignores a NaN, the sum of squares carries it
+  auto take = [&](double2 v) {
+    mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
+    ss = fma(v.x, v.x, fma(v.y, v.y, ss));
+  };
+  if (KC) {
+    const int r = blockIdx.x;
+    const double2* x = X + (long)r * ld;
+#pragma unroll 4
+    for (int k = k0 + threadIdx.x; k < k1; k += 256) take(x[k]);
+    for (int o = 16; o > 0; o >>= 1) {
+      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    }
+    __shared__ double2 red[8];
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_double2(mx, ss);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < 8; ++w) {
+        mx = fmax(mx, red[w].x);
+        ss += red[w].y;
+      }
+      part[(long)blockIdx.y * R + r] = make_double2(mx, ss);
+    }
+  } else {
+    const int r = blockIdx.x * 256 + threadIdx.x;
+    if (r >= R) return;
+#pragma unroll 4
+    for (int k = k0; k < k1; ++k) take(X[(long)k * ld + r]);
+    part[(long)blockIdx.y * R + r] = make_double2(mx, ss);
+  }
+}
+
+// Exponent e of every row: the entries times 2^e have norm <= 2^58.
+__global__ void k_i8_scale(const double2* __restrict__ part, int R, int chunks, int K, int* __restrict__ ex) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= R) return;
+  double mx = 0.0, ss = 0.0;
+  for (int c = 0; c < chunks; ++c) {
+    const double2 v = part[(long)c * R + r];
+    mx = fmax(mx, v.x);
+    ss += v.y;
+  }
+  int e;
+  if (isnan(ss) || isinf(mx)) {
+    e = I8_BAD;
+  } else if (mx == 0.0) {
+    e = 0;
+  } else if (ss > 1e-280 && ss < 1e300) {
+    frexp(sqrt(ss) * (1.0 + 1e-12), &e);  // norm < 2^e (1e-12: the rounding of the sum of squares)
+    e = I8_NORM_EXP - e;
+  } else {  // the squares over- or underflow: norm <= sqrt(2 K) max
+    int em, ek;
+    frexp(mx, &em);
+    frexp(sqrt(2.0 * K), &ek);
+    e = I8_NORM_EXP - em - ek;
+  }
+  ex[r] = e;
+}
+
+// ---- residue tiles ------------------------------------------------------------------------------
+// int8 residues in the MMA's shared-memory image: per modulus, plane (x + wy, x - wy) and 64-deep K
+// block, the operand's 8-row groups of four 8 x 16-byte core matrices one after another, so any range of
+// row groups of a K block is one contiguous block.  A 128-row read may run past the last row group (of
+// the buffer, by up to I8_SLACK); what it brings there only reaches outputs beyond the matrix.
+constexpr int I8_KB = 64;
+constexpr size_t I8_SLACK = 16 * 8 * I8_KB;
+static size_t i8_groups(long R) { return (size_t)((R + 7) / 8); }
+static size_t i8_tile_bytes(long R, long K) {
+  return (size_t)2 * I8_MODS * ((K + I8_KB - 1) / I8_KB) * i8_groups(R) * 8 * I8_KB + I8_SLACK;
+}
+
+struct I8Tiles {
+  unsigned char* p;
+  size_t plane, kb;  // strides in bytes; the planes of a modulus are neighbours, the moduli 2 planes apart
+};
+
+// Residue in the low byte of T, the bit pattern of F = 2^23 * 1.5 + t with F = the value sought modulo P (the
+// dot products' start carries what that takes).  The product's rounding can move a quotient that is
+// within 0.008 of a half to the other side: |residue| <= (P + 1) / 2 instead of (P - 1) / 2.
+template <int P>
+__device__ __forceinline__ unsigned i8_reduce(unsigned T) {
+  const float g = fmaf(__uint_as_float(T), 1.0f / P, 12582912.f);  // rint(F / P) in the low mantissa bits
+  return T - __float_as_uint(g) * (unsigned)P;                      // 0x4B400000 and 12582912 have zero low bytes
+}
+
+__device__ __forceinline__ unsigned i8_dot(unsigned lo, unsigned hi, unsigned clo, unsigned chi, unsigned add) {
+  unsigned t;
+  asm("{\n\t.reg .s32 t;\n\tdp4a.u32.s32 t, %1, %2, %5;\n\tdp4a.u32.s32 %0, %3, %4, t;\n\t}"
+      : "=r"(t)
+      : "r"(lo), "r"(clo), "r"(hi), "r"(chi), "r"(add));
+  return t;
+}
+
+template <int I>
+__device__ __forceinline__ void i8_store(const unsigned (&lo)[8], const unsigned (&hi)[8], unsigned char* o, size_t plane, bool conj) {
+  if constexpr (I < I8_MODS) {
+    constexpr int P = kI8P[I], W = i8_root(P);
+    constexpr unsigned xl = i8_coef(0, 1, P), xh = i8_coef(1, 1, P), yl = i8_coef(0, W, P), yh = i8_coef(1, W, P);
+    constexpr unsigned xo = 0x4B400000u + (unsigned)(i8_off(1, P) - 12582912 % P), yo = (unsigned)i8_off(W, P);
+    unsigned u[4], v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const unsigned x = i8_dot(lo[j], hi[j], xl, xh, xo), y = i8_dot(lo[4 + j], hi[4 + j], yl, yh, yo);
+      u[j] = i8_reduce<P>(x + y);
+      v[j] = i8_reduce<P>(x - y);
+    }
+    auto pack = [](const unsigned (&a)[4]) {
+      return __byte_perm(__byte_perm(a[0], a[1], 0x0040), __byte_perm(a[2], a[3], 0x0040), 0x5410);
+    };
+    *reinterpret_cast<unsigned*>(o + (conj ? plane : 0)) = pack(u);
+    *reinterpret_cast<unsigned*>(o + (conj ? 0 : plane)) = pack(v);
+    i8_store<I + 1>(lo, hi, o + 2 * plane, plane, conj);
+  }
+}
+
+// One warp per core matrix (8 rows x 16 K), lane = 4 row + quad: four consecutive K of one row; the
+// warp writes 128 contiguous bytes per modulus and plane.  Rows r0 .. r0 + rows of X, K k0 .. k0 + kn;
+// X(r, k) = X[r * ld + k] when kc, else X[k * ld + r].  grid.x: row groups, grid.y: warps along K.
+// 16 bytes read and 32 written per entry: 110e6 entries in 1.18 ms, 4.5 TB/s, with the integer pipes at
+// three quarters of their rate (about 13 instructions per entry and modulus).
+__global__ void __launch_bounds__(256) k_i8_tiles(const double2* __restrict__ X, long ld, bool kc, bool conj, int r0, int rows,
+                                                  int k0, int kn, const int* __restrict__ ex, I8Tiles out) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kcm = blockIdx.y * 8 + warp;  // core matrix along K
+  if (kcm >= (kn + I8_KB - 1) / I8_KB * (I8_KB / 16)) return;
+  const int rg = blockIdx.x, row = rg * 8 + (lane >> 2), kk = kcm * 16 + (lane & 3) * 4;
+  unsigned lo[8], hi[8];
+  double p1 = 0.0, p2 = 0.0;
+  if (row < rows) {
+    const int e = ex[r0 + row];
+    if (e != I8_BAD) {  // 2^e as two factors: e may be beyond a double's own range
+      const int h = e / 2;
+      p1 = __hiloint2double((1023 + h) << 20, 0);
+      p2 = __hiloint2double((1023 + e - h) << 20, 0);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    double2 x = make_double2(0.0, 0.0);
+    if (p1 != 0.0 && kk + j < kn) x = kc ? X[(long)(r0 + row) * ld + k0 + kk + j] : X[(long)(k0 + kk + j) * ld + r0 + row];
+    const long long a = __double2ll_rn(x.x * p1 * p2) + I8_OFFSET, b = __double2ll_rn(x.y * p1 * p2) + I8_OFFSET;
+    lo[j] = (unsigned)a; hi[j] = (unsigned)(a >> 32);
+    lo[4 + j] = (unsigned)b; hi[4 + j] = (unsigned)(b >> 32);
+  }
+  unsigned char* o = out.p + (size_t)(kcm >> 2) * out.kb + (size_t)rg * (8 * I8_KB) + (kcm & 3) * 128 + lane * 4;
+  i8_store<0>(lo, hi, o, out.plane, conj);
+}
+
+// ---- the residue products -----------------------------------------------------------------------
+// Persistent kernel on CTA pairs (clusters of two, one CTA per SM); a work item is a 256 x tn tile
+// (tn <= 256) of one plane of one modulus over one K split.  Each CTA holds 128 rows of A and half of
+// the tile's rows of B, 128 deep in K, per slot of a six-slot ring (two K blocks, one bulk copy of up to
+// 8 KB per operand and block); the pair's leader issues tcgen05.mma.cta_group::2 (M = 256, N = tn), which
+// reads both CTAs' shared memory, and its commits free the slot in both.  A CTA reads 32 KB per 512 cycles of MMA, two thirds of what a
+// single-CTA 128 x 256 tile would: the reads from L2 are the bound.  TMEM holds two accumulators: eight
+// warps reduce a finished one to residues while the next item's MMAs run.  The producing and issuing warps run
+// their loops with all lanes and elect one for the copies and MMAs: from inside a divergent branch the same
+// loop took three times as long.  1344 x 448 x 61565 (a sixth of its tiles padding): 0.88 ms, 2.7e15 useful
+// operations/s of 4.5e15 nominal; the single-CTA form with four products per complex one took 2.0 ms.
+constexpr int I8_STAGES = 6;
+constexpr int I8_HALF = 128 * I8_KB;  // bytes of 128 rows of a K block
+constexpr int I8_SLOT = 4 * I8_HALF;  // A, then B, of two K blocks
+constexpr int I8_SMEM = I8_STAGES * I8_SLOT;
+constexpr int I8_EPI = 8, I8_THREADS = 32 * (I8_EPI + 2);
+constexpr int I8_MAX_K = 65536;  // of one split: K 121^2 < 2^30 in the int32 accumulators
+constexpr long long I8_WAIT_CYCLES = 1LL << 33;  // about four seconds
+constexpr int I8_PAIRS = 74;
+
+struct I8Mod {
+  unsigned p[I8_MODS], magic[I8_MODS], off[I8_MODS], shift[I8_MODS];  // x mod p = y - p (umulhi(y, magic) >> shift), y = x + off
+};
+struct I8Gemm {
+  const unsigned char *A, *B;
+  size_t a_plane, a_kb, b_plane, b_kb;
+  int M, N, Npad, mt, nt, tn, kblocks, splits, kps;  // kps: K blocks per split
+  int rga, rgb;                                      // row groups of A and B
+  unsigned char* out;                                // [split][mod][plane][M][Npad]
+  int* err;
+  I8Mod mod;
+};
+
+__device__ __forceinline__ bool i8_try(uint32_t mbar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(done)
+      : "r"(mbar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+__device__ __noinline__ bool i8_wait_long(uint32_t mbar, uint32_t parity) {
+  const long long t0 = clock64();
+  do {
+    if (i8_try(mbar, parity)) return true;
+  } while (clock64() - t0 < I8_WAIT_CYCLES);
+  return false;
+}
+// Bounded wait for the phase with the given parity; all lanes of the warp.
+__device__ __forceinline__ bool i8_wait(uint32_t mbar, uint32_t parity) {
+  return __all_sync(0xffffffffu, i8_try(mbar, parity) || i8_try(mbar, parity) || i8_wait_long(mbar, parity));
+}
+__device__ __forceinline__ bool i8_elect() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
+__device__ __forceinline__ void i8_arrive_leader(uint32_t mbar) {  // on the same barrier of the pair's first CTA
+  asm volatile(
+      "{\n\t.reg .b32 a;\n\t"
+      "mapa.shared::cluster.u32 a, %0, 0;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [a];\n\t}\n" ::"r"(mbar)
+      : "memory");
+}
+__device__ __forceinline__ void i8_bulk(uint32_t dst, const unsigned char* src, uint32_t bytes, uint32_t mbar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(dst), "l"(src),
+               "r"(bytes), "r"(mbar)
+               : "memory");
+}
+__device__ __forceinline__ uint64_t i8_desc(uint32_t addr) {
+  // start >> 4 | LBO 128 B (next core matrix along K) | SBO 512 B (next 8 rows) | version 1 (sm_100)
+  return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) | (1ULL << 46);
+}
+__device__ __forceinline__ void i8_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accum) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accum ? 1 : 0));
+}
+__device__ __forceinline__ void i8_commit(uint32_t mbar) {  // arrives on the barrier in both CTAs
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(mbar),
+               "h"((unsigned short)3)
+               : "memory");
+}
+__device__ __forceinline__ void i8_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ void i8_ld16(uint32_t (&v)[16], uint32_t addr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+        "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr));
+}
+__device__ __forceinline__ unsigned i8_mod4(const uint32_t* x, unsigned p, unsigned magic, unsigned off, unsigned shift) {
+  unsigned r[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const unsigned y = x[j] + off;
+    r[j] = y - p * (__umulhi(y, magic) >> shift);
+  }
+  return __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+}
+
+__global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant__ I8Gemm g) {
+  extern __shared__ __align__(1024) unsigned char ism[];
+  __shared__ __align__(8) uint64_t bars[3 * I8_STAGES + 5];
+  __shared__ uint32_t tmem_slot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = blockIdx.x & 1, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(ism);
+  // full: this CTA's copies; peer: the second CTA's, relayed to the leader; empty: the slot's MMAs are done
+  const uint32_t full = (uint32_t)__cvta_generic_to_shared(bars), empty = full + 8 * I8_STAGES, peer = empty + 8 * I8_STAGES;
+  const uint32_t acc_full = peer + 8 * I8_STAGES, acc_empty = acc_full + 16, fin = acc_full + 32;
+  const int items = g.mt * g.nt * g.splits * I8_MODS * 2;
+  if (tid == 0) {
+    for (int q = 0; q < 3 * I8_STAGES + 2; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(full + 8 * q));
+    for (int q = 0; q < 2; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(acc_empty + 8 * q), "r"(2 * I8_EPI));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(fin));
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
+  }
+  if (warp == I8_EPI + 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(
+        (uint32_t)__cvta_generic_to_shared(&tmem_slot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+  __syncthreads();
+  i8_cluster_sync();  // both CTAs' barriers are initialised
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+  const uint32_t tmem = tmem_slot;
+  // A role whose wait runs out records it and stops; the others' waits then run out too.
+  auto late = [&] {
+    if (lane == 0) atomicExch(g.err, 1);
+  };
+  // item: nt fastest, then mt, split, plane (the pairs at work share a few planes' tiles in L2)
+  struct Item {
+    int n, m, split, plane, kb0, kbs;
+  };
+  auto item_of = [&](int it) {
+    Item r;
+    r.n = it % g.nt;
+    it /= g.nt;
+    r.m = it % g.mt;
+    it /= g.mt;
+    r.split = it % g.splits;
+    r.plane = it / g.splits;
+    r.kb0 = r.split * g.kps;
+    r.kbs = min(g.kps, g.kblocks - r.kb0);
+    return r;
+  };
+  if (warp < I8_EPI) {
+    // ---- residues of the finished accumulators ----
+    const int quarter = warp & 3, half = warp >> 2;
+    int j = 0;
+    for (int it = pair; it < items; it += pairs, ++j) {
+      const Item w = item_of(it);
+      const int buf = j & 1;
+      if (!i8_wait(acc_full + 8 * buf, (uint32_t)((j >> 1) & 1))) {
+        late();
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+      const int mod = w.plane >> 1;
+      const unsigned p = g.mod.p[mod], magic = g.mod.magic[mod], off = g.mod.off[mod], shift = g.mod.shift[mod];
+      const int row = w.m * 256 + rank * 128 + quarter * 32 + lane;
+      const uint32_t acc = tmem + buf * 256 + ((uint32_t)(quarter * 32) << 16);
+      const int c0 = w.n * g.tn, cols = min(g.tn, g.Npad - c0);
+      unsigned char* o = g.out + ((size_t)(w.split * I8_MODS * 2 + w.plane) * g.M + row) * g.Npad + c0;
+      for (int c = half * 32; c < cols; c += 64) {
+        uint32_t x[16], y[16];
+        i8_ld16(x, acc + c);
+        i8_ld16(y, acc + c + 16);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        if (row < g.M) {
+          uint4 a, b;
+          a.x = i8_mod4(x, p, magic, off, shift); a.y = i8_mod4(x + 4, p, magic, off, shift);
+          a.z = i8_mod4(x + 8, p, magic, off, shift); a.w = i8_mod4(x + 12, p, magic, off, shift);
+          b.x = i8_mod4(y, p, magic, off, shift); b.y = i8_mod4(y + 4, p, magic, off, shift);
+          b.z = i8_mod4(y + 8, p, magic, off, shift); b.w = i8_mod4(y + 12, p, magic, off, shift);
+          *reinterpret_cast<uint4*>(o + c) = a;  // tn and Npad are multiples of 32
+          *reinterpret_cast<uint4*>(o + c + 16) = b;
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+      __syncwarp();
+      if (lane == 0) i8_arrive_leader(acc_empty + 8 * buf);
+    }
+  } else if (warp == I8_EPI) {
+    // ---- bulk copies ----
+    int t = 0;
+    bool ok = true;
+    const uint32_t bb = (uint32_t)(g.tn / 2 * I8_KB);
+    for (int it = pair; it < items && ok; it += pairs) {
+      const Item w = item_of(it);
+      const int ra = min(w.m * 32 + rank * 16, g.rga - 1), rb = min((w.n * g.tn + rank * (g.tn / 2)) / 8, g.rgb - 1);
+      const unsigned char* a = g.A + (size_t)w.plane * g.a_plane + (size_t)w.kb0 * g.a_kb + (size_t)ra * (8 * I8_KB);
+      const unsigned char* b = g.B + (size_t)w.plane * g.b_plane + (size_t)w.kb0 * g.b_kb + (size_t)rb * (8 * I8_KB);
+      for (int k = 0; k < w.kbs; k += 2, ++t) {
+        const int q = t % I8_STAGES;
+        if (t >= I8_STAGES && !i8_wait(empty + 8 * q, (uint32_t)((t / I8_STAGES - 1) & 1))) {
+          late();
+          ok = false;
+          break;
+        }
+        const uint32_t bar = full + 8 * q, dst = ring + q * I8_SLOT;
+        const bool two = k + 1 < w.kbs;
+        if (i8_elect()) {
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"((two ? 2 : 1) * (I8_HALF + bb)) : "memory");
+          i8_bulk(dst, a, I8_HALF, bar);
+          i8_bulk(dst + 2 * I8_HALF, b, bb, bar);
+          if (two) {
+            i8_bulk(dst + I8_HALF, a + g.a_kb, I8_HALF, bar);
+            i8_bulk(dst + 3 * I8_HALF, b + g.b_kb, bb, bar);
+          }
+        }
+        __syncwarp();
+        a += 2 * g.a_kb;
+        b += 2 * g.b_kb;
+      }
+    }
+    // no copy may be in flight when the CTA exits, nor a commit on its way to this CTA's barriers
+    const uint32_t last = ok ? empty : full;
+    for (int u = max(0, t - I8_STAGES); u < t; ++u)
+      if (!i8_wait(last + 8 * (u % I8_STAGES), (uint32_t)((u / I8_STAGES) & 1))) late();
+  } else if (rank == 1) {
+    // ---- the second CTA tells the leader that its copies have landed ----
+    int t = 0;
+    bool ok = true;
+    for (int it = pair; it < items && ok; it += pairs) {
+      const int kbs = item_of(it).kbs;
+      for (int k = 0; k < kbs; k += 2, ++t) {
+        const int q = t % I8_STAGES;
+        if (!i8_wait(full + 8 * q, (uint32_t)((t / I8_STAGES) & 1))) {
+          late();
+          ok = false;
+          break;
+        }
+        if (i8_elect()) i8_arrive_leader(peer + 8 * q);
+        __syncwarp();
+      }
+    }
+  } else {
+    // ---- MMA issuer ----
+    int t = 0, j = 0;
+    bool ok = true;
+    // D = S32 (2 at bit 4), A and B = S8 (1 at bits 7 and 10), K-major, N = tn, M = 256
+    const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(g.tn >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+    const uint64_t desc0 = i8_desc(ring);
+    for (int it = pair; it < items && ok; it += pairs, ++j) {
+      const int kbs = item_of(it).kbs, buf = j & 1;
+      if (j >= 2 && !i8_wait(acc_empty + 8 * buf, (uint32_t)((j / 2 - 1) & 1))) {
+        late();
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+      const uint32_t d = tmem + buf * 256;
+      for (int k = 0; k < kbs; k += 2, ++t) {
+        const int q = t % I8_STAGES;
+        const uint32_t par = (uint32_t)((t / I8_STAGES) & 1);
+        if (!i8_wait(full + 8 * q, par) || !i8_wait(peer + 8 * q, par)) {
+          late();
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
+        if (i8_elect()) {
+          const uint64_t a = desc0 + (uint64_t)(q * (I8_SLOT >> 4)), b = a + (2 * I8_HALF >> 4);
+          i8_mma(d, a, b, idesc, k > 0);
+          i8_mma(d, a + (256 >> 4), b + (256 >> 4), idesc, true);
+          if (k + 1 < kbs) {
+            i8_mma(d, a + (I8_HALF >> 4), b + (I8_HALF >> 4), idesc, true);
+            i8_mma(d, a + ((I8_HALF + 256) >> 4), b + ((I8_HALF + 256) >> 4), idesc, true);
+          }
+          i8_commit(empty + 8 * q);
+          if (k + 2 >= kbs) i8_commit(acc_full + 8 * buf);
+        }
+        __syncwarp();
+      }
+    }
+    // every MMA issued is done before TMEM is freed
+    if (i8_elect())
+      asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(fin) : "memory");
+    __syncwarp();
+    if (!i8_wait(fin, 0u)) late();
+  }
+  __syncwarp();
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
+  __syncthreads();
+  i8_cluster_sync();  // neither CTA leaves while the other may reach its shared memory
+  if (warp == I8_EPI + 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;\n" ::"r"(tmem));
+}
+
+// ---- reconstruction -----------------------------------------------------------------------------
+// With s and d the sum and difference of the two planes' residues (summed over the splits),
+//   Re = P frac(sum_i s_i inv(2) inv_i / p_i),  Im = P frac(sum_i d_i inv(2 w_i) inv_i / p_i),
+// inv_i the inverse of P / p_i modulo p_i; the coefficients held to 76 bits, the fractions taken in
+// [-1/2, 1/2).
+constexpr int I8_MAX_SPLITS = 64;
+struct I8Frac {
+  unsigned long long hi;
+  unsigned lo;  // 12 bits below hi's 2^-64
+};
+__host__ __device__ constexpr I8Frac i8_crt(int i, int part) {
+  const int p = kI8P[i];
+  long den = part == 0 ? 2 : 2 * i8_root(p);
+  for (int j = 0; j < I8_MODS; ++j)
+    if (j != i) den = den * kI8P[j] % p;
+  long inv = 1;
+  while (den * inv % p != 1) ++inv;
+  // inv / p in binary, 12 bits at a time (76 = 6 * 12 + 4)
+  unsigned long long hi = (unsigned long long)inv * 16 / p;
+  unsigned long rem = (unsigned long)inv * 16 % p;
+  unsigned lo = 0;
+  for (int k = 0; k < 6; ++k) {
+    lo = (unsigned)(rem * 4096 / p);
+    rem = rem * 4096 % p;
+    if (k < 5) hi = hi << 12 | lo;
+  }
+  return {hi, lo};
+}
+
+struct I8Less {
+  unsigned long long hi;
+  long long lo;
+};
+__host__ __device__ constexpr I8Less i8_less_one() {
+  I8Less r{0, 0};
+  for (int i = 0; i < I8_MODS; ++i) {
+    const I8Frac f = i8_crt(i, 1);
+    r.hi += f.hi * (unsigned long long)kI8P[i];
+    r.lo += (long long)f.lo * kI8P[i];
+  }
+  return r;
+}
+constexpr I8Less kI8Less = i8_less_one();
+
+struct I8Sum {
+  unsigned long long h[2] = {0, 0};
+  unsigned l[2] = {0, 0};
+  template <int I>
+  __device__ __forceinline__ void add(unsigned s, unsigned d) {
+    constexpr I8Frac re = i8_crt(I, 0), im = i8_crt(I, 1);
+    h[0] += re.hi * s;
+    l[0] += re.lo * s;
+    h[1] += im.hi * d;
+    l[1] += im.lo * d;
+  }
+  // less: what the moduli added to each split's differences put into the imaginary part (so that a sum of
+  // zeros is exactly zero)
+  __device__ __forceinline__ double2 value(int ea, int eb, double scale, I8Less less) const {
+    double v[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const long long ll = (long long)l[q] - (q ? less.lo : 0);
+      const long long hh = (long long)(h[q] - (q ? less.hi : 0ULL) + (unsigned long long)(ll >> 12));
+      const double f = (double)hh + (double)(int)(ll & 4095) * (1.0 / 4096.0);
+      v[q] = (ea == I8_BAD || eb == I8_BAD) ? __longlong_as_double(0x7ff8000000000000LL) : scalbn(f * scale, -(ea + eb));
+    }
+    return make_double2(v[0], v[1]);
+  }
+};
+
+// Moduli I, I + 1, ... of four neighbouring columns: w holds each plane's four residues, summed over the
+// splits, as 16-bit pairs (columns 0 and 2, then 1 and 3).
+template <int I, int I0, int I1>
+__device__ __forceinline__ void i8_group(I8Sum (&x)[4], const uint2* w, unsigned splits) {
+  if constexpr (I < I1) {
+    const unsigned p = (unsigned)std::integral_constant<int, kI8P[I]>::value * splits;
+    const uint2 u = w[2 * (I - I0)], v = w[2 * (I - I0) + 1];
+    x[0].template add<I>((u.x & 0xffffu) + (v.x & 0xffffu), (u.x & 0xffffu) + p - (v.x & 0xffffu));
+    x[1].template add<I>((u.y & 0xffffu) + (v.y & 0xffffu), (u.y & 0xffffu) + p - (v.y & 0xffffu));
+    x[2].template add<I>((u.x >> 16) + (v.x >> 16), (u.x >> 16) + p - (v.x >> 16));
+    x[3].template add<I>((u.y >> 16) + (v.y >> 16), (u.y >> 16) + p - (v.y >> 16));
+    i8_group<I + 1, I0, I1>(x, w, splits);
+  }
+}
+// In groups of eight moduli: all of a group's loads of one split are in flight together.
+template <int I, bool ONE>
+__device__ __forceinline__ void i8_sums(I8Sum (&x)[4], const unsigned char* q, size_t plane, int splits) {
+  if constexpr (I < I8_MODS) {
+    constexpr int G = 8;
+    uint2 w[2 * G];
+#pragma unroll
+    for (int i = 0; i < 2 * G; ++i) w[i] = make_uint2(0, 0);
+    for (int z = 0; z < (ONE ? 1 : splits); ++z) {
+      const unsigned char* o = q + (size_t)z * (2 * I8_MODS) * plane;
+      unsigned r[2 * G];
+#pragma unroll
+      for (int i = 0; i < 2 * G; ++i) r[i] = __ldg(reinterpret_cast<const unsigned*>(o + i * plane));
+#pragma unroll
+      for (int i = 0; i < 2 * G; ++i) {
+        w[i].x += r[i] & 0x00ff00ffu;
+        w[i].y += (r[i] >> 8) & 0x00ff00ffu;
+      }
+    }
+    i8_group<I, I, I + G>(x, w, ONE ? 1u : (unsigned)splits);
+    i8_sums<I + G, ONE>(x, q + 2 * G * plane, plane, splits);
+  }
+}
+
+__device__ __forceinline__ void i8_put(double2* o, double2 s, double alpha, double beta) {
+  double2 v = make_double2(alpha * s.x, alpha * s.y);
+  if (beta != 0.0) {
+    const double2 old = *o;
+    v.x += beta * old.x;
+    v.y += beta * old.y;
+  }
+  *o = v;
+}
+
+// A thread takes four columns of a row and passes its results through shared memory, so that a warp's
+// stores are contiguous.  TR = false: a warp takes 128 columns of one row.  TR = true (consecutive rows
+// are neighbours in the destination): a block takes 32 rows x 32 columns.
+template <bool TR, bool ONE>
+__global__ void __launch_bounds__(256, 2) k_i8_out(const unsigned char* __restrict__ res, int M, int N, int Npad, int splits,
+                                                const int* __restrict__ exa, const int* __restrict__ exb, double2* __restrict__ O,
+                                                long ldo_r, long ldo_c, double alpha, double beta, double scale, I8Less less) {
+  constexpr int COLS = TR ? 32 : 128, ROWS = 1024 / COLS;
+  __shared__ double2 tile[ROWS][TR ? COLS + 1 : COLS];
+  const int cl = threadIdx.x % (COLS / 4) * 4;
+  const int r0 = blockIdx.y * ROWS, c0 = blockIdx.x * COLS, c = c0 + cl;
+  const size_t plane = (size_t)M * Npad;
+  {
+    const int rl = threadIdx.x / (COLS / 4), r = r0 + rl;
+    if (r < M && c < N) {
+      I8Sum x[4];
+      i8_sums<0, ONE>(x, res + (size_t)r * Npad + c, plane, splits);
+      const int ea = exa[r];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < N) tile[rl][cl + j] = x[j].value(ea, exb[c + j], scale, less);
+    }
+  }
+  if (TR) {
+    __syncthreads();
+    const int rr = r0 + (threadIdx.x & 31);
+    for (int k = threadIdx.x >> 5; k < COLS; k += 8)
+      if (rr < M && c0 + k < N) i8_put(O + (long)rr * ldo_r + (long)(c0 + k) * ldo_c, tile[threadIdx.x & 31][k], alpha, beta);
+  } else {
+    __syncwarp();
+    const int rl = threadIdx.x >> 5, r = r0 + rl;
+    if (r < M)
+      for (int k = threadIdx.x & 31; k < COLS; k += 32)
+        if (c0 + k < N) i8_put(O + (long)r * ldo_r + (long)(c0 + k) * ldo_c, tile[rl][k], alpha, beta);
+  }
+}
+
+// ---- host side ----------------------------------------------------------------------------------
+
+static const I8Mod& i8_mods() {
+  static const I8Mod m = [] {
+    I8Mod r;
+    for (int i = 0; i < I8_MODS; ++i) {
+      const unsigned long long p = kI8P[i];
+      r.shift[i] = p > 128 ? 7 : 6;
+      // ceil(2^(32 + shift) / p) exceeds the quotient by less than p / p: exact for y < 2^31, p <= 2^(shift + 1)
+      r.p[i] = (unsigned)p;
+      r.magic[i] = (unsigned)(((1ULL << (32 + r.shift[i])) + p - 1) / p);
+      r.off[i] = (unsigned)(p * (((1ULL << 30) + p - 1) / p));
+    }
+    return r;
+  }();
+  return m;
+}
+
+static double i8_scale() {  // P 2^-64
+  static const double v = [] {
+    long double P = 1.0L;
+    for (int p : kI8P) P *= p;
+    return (double)(P / 18446744073709551616.0L);
+  }();
+  return v;
+}
+
+// Split-K of one launch: the split count with the shortest estimated time on 74 pairs, a K block costing
+// two MMAs of 128 cycles, an item the fill of its ring, and a split 32 bytes per output, written and read
+// back at about 2.5 TB/s.
+static int i8_splits(long M, long N, int kblocks) {
+  const long tiles = (M + 255) / 256 * ((N + 255) / 256);
+  long best = 1;
+  double best_t = 1e300;
+  const int least = (kblocks * I8_KB + I8_MAX_K - 1) / I8_MAX_K;
+  for (int s = least; s <= std::max(least, std::min(kblocks / 8, 16)); ++s) {
+    const int kps = (kblocks + s - 1) / s;
+    const long items = tiles * I8_MODS * 2 * ((kblocks + kps - 1) / kps);
+    const double t = (double)((items + I8_PAIRS - 1) / I8_PAIRS) * (kps * 256.0 + 500.0) + 0.025 * s * (double)M * N;
+    if (t < best_t * 0.98) {
+      best_t = t;
+      best = s;
+    }
+  }
+  return (int)best;
+}
+
+static bool i8_enabled() {
+  static const bool v = [] {
+    const char* e = std::getenv("DFTCUDA_ZGEMM");
+    return !e || std::string(e) == "i8";
+  }();
+  return v;
+}
+
+// The line between the residue form and the FP64 tensor cores (k_zgemm_dmma3m), from both sides' measured rates:
+// the residue form reads an operand twice and writes 32 bytes per entry at 4.5 TB/s together, multiplies at
+// 3.1e15 operations/s on its padded tiles, writes and reads 32 bytes per output at 2 TB/s, and costs
+// 50 us in launches and short kernels; the other runs at 31 TFLOP/s on its padded tiles.  share: the part of
+// an operand's conversion that this product pays for (an operand that its owner keeps is converted once for
+// several).  Measured, us, FP64 tensor cores / residues: V^H W 1344 x 448 x 61565 9390 / 2580, 536 x 132 x 18000
+// 548 / 306, 132 x 132 x 18000 224 / 171, 200 x 200 x 8000 185 / 135, 256 x 256 x 3000 97 / 105, 100 x 100 x 20000
+// 147 / 194, 34 x 61565 x 1080 1004 / 1462.
+static double i8_seconds(double M, double N, double K, double share_m, double share_n) {
+  auto up = [](double v, double u) { return std::ceil(v / u) * u; };
+  const double padded = std::min(up(M, 256) * up(N, 32), up(N, 256) * up(M, 32));
+  return 64.0 * K * (M * share_m + N * share_n) / 4.5e12 + 64.0 * padded * K / 3.1e15 + 64.0 * M * N / 2e12 + 50e-6;
+}
+
+bool zgemm_i8_worthwhile(int M, int N, int K, double share_m, double share_n) {
+  if (!i8_enabled() || M <= 0 || N <= 0 || K < 64) return false;
+  const double dmma = 8.0 * ((M + 63) / 64 * 64.0) * ((N + 63) / 64 * 64.0) * K / 31e12 + 12e-6;
+  return i8_seconds(M, N, K, share_m, share_n) < dmma;
+}
+
+// The same against the split TF32 form (105 TFLOP/s with its own conversions), for the projector products.
+bool zgemm_i8_beats_split_tf32(int M, int N, int K, double share_m, double share_n) {
+  return zgemm_i8_worthwhile(M, N, K, share_m, share_n) && i8_seconds(M, N, K, share_m, share_n) < 8.0 * M * (double)N * K / 105e12 + 10e-6;
+}
+
+constexpr size_t kI8ChunkElems = (size_t)1 << 25;  // entries of one operand whose tiles are held at a time
+constexpr long kI8ChunkOut = 1L << 26;             // outputs whose residues are held at a time
+
+size_t zgemm_i8_cache_bytes(int R, int K) { return ((size_t)R * 4 + 255) / 256 * 256 + i8_tile_bytes(R, K); }
+
+int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, bool* done) {
+  *done = false;
+  GemmArgs g = g0;
+  // The MMA's M side pads to 256 rows, its N side to 32 per tile: the orientation with less padding, or, within
+  // a tenth, the one whose N side is contiguous in the output.
+  auto tile_n = [](long n) { const long nt = (n + 255) / 256; return (n + 32 * nt - 1) / (32 * nt) * 32; };
+  auto padded = [&](long m, long n) { return (double)((m + 255) / 256 * 256) * ((n + tile_n(n) - 1) / tile_n(n) * tile_n(n)); };
+  const double keep = padded(g0.M, g0.N) * (g0.ldo_c <= g0.ldo_r ? 1.0 : 1.1);
+  const double turn = padded(g0.N, g0.M) * (g0.ldo_r <= g0.ldo_c ? 1.0 : 1.1);
+  if (turn < keep) {
+    std::swap(g.M, g.N);
+    std::swap(g.A, g.B);
+    std::swap(g.lda, g.ldb);
+    std::swap(g.a_kc, g.b_kc);
+    std::swap(g.conj_a, g.conj_b);
+    std::swap(g.ldo_r, g.ldo_c);
+    std::swap(g.a_cache, g.b_cache);
+  }
+  // chunks: equal parts of K, then of the rows, so that the tiles held are bounded
+  auto parts = [](long n, long most, long unit) {  // size of the equal parts of n, a multiple of unit
+    const long c = (n + most - 1) / most;
+    return std::min(n, ((n + c - 1) / c + unit - 1) / unit * unit);
+  };
+  const long Kc = parts(g.K, std::max<long>(8192, std::min<long>(I8_MAX_K, (long)(kI8ChunkElems / std::max(g.M, g.N)))), I8_KB);
+  const long rmax = std::max<long>(256, (long)(kI8ChunkElems / Kc));
+  const long Mc = parts(g.M, rmax, 256), Nc = parts(g.N, std::min(rmax, std::max<long>(256, kI8ChunkOut / Mc)), 256);
+  const int nk = (int)((g.K + Kc - 1) / Kc), KBc = (int)((Kc + I8_KB - 1) / I8_KB), KB = (g.K + I8_KB - 1) / I8_KB;
+  const int splits = i8_splits(Mc, Nc, KBc);
+  const int kps = (KBc + splits - 1) / splits;
+  int total_splits = 0;
+  for (int k = 0; k < nk; ++k) {
+    const int kb = (int)((std::min<long>(Kc, g.K - k * Kc) + I8_KB - 1) / I8_KB);
+    total_splits += (kb + kps - 1) / kps;
+  }
+  if (total_splits > I8_MAX_SPLITS) return DFTCUDA_OK;
+  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+  // norm chunks: enough blocks to cover the latency of their loads
+  auto norm_chunks = [&](bool kc, long R) {
+    const long blocks = kc ? R : (R + 255) / 256, least = kc ? 2048 : 32;
+    return (int)std::max<long>(1, std::min<long>({64, g.K / least, (1184 + blocks - 1) / blocks}));
+  };
+  size_t off = 0;
+  auto take = [&](size_t b) { const size_t o = off; off += up(b); return o; };
+  const size_t o_exa = take(4 * (size_t)g.M), o_exb = take(4 * (size_t)g.N);
+  const size_t o_part = take(sizeof(double2) * std::max((size_t)norm_chunks(g.a_kc, g.M) * g.M, (size_t)norm_chunks(g.b_kc, g.N) * g.N));
+  const size_t o_a = take(g.a_cache ? 0 : i8_tile_bytes(Mc, Kc));
+  const size_t o_b = take(g.b_cache ? 0 : i8_tile_bytes(Nc, Kc));
+  const size_t o_res = take((size_t)total_splits * I8_MODS * 2 * Mc * ((Nc + 255) / 256 * tile_n(Nc)));
+  auto no_room = [] {  // not done: the caller's other kernel runs, and must not meet this failure
+    cudaGetLastError();
+    return DFTCUDA_OK;
+  };
+  if (scratch->ensure(off) != DFTCUDA_OK) return no_room();
+  unsigned char* base = static_cast<unsigned char*>(scratch->p);
+
+  struct Op {
+    const double2* X;
+    long ld;
+    bool kc, cj;
+    int R;
+    TcScratch* cache;
+    int* ex;
+    I8Tiles t;        // of the whole operand (cache) or of the current chunk
+    long at_r, at_k;  // chunk held (no cache)
+  };
+  Op oa{g.A, g.lda, g.a_kc, g.conj_a, g.M, g.a_cache, (int*)(base + o_exa), {base + o_a, 0, 0}, -1, -1};
+  Op ob{g.B, g.ldb, g.b_kc, g.conj_b, g.N, g.b_cache, (int*)(base + o_exb), {base + o_b, 0, 0}, -1, -1};
+  auto exponents = [&](const Op& o) {
+    double2* part = reinterpret_cast<double2*>(base + o_part);
+    const int nch = norm_chunks(o.kc, o.R), kchunk = (g.K + nch - 1) / nch;
+    if (o.kc) k_i8_norm<true><<<dim3(o.R, nch), 256, 0, s>>>(o.X, o.ld, o.R, g.K, kchunk, part);
+    else k_i8_norm<false><<<dim3(ceil_div(o.R, 256), nch), 256, 0, s>>>(o.X, o.ld, o.R, g.K, kchunk, part);
+    k_i8_scale<<<ceil_div(o.R, 256), 256, 0, s>>>(part, o.R, nch, g.K, o.ex);
+    count_launch(2);
+  };
+  auto convert = [&](Op& o, long r0, int rows, long k0, int kn) {
+    const size_t kbs = (size_t)(kn + I8_KB - 1) / I8_KB;
+    o.t.kb = i8_groups(rows) * 8 * I8_KB;
+    o.t.plane = o.t.kb * kbs;
+    k_i8_tiles<<<dim3((unsigned)i8_groups(rows), ceil_div(kbs * (I8_KB / 16), 8)), 256, 0, s>>>(o.X, o.ld, o.kc, o.cj, (int)r0, rows,
+                                                                                             (int)k0, kn, o.ex, o.t);
+    count_launch();
+    o.at_r = r0;
+    o.at_k = k0;
+  };
+  for (Op* o : {&oa, &ob}) {
+    if (!o->cache) {
+      exponents(*o);
+      continue;
+    }
+    // an operand that its owner keeps: exponents and tiles of all of it
+    unsigned long long key = 0x69386b6579ULL;
+    for (unsigned long long v : {(unsigned long long)(uintptr_t)o->X, (unsigned long long)o->ld, (unsigned long long)o->kc,
+                                 (unsigned long long)o->cj, (unsigned long long)o->R, (unsigned long long)g.K})
+      key = key * 1000003ULL ^ v;
+    const size_t head = up((size_t)o->R * 4), need = zgemm_i8_cache_bytes(o->R, g.K);
+    const bool have = o->cache->valid && o->cache->key == key && o->cache->bytes >= need;
+    if (!have) {
+      o->cache->valid = false;
+      if (o->cache->ensure(need) != DFTCUDA_OK) return no_room();
+    }
+    o->ex = static_cast<int*>(o->cache->p);
+    o->t.p = static_cast<unsigned char*>(o->cache->p) + head;
+    o->t.kb = i8_groups(o->R) * 8 * I8_KB;
+    o->t.plane = o->t.kb * KB;
+    if (!have) {
+      exponents(*o);
+      convert(*o, 0, o->R, 0, g.K);
+      o->cache->key = key;
+      o->cache->valid = true;
+    }
+  }
+  DFT_TRY(ensure_max_dynamic_smem((const void*)k_i8_gemm, I8_SMEM));
+  for (long n0 = 0; n0 < g.N; n0 += Nc) {
+    for (long m0 = 0; m0 < g.M; m0 += Mc) {
+      const int rm = (int)std::min<long>(Mc, g.M - m0), rn = (int)std::min<long>(Nc, g.N - n0);
+      I8Gemm a{};
+      a.M = rm; a.N = rn;
+      a.mt = (rm + 255) / 256; a.nt = (rn + 255) / 256;
+      a.tn = (int)tile_n(rn);
+      a.Npad = a.nt * a.tn;
+      a.kps = kps;
+      a.err = err;
+      a.mod = i8_mods();
+      int z = 0;
+      for (int k = 0; k < nk; ++k) {
+        const long k0 = k * Kc;
+        const int kn = (int)std::min<long>(Kc, g.K - k0);
+        for (Op* o : {&oa, &ob}) {
+          const long r0 = o == &oa ? m0 : n0;
+          const int rows = o == &oa ? rm : rn;
+          if (!o->cache && (o->at_r != r0 || o->at_k != k0)) convert(*o, r0, rows, k0, kn);
+          const size_t at = o->cache ? (size_t)(k0 / I8_KB) * o->t.kb + (size_t)(r0 / 8) * 8 * I8_KB : 0;
+          (o == &oa ? a.A : a.B) = o->t.p + at;
+          (o == &oa ? a.a_plane : a.b_plane) = o->t.plane;
+          (o == &oa ? a.a_kb : a.b_kb) = o->t.kb;
+          (o == &oa ? a.rga : a.rgb) = (int)i8_groups(rows);
+        }
+        a.kblocks = (kn + I8_KB - 1) / I8_KB;
+        a.splits = (a.kblocks + kps - 1) / kps;
+        a.out = base + o_res + (size_t)z * I8_MODS * 2 * rm * a.Npad;
+        const int items = a.mt * a.nt * a.splits * I8_MODS * 2;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(2 * std::min(items, I8_PAIRS));
+        cfg.blockDim = dim3(I8_THREADS);
+        cfg.dynamicSmemBytes = I8_SMEM;
+        cfg.stream = s;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 2;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        DFT_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_i8_gemm, a));
+        count_launch();
+        z += a.splits;
+      }
+      double2* o = g.O + m0 * g.ldo_r + n0 * g.ldo_c;
+      const bool tr = g.ldo_r < g.ldo_c;
+      const dim3 grid = tr ? dim3(ceil_div(rn, 32), ceil_div(rm, 32)) : dim3(ceil_div(rn, 128), ceil_div(rm, 8));
+      auto* kernel = tr ? (z == 1 ? k_i8_out<true, true> : k_i8_out<true, false>) : (z == 1 ? k_i8_out<false, true> : k_i8_out<false, false>);
+      kernel<<<grid, 256, 0, s>>>(base + o_res, rm, rn, a.Npad, z, oa.ex + m0, ob.ex + n0, o, g.ldo_r, g.ldo_c, g.alpha, g.beta, i8_scale(), I8Less{kI8Less.hi * (unsigned long long)z, kI8Less.lo * z});
+      count_launch();
+    }
+  }
+  DFT_CUDA_TRY(cudaGetLastError());
+  *done = true;
+  return DFTCUDA_OK;
+}
+
+}  // namespace dftcuda
