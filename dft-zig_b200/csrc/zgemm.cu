@@ -316,14 +316,17 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_dmma16(int M, int N, int K, co
 //   T1 = ar (br + bi),  T2 = (ar + ai) bi,  T3 = (ai - ar) br;   Re = T1 - T2,  Im = T1 + T3.
 // The m8n8k4 kernel's tiling and fragments with a third accumulator per 8 x 8 tile: a quarter
 // fewer FP64 MMAs, the FP64 tensor pipe being the bound of the four-product form.
-template <bool AKC, bool BKC, bool CJA, bool CJB>
-__global__ void __launch_bounds__(256, 2) k_zgemm_dmma3m(int M, int N, int K, const double2* __restrict__ A, long lda,
+// ST K slices in shared memory: two for products that fill the chip (two CTAs per SM; a third slice
+// measured 2-3 % slower), four where there is at most one CTA per SM, whose time is the latency of its
+// loads: three slices are then in flight instead of one.
+template <bool AKC, bool BKC, bool CJA, bool CJB, int ST>
+__global__ void __launch_bounds__(256, ST == 2 ? 2 : 1) k_zgemm_dmma3m(int M, int N, int K, const double2* __restrict__ A, long lda,
                                                          const double2* __restrict__ B, long ldb, double2* __restrict__ O,
                                                          long ldo_r, long ldo_c, double alpha, double beta, int kps,
                                                          double2* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char zsm[];
   double2(*As)[BK][BM + kZmPad] = reinterpret_cast<double2(*)[BK][BM + kZmPad]>(zsm);
-  double2(*Bs)[BK][BN + kZmPad] = reinterpret_cast<double2(*)[BK][BN + kZmPad]>(zsm + 2 * sizeof(double2) * BK * (BM + kZmPad));
+  double2(*Bs)[BK][BN + kZmPad] = reinterpret_cast<double2(*)[BK][BN + kZmPad]>(zsm + ST * sizeof(double2) * BK * (BM + kZmPad));
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int wr = warp >> 1, wc = warp & 1;
@@ -338,12 +341,17 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_dmma3m(int M, int N, int K, co
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h) t1[i][j][h] = t2[i][j][h] = t3[i][j][h] = 0.0;
-  if (kbeg < kend) zgemm_fetch<AKC, BKC, kZmPad>(As[0], Bs[0], M, N, kend, r0, c0, kbeg, A, lda, B, ldb, tid);
+  auto fetch = [&](int k, int b) {  // one group per slice, empty past the end
+    if (k < kend) zgemm_fetch<AKC, BKC, kZmPad>(As[b], Bs[b], M, N, kend, r0, c0, k, A, lda, B, ldb, tid);
+    else cp_async_commit();
+  };
+#pragma unroll
+  for (int i = 0; i + 1 < ST; ++i) fetch(kbeg + i * BK, i);
   int buf = 0;
   for (int k0 = kbeg; k0 < kend; k0 += BK) {
-    cp_async_wait_all();
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2));
     __syncthreads();
-    if (k0 + BK < kend) zgemm_fetch<AKC, BKC, kZmPad>(As[buf ^ 1], Bs[buf ^ 1], M, N, kend, r0, c0, k0 + BK, A, lda, B, ldb, tid);
+    fetch(k0 + (ST - 1) * BK, (buf + ST - 1) % ST);
 #pragma unroll
     for (int k4 = 0; k4 < BK; k4 += 4) {
       double ar[2], as_[2], ad[2], bs[4], bi[4], br[4];
@@ -371,7 +379,7 @@ __global__ void __launch_bounds__(256, 2) k_zgemm_dmma3m(int M, int N, int K, co
           dmma(t3[i][j][0], t3[i][j][1], ad[i], br[j]);
         }
     }
-    buf ^= 1;
+    buf = (buf + 1) % ST;
   }
 #pragma unroll
   for (int i = 0; i < 2; ++i)
@@ -459,8 +467,11 @@ static int zgemm_kind() {
 template <bool AKC, bool BKC, bool CJA, bool CJB>
 static void launch(const GemmArgs& g, dim3 grid, int kps, double2* part, cudaStream_t s) {
   if (zgemm_kind() == 3) {
-    ensure_max_dynamic_smem((const void*)k_zgemm_dmma3m<AKC, BKC, CJA, CJB>, (int)kZgemmDmmaSmem);
-    k_zgemm_dmma3m<AKC, BKC, CJA, CJB><<<grid, 256, kZgemmDmmaSmem, s>>>(g.M, g.N, g.K, g.A, g.lda, g.B, g.ldb, g.O, g.ldo_r,
+    const bool few = (long)grid.x * grid.y * grid.z <= 148;
+    const size_t smem = few ? 2 * kZgemmDmmaSmem : kZgemmDmmaSmem;
+    auto* kernel = few ? k_zgemm_dmma3m<AKC, BKC, CJA, CJB, 4> : k_zgemm_dmma3m<AKC, BKC, CJA, CJB, 2>;
+    ensure_max_dynamic_smem((const void*)kernel, (int)smem);
+    kernel<<<grid, 256, smem, s>>>(g.M, g.N, g.K, g.A, g.lda, g.B, g.ldb, g.O, g.ldo_r,
                                                                         g.ldo_c, g.alpha, g.beta, kps, part);
     count_launch();
     return;
@@ -490,6 +501,11 @@ int zgemm(const GemmArgs& g, cudaStream_t s, double2* ws, size_t ws_elems) {
     // out = beta * out
     return fail(DFTCUDA_ERR_INVALID_ARGUMENT, "zgemm: K must be positive");
   }
+  if (g.i8 && g.err && zgemm_i8_worthwhile(g.M, g.N, g.K, g.a_share, g.b_share)) {
+    bool done = false;
+    DFT_TRY(zgemm_i8(g, s, g.i8, g.err, &done));
+    if (done) return DFTCUDA_OK;
+  }
   int splits = g.splits > 0 ? std::min(g.splits, std::max(1, g.K / 32)) : pick_splits(g.M, g.N, g.K);
   if (splits > 1) splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ws_elems / ((size_t)g.M * g.N)));  // what fits the workspace
   int kps = (g.K + splits - 1) / splits;
@@ -501,11 +517,6 @@ int zgemm(const GemmArgs& g, cudaStream_t s, double2* ws, size_t ws_elems) {
   switch (key) {
     case 0: launch<false, false, false, false>(g, grid, kps, part, s); break;
     case 1: launch<false, false, false, true>(g, grid, kps, part, s); break;
-  if (g.i8 && g.err && zgemm_i8_worthwhile(g.M, g.N, g.K, g.a_share, g.b_share)) {
-    bool done = false;
-    DFT_TRY(zgemm_i8(g, s, g.i8, g.err, &done));
-    if (done) return DFTCUDA_OK;
-  }
     case 2: launch<false, false, true, false>(g, grid, kps, part, s); break;
     case 3: launch<false, false, true, true>(g, grid, kps, part, s); break;
     case 4: launch<false, true, false, false>(g, grid, kps, part, s); break;
