@@ -20,14 +20,14 @@
 
 namespace dftcuda {
 
-// Roots exp(2 pi i e / L) for the sub-DFT lengths, concatenated: L = 2,3,4,5,6,8,9,10,12,15,16.
-constexpr int kRootLens[] = {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16};
+// Roots exp(2 pi i e / L) for the sub-DFT lengths, concatenated: L = 2,3,4,5,6,8,9,10,12,15,16,18.
+constexpr int kRootLens[] = {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18};
 constexpr int kNumRootLens = sizeof(kRootLens) / sizeof(int);
 __host__ __device__ constexpr int root_off(int L) {
   return L == 2 ? 0 : L == 3 ? 2 : L == 4 ? 5 : L == 5 ? 9 : L == 6 ? 14 : L == 8 ? 20 : L == 9 ? 28
-       : L == 10 ? 37 : L == 12 ? 47 : L == 15 ? 59 : L == 16 ? 74 : -1;
+       : L == 10 ? 37 : L == 12 ? 47 : L == 15 ? 59 : L == 16 ? 74 : L == 18 ? 90 : -1;
 }
-constexpr int kRootTotal = root_off(16) + 16;
+constexpr int kRootTotal = root_off(18) + 18;
 
 // Defined here (not extern): the library is compiled without relocatable device code, so every
 // translation unit that includes this header has its own copy of the tables, and must fill it with
@@ -155,7 +155,7 @@ struct RegDft<T, 1> {
   static __device__ __forceinline__ void run(cplx<T>*, T) {}
 };
 
-// Factorisation N = N1 * N2 used by the four-step kernels (N1 >= N2, both <= 16).
+// Factorisation N = N1 * N2 used by the four-step kernels (N1 >= N2, both <= 16; XSplit below: <= 18).
 template <int N> struct Split;
 #define DFTCUDA_SPLIT(N, A, B) \
   template <> struct Split<N> { static constexpr int N1 = A, N2 = B; };
@@ -180,6 +180,27 @@ DFTCUDA_SPLIT(108, 12, 9)
 DFTCUDA_SPLIT(120, 12, 10)
 DFTCUDA_SPLIT(128, 16, 8)
 #undef DFTCUDA_SPLIT
+
+// The split of the warp-synchronous x lines, where one warp's lanes serve floor(32 / N2) lines in all steps and
+// each takes ceil(N1 / N2) rows of the middle step, the dearest one: N1 a multiple of N2, or nearly, and
+// 32 nearly a multiple of N2 keep the lanes busy (108 = 12 x 9 leaves 44 % of the middle step idle, 18 x 6
+// leaves 6 %).
+template <int N> struct XSplit {
+  static constexpr int N1 = Split<N>::N1, N2 = Split<N>::N2;
+};
+#define DFTCUDA_XSPLIT(N, A, B) \
+  template <> struct XSplit<N> { static constexpr int N1 = A, N2 = B; };
+DFTCUDA_XSPLIT(20, 10, 2)
+DFTCUDA_XSPLIT(24, 8, 3)
+DFTCUDA_XSPLIT(30, 10, 3)
+DFTCUDA_XSPLIT(48, 12, 4)
+DFTCUDA_XSPLIT(72, 12, 6)
+DFTCUDA_XSPLIT(80, 16, 5)
+DFTCUDA_XSPLIT(90, 18, 5)
+DFTCUDA_XSPLIT(96, 16, 6)
+DFTCUDA_XSPLIT(108, 18, 6)
+DFTCUDA_XSPLIT(120, 15, 8)
+#undef DFTCUDA_XSPLIT
 
 // Lengths with a four-step kernel (keep in sync with the Split table and the dispatch switches).
 #define DFTCUDA_FOUR_STEP_LENGTHS(X) \

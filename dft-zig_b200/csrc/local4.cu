@@ -477,90 +477,92 @@ __global__ void __launch_bounds__(256) k_xline4(cplx<T>* __restrict__ W, int n_a
 }
 
 // Geometry of the warp-synchronous x-line pass: a line's x transform is done by N2 lanes of one
-// warp (LW lines per warp).  Exchange-buffer stride S >= NX with S = N2 (mod 8), so the step-A writes
-// of the N2 lanes of consecutive lines fall in distinct 16-byte bank groups.
+// warp (LW lines per warp).  Exchange buffer per line: N1 rows of N2 entries, row stride RP odd, line
+// stride S = N2 (mod 8), so that a quarter warp's 16-byte accesses fall in distinct bank groups along the
+// rows (lanes over t) and across them (lanes over k1).
 template <int NX> struct XLineGeom {
-  static constexpr int N1 = Split<NX>::N1, N2 = Split<NX>::N2;
+  static constexpr int N1 = XSplit<NX>::N1, N2 = XSplit<NX>::N2;
   static constexpr int LW = 32 / N2;
   static constexpr int Q = (N1 + N2 - 1) / N2;
-  static constexpr int S = NX + ((N2 - NX) % 8 + 8) % 8;
+  static constexpr int RP = N2 | 1;
+  static constexpr int S = N1 * RP + ((N2 - N1 * RP) % 8 + 8) % 8;
 };
 constexpr int kXlWarps = 3;
 
 // x-line pass with every lane busy in every phase: lane t of a line
 //   1. inverse step A for index t: DFT_N1 over the inputs x = m N2 + t (the active slots),
 //   2. for its rows k1 = t, t + N2, ... < N1: inverse step B (DFT_N2), x V(r) at x = k1 + N1 k2,
-//      forward step A (DFT_N2, lengths swapped) and its twiddles,
+//      forward step A (DFT_N2, lengths swapped) and its twiddles, back into the same row,
 //   3. forward step B for frequency index t: DFT_N1, outputs x = t + N2 m back to the active slots.
-// The exchanges go through two per-warp shared buffers with __syncwarp only (no block barriers);
-// the input and output slot sets of a lane coincide ({t + N2 m}).  V(r) and the slot table are read
-// through L1 (reused by the CTA's columns) instead of being held in registers.
+// The exchanges go through one per-warp shared buffer with __syncwarp only (no block barriers); a
+// lane's slots ({t + N2 m}, the same for input and output) stay in registers, the twiddles in shared
+// memory in the order the lanes read them.  V(r) is read through L1 (reused by the CTA's columns).
 template <typename T, int NX>
 __global__ void __launch_bounds__(kXlWarps * 32, 5) k_xline5(cplx<T>* __restrict__ W, int n_act, const int* __restrict__ slot_of_x,
                                                              const T* __restrict__ Vt, int P, int ncols, int cols_per_cta,
                                                              const cplx<T>* __restrict__ tw) {
   using C = cplx<T>;
   using G = XLineGeom<NX>;
-  constexpr int N1 = G::N1, N2 = G::N2, LW = G::LW, Q = G::Q, S = G::S;
+  constexpr int N1 = G::N1, N2 = G::N2, LW = G::LW, Q = G::Q, RP = G::RP;
   extern __shared__ __align__(16) unsigned char smraw[];
+  C* twa = reinterpret_cast<C*>(smraw);  // [k1][t] = w^(t k1)
+  C* twb = twa + NX;                     // [k2][k1] = w^-(k1 k2)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int L = lane / N2, t = lane - L * N2;
   const bool lane_ok = L < LW;
-  C* B1 = reinterpret_cast<C*>(smraw) + ((size_t)warp * LW + (lane_ok ? L : 0)) * S;
-  C* B2 = B1 + (size_t)kXlWarps * LW * S;
+  C* B = twb + NX + ((size_t)warp * LW + (lane_ok ? L : 0)) * G::S;
   const int j = (blockIdx.x * kXlWarps + warp) * LW + L;
   const bool lv = lane_ok && j < P;
   const int c0 = blockIdx.y * cols_per_cta;
   const int c1 = min(ncols, c0 + cols_per_cta);
-  const int* slt = slot_of_x + t;  // slot of x = t + N2 m at slt[N2 m]
+  for (int i = threadIdx.x; i < NX; i += blockDim.x) {
+    twa[i] = tw_ld<T>(tw, ((i / N2) * (i % N2)) % NX, (T)1);
+    twb[i] = tw_ld<T>(tw, ((i / N1) * (i % N1)) % NX, (T)-1);
+  }
+  int sl[N1];  // slots of x = t + N2 m
+#pragma unroll
+  for (int m = 0; m < N1; ++m) sl[m] = lv ? __ldg(slot_of_x + t + N2 * m) : -1;
+  __syncthreads();
   for (int c = c0; c < c1; ++c) {
     C* Wc = W + (long)c * n_act * P + j;
     {  // 1. inverse step A
       C v[N1];
 #pragma unroll
-      for (int m = 0; m < N1; ++m) {
-        const int sm = lv ? __ldg(slt + N2 * m) : -1;
-        v[m] = sm >= 0 ? Wc[(long)sm * P] : mk<C>(0.0, 0.0);
-      }
+      for (int m = 0; m < N1; ++m) v[m] = sl[m] >= 0 ? Wc[(long)sl[m] * P] : mk<C>(0.0, 0.0);
       RegDft<T, N1>::run(v, (T)1);
-#pragma unroll
-      for (int k1 = 1; k1 < N1; ++k1)
-        if (t) v[k1] = cmul(v[k1], tw_ld<T>(tw, (t * k1) % NX, (T)1));
       if (lane_ok) {
+        B[t] = v[0];
 #pragma unroll
-        for (int k1 = 0; k1 < N1; ++k1) B1[k1 * N2 + t] = v[k1];
+        for (int k1 = 1; k1 < N1; ++k1) B[k1 * RP + t] = cmul(v[k1], twa[k1 * N2 + t]);
       }
     }
     __syncwarp();
 #pragma unroll
-    for (int q = 0; q < Q; ++q) {  // 2. inverse step B, x V(r), forward step A
+    for (int q = 0; q < Q; ++q) {  // 2. inverse step B, x V(r), forward step A, row k1 in place
       const int k1 = t + N2 * q;
-      if (lane_ok && k1 < N1) {
+      if (lv && k1 < N1) {
+        C* row = B + k1 * RP;
         C u[N2];
 #pragma unroll
-        for (int tt = 0; tt < N2; ++tt) u[tt] = B1[k1 * N2 + tt];
+        for (int tt = 0; tt < N2; ++tt) u[tt] = row[tt];
         RegDft<T, N2>::run(u, (T)1);
 #pragma unroll
-        for (int k2 = 0; k2 < N2; ++k2) u[k2] = cscale(u[k2], lv ? __ldg(Vt + (long)(k1 + N1 * k2) * P + j) : (T)0);
+        for (int k2 = 0; k2 < N2; ++k2) u[k2] = cscale(u[k2], __ldg(Vt + (long)(k1 + N1 * k2) * P + j));
         RegDft<T, N2>::run(u, (T)-1);
+        row[0] = u[0];
 #pragma unroll
-        for (int k1f = 1; k1f < N2; ++k1f)
-          if (k1) u[k1f] = cmul(u[k1f], tw_ld<T>(tw, (k1 * k1f) % NX, (T)-1));
-#pragma unroll
-        for (int k1f = 0; k1f < N2; ++k1f) B2[k1f * N1 + k1] = u[k1f];
+        for (int kf = 1; kf < N2; ++kf) row[kf] = cmul(u[kf], twb[kf * N1 + k1]);
       }
     }
     __syncwarp();
     {  // 3. forward step B for frequency index t
       C v[N1];
 #pragma unroll
-      for (int tf = 0; tf < N1; ++tf) v[tf] = lane_ok ? B2[t * N1 + tf] : mk<C>(0.0, 0.0);
+      for (int tf = 0; tf < N1; ++tf) v[tf] = lane_ok ? B[tf * RP + t] : mk<C>(0.0, 0.0);
       RegDft<T, N1>::run(v, (T)-1);
 #pragma unroll
-      for (int m = 0; m < N1; ++m) {
-        const int sm = lv ? __ldg(slt + N2 * m) : -1;
-        if (sm >= 0) Wc[(long)sm * P] = v[m];
-      }
+      for (int m = 0; m < N1; ++m)
+        if (sl[m] >= 0) Wc[(long)sl[m] * P] = v[m];
     }
     __syncwarp();
   }
@@ -693,7 +695,7 @@ static int launch_xline4(dftcuda_kctx* c, cplx<T>* W, size_t ncols, cudaStream_t
   const cplx<T>* tw = std::is_same<T, double>::value ? (const cplx<T>*)c->d_tw4x64 : (const cplx<T>*)c->d_tw4x32;
   if (!fft4_legacy()) {
     using G = XLineGeom<NX>;
-    const size_t smem5 = 2 * sizeof(cplx<T>) * (size_t)kXlWarps * G::LW * G::S;
+    const size_t smem5 = sizeof(cplx<T>) * (2 * NX + (size_t)kXlWarps * G::LW * G::S);
     DFT_TRY(ensure_max_dynamic_smem((const void*)k_xline5<T, NX>, (int)kSmem4));
     const int cpc = 4;
     dim3 g(ceil_div(c->P, kXlWarps * G::LW), ceil_div(ncols, cpc));

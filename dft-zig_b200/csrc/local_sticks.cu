@@ -36,9 +36,8 @@ namespace {
 constexpr int kStickTile = 32;    // sticks per CTA of the stick passes
 constexpr int kStickPad = kStickTile + 1;
 constexpr int kStickThreads = 256;
-// warps of a z-plane CTA (128 registers per lane)
-template <typename T> constexpr int plane_max_warps() { return 16; }
-template <typename T> constexpr int kDensityWarps() { return 16; }
+// most warps of a z-plane CTA: 168 registers per lane for the FP64 lines, 128 for the FP32 ones
+template <typename T> constexpr int plane_max_warps() { return sizeof(T) == 8 ? 12 : 16; }
 
 template <typename T> __device__ __forceinline__ cplx<T> twl(const cplx<T>* tw, int e, T sg) {
   cplx<T> w = tw[e];
@@ -181,8 +180,9 @@ __global__ void __launch_bounds__(kStickThreads) k_stick_fwd(const cplx<T>* __re
 // Exchange buffer of one x line: N1 rows of N2 entries, row stride RP odd, so that a quarter warp's
 // 16-byte accesses fall on distinct bank groups both along a row (lanes over t) and down a column of rows
 // (lanes over k1); line stride S = N2 modulo 8 entries, which continues the pattern across a warp's lines.
-template <int NX> struct PlaneXGeom {
-  static constexpr int N1 = Split<NX>::N1, N2 = Split<NX>::N2;
+template <int NX, typename X = XSplit<NX>> struct PlaneXGeom {
+  static constexpr int N1 = X::N1, N2 = X::N2;
+  static constexpr int Y1 = Split<NX>::N1, Y2 = Split<NX>::N2;       // the y transforms' split
   static constexpr int LW = 32 / N2;                                 // lines per warp
   static constexpr int Q = (N1 + N2 - 1) / N2;                       // phase-2 rows per lane
   static constexpr int RP = N2 | 1;
@@ -225,9 +225,8 @@ __device__ __forceinline__ void plane_y_inverse(const cplx<T>* Srow, const int* 
 
 // Per (z plane, column): inverse y, then per y line inverse x, x V(r), forward x, then forward y.  The
 // plane's sticks are read by the first step and written by the last one; the x lines exchange through a
-// per-warp buffer in which a lane's rows stay its own from the inverse step B to the forward step A, so one
-// row at a time is in registers and 16 FP64 warps fit an SM (128 registers; the two rows that a transposed
-// layout held at once allowed 12).  The four-step twiddles sit in shared memory in the order the lanes
+// per-warp buffer in which a lane's rows stay its own from the inverse step B to the forward step A, so that
+// one row at a time is in registers and the lines can take the split that keeps the lanes busy (XSplit).  The four-step twiddles sit in shared memory in the order the lanes
 // read them.  Bound by shared memory / L1 wavefronts and the FP64 pipe, about equally.
 template <typename T, int N>
 __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>* __restrict__ S, int n_st, const int* __restrict__ st_of,
@@ -236,12 +235,14 @@ __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>
                                                                      int cols_per_cta, const cplx<T>* __restrict__ tw) {
   using C = cplx<T>;
   using G = PlaneXGeom<N>;
-  constexpr int N1 = G::N1, N2 = G::N2, LW = G::LW, QR = G::Q, RP = G::RP;
+  constexpr int N1 = G::N1, N2 = G::N2, Y1 = G::Y1, Y2 = G::Y2, LW = G::LW, QR = G::Q, RP = G::RP;
   constexpr int QS = N + 1;  // Q row stride: odd, so lanes over slots hit distinct banks
   extern __shared__ __align__(16) unsigned char smraw[];
-  C* twa = reinterpret_cast<C*>(smraw);  // [k1][t] = w^(t k1)
-  C* twb = twa + N;                      // [k2][k1] = w^-(k1 k2)
-  C* Q = twb + N;                        // [n_act][QS]
+  C* twa = reinterpret_cast<C*>(smraw);  // x split: [k1][t] = w^(t k1)
+  C* twb = twa + N;                      // x split: [k2][k1] = w^-(k1 k2)
+  C* ya = twb + N;                       // the same of the y split
+  C* yb = ya + N;
+  C* Q = yb + N;                         // [n_act][QS]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   C* Bw = Q + (size_t)n_act * QS + (size_t)warp * LW * G::S;  // this warp's exchange buffer
   const int z = blockIdx.x;
@@ -255,6 +256,8 @@ __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
     twa[i] = twl<T>(tw, ((i / N2) * (i % N2)) % N, (T)1);
     twb[i] = twl<T>(tw, ((i / N1) * (i % N1)) % N, (T)-1);
+    ya[i] = twl<T>(tw, ((i / Y2) * (i % Y2)) % N, (T)1);
+    yb[i] = twl<T>(tw, ((i / Y1) * (i % Y1)) % N, (T)-1);
   }
   int so[N1];  // Q offsets of this lane's slots along x, or -1
 #pragma unroll
@@ -265,12 +268,12 @@ __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>
   for (int c = c0; c < c1; ++c) {
     C* Srow = S + ((long)c * gridDim.x + r) * n_st;
     __syncthreads();  // the previous column's last step has read Q
-    plane_y_inverse<T, N>(Srow, st_of, n_act, Q, twa);
+    plane_y_inverse<T, N>(Srow, st_of, n_act, Q, ya);
     // x lines: LW lines per warp; line y sits in column col(y) of every active slot
     for (int lt = warp; lt * LW < N; lt += nwarp) {
       const int yl = lt * LW + L;
       const bool lv = lane_ok && yl < N;
-      const int col = lv ? (yl % N1) * N2 + yl / N1 : 0;
+      const int col = lv ? (yl % Y1) * Y2 + yl / Y1 : 0;
       {  // inverse step A over x = t + N2 m
         C v[N1];
 #pragma unroll
@@ -314,35 +317,39 @@ __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>
       __syncwarp();
     }
     __syncthreads();
-    // forward y (split swapped), step A: task (t < N1, slot) reads columns t N2 + j
-    for (int w = threadIdx.x; w < N1 * n_act; w += blockDim.x) {
+    // forward y (split swapped), step A: task (t < Y1, slot) reads columns t Y2 + j
+    for (int w = threadIdx.x; w < Y1 * n_act; w += blockDim.x) {
       const int sl = w % n_act, tt = w / n_act;
-      C* q = Q + sl * QS + tt * N2;
-      C v[N2];
+      C* q = Q + sl * QS + tt * Y2;
+      C v[Y2];
 #pragma unroll
-      for (int j = 0; j < N2; ++j) v[j] = q[j];
-      RegDft<T, N2>::run(v, (T)-1);
+      for (int j = 0; j < Y2; ++j) v[j] = q[j];
+      RegDft<T, Y2>::run(v, (T)-1);
       q[0] = v[0];
 #pragma unroll
-      for (int k = 1; k < N2; ++k) q[k] = cmul(v[k], twb[k * N1 + tt]);
+      for (int k = 1; k < Y2; ++k) q[k] = cmul(v[k], yb[k * Y1 + tt]);
     }
     __syncthreads();
-    // forward y, step B: task (k < N2, slot), frequencies k + N2 m to their sticks
-    for (int w = threadIdx.x; w < N2 * n_act; w += blockDim.x) {
+    // forward y, step B: task (k < Y2, slot), frequencies k + Y2 m to their sticks
+    for (int w = threadIdx.x; w < Y2 * n_act; w += blockDim.x) {
       const int sl = w % n_act, k = w / n_act;
       const C* q = Q + sl * QS;
-      C u[N1];
+      C u[Y1];
 #pragma unroll
-      for (int tt = 0; tt < N1; ++tt) u[tt] = q[tt * N2 + k];
-      RegDft<T, N1>::run(u, (T)-1);
+      for (int tt = 0; tt < Y1; ++tt) u[tt] = q[tt * Y2 + k];
+      RegDft<T, Y1>::run(u, (T)-1);
 #pragma unroll
-      for (int m = 0; m < N1; ++m) {
-        const int g = __ldg(st_of + (k + N2 * m) * n_act + sl);
+      for (int m = 0; m < Y1; ++m) {
+        const int g = __ldg(st_of + (k + Y2 * m) * n_act + sl);
         if (g >= 0) Srow[g] = u[m];
       }
     }
   }
 }
+
+// The density pass holds all rows of its middle step while the parts of the exchange pass one after the other:
+// the split with fewer of them.
+template <int N> using DensityGeom = PlaneXGeom<N, Split<N>>;
 
 // Doubles reserved for the density kernel's N x N plane: rounded up to an even count, so the complex
 // plane after it starts on a 16-byte boundary (N^2 is odd for odd N).
@@ -354,18 +361,19 @@ template <int N> __host__ __device__ constexpr int density_plane_words() { retur
 // added to the global density once at the end (several CTAs share a plane: atomics).
 // ------------------------------------------------------------------------------------------
 template <typename T, int N>
-__global__ void __launch_bounds__(kDensityWarps<T>() * 32, 1) k_zplane_density(const cplx<T>* __restrict__ S, int n_st, const int* __restrict__ st_of,
+__global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane_density(const cplx<T>* __restrict__ S, int n_st, const int* __restrict__ st_of,
                                                            int n_act, const int* __restrict__ slot_of_x, int n1z, int n2z, int ncols,
                                                            int cols_per_cta, const cplx<T>* __restrict__ tw,
                                                            const double* __restrict__ wgt, double inv_vol, double* __restrict__ rho) {
   using C = cplx<T>;
-  using G = PlaneXGeom<N>;
-  constexpr int N1 = G::N1, N2 = G::N2, LW = G::LW, QR = G::Q, RP = G::RP;
+  using G = DensityGeom<N>;
+  constexpr int N1 = G::N1, N2 = G::N2, Y1 = G::Y1, Y2 = G::Y2, LW = G::LW, QR = G::Q, RP = G::RP;
   constexpr int QS = N + 1;
   extern __shared__ __align__(16) unsigned char smraw[];
   double* R = reinterpret_cast<double*>(smraw);                 // [N][N] density plane, x fastest
-  C* twa = reinterpret_cast<C*>(R + density_plane_words<N>());  // [k1][t] = w^(t k1), 16-byte aligned
-  C* Q = twa + N;                                               // [n_act][QS]
+  C* twa = reinterpret_cast<C*>(R + density_plane_words<N>());  // x split: [k1][t] = w^(t k1), 16-byte aligned
+  C* ya = twa + N;                                              // the same of the y split
+  C* Q = ya + N;                                                // [n_act][QS]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   T* Bw = reinterpret_cast<T*>(Q + (size_t)n_act * QS) + (size_t)warp * LW * G::S;  // one part at a time
   const int z = blockIdx.x;
@@ -375,7 +383,10 @@ __global__ void __launch_bounds__(kDensityWarps<T>() * 32, 1) k_zplane_density(c
   const int L = lane / N2, t = lane - L * N2;
   const bool lane_ok = L < LW;
   T* B = Bw + (lane_ok ? L : 0) * G::S;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) twa[i] = twl<T>(tw, ((i / N2) * (i % N2)) % N, (T)1);
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    twa[i] = twl<T>(tw, ((i / N2) * (i % N2)) % N, (T)1);
+    ya[i] = twl<T>(tw, ((i / Y2) * (i % Y2)) % N, (T)1);
+  }
   for (int i = threadIdx.x; i < N * N; i += blockDim.x) R[i] = 0.0;
   int so[N1];
 #pragma unroll
@@ -387,11 +398,11 @@ __global__ void __launch_bounds__(kDensityWarps<T>() * 32, 1) k_zplane_density(c
     const C* Srow = S + ((long)c * gridDim.x + r) * n_st;
     const double wc = __ldg(wgt + c) * inv_vol;
     __syncthreads();
-    plane_y_inverse<T, N>(Srow, st_of, n_act, Q, twa);
+    plane_y_inverse<T, N>(Srow, st_of, n_act, Q, ya);
     for (int lt = warp; lt * LW < N; lt += nwarp) {
       const int yl = lt * LW + L;
       const bool lv = lane_ok && yl < N;
-      const int col = lv ? (yl % N1) * N2 + yl / N1 : 0;
+      const int col = lv ? (yl % Y1) * Y2 + yl / Y1 : 0;
       C v[N1];
 #pragma unroll
       for (int m = 0; m < N1; ++m) v[m] = so[m] >= 0 ? Q[so[m] + col] : mk<C>(0.0, 0.0);
@@ -452,7 +463,7 @@ static size_t stick_smem(size_t cs, int nz) { return cs * (size_t)nz * kStickPad
 // fewer idle warps in the short y steps of small planes), else as many as fit one.
 template <int N> static int plane_warps(size_t cs, int n_act) {
   using G = PlaneXGeom<N>;
-  const size_t q = cs * ((size_t)n_act * (N + 1) + 2 * N);
+  const size_t q = cs * ((size_t)n_act * (N + 1) + 4 * N);
   const size_t per_warp = cs * (size_t)G::LW * G::S;
   if (2 * (q + 8 * per_warp + 1024) <= (size_t)kSmemSticks) return 8;
   const int maxw = cs == sizeof(double2) ? plane_max_warps<double>() : plane_max_warps<float>();
@@ -520,7 +531,7 @@ static int launch_zplane(dftcuda_kctx* c, cplx<T>* S, size_t ncols, cudaStream_t
   const size_t cs = sizeof(cplx<T>);
   const int nw = plane_warps<N>(cs, c->n_act);
   if (nw < 1) return fail(DFTCUDA_ERR_UNSUPPORTED, "z-plane pass does not fit shared memory");
-  const size_t smem = cs * ((size_t)c->n_act * (N + 1) + 2 * N + (size_t)nw * G::LW * G::S);
+  const size_t smem = cs * ((size_t)c->n_act * (N + 1) + 4 * N + (size_t)nw * G::LW * G::S);
   DFT_TRY(ensure_max_dynamic_smem((const void*)k_zplane<T, N>, (int)smem));
   const T* vn = std::is_same<T, double>::value ? (const T*)c->d_vn : (const T*)c->d_vn32;
   const cplx<T>* tw = std::is_same<T, double>::value ? (const cplx<T>*)c->d_twx64 : (const cplx<T>*)c->d_twx32;
@@ -545,14 +556,14 @@ static int launch_zplane(dftcuda_kctx* c, cplx<T>* S, size_t ncols, cudaStream_t
 }
 
 template <typename T, int N> static size_t density_plane_smem(int n_act, int warps) {
-  using G = PlaneXGeom<N>;
-  return sizeof(double) * (size_t)density_plane_words<N>() + sizeof(cplx<T>) * ((size_t)n_act * (N + 1) + N) +
+  using G = DensityGeom<N>;
+  return sizeof(double) * (size_t)density_plane_words<N>() + sizeof(cplx<T>) * ((size_t)n_act * (N + 1) + 2 * N) +
          sizeof(T) * (size_t)warps * G::LW * G::S;
 }
 // Warps of the density pass, likewise; eight at least, or the pass is not used.
 template <typename T, int N> static int density_warps(int n_act) {
   if (2 * (density_plane_smem<T, N>(n_act, 8) + 1024) <= (size_t)kSmemSticks) return 8;
-  for (int w = kDensityWarps<T>(); w >= 8; --w)
+  for (int w = plane_max_warps<T>(); w >= 8; --w)
     if (density_plane_smem<T, N>(n_act, w) <= (size_t)kSmemSticks) return w;
   return 0;
 }
