@@ -8,8 +8,7 @@
 //  * random start: the reference's LCG (common.zig:287-319) evaluated in closed form per element
 //    (s_k = a^k s0 + sum_{j<k} a^j mod 2^64), so the device draws exactly the reference's numbers;
 //  * T = V^H W, Hermitised (common.zig:231-259): FP64 complex GEMM on the new columns only + k_gram_finish;
-//  * small eigenproblem (zheev, common.zig:440-508): cyclic two-sided complex Jacobi in one CTA
-//    below 96 columns, the tridiagonal solver of heev.cu (lowest nbands pairs) from there on;
+//  * small eigenproblem (zheev, common.zig:440-508): the tridiagonal solver of heev.cu (lowest nbands pairs);
 //  * Ritz vectors V C, W C and residuals r_b = W c_b - lambda_b V c_b with norms (serial.zig:201-227);
 //  * new directions: r_b / (diag - lambda_b) clamped at |den| >= 1e-8 (common.zig:214-226), then
 //    modified Gram-Schmidt against V with a drop when the remaining norm is < 1e-8
@@ -697,13 +696,12 @@ static int block_orthonormalize(dftcuda_kctx* c, int m, double2* Q, int k, doubl
   return DFTCUDA_OK;
 }
 
-// Subspace sizes from which the tridiagonal solver replaces the one-CTA Jacobi sweeps (whose cost
-// grows as m^3 on a single SM).  DFTCUDA_SUBSPACE_EIG=jacobi|tridiag forces either.
-constexpr int kTridiagMinM = 96;
+// The tridiagonal solver at every size; DFTCUDA_SUBSPACE_EIG=jacobi selects the one-CTA Jacobi sweeps (a
+// second method to check it against).
 
 static int small_eig(KCtxImpl* e, int m, int nev, cudaStream_t s) {
   const char* force = std::getenv("DFTCUDA_SUBSPACE_EIG");
-  const bool tri = force ? (std::strcmp(force, "tridiag") == 0) : (m >= kTridiagMinM);
+  const bool tri = !force || std::strcmp(force, "tridiag") == 0;
   if (tri) return heev_lowest(e->T, m, nev, e->evals, e->E, m, e->hw, e->status, s);
   const int m2 = m + (m & 1);
   const size_t smem = (sizeof(int2) + 2 * sizeof(double) + sizeof(double2)) * (size_t)(m2 / 2);
@@ -862,8 +860,8 @@ static int run_init(EigRun& r, const double* diag, const double* init_vecs, size
                                  is_device_pointer(init_vecs) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
   }
   DFT_TRY(orthonormalize_all(c, (int)m, r.seed, s));
-      cudaGetLastError();
   DFT_TRY(kctx_apply_h_dev(c, e->V, e->W, m, s));
+      cudaGetLastError();
   r.applies = m;
   r.m = m;
   return DFTCUDA_OK;
@@ -913,7 +911,7 @@ static int run_decide(EigRun& r) {
   if (*e->h_st == kBarrierTimeoutFlag)
     return fail(DFTCUDA_ERR_TIMEOUT, "eig_solve: a grid barrier of the subspace eigensolver timed out");
   if (*e->h_st != 0)
-    return fail(DFTCUDA_ERR_EIGENSOLVER_FAILURE, "eig_solve: subspace eigensolver failed (Jacobi not converged)");
+    return fail(DFTCUDA_ERR_EIGENSOLVER_FAILURE, "eig_solve: subspace eigensolver failed (a matrix that is not finite, or Jacobi not converged)");
   r.max_res = 0.0;
   for (size_t b = 0; b < r.nbands; ++b) r.max_res = std::max(r.max_res, e->h_nr[b]);
   if (r.max_res < r.opts.tol) {

@@ -5,9 +5,10 @@
 //   1. Householder reduction to real symmetric tridiagonal form Q^H A Q = T, reflectors chosen as
 //      in LAPACK's zlarfg so the off-diagonal of T is real.  One cooperative launch; the matrix
 //      stays in L2 (m = 2048: 64 MB) and each column costs one grid barrier (bounded waits): the
-//      rank-2 update of step k and the matrix-vector product of step k+1 share one sweep.
-//   2. The nev lowest eigenvalues of T by Sturm-count multisection: one warp per eigenvalue, its
-//      32 lanes evaluate the count at 32 interior points, so the bracket shrinks 33x per round.
+//      rank-2 update of step k and the matrix-vector product of step k+1 share one sweep.  Up to
+//      m = 95 one block does it with the matrix in shared memory.
+//   2. The nev lowest eigenvalues of T by Sturm-count multisection: one block per eigenvalue, one
+//      to eight warps whose threads each evaluate the count at an interior point.
 //   3. Eigenvectors of T by inverse iteration on a row-pivoted LU of T - lambda I (three sweeps
 //      from a hashed start vector), one warp per group of eigenvalues closer than 1e-5 ||T||: its
 //      vectors are computed in order, re-orthogonalised (modified Gram-Schmidt, all lanes) after
@@ -31,7 +32,7 @@ namespace {
 
 constexpr int HT_THREADS = 512;              // tridiagonalisation block
 constexpr int HT_WARPS = HT_THREADS / 32;
-constexpr int BS_WARPS = 8;                  // bisection: eigenvalues per block
+constexpr int BS_WARPS = 8;                  // bisection: most warps per eigenvalue
 constexpr int BT_WARPS = 4;                  // back-transformation: eigenvectors per block
 constexpr long kBarrierSpin = 1L << 24;      // polls (with 32 ns sleeps) before a barrier gives up
 constexpr double kGroupTol = 1e-5;           // eigenvalue grouping, relative to ||T||
@@ -397,6 +398,163 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd1(double2* __restrict__ A, 
   }
 }
 
+// Step 1 for m <= kHtSmallM in one block, the matrix in shared memory (m = 95: 144 KB): no grid barrier, so
+// that the small subspaces of many concurrent runs do not queue for co-resident grids.  The algebra of
+// k_hetrd1; warp 0 forms w, the next column and its reflector with warp reductions alone (at most
+// three entries per lane) between the two block barriers of a column, and all warps then update the
+// trailing columns and take their products with the new reflector.  Bound by the latency of those
+// reductions.  The cyclic Jacobi sweeps that used to serve these sizes took 2.9 ms at m = 40-88.
+// status: 1 when the tridiagonal form is not finite.
+constexpr int kHtSmallM = 95;
+
+__global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict__ A, int m, double* __restrict__ dd,
+                                                            double* __restrict__ ee, double2* __restrict__ tau, int* __restrict__ status) {
+  extern __shared__ double2 hsm[];
+  double2* const a = hsm;  // column-major, leading dimension m
+  __shared__ double2 sv[2][kHtSmallM + 1], sw[kHtSmallM + 1], sy[kHtSmallM + 1];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < m * m; i += HT_THREADS) a[i] = A[i];
+  __syncthreads();
+  constexpr int Q = (kHtSmallM + 31) / 32;
+  double2 t = make_double2(0.0, 0.0);  // warp 0: tau and beta of the current reflector
+  double beta = 0.0;
+  bool finite = true;
+  // warp 0: the reflector of x[0 .. n) (lane holds entries lane + 32 q), v to out; as block_reflector
+  auto reflector = [&](double2 (&x)[Q], int n, double2* out) {
+    double ss = 0.0;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int i = lane + 32 * q;
+      if (i > 0 && i < n) ss += x[q].x * x[q].x + x[q].y * x[q].y;
+    }
+    ss = warp_sum(ss);
+    const double2 alpha = make_double2(__shfl_sync(0xffffffffu, x[0].x, 0), __shfl_sync(0xffffffffu, x[0].y, 0));
+    t = make_double2(0.0, 0.0);
+    beta = alpha.x;
+    double2 sc = make_double2(0.0, 0.0);
+    if (!(ss == 0.0 && alpha.y == 0.0)) {
+      beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + ss), alpha.x);
+      const double2 den = make_double2(alpha.x - beta, alpha.y);
+      const double dn2 = den.x * den.x + den.y * den.y, ib = 1.0 / beta, id = 1.0 / dn2;
+      t = make_double2(-den.x * ib, -den.y * ib);
+      sc = make_double2(den.x * id, -den.y * id);
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int i = lane + 32 * q;
+      if (i < n) out[i] = i == 0 ? make_double2(1.0, 0.0) : cmul(x[q], sc);
+    }
+    finite = finite && isfinite(beta);
+  };
+  if (warp == 0) {
+    double2 x[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) x[q] = lane + 32 * q < m - 1 ? a[1 + lane + 32 * q] : make_double2(0.0, 0.0);
+    reflector(x, m - 1, sv[0]);
+    if (lane == 0) {
+      dd[0] = a[0].x;
+      ee[0] = beta;
+      tau[0] = t;
+    }
+    finite = finite && isfinite(a[0].x);
+  }
+  __syncthreads();
+  for (int r = 1 + warp; r < m; r += HT_WARPS) {  // products of step 0: conj(a) v
+    double sx = 0.0, sz = 0.0;
+    for (int i = lane; i < m - 1; i += 32) {
+      const double2 e = a[r * m + 1 + i], v = sv[0][i];
+      sx += e.x * v.x + e.y * v.y;
+      sz += e.x * v.y - e.y * v.x;
+    }
+    sx = warp_sum(sx);
+    sz = warp_sum(sz);
+    if (lane == 0) sy[r] = make_double2(sx, sz);
+  }
+  __syncthreads();
+  for (int k = 0; k + 1 < m; ++k) {
+    const int n1 = m - k - 1;
+    double2* const v = sv[k & 1];
+    double2* const vn = sv[(k + 1) & 1];
+    const bool next = k + 2 < m;
+    if (warp == 0) {
+      // y = tau A22 v, w = y + alpha v, alpha = -tau (y^H v) / 2; column k takes its reflector
+      double2 y[Q], x[Q];
+      double px = 0.0, pz = 0.0;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int i = lane + 32 * q;
+        y[q] = make_double2(0.0, 0.0);
+        if (i >= n1) continue;
+        y[q] = cmul(t, sy[k + 1 + i]);
+        px += y[q].x * v[i].x + y[q].y * v[i].y;
+        pz += y[q].x * v[i].y - y[q].y * v[i].x;
+      }
+      px = warp_sum(px);
+      pz = warp_sum(pz);
+      const double2 al = cscale(cmul(t, make_double2(px, pz)), -0.5);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int i = lane + 32 * q;
+        if (i >= n1) continue;
+        y[q] = cadd(y[q], cmul(al, v[i]));
+        sw[i] = y[q];
+        a[k * m + k + 1 + i] = i == 0 ? make_double2(beta, 0.0) : v[i];
+      }
+      const double2 w0c = make_double2(__shfl_sync(0xffffffffu, y[0].x, 0), -__shfl_sync(0xffffffffu, y[0].y, 0));
+      // column k + 1 after the update: its diagonal, and the entries below it shifted up by one
+      double2 c[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int i = lane + 32 * q;
+        c[q] = i < n1 ? csub(a[(k + 1) * m + k + 1 + i], cadd(cmul(v[i], w0c), y[q])) : make_double2(0.0, 0.0);
+      }
+      if (lane == 0) dd[k + 1] = c[0].x;
+      finite = finite && isfinite(__shfl_sync(0xffffffffu, c[0].x, 0));
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        x[q].x = __shfl_down_sync(0xffffffffu, c[q].x, 1);
+        x[q].y = __shfl_down_sync(0xffffffffu, c[q].y, 1);
+        const double nx = q + 1 < Q ? __shfl_sync(0xffffffffu, c[q + 1 < Q ? q + 1 : q].x, 0) : 0.0;
+        const double ny = q + 1 < Q ? __shfl_sync(0xffffffffu, c[q + 1 < Q ? q + 1 : q].y, 0) : 0.0;
+        if (lane == 31) x[q] = make_double2(nx, ny);
+      }
+      if (next) {
+        reflector(x, n1 - 1, vn);
+        if (lane == 0) {
+          ee[k + 1] = beta;
+          tau[k + 1] = t;
+        }
+      }
+    }
+    __syncthreads();
+    if (!next) break;
+    // rank-2 update of columns k + 2 .. (rows k + 2 ..) and their products with the new reflector (a warp's
+    // columns unrolled side by side measured 10-30 % slower)
+    for (int c = 1 + warp; c < n1; c += HT_WARPS) {
+      const double2 wr = cconj(sw[c]), vr = cconj(v[c]);
+      double2* col = a + (k + 1 + c) * m + k + 1;
+      double sx = 0.0, sz = 0.0;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int i = lane + 32 * q;
+        if (i < 1 || i >= n1) continue;
+        const double2 e = csub(col[i], cadd(cmul(v[i], wr), cmul(sw[i], vr)));
+        col[i] = e;
+        const double2 u = vn[i - 1];
+        sx += e.x * u.x + e.y * u.y;
+        sz += e.x * u.y - e.y * u.x;
+      }
+      sx = warp_sum(sx);
+      sz = warp_sum(sz);
+      if (lane == 0) sy[k + 1 + c] = make_double2(sx, sz);
+    }
+    __syncthreads();
+  }
+  // the reflectors, for the back-transformation
+  for (int i = tid; i < m * m; i += HT_THREADS) A[i] = a[i];
+  if (warp == 0 && lane == 0 && !finite) *status = 1;
+}
+
 // Number of eigenvalues of T below x (Sturm sequence of the LDL^T pivots).
 __device__ __forceinline__ int sturm_count(const double* d, const double* e2, int m, double x, double pivmin) {
   double q = d[0] - x;
@@ -419,7 +577,7 @@ __global__ void __launch_bounds__(BS_WARPS * 32) k_tridiag_bisect(const double* 
   double* d = bsm;
   double* e2 = bsm + m;
   __shared__ double red[3][BS_WARPS];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwarps = blockDim.x >> 5;
   double lo = DBL_MAX, hi = -DBL_MAX, emax = 0.0;
   for (int i = tid; i < m; i += blockDim.x) {
     const double di = dd[i];
@@ -445,7 +603,7 @@ __global__ void __launch_bounds__(BS_WARPS * 32) k_tridiag_bisect(const double* 
   lo = red[0][0];
   hi = red[1][0];
   emax = red[2][0];
-  for (int i = 1; i < BS_WARPS; ++i) {
+  for (int i = 1; i < nwarps; ++i) {
     lo = fmin(lo, red[0][i]);
     hi = fmax(hi, red[1][i]);
     emax = fmax(emax, red[2][i]);
@@ -456,29 +614,30 @@ __global__ void __launch_bounds__(BS_WARPS * 32) k_tridiag_bisect(const double* 
   const double fudge = 2.0 * DBL_EPSILON * tnorm + 4.0 * pivmin;
   lo -= fudge;
   hi += fudge;
-  const int j = blockIdx.x * BS_WARPS + wid;
-  if (j >= nev) return;
+  // One interior point per thread: with eight warps the bracket shrinks 257x a round, seven rounds where
+  // one warp's 33-section takes eleven.
+  const int PTS = blockDim.x;
+  __shared__ int first[2][BS_WARPS];
+  __shared__ double at[BS_WARPS * 32];
+  const int j = blockIdx.x;
   const double abstol = DBL_EPSILON * tnorm;
   for (int it = 0; it < 64; ++it) {
     const double width = hi - lo;
     if (width <= fmax(abstol, 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi))) + pivmin) break;
-    const double x = lo + width * (double)(lane + 1) / 33.0;
-    const int c = sturm_count(d, e2, m, x, pivmin);
-    const unsigned ball = __ballot_sync(0xffffffffu, c > j);
-    if (ball) {
-      const int f = __ffs(ball) - 1;
-      const double nhi = __shfl_sync(0xffffffffu, x, f);
-      const double nlo = f > 0 ? __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0) : lo;
-      if (nhi >= hi && nlo <= lo) break;  // no progress: bracket at rounding level
-      lo = nlo;
-      hi = nhi;
-    } else {
-      const double nlo = __shfl_sync(0xffffffffu, x, 31);
-      if (nlo <= lo) break;
-      lo = nlo;
-    }
+    const double x = lo + width * (double)(tid + 1) / (double)(PTS + 1);
+    at[tid] = x;
+    const unsigned ball = __ballot_sync(0xffffffffu, sturm_count(d, e2, m, x, pivmin) > j);
+    if (lane == 0) first[it & 1][wid] = ball ? wid * 32 + __ffs(ball) - 1 : PTS;
+    __syncthreads();
+    int f = PTS;
+    for (int i = 0; i < nwarps; ++i) f = min(f, first[it & 1][i]);
+    const double nlo = f > 0 ? at[f - 1] : lo, nhi = f < PTS ? at[f] : hi;
+    __syncthreads();  // at is written again by the next round
+    if (nhi >= hi && nlo <= lo) break;  // no progress: bracket at rounding level
+    lo = nlo;
+    hi = nhi;
   }
-  if (lane == 0) w[j] = 0.5 * (lo + hi);
+  if (tid == 0) w[j] = 0.5 * (lo + hi);
 }
 
 __device__ __forceinline__ double hashed_unit(uint64_t a, uint64_t b) {
@@ -664,26 +823,39 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(const double* __restrict__
   }
 }
 
-// Step 4.  E[:, j] = H_0 H_1 ... H_{m-2} Z[:, j] (applied right to left), one warp per column.
+// Step 4.  E[:, j] = H_0 H_1 ... H_{m-2} Z[:, j] (applied right to left), one warp per column.  SMALL
+// (m <= kHtSmallM): the block first copies the reflectors to shared memory, so that a step's time is not the
+// latency of its global loads (0.75 us a reflector).
+template <bool SMALL>
 __global__ void __launch_bounds__(BT_WARPS * 32) k_hetrd_back(const double2* __restrict__ A, const double2* __restrict__ tau,
                                                               int m, int nev, const double* __restrict__ Z,
                                                               double2* __restrict__ E, long lde) {
   extern __shared__ double2 esm[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int j = blockIdx.x * BT_WARPS + wid;
+  const double2* refl = A;
+  const double2* tk = tau;
+  if (SMALL) {
+    double2* s = esm + (size_t)BT_WARPS * m;
+    for (int i = threadIdx.x; i < m * m; i += blockDim.x) s[i] = A[i];
+    for (int i = threadIdx.x; i < m; i += blockDim.x) s[m * m + i] = tau[i];
+    __syncthreads();
+    refl = s;
+    tk = s + m * m;
+  }
   if (j >= nev) return;
   double2* ev = esm + (size_t)wid * m;
   const double* zj = Z + (size_t)j * m;
   for (int i = lane; i < m; i += 32) ev[i] = make_double2(zj[i], 0.0);
   __syncwarp();
   for (int k = m - 2; k >= 0; --k) {
-    const double2 t = tau[k];
+    const double2 t = tk[k];
     if (t.x == 0.0 && t.y == 0.0) continue;
     const int n1 = m - k - 1;
-    const double2* vk = A + (long)k * m + (k + 1);
+    const double2* vk = refl + (long)k * m + (k + 1);
     double sx = 0.0, sy = 0.0;
     for (int i = lane; i < n1; i += 32) {
-      const double2 v = i == 0 ? make_double2(1.0, 0.0) : __ldg(vk + i);
+      const double2 v = i == 0 ? make_double2(1.0, 0.0) : vk[i];
       const double2 x = ev[k + 1 + i];
       sx += v.x * x.x + v.y * x.y;  // conj(v) x
       sy += v.x * x.y - v.y * x.x;
@@ -692,7 +864,7 @@ __global__ void __launch_bounds__(BT_WARPS * 32) k_hetrd_back(const double2* __r
     sy = warp_sum(sy);
     const double2 ts = cmul(t, make_double2(sx, sy));
     for (int i = lane; i < n1; i += 32) {
-      const double2 v = i == 0 ? make_double2(1.0, 0.0) : __ldg(vk + i);
+      const double2 v = i == 0 ? make_double2(1.0, 0.0) : vk[i];
       ev[k + 1 + i] = csub(ev[k + 1 + i], cmul(ts, v));
     }
     __syncwarp();
@@ -913,7 +1085,7 @@ int heev_lowest(double2* A, int m, int nev, double* evals, double2* E, long lde,
   const int hetrd_bufs = two_barrier ? 2 : 3;  // shared-memory vectors of m entries
   const size_t smem_tr = sizeof(double2) * hetrd_bufs * 2048;
   DFT_TRY(ensure_max_dynamic_smem(hetrd_fn, (int)smem_tr));
-  DFT_TRY(ensure_max_dynamic_smem((const void*)k_hetrd_back, (int)(sizeof(double2) * BT_WARPS * 2048)));
+  DFT_TRY(ensure_max_dynamic_smem((const void*)k_hetrd_back<false>, (int)(sizeof(double2) * BT_WARPS * 2048)));
   DFT_TRY(ensure_max_dynamic_smem((const void*)k_wy_t_all, (int)kWyTSmem));
   DFT_TRY(ensure_max_dynamic_smem((const void*)k_tridiag_invit, (int)invit_smem(2048)));
   // SM count and the reduction kernel's occupancy, per device (several host threads may ask at once)
@@ -935,7 +1107,11 @@ int heev_lowest(double2* A, int m, int nev, double* evals, double2* E, long lde,
   if (per_sm < 1) return fail(DFTCUDA_ERR_UNSUPPORTED, "heev: tridiagonalisation kernel does not fit an SM");
   DFT_CUDA_TRY(cudaMemsetAsync(w.bar, 0, 2 * sizeof(unsigned), s));
   DFT_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
-  if (m > 1) {
+  if (m > 1 && m <= kHtSmallM && !two_barrier) {
+    DFT_TRY(ensure_max_dynamic_smem((const void*)k_hetrd_small, (int)(sizeof(double2) * kHtSmallM * kHtSmallM)));
+    k_hetrd_small<<<1, HT_THREADS, sizeof(double2) * m * m, s>>>(A, m, w.d, w.e, w.tau, status);
+    count_launch();
+  } else if (m > 1) {
     GridBarrier bar{w.bar, status, 0};
     const WaitLimits wl = wait_limits();
     if (wl.polls > 0) bar.spin = wl.polls;
@@ -962,14 +1138,23 @@ int heev_lowest(double2* A, int m, int nev, double* evals, double2* E, long lde,
     DFT_CUDA_TRY(cudaMemcpyAsync(w.d, A, sizeof(double), cudaMemcpyDeviceToDevice, s));
     DFT_CUDA_TRY(cudaMemsetAsync(w.tau, 0, sizeof(double2), s));
   }
-  k_tridiag_bisect<<<ceil_div(nev, BS_WARPS), BS_WARPS * 32, sizeof(double) * 2 * m, s>>>(w.d, w.e, m, nev, evals, w.tnorm);
+  // as many warps per eigenvalue as keep four to a scheduler, where the divisions' latency, not their
+  // rate, still sets the time
+  int bw = BS_WARPS;
+  while (bw > 1 && bw * nev > 4 * 4 * n_sm) bw /= 2;
+  k_tridiag_bisect<<<nev, bw * 32, sizeof(double) * 2 * m, s>>>(w.d, w.e, m, nev, evals, w.tnorm);
   count_launch();
   k_tridiag_invit<<<nev, 32, invit_smem(m), s>>>(w.d, w.e, m, nev, evals, w.tnorm, w.z);
   count_launch();
   if (m >= 192 && nev >= 32) {
     DFT_TRY(heev_back_blocked(A, w.tau, m, nev, w.z, E, lde, w, s));
+  } else if (m <= kHtSmallM) {
+    const size_t smem = sizeof(double2) * ((size_t)BT_WARPS * m + (size_t)m * m + m);
+    DFT_TRY(ensure_max_dynamic_smem((const void*)k_hetrd_back<true>, (int)(sizeof(double2) * (kHtSmallM + BT_WARPS + 1) * kHtSmallM)));
+    k_hetrd_back<true><<<ceil_div(nev, BT_WARPS), BT_WARPS * 32, smem, s>>>(A, w.tau, m, nev, w.z, E, lde);
+    count_launch();
   } else {
-    k_hetrd_back<<<ceil_div(nev, BT_WARPS), BT_WARPS * 32, sizeof(double2) * BT_WARPS * m, s>>>(A, w.tau, m, nev, w.z, E, lde);
+    k_hetrd_back<false><<<ceil_div(nev, BT_WARPS), BT_WARPS * 32, sizeof(double2) * BT_WARPS * m, s>>>(A, w.tau, m, nev, w.z, E, lde);
     count_launch();
   }
   DFT_CUDA_TRY(cudaGetLastError());
@@ -1027,6 +1212,6 @@ extern "C" int dftcuda_hermitian_eigen_decomp(size_t n, const double* a, size_t 
   DFT_CUDA_TRY(cudaMemcpyAsync(vectors, E, sizeof(double2) * n * nev,
                                is_device_pointer(vectors) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
   DFT_CUDA_TRY(cudaStreamSynchronize(s));
-  if (h_status != 0) return fail(DFTCUDA_ERR_TIMEOUT, "hermitian_eigen_decomp: grid barrier timed out");
+  if (h_status == kBarrierTimeoutFlag) return fail(DFTCUDA_ERR_TIMEOUT, "hermitian_eigen_decomp: grid barrier timed out");
   return DFTCUDA_OK;
 }
