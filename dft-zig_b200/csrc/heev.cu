@@ -6,7 +6,8 @@
 //      in LAPACK's zlarfg so the off-diagonal of T is real.  One cooperative launch; the matrix
 //      stays in L2 (m = 2048: 64 MB) and each column costs one grid barrier (bounded waits): the
 //      rank-2 update of step k and the matrix-vector product of step k+1 share one sweep.  Up to
-//      m = 95 one block does it with the matrix in shared memory.
+//      m = 95 one block does it with the matrix in shared memory, up to about 1200 the grid's blocks
+//      each keep their columns in shared memory.
 //   2. The nev lowest eigenvalues of T by Sturm-count multisection: one block per eigenvalue, one
 //      to eight warps whose threads each evaluate the count at an interior point.
 //   3. Eigenvectors of T by inverse iteration on a row-pivoted LU of T - lambda I (three sweeps
@@ -78,8 +79,7 @@ __device__ bool grid_sync(const GridBarrier& b, unsigned& epoch) {
       }
       __nanosleep(32);
     }
-    __threadfence();
-    s_ok = ok;
+    s_ok = ok;  // the acquiring load and the block barrier order what follows, read through L2
   }
   __syncthreads();
   return s_ok != 0;
@@ -398,12 +398,182 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd1(double2* __restrict__ A, 
   }
 }
 
+// The same reduction with the matrix resident in the grid's shared memory, each block holding every nb-th
+// column: a column's step then exchanges through L2 only the partial products and the next column, and the
+// grid barrier's fence has no trailing matrix to wait for.  Bound by the latency of that exchange and of the
+// two block reductions of a column.  Whole solves, us, matrix in L2 / resident: m = 136 749 / 684, 268 1505 /
+// 1410, 400 2485 / 2267, 536 3495 / 3138, 900 7453 / 5966.
+__global__ void __launch_bounds__(HT_THREADS) k_hetrd_res(double2* __restrict__ A, int m, double* __restrict__ dd,
+                                                       double* __restrict__ ee, double2* __restrict__ tau,
+                                                       double2* __restrict__ y, GridBarrier bar) {
+  extern __shared__ double2 hsm[];
+  double2* sv = hsm;          // v_k (n1 entries)
+  double2* sw = hsm + m;      // w_k
+  double2* sn = hsm + 2 * m;  // v_{k+1}
+  double2* const own = hsm + 3 * m;  // columns r = blockIdx.x + l gridDim.x at own + l m
+  __shared__ double2 red[HT_WARPS];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = tid >> 5, nb = gridDim.x;
+  unsigned epoch = 0;
+  // prologue: reflector 0 and the partial products of step 0
+  double2 t;
+  double beta;
+  {
+    const int n1 = m - 1;
+    for (int i = tid; i < n1; i += HT_THREADS) sv[i] = __ldcg(A + 1 + i);
+    __syncthreads();
+    block_reflector(sv, n1, red, t, beta);
+    if (blockIdx.x == 0 && tid == 0) {
+      dd[0] = __ldcg(A).x;
+      ee[0] = beta;
+      tau[0] = t;
+    }
+  }
+  for (int l = 0, r = blockIdx.x; r < m; ++l, r += nb)
+    for (int i = tid; i < m; i += HT_THREADS) own[(long)l * m + i] = __ldcg(A + (long)r * m + i);
+  __syncthreads();
+  // warps per column: the same for every block at a step, so that all know how many partials there are
+  auto split = [&](int ncols) { return max(1, min(kHtMaxSplit, HT_WARPS / ((ncols + nb - 1) / nb))); };
+  // first owned column >= r, as a local index
+  auto first = [&](int r) { return max(0, (r - (int)blockIdx.x + nb - 1) / nb); };
+  int S_prev;
+  {
+    const int n1 = m - 1;
+    const int S = split(max(n1, 1));
+    const int chunk = (n1 + S - 1) / S;
+    for (int g = warp;; g += HT_WARPS) {
+      const int l = first(1) + g / S, sidx = g % S, r = blockIdx.x + l * nb;
+      if (r >= m) break;
+      const int i0 = sidx * chunk, i1 = min(n1, i0 + chunk);
+      const double2* ac = own + (long)l * m + 1;
+      double sx = 0.0, sy = 0.0;
+#pragma unroll 4
+      for (int i = i0 + lane; i < i1; i += 32) {
+        const double2 a = ac[i], v = sv[i];
+        sx += a.x * v.x + a.y * v.y;  // conj(a) v
+        sy += a.x * v.y - a.y * v.x;
+      }
+      sx = warp_sum(sx);
+      sy = warp_sum(sy);
+      if (lane == 0) y[(long)sidx * m + r] = make_double2(sx, sy);
+    }
+    S_prev = S;
+  }
+  if (!grid_sync(bar, epoch)) return;
+  for (int k = 0; k + 1 < m; ++k) {
+    const int n1 = m - k - 1;
+    const double2* yk = y + (size_t)(k & 1) * kHtMaxSplit * m;      // step k's partials
+    double2* yn = y + (size_t)((k + 1) & 1) * kHtMaxSplit * m;      // step k+1's
+    // column k+1 as the previous sweep left it (rows k+1 ..), loaded with step k's partials
+    double2 colr[kHtColRegs];
+    {
+      const double2* col = A + (long)(k + 1) * m + (k + 1);
+#pragma unroll
+      for (int q = 0; q < kHtColRegs; ++q) {
+        const int i = tid + q * HT_THREADS;
+        colr[q] = i < n1 ? __ldcg(col + i) : make_double2(0.0, 0.0);
+      }
+    }
+    // (1) y = tau A22 v from the partial products; w = y + alpha v, alpha = -tau (y^H v) / 2
+    {
+      double2 p2 = make_double2(0.0, 0.0);
+      for (int i = tid; i < n1; i += HT_THREADS) {
+        double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 8
+        for (int q = 0; q < S_prev; ++q) acc = cadd(acc, __ldcg(yk + (long)q * m + k + 1 + i));
+        const double2 yi = cmul(t, acc), vi = sv[i];
+        sw[i] = yi;
+        p2.x += yi.x * vi.x + yi.y * vi.y;
+        p2.y += yi.x * vi.y - yi.y * vi.x;
+      }
+      const double2 sdot = block_sum2(p2, red);
+      const double2 al = cscale(cmul(t, sdot), -0.5);
+      for (int i = tid; i < n1; i += HT_THREADS) sw[i] = cadd(sw[i], cmul(al, sv[i]));
+      if (blockIdx.x == 0) {
+        // column k now holds its reflector (no block reads column k any more)
+        double2* cw = A + (long)k * m + (k + 1);
+        for (int i = tid; i < n1; i += HT_THREADS) cw[i] = i == 0 ? make_double2(beta, 0.0) : sv[i];
+      }
+      __syncthreads();
+    }
+    // (2) column k+1 after step k's update (rows k+1 .. m-1), its diagonal, and reflector k+1
+    const bool next = k + 2 < m;  // a reflector k+1 exists
+    double2 tn = make_double2(0.0, 0.0);
+    double betan = 0.0;
+    {
+      const double2 w0c = cconj(sw[0]);  // v_0 = 1
+#pragma unroll
+      for (int q = 0; q < kHtColRegs; ++q) {
+        const int i = tid + q * HT_THREADS;
+        if (i >= n1) break;
+        const double2 x = csub(colr[q], cadd(cmul(sv[i], w0c), sw[i]));
+        if (i == 0) {
+          if (blockIdx.x == 0) dd[k + 1] = x.x;
+        } else {
+          sn[i - 1] = x;
+        }
+      }
+      __syncthreads();
+      if (next) {
+        block_reflector(sn, n1 - 1, red, tn, betan);
+        if (blockIdx.x == 0 && tid == 0) {
+          ee[k + 1] = betan;
+          tau[k + 1] = tn;
+        }
+      }
+    }
+    if (!next) break;
+    // (3) rank-2 update of the owned columns >= k+2 (rows k+2 ..), in shared memory, and their partial
+    // products of step k+1; column k+2, which every block reads next, goes to global memory as well
+    {
+      const int S = split(n1 - 1);
+      const int chunk = (n1 + S - 1) / S;
+      for (int g = warp;; g += HT_WARPS) {
+        const int l = first(k + 2) + g / S, sidx = g % S, r = blockIdx.x + l * nb;
+        if (r >= m) break;
+        const int c = r - (k + 1);
+        const int i0 = sidx * chunk, i1 = min(n1, i0 + chunk);
+        const double2 wr = cconj(sw[c]), vr = cconj(sv[c]);
+        double2* ac = own + (long)l * m + (k + 1);
+        double2* pub = r == k + 2 ? A + (long)r * m + (k + 1) : nullptr;
+        double sx = 0.0, sy = 0.0;
+#pragma unroll 4
+        for (int i = i0 + lane; i < i1; i += 32) {
+          if (i == 0) continue;
+          double2 a = ac[i];
+          a = csub(a, cadd(cmul(sv[i], wr), cmul(sw[i], vr)));
+          ac[i] = a;
+          if (pub) pub[i] = a;
+          const double2 v = sn[i - 1];
+          sx += a.x * v.x + a.y * v.y;  // conj(a) v
+          sy += a.x * v.y - a.y * v.x;
+        }
+        sx = warp_sum(sx);
+        sy = warp_sum(sy);
+        if (lane == 0) yn[(long)sidx * m + r] = make_double2(sx, sy);
+      }
+      S_prev = S;
+    }
+    if (!grid_sync(bar, epoch)) return;
+    double2* tmp = sv;
+    sv = sn;
+    sn = tmp;
+    t = tn;
+    beta = betan;
+  }
+}
+
+// Shared memory of k_hetrd_res on nb blocks.
+constexpr size_t hetrd_res_smem(int m, int nb) { return sizeof(double2) * (size_t)m * (3 + (m + nb - 1) / nb); }
+constexpr size_t kHtResSmem = 226 * 1024;
+
 // Step 1 for m <= kHtSmallM in one block, the matrix in shared memory (m = 95: 144 KB): no grid barrier, so
 // that the small subspaces of many concurrent runs do not queue for co-resident grids.  The algebra of
 // k_hetrd1; warp 0 forms w, the next column and its reflector with warp reductions alone (at most
 // three entries per lane) between the two block barriers of a column, and all warps then update the
 // trailing columns and take their products with the new reflector.  Bound by the latency of those
-// reductions.  The cyclic Jacobi sweeps that used to serve these sizes took 2.9 ms at m = 40-88.
+// reductions (119 us on average over m = 20-88).  The cyclic Jacobi sweeps that used to serve these sizes took 2.9 ms at
+// m = 40-88.
 // status: 1 when the tridiagonal form is not finite.
 constexpr int kHtSmallM = 95;
 
@@ -1124,6 +1294,11 @@ int heev_lowest(double2* A, int m, int nev, double* evals, double2* E, long lde,
     }();
     const int want = (m * kHtMaxSplit + HT_WARPS - 1) / HT_WARPS;
     bar.nblocks = (unsigned)std::max(1, std::min(want, n_sm * std::min(per_sm, bps)));
+    // resident wherever the columns fit (m <= 1205 on 148 SMs; faster at every size below), on two columns per
+    // block or one block per SM
+    const int res_blocks = std::max(1, std::min(n_sm, (m + 1) / 2));
+    const bool resident = !two_barrier && hetrd_res_smem(m, res_blocks) <= kHtResSmem;
+    if (resident) bar.nblocks = (unsigned)res_blocks;
     double2* a_ = A;
     int m_ = m;
     double* d_ = w.d;
@@ -1131,8 +1306,14 @@ int heev_lowest(double2* A, int m, int nev, double* evals, double2* E, long lde,
     double2* t_ = w.tau;
     double2* y_ = w.y;
     void* args[] = {&a_, &m_, &d_, &e_, &t_, &y_, &bar};
-    DFT_CUDA_TRY(cudaLaunchCooperativeKernel(hetrd_fn, dim3(bar.nblocks), dim3(HT_THREADS), args,
-                                             sizeof(double2) * hetrd_bufs * m, s));
+    if (resident) {
+      DFT_TRY(ensure_max_dynamic_smem((const void*)k_hetrd_res, (int)kHtResSmem));
+      DFT_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_hetrd_res, dim3(bar.nblocks), dim3(HT_THREADS), args,
+                                               hetrd_res_smem(m, res_blocks), s));
+    } else {
+      DFT_CUDA_TRY(cudaLaunchCooperativeKernel(hetrd_fn, dim3(bar.nblocks), dim3(HT_THREADS), args,
+                                               sizeof(double2) * hetrd_bufs * m, s));
+    }
     count_launch();
   } else {
     DFT_CUDA_TRY(cudaMemcpyAsync(w.d, A, sizeof(double), cudaMemcpyDeviceToDevice, s));
