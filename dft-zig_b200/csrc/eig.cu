@@ -278,59 +278,80 @@ __global__ void k_precondition(double2* __restrict__ Q, const double2* __restric
   Q[idx] = make_double2(v.x * inv, v.y * inv);
 }
 
+// Rows [0, rows) of an upper triangle in shared memory (row r, column c at cps[r * nc + c]) factored in
+// order: s_inv[r] becomes 1 / pivot, or -1 where the row is dropped, and j0 + r of each kept row is appended
+// to kept[nk ..).  The rows stay unscaled (chol_entry gives R), so that a row costs one block barrier: the
+// updates scale what they read, one warp per row below, and the lane that updates the next diagonal also
+// takes its root.  Bound by the latency of a row's chain.  With a barrier each for the pivot, the scaled row and
+// the update (and the small triangle in L2) a 32-row panel of up to 132 columns took 33.7 us, now 21.8, and a
+// block of about 20 columns 16.6, now 10.0.
+__device__ __forceinline__ double chol_pivot(double d) { return d > 0.0 ? sqrt(d) : 0.0; }
+__device__ __forceinline__ double chol_pivot_inv(double d, double drop) {
+  const double piv = chol_pivot(d);
+  return !(piv >= drop) || piv == 0.0 ? -1.0 : 1.0 / piv;
+}
+__device__ __forceinline__ int chol_rows(double2* cps, int nc, int rows, double drop, int j0, double* s_inv,
+                                         int* __restrict__ kept, int nk) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (threadIdx.x == 0 && rows > 0) s_inv[0] = chol_pivot_inv(cps[0].x, drop);
+  __syncthreads();
+  for (int jl = 0; jl < rows; ++jl) {
+    const double2* rj = cps + (long)jl * nc;
+    const double inv = s_inv[jl];
+    const bool keep = inv >= 0.0;
+    if (keep) {
+      if (threadIdx.x == 0) kept[nk] = j0 + jl;
+      ++nk;
+    }
+    for (int rr = jl + 1 + warp; rr < rows; rr += nw) {
+      double2* t = cps + (long)rr * nc;
+      if (keep) {
+        const double2 x = make_double2(rj[rr].x * inv, rj[rr].y * inv);
+        for (int c = rr + lane; c < nc; c += 32) {
+          const double2 y = make_double2(rj[c].x * inv, rj[c].y * inv);
+          double2 v = t[c];
+          v.x -= x.x * y.x + x.y * y.y;
+          v.y -= x.x * y.y - x.y * y.x;
+          t[c] = v;
+        }
+      }
+      if (rr == jl + 1 && lane == 0) s_inv[rr] = chol_pivot_inv(t[rr].x, drop);
+    }
+    __syncthreads();
+  }
+  return nk;
+}
+// Entry (r, c) of R, c >= r, from the factored rows.
+__device__ __forceinline__ double2 chol_entry(const double2* cps, int nc, const double* s_inv, int r, int c) {
+  const double inv = s_inv[r];
+  const double2 v = cps[(long)r * nc + c];
+  if (inv < 0.0) return make_double2(0.0, 0.0);
+  return c == r ? make_double2(chol_pivot(v.x), 0.0) : make_double2(v.x * inv, v.y * inv);
+}
+
 // Cholesky of the k x k Gram matrix G (column-major) in column order with the MGS drop rule: column
 // j is dropped when its pivot sqrt(d) < drop, where d, the Schur-complement diagonal after the kept
 // columns before j, is exactly the squared norm MGS leaves (common.zig:263-284).  Right-looking: each
-// kept column scales its row and updates the whole trailing upper triangle in parallel; dropped
-// columns update nothing.  A: k x k row-major workspace (its kept rows end up as R); kept[0..kk),
-// *kk_out.  One CTA; the working triangle stays in L2.
-__global__ void __launch_bounds__(1024) k_chol_right(const double2* __restrict__ G, int k, double drop,
+// kept row updates the whole trailing upper triangle in parallel; dropped rows update nothing.  A: k x k
+// row-major, its kept rows end up as R; kept[0..kk), *kk_out.  One CTA; the triangle stays in shared
+// memory (k <= kChSmallK: 144 KB).
+constexpr int kChSmallK = 96, kChThreads = 512;
+__global__ void __launch_bounds__(kChThreads) k_chol_right(const double2* __restrict__ G, int k, double drop,
                                                      double2* __restrict__ A, int* __restrict__ kept, int* __restrict__ kk_out) {
-  __shared__ double s_piv;
-  __shared__ int s_nk;
+  extern __shared__ double2 cps[];  // [k][k]
+  __shared__ double s_inv[kChSmallK];
   const int tid = threadIdx.x, nt = blockDim.x;
-  for (long idx = tid; idx < (long)k * k; idx += nt) {
-    const int j = (int)(idx / k), l = (int)(idx - (long)j * k);
-    if (l >= j) A[idx] = G[j + (long)l * k];
+  for (int idx = tid; idx < k * k; idx += nt) {
+    const int l = idx / k, j = idx - l * k;
+    if (l >= j) cps[j * k + l] = G[idx];
   }
-  if (tid == 0) s_nk = 0;
   __syncthreads();
-  for (int j = 0; j < k; ++j) {
-    if (tid == 0) {
-      const double d = A[(long)j * k + j].x;
-      s_piv = d > 0.0 ? sqrt(d) : 0.0;
-    }
-    __syncthreads();
-    const double piv = s_piv;
-    if (!(piv >= drop) || piv == 0.0) {
-      __syncthreads();
-      continue;
-    }
-    const double inv = 1.0 / piv;
-    double2* rj = A + (long)j * k;
-    for (int l = j + 1 + tid; l < k; l += nt) rj[l] = make_double2(rj[l].x * inv, rj[l].y * inv);
-    if (tid == 0) {
-      rj[j] = make_double2(piv, 0.0);
-      kept[s_nk] = j;
-      s_nk = s_nk + 1;
-    }
-    __syncthreads();
-    // A[l1][l2] -= conj(R[j][l1]) R[j][l2] for j < l1 <= l2 < k
-    const int n = k - j - 1;
-    for (long idx = tid; idx < (long)n * n; idx += nt) {
-      const int a1 = (int)(idx / n), a2 = (int)(idx - (long)a1 * n);
-      if (a1 > a2) continue;
-      const int l1 = j + 1 + a1, l2 = j + 1 + a2;
-      const double2 x = rj[l1], y = rj[l2];
-      double2* t = A + (long)l1 * k + l2;
-      double2 v = *t;
-      v.x -= x.x * y.x + x.y * y.y;
-      v.y -= x.x * y.y - x.y * y.x;
-      *t = v;
-    }
-    __syncthreads();
+  const int nk = chol_rows(cps, k, k, drop, 0, s_inv, kept, 0);
+  for (int idx = tid; idx < k * k; idx += nt) {
+    const int r = idx / k, c = idx - r * k;
+    if (c >= r) A[idx] = chol_entry(cps, k, s_inv, r, c);
   }
-  if (tid == 0) *kk_out = s_nk;
+  if (tid == 0) *kk_out = nk;
 }
 
 // Blocked form of the same factorisation for larger blocks.  k_chol_init copies G's upper triangle
@@ -350,72 +371,33 @@ __global__ void k_chol_init(const double2* __restrict__ G, int k, double2* __res
   if (l >= j) A[idx] = G[j + (long)l * k];
 }
 
-__global__ void __launch_bounds__(1024) k_chol_panel(double2* __restrict__ A, int k, double drop, int* __restrict__ kept,
+__global__ void __launch_bounds__(kChThreads) k_chol_panel(double2* __restrict__ A, int k, double drop, int* __restrict__ kept,
                                                      int* __restrict__ kk, int j0, int j1) {
-  extern __shared__ double2 cps[];  // [j1 - j0][k - j0]: row j0 + r, column j0 + c at cps[r * nc + c]
-  __shared__ double s_piv;
-  __shared__ int s_nk;
-  const int tid = threadIdx.x, nt = blockDim.x;
+  extern __shared__ double2 cps[];  // [j1 - j0][k - j0]
+  __shared__ double s_inv[kChPanelMax];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const int nc = k - j0, rows = j1 - j0;
-  for (long idx = tid; idx < (long)rows * nc; idx += nt) {
-    const int r = (int)(idx / nc), c = (int)(idx - (long)r * nc);
-    cps[idx] = A[(long)(j0 + r) * k + j0 + c];
-  }
-  if (tid == 0) s_nk = *kk;
+  for (int r = warp; r < rows; r += nw)
+    for (int c = r + lane; c < nc; c += 32) cps[(long)r * nc + c] = A[(long)(j0 + r) * k + j0 + c];
+  const int nk0 = *kk;
   __syncthreads();
-  for (int jl = 0; jl < rows; ++jl) {  // row j = j0 + jl; its diagonal at column jl
-    double2* rj = cps + (long)jl * nc;
-    if (tid == 0) {
-      const double d = rj[jl].x;
-      s_piv = d > 0.0 ? sqrt(d) : 0.0;
-    }
-    __syncthreads();
-    const double piv = s_piv;
-    if (!(piv >= drop) || piv == 0.0) {
-      for (int c = jl + tid; c < nc; c += nt) rj[c] = make_double2(0.0, 0.0);
-      __syncthreads();
-      continue;
-    }
-    const double inv = 1.0 / piv;
-    for (int c = jl + 1 + tid; c < nc; c += nt) rj[c] = make_double2(rj[c].x * inv, rj[c].y * inv);
-    if (tid == 0) {
-      rj[jl] = make_double2(piv, 0.0);
-      kept[s_nk] = j0 + jl;
-      s_nk = s_nk + 1;
-    }
-    __syncthreads();
-    // the panel's rows after j: A[j'][l] -= conj(R[j][j']) R[j][l] for l >= j'
-    const int nr = rows - jl - 1, nu = nc - jl - 1;
-    for (long idx = tid; idx < (long)nr * nu; idx += nt) {
-      const int a = (int)(idx / nu), b = (int)(idx - (long)a * nu);
-      const int rr = jl + 1 + a, c = jl + 1 + b;
-      if (c < rr) continue;
-      const double2 x = rj[rr], y = rj[c];
-      double2* t = cps + (long)rr * nc + c;
-      double2 v = *t;
-      v.x -= x.x * y.x + x.y * y.y;
-      v.y -= x.x * y.y - x.y * y.x;
-      *t = v;
-    }
-    __syncthreads();
-  }
-  for (long idx = tid; idx < (long)rows * nc; idx += nt) {
-    const int r = (int)(idx / nc), c = (int)(idx - (long)r * nc);
-    A[(long)(j0 + r) * k + j0 + c] = cps[idx];
-  }
-  if (tid == 0) *kk = s_nk;
+  const int nk = chol_rows(cps, nc, rows, drop, j0, s_inv, kept, nk0);
+  for (int r = warp; r < rows; r += nw)
+    for (int c = r + lane; c < nc; c += 32) A[(long)(j0 + r) * k + j0 + c] = chol_entry(cps, nc, s_inv, r, c);
+  if (tid == 0) *kk = nk;
 }
 
 // Z (k x k columns, ld k): column b < kk solves R_kept z = e_b on the kept rows (rows of dropped
-// columns zero), so Q Z has orthonormal columns; columns b >= kk are zeroed.  One warp per column,
-// the back substitution's dot products split over the lanes; the column being solved and the kept
-// index table live in shared memory, so each of the (up to k - 1) dependent steps waits only on
-// shared-memory and L1 latency.
-constexpr int kCiWarps = 4;
+// columns zero), so Q Z has orthonormal columns; columns b >= kk are zeroed.  One warp per column.  The
+// substitution goes up in blocks of eight kept rows: eight lanes solve the block's triangle held in
+// their registers, then all lanes take the block out of the rows above, whose loads do not depend on one
+// another.  A dot product per row, each waiting for its own loads and a warp reduction, took 133 us at
+// k = 132, the blocks take 50.
+constexpr int kCiWarps = 4, kCiBlock = 8;
 __global__ void __launch_bounds__(kCiWarps * 32) k_chol_inv(const double2* __restrict__ A, int k, const int* __restrict__ kept,
                                                             const int* __restrict__ kk_p, double2* __restrict__ Z) {
   extern __shared__ __align__(16) unsigned char cism[];
-  double2* zs = reinterpret_cast<double2*>(cism);                // [kCiWarps][k]
+  double2* zs = reinterpret_cast<double2*>(cism);                // [kCiWarps][k]: entry u at the u-th kept row
   int* skept = reinterpret_cast<int*>(zs + (size_t)kCiWarps * k);  // [k]
   const int kk = *kk_p;
   for (int i = threadIdx.x; i < kk; i += blockDim.x) skept[i] = kept[i];
@@ -424,38 +406,45 @@ __global__ void __launch_bounds__(kCiWarps * 32) k_chol_inv(const double2* __res
   const int b = blockIdx.x * kCiWarps + w;
   if (b >= k) return;
   double2* z = zs + (size_t)w * k;
-  for (int i = lane; i < k; i += 32) z[i] = make_double2(0.0, 0.0);
-  __syncwarp();
-  if (b < kk) {
-    const int kb = skept[b];
-    if (lane == 0) z[kb] = make_double2(1.0 / A[(long)kb * k + kb].x, 0.0);
-    __syncwarp();
-    for (int a = b - 1; a >= 0; --a) {
-      const int ka = skept[a];
-      const double2* ra = A + (long)ka * k;
-      double sx = 0.0, sy = 0.0;
-      for (int u = a + 1 + lane; u <= b; u += 32) {
-        const int ku = skept[u];
-        const double2 r = __ldg(ra + ku), zz = z[ku];
-        sx += r.x * zz.x - r.y * zz.y;
-        sy += r.x * zz.y + r.y * zz.x;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        sx += __shfl_xor_sync(0xffffffffu, sx, o);
-        sy += __shfl_xor_sync(0xffffffffu, sy, o);
-      }
-      if (lane == 0) {
-        const double d = ra[ka].x;
-        z[ka] = make_double2(-sx / d, -sy / d);
-      }
-      __syncwarp();
-    }
-  }
   double2* zo = Z + (long)b * k;
-  for (int i = lane; i < k; i += 32) zo[i] = z[i];
+  for (int i = lane; i < k; i += 32) zo[i] = make_double2(0.0, 0.0);
+  if (b >= kk) return;
+  for (int i = lane; i <= b; i += 32) z[i] = make_double2(i == b ? 1.0 : 0.0, 0.0);  // right-hand side, then the solution
+  __syncwarp();
+  for (int a1 = b; a1 >= 0; a1 -= kCiBlock) {
+    const int a0 = max(0, a1 - kCiBlock + 1), nb = a1 - a0 + 1;
+    // lane i < nb: row a0 + i of the triangle, its right-hand side and the reciprocal of its diagonal
+    double2 r[kCiBlock], x = make_double2(0.0, 0.0);
+    double inv = 0.0;
+    const double2* ra = A + (long)skept[a0 + min(lane, nb - 1)] * k;
+#pragma unroll
+    for (int j = 0; j < kCiBlock; ++j) r[j] = j > lane && j < nb ? ra[skept[a0 + j]] : make_double2(0.0, 0.0);
+    if (lane < nb) {
+      inv = 1.0 / ra[skept[a0 + lane]].x;
+      x = z[a0 + lane];
+    }
+    double2 s[kCiBlock];  // the block's solution, in every lane
+#pragma unroll
+    for (int j = kCiBlock - 1; j >= 0; --j) {
+      const double sx = __shfl_sync(0xffffffffu, x.x * inv, j), sy = __shfl_sync(0xffffffffu, x.y * inv, j);
+      s[j] = j < nb ? make_double2(sx, sy) : make_double2(0.0, 0.0);
+      if (lane < j) x = csub(x, cmul(r[j], s[j]));
+    }
+#pragma unroll
+    for (int j = 0; j < kCiBlock; ++j)
+      if (lane == j && j < nb) z[a0 + j] = s[j];
+    for (int u = lane; u < a0; u += 32) {
+      const double2* ra = A + (long)skept[u] * k;
+      double2 y = z[u];
+#pragma unroll
+      for (int j = 0; j < kCiBlock; ++j)
+        if (j < nb) y = csub(y, cmul(ra[skept[a0 + j]], s[j]));
+      z[u] = y;
+    }
+    __syncwarp();
+  }
+  for (int i = lane; i <= b; i += 32) zo[skept[i]] = z[i];
 }
-
 
 // ------------------------------------------------------------------------------------------
 
@@ -611,8 +600,9 @@ static int combine(KCtxImpl* e, const double2* X, int mx, const double2* C, int 
 // Cholesky with the drop rule of the k x k Gram matrix G into e->R / e->kept, kept count at kk_dev,
 // then Z = the inverse on the kept rows.  One CTA below 97 columns, the panel form above.
 static int chol_drop(KCtxImpl* e, const double2* G, int k, double drop, int* kk_dev, cudaStream_t s) {
-  if (k <= 96) {
-    k_chol_right<<<1, 1024, 0, s>>>(G, k, drop, e->R, e->kept, kk_dev);
+  if (k <= kChSmallK) {
+    DFT_TRY(ensure_max_dynamic_smem((const void*)k_chol_right, (int)(sizeof(double2) * kChSmallK * kChSmallK)));
+    k_chol_right<<<1, kChThreads, sizeof(double2) * (size_t)k * k, s>>>(G, k, drop, e->R, e->kept, kk_dev);
     count_launch();
   } else {
     k_chol_init<<<ceil_div((size_t)k * k, 256), 256, 0, s>>>(G, k, e->R, kk_dev);
@@ -621,7 +611,7 @@ static int chol_drop(KCtxImpl* e, const double2* G, int k, double drop, int* kk_
     for (int j0 = 0; j0 < k;) {
       const int w = (int)std::max<size_t>(1, std::min<size_t>(kChPanelMax, kChPanelSmem / (sizeof(double2) * (size_t)(k - j0))));
       const int j1 = std::min(k, j0 + w);
-      k_chol_panel<<<1, 1024, sizeof(double2) * (size_t)(j1 - j0) * (k - j0), s>>>(e->R, k, drop, e->kept, kk_dev, j0, j1);
+      k_chol_panel<<<1, kChThreads, sizeof(double2) * (size_t)(j1 - j0) * (k - j0), s>>>(e->R, k, drop, e->kept, kk_dev, j0, j1);
       count_launch();
       if (j1 < k) {
         // A[l1][l2] -= sum_{j in panel} conj(R[j][l1]) R[j][l2], l1, l2 >= j1 (the lower triangle
@@ -827,6 +817,7 @@ static int run_init(EigRun& r, const double* diag, const double* init_vecs, size
     } else {
       e->vt_gram.release();
       e->vt_comb.release();
+      cudaGetLastError();
     }
   }
   e->tc_min_flops = c->tc_min_flops;
@@ -861,7 +852,6 @@ static int run_init(EigRun& r, const double* diag, const double* init_vecs, size
   }
   DFT_TRY(orthonormalize_all(c, (int)m, r.seed, s));
   DFT_TRY(kctx_apply_h_dev(c, e->V, e->W, m, s));
-      cudaGetLastError();
   r.applies = m;
   r.m = m;
   return DFTCUDA_OK;
