@@ -1006,7 +1006,9 @@ static double now_s() {
 // Host threads that issue the runs' kernels in each phase: many small runs (k-points, cells) spend
 // most of their time in the host's launch calls, and the runs are independent (each has its own
 // context, stream and workspace), so their issue spreads over threads.  DFTCUDA_ISSUE_THREADS
-// overrides the default (up to 8 threads, one per 8 runs; 1 = issue serially).
+// overrides the default (up to 8 threads, one per run; 1 = issue serially).  A run's phase takes the host
+// 30 to 60 us to issue, several times what a thread costs to start: eight k-points of an 8-atom cell take
+// 52.5 / 43.1 / 37.9 / 35.0 ms on 1 / 2 / 4 / 8 threads.
 static int issue_threads(size_t nruns) {
   static const int env = [] {
     const char* e = std::getenv("DFTCUDA_ISSUE_THREADS");
@@ -1014,7 +1016,7 @@ static int issue_threads(size_t nruns) {
   }();
   if (env > 0) return (int)std::min<size_t>(env, std::max<size_t>(nruns, 1));
   const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-  return (int)std::max<size_t>(1, std::min<size_t>({(size_t)8, (size_t)hw, nruns / 8}));
+  return (int)std::max<size_t>(1, std::min<size_t>({(size_t)8, (size_t)hw, nruns}));
 }
 
 // fn(run) for every run, on up to issue_threads() host threads (dynamic assignment).
