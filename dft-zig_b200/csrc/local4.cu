@@ -236,10 +236,18 @@ template <typename T, int NP> __host__ __device__ constexpr int plane_min_ctas()
   return sizeof(cplx<T>) * NP * NP <= 113 * 1024 ? 2 : 1;
 }
 
-template <int NP> __device__ __forceinline__ int dperm(int f) {
-  constexpr int N1 = Split<NP>::N1, N2 = Split<NP>::N2;
-  return (f % N1) * N2 + f / N1;
-}
+// A plane's row in shared memory: N1 groups of N2 entries, group stride RP.  Lanes step by a group in both
+// directions' second steps and over the stick columns, so that an even N2 (72 = 9 x 8: eight 16-byte lanes on the
+// same banks) takes a group stride of N2 + 1 where the plane then still fits its CTAs per SM.  72^3, 36 columns:
+// k_plane_fwd5 99 to 42 us (with its first step reading HBM itself), k_plane_inv5 60 to 43.
+template <typename T, int NP> struct PlaneRow {
+  static constexpr int N1 = Split<NP>::N1, N2 = Split<NP>::N2;
+  static constexpr size_t kRoom = plane_min_ctas<T, NP>() == 2 ? 112 * 1024 : 224 * 1024;
+  static constexpr int RP = sizeof(cplx<T>) * NP * N1 * (N2 | 1) <= kRoom ? N2 | 1 : N2;
+  static constexpr int RS = N1 * RP;  // row stride
+  static __device__ __forceinline__ int at(int y) { return y / N2 * RP + y % N2; }     // natural index y
+  static __device__ __forceinline__ int freq(int f) { return f % N1 * RP + f / N1; }  // frequency f after step B
+};
 
 template <typename T, int NP>
 __global__ void __launch_bounds__(kPlaneThreads, plane_min_ctas<T, NP>()) k_plane_inv5(const double2* __restrict__ x, long npw, cplx<T>* __restrict__ W,
@@ -247,10 +255,11 @@ __global__ void __launch_bounds__(kPlaneThreads, plane_min_ctas<T, NP>()) k_plan
                                                     const int* __restrict__ stick_off, const int* __restrict__ stick_y,
                                                     const cplx<T>* __restrict__ tw) {
   using C = cplx<T>;
-  constexpr int N1 = Split<NP>::N1, N2 = Split<NP>::N2, P = NP * NP;
+  using R = PlaneRow<T, NP>;
+  constexpr int N1 = R::N1, N2 = R::N2, RP = R::RP, RS = R::RS, P = NP * NP;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* S = reinterpret_cast<C*>(smraw);
-  int* sy = reinterpret_cast<int*>(S + P);
+  int* sy = reinterpret_cast<int*>(S + NP * RS);
   unsigned char* isst = reinterpret_cast<unsigned char*>(sy + NP);
   const int slot = blockIdx.x;
   const long b = blockIdx.y;
@@ -268,7 +277,7 @@ __global__ void __launch_bounds__(kPlaneThreads, plane_min_ctas<T, NP>()) k_plan
   const double2* xb = x + b * npw;
   // z transform, step A: thread (t, stick), rows k1 N2 + t of column y
   for (int w = tid; w < N2 * ns; w += nt) {
-    const int s = w % ns, t = w / ns, y = sy[s];
+    const int s = w % ns, t = w / ns, y = sy[s], col = R::at(y);
     C v[N1];
 #pragma unroll
     for (int j = 0; j < N1; ++j) {
@@ -285,18 +294,18 @@ __global__ void __launch_bounds__(kPlaneThreads, plane_min_ctas<T, NP>()) k_plan
     for (int k1 = 1; k1 < N1; ++k1)
       if (t) v[k1] = cmul(v[k1], tw_ld<T>(tw, (t * k1) % NP, (T)1));
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) S[(k1 * N2 + t) * NP + y] = v[k1];
+    for (int k1 = 0; k1 < N1; ++k1) S[(k1 * N2 + t) * RS + col] = v[k1];
   }
   __syncthreads();
   // z transform, step B in place: z frequency k1 + N1 k2 lands in row k1 N2 + k2
   for (int w = tid; w < N1 * ns; w += nt) {
-    const int s = w % ns, k1 = w / ns, y = sy[s];
+    const int s = w % ns, k1 = w / ns, col = R::at(sy[s]);
     C u[N2];
 #pragma unroll
-    for (int t = 0; t < N2; ++t) u[t] = S[(k1 * N2 + t) * NP + y];
+    for (int t = 0; t < N2; ++t) u[t] = S[(k1 * N2 + t) * RS + col];
     RegDft<T, N2>::run(u, (T)1);
 #pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) S[(k1 * N2 + k2) * NP + y] = u[k2];
+    for (int k2 = 0; k2 < N2; ++k2) S[(k1 * N2 + k2) * RS + col] = u[k2];
   }
   __syncthreads();
   // y transform, step A in place on every row r (a permuted z); columns without plane waves are zero
@@ -306,14 +315,14 @@ __global__ void __launch_bounds__(kPlaneThreads, plane_min_ctas<T, NP>()) k_plan
 #pragma unroll
     for (int j = 0; j < N1; ++j) {
       const int y = j * N2 + t;
-      v[j] = isst[y] ? S[r * NP + y] : mk<C>(0.0, 0.0);
+      v[j] = isst[y] ? S[r * RS + j * RP + t] : mk<C>(0.0, 0.0);
     }
     RegDft<T, N1>::run(v, (T)1);
 #pragma unroll
     for (int k1 = 1; k1 < N1; ++k1)
       if (t) v[k1] = cmul(v[k1], tw_ld<T>(tw, (t * k1) % NP, (T)1));
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) S[r * NP + k1 * N2 + t] = v[k1];
+    for (int k1 = 0; k1 < N1; ++k1) S[r * RS + k1 * RP + t] = v[k1];
   }
   __syncthreads();
   // y transform, step B: thread (k1, row); the plane to HBM in natural (z, y) order
@@ -323,7 +332,7 @@ __global__ void __launch_bounds__(kPlaneThreads, plane_min_ctas<T, NP>()) k_plan
     const int z = (r / N2) + N1 * (r % N2);
     C u[N2];
 #pragma unroll
-    for (int t = 0; t < N2; ++t) u[t] = S[r * NP + k1 * N2 + t];
+    for (int t = 0; t < N2; ++t) u[t] = S[r * RS + k1 * RP + t];
     RegDft<T, N2>::run(u, (T)1);
 #pragma unroll
     for (int k2 = 0; k2 < N2; ++k2) Wp[z * NP + k1 + N1 * k2] = u[k2];
@@ -337,30 +346,29 @@ __global__ void __launch_bounds__(kPlaneThreads, plane_min_ctas<T, NP>()) k_plan
                                                     double2* __restrict__ y_out, long npw,
                                                     const double* __restrict__ kinetic, double invN) {
   using C = cplx<T>;
-  constexpr int N1 = Split<NP>::N1, N2 = Split<NP>::N2, P = NP * NP;
+  using R = PlaneRow<T, NP>;
+  constexpr int N1 = R::N1, N2 = R::N2, RP = R::RP, RS = R::RS, P = NP * NP;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* S = reinterpret_cast<C*>(smraw);
-  int* sy = reinterpret_cast<int*>(S + P);
+  int* sy = reinterpret_cast<int*>(S + NP * RS);
   const int slot = blockIdx.x;
   const long b = blockIdx.y;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int s0 = stick_off[slot], ns = stick_off[slot + 1] - s0;
   const C* Wp = W + (b * n_act + slot) * (long)P;
-  for (int i = tid; i < P; i += nt) S[i] = Wp[i];
   for (int i = tid; i < ns; i += nt) sy[i] = stick_y[s0 + i];
-  __syncthreads();
-  // y transform, step A in place: thread (t, z)
+  // y transform, step A: thread (t, z), read from HBM
   for (int w = tid; w < N2 * NP; w += nt) {
     const int t = w % N2, z = w / N2;
     C v[N1];
 #pragma unroll
-    for (int j = 0; j < N1; ++j) v[j] = S[z * NP + j * N2 + t];
+    for (int j = 0; j < N1; ++j) v[j] = Wp[z * NP + j * N2 + t];
     RegDft<T, N1>::run(v, (T)-1);
 #pragma unroll
     for (int k1 = 1; k1 < N1; ++k1)
       if (t) v[k1] = cmul(v[k1], tw_ld<T>(tw, (t * k1) % NP, (T)-1));
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) S[z * NP + k1 * N2 + t] = v[k1];
+    for (int k1 = 0; k1 < N1; ++k1) S[z * RS + k1 * RP + t] = v[k1];
   }
   __syncthreads();
   // y transform, step B in place: y frequency k1 + N1 k2 lands in column k1 N2 + k2
@@ -368,33 +376,33 @@ __global__ void __launch_bounds__(kPlaneThreads, plane_min_ctas<T, NP>()) k_plan
     const int k1 = w % N1, z = w / N1;
     C u[N2];
 #pragma unroll
-    for (int t = 0; t < N2; ++t) u[t] = S[z * NP + k1 * N2 + t];
+    for (int t = 0; t < N2; ++t) u[t] = S[z * RS + k1 * RP + t];
     RegDft<T, N2>::run(u, (T)-1);
 #pragma unroll
-    for (int k2 = 0; k2 < N2; ++k2) S[z * NP + k1 * N2 + k2] = u[k2];
+    for (int k2 = 0; k2 < N2; ++k2) S[z * RS + k1 * RP + k2] = u[k2];
   }
   __syncthreads();
-  // z transform, step A in place on the stick columns (stick y sits at column dperm(y))
+  // z transform, step A in place on the stick columns (stick y sits at column freq(y))
   for (int w = tid; w < N2 * ns; w += nt) {
-    const int s = w % ns, t = w / ns, col = dperm<NP>(sy[s]);
+    const int s = w % ns, t = w / ns, col = R::freq(sy[s]);
     C v[N1];
 #pragma unroll
-    for (int j = 0; j < N1; ++j) v[j] = S[(j * N2 + t) * NP + col];
+    for (int j = 0; j < N1; ++j) v[j] = S[(j * N2 + t) * RS + col];
     RegDft<T, N1>::run(v, (T)-1);
 #pragma unroll
     for (int k1 = 1; k1 < N1; ++k1)
       if (t) v[k1] = cmul(v[k1], tw_ld<T>(tw, (t * k1) % NP, (T)-1));
 #pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) S[(k1 * N2 + t) * NP + col] = v[k1];
+    for (int k1 = 0; k1 < N1; ++k1) S[(k1 * N2 + t) * RS + col] = v[k1];
   }
   __syncthreads();
   // z transform, step B: thread (k1, stick); gather x 1/N plus kinetic into the output column
   const int* pm = pwmap + (long)slot * P;
   for (int w = tid; w < N1 * ns; w += nt) {
-    const int s = w % ns, k1 = w / ns, y = sy[s], col = dperm<NP>(y);
+    const int s = w % ns, k1 = w / ns, y = sy[s], col = R::freq(y);
     C u[N2];
 #pragma unroll
-    for (int t = 0; t < N2; ++t) u[t] = S[(k1 * N2 + t) * NP + col];
+    for (int t = 0; t < N2; ++t) u[t] = S[(k1 * N2 + t) * RS + col];
     RegDft<T, N2>::run(u, (T)-1);
 #pragma unroll
     for (int k2 = 0; k2 < N2; ++k2) {
@@ -496,7 +504,10 @@ constexpr int kXlWarps = 3;
 //   3. forward step B for frequency index t: DFT_N1, outputs x = t + N2 m back to the active slots.
 // The exchanges go through one per-warp shared buffer with __syncwarp only (no block barriers); a
 // lane's slots ({t + N2 m}, the same for input and output) stay in registers, the twiddles in shared
-// memory in the order the lanes read them.  V(r) is read through L1 (reused by the CTA's columns).
+// memory in the order the lanes read them.  V(r) is read through L1 (reused by the CTA's columns).  A row stays
+// in its lane from step B to step A, so one buffer serves both exchanges and one row at a time is in registers:
+// 75^3, 164 columns of H|psi>, 1,597 us against 1,736 with a second buffer and all rows held.  Five blocks per SM:
+// six take 75^3 to 1,567 but spill at 72 and cost the 8-atom cells' boxes as much.
 template <typename T, int NX>
 __global__ void __launch_bounds__(kXlWarps * 32, 5) k_xline5(cplx<T>* __restrict__ W, int n_act, const int* __restrict__ slot_of_x,
                                                              const T* __restrict__ Vt, int P, int ncols, int cols_per_cta,
@@ -628,7 +639,8 @@ static size_t plane_smem_bytes(size_t cs, int N, int buffers) {
 }
 template <typename T, int N>
 static size_t plane_smem(int buffers) {
-  return plane_smem_bytes(sizeof(cplx<T>), N, buffers);
+  const size_t pad = buffers == 1 ? sizeof(cplx<T>) * (size_t)N * (PlaneRow<T, N>::RS - N) : 0;
+  return plane_smem_bytes(sizeof(cplx<T>), N, buffers) + pad;
 }
 
 // DFTCUDA_FFT4=legacy selects the earlier two-buffer plane passes and the block-barrier x-line
