@@ -91,20 +91,46 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Sum over the block (HT_THREADS threads), returned to every thread.
-__device__ double2 block_sum2(double2 v, double2* red) {
-  v.x = warp_sum(v.x);
-  v.y = warp_sum(v.y);
+// Sums over the block (HT_THREADS threads), returned to every thread.  The callers pass a block barrier between
+// two uses of the same red.  In a warp one exchange leaves x to the lower and y to the upper lanes, so that
+// either sum is one chain of additions; the warps' sums are added by lanes again (16 additions in a row by
+// every thread took most of 1,080 cycles per sum).
+static_assert(HT_WARPS == 16, "the block sums add 16 warps by half a warp's lanes");
+__device__ __forceinline__ double half_sum(double v) {
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ double2 block_sum2(double2 v, double2* red) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double* const r = reinterpret_cast<double*>(red);
+  double keep = lane < 16 ? v.x : v.y;
+  keep += __shfl_xor_sync(0xffffffffu, lane < 16 ? v.y : v.x, 16);
+  keep = half_sum(keep);
+  if ((lane & 15) == 0) r[2 * w + (lane >> 4)] = keep;
   __syncthreads();
-  if (lane == 0) red[w] = v;
+  const double t = half_sum(r[2 * (lane & 15) + (lane >> 4)]);
+  return make_double2(__shfl_sync(0xffffffffu, t, 0), __shfl_sync(0xffffffffu, t, 16));
+}
+__device__ __forceinline__ double block_sum1(double v, double2* red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  v = warp_sum(v);
+  if (lane == 0) red[w].x = v;
   __syncthreads();
-  double2 t = make_double2(0.0, 0.0);
-  for (int i = 0; i < HT_WARPS; ++i) {
-    t.x += red[i].x;
-    t.y += red[i].y;
-  }
-  return t;
+  return half_sum(red[lane & 15].x);
+}
+
+// The reflector (zlarfg) of a column with first entry alpha and squared norm xnorm2 below it:
+// v = x sc with v_0 = 1, H = I - t v v^H, H^H x = beta e_1.
+__device__ __forceinline__ void reflector_scalars(double2 alpha, double xnorm2, double2& t, double& beta, double2& sc) {
+  t = sc = make_double2(0.0, 0.0);
+  beta = alpha.x;
+  if (xnorm2 == 0.0 && alpha.y == 0.0) return;
+  beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2), alpha.x);
+  const double2 den = make_double2(alpha.x - beta, alpha.y);  // v = x / (alpha - beta)
+  const double ib = 1.0 / beta, id = 1.0 / (den.x * den.x + den.y * den.y);
+  t = make_double2(-den.x * ib, -den.y * ib);
+  sc = make_double2(den.x * id, -den.y * id);
 }
 
 // Step 1.  A: m x m Hermitian, column-major, both triangles.  Column k of the result holds the
@@ -218,21 +244,11 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd(double2* __restrict__ A, i
 // block: x becomes v (v[0] = 1), returns tau and beta with H^H x = beta e_1, H = I - tau v v^H.
 __device__ void block_reflector(double2* x, int n, double2* red, double2& t, double& beta) {
   const int tid = threadIdx.x;
-  double2 part = make_double2(0.0, 0.0);
-  for (int i = tid + 1; i < n; i += HT_THREADS) part.x += x[i].x * x[i].x + x[i].y * x[i].y;
-  const double xnorm2 = block_sum2(part, red).x;
+  double part = 0.0;
+  for (int i = tid + 1; i < n; i += HT_THREADS) part += x[i].x * x[i].x + x[i].y * x[i].y;
   const double2 alpha = x[0];
-  t = make_double2(0.0, 0.0);
-  beta = alpha.x;
-  if (!(xnorm2 == 0.0 && alpha.y == 0.0)) {
-    beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2), alpha.x);
-    t = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
-  }
-  const bool active = !(t.x == 0.0 && t.y == 0.0);
-  const double2 den = make_double2(alpha.x - beta, alpha.y);  // v = x / (alpha - beta)
-  const double dn2 = den.x * den.x + den.y * den.y;
-  const double2 sc = active ? make_double2(den.x / dn2, -den.y / dn2) : make_double2(0.0, 0.0);
-  __syncthreads();
+  double2 sc;
+  reflector_scalars(alpha, block_sum1(part, red), t, beta, sc);
   for (int i = tid; i < n; i += HT_THREADS) x[i] = i == 0 ? make_double2(1.0, 0.0) : cmul(x[i], sc);
   __syncthreads();
 }
@@ -399,10 +415,13 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd1(double2* __restrict__ A, 
 }
 
 // The same reduction with the matrix resident in the grid's shared memory, each block holding every nb-th
-// column: a column's step then exchanges through L2 only the partial products and the next column, and the
+// column: a column's step then exchanges through L2 only the products and the next column, and the
 // grid barrier's fence has no trailing matrix to wait for.  Bound by the latency of that exchange and of the
-// two block reductions of a column.  Whole solves, us, matrix in L2 / resident: m = 136 749 / 684, 268 1505 /
-// 1410, 400 2485 / 2267, 536 3495 / 3138, 900 7453 / 5966.
+// two block reductions of a column (m = 400, cycles before the sums below: 2,700 of barrier, 1,700 and 1,100 of the
+// two sums, 1,800 of the reflector, 1,900 of the update).  The reduction, us, matrix in L2 / resident / with the
+// products summed before they are published, lane-wise block sums and a column's entries kept in registers:
+// m = 136 749 / 684 / 557, 268 1505 / 1410 / 1134, 400 2485 / 2267 / 1740, 536 3495 / 3138 / 2444, 900 7453 /
+// 5966 / 4659.
 __global__ void __launch_bounds__(HT_THREADS) k_hetrd_res(double2* __restrict__ A, int m, double* __restrict__ dd,
                                                        double* __restrict__ ee, double2* __restrict__ tau,
                                                        double2* __restrict__ y, GridBarrier bar) {
@@ -411,7 +430,7 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_res(double2* __restrict__ 
   double2* sw = hsm + m;      // w_k
   double2* sn = hsm + 2 * m;  // v_{k+1}
   double2* const own = hsm + 3 * m;  // columns r = blockIdx.x + l gridDim.x at own + l m
-  __shared__ double2 red[HT_WARPS];
+  __shared__ double2 red[2][HT_WARPS], part[HT_WARPS], s_y0, s_alpha;
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = tid >> 5, nb = gridDim.x;
   unsigned epoch = 0;
@@ -422,7 +441,7 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_res(double2* __restrict__ 
     const int n1 = m - 1;
     for (int i = tid; i < n1; i += HT_THREADS) sv[i] = __ldcg(A + 1 + i);
     __syncthreads();
-    block_reflector(sv, n1, red, t, beta);
+    block_reflector(sv, n1, red[0], t, beta);
     if (blockIdx.x == 0 && tid == 0) {
       dd[0] = __ldcg(A).x;
       ee[0] = beta;
@@ -432,11 +451,21 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_res(double2* __restrict__ 
   for (int l = 0, r = blockIdx.x; r < m; ++l, r += nb)
     for (int i = tid; i < m; i += HT_THREADS) own[(long)l * m + i] = __ldcg(A + (long)r * m + i);
   __syncthreads();
-  // warps per column: the same for every block at a step, so that all know how many partials there are
+  // warps per column: the same for every block at a step
   auto split = [&](int ncols) { return max(1, min(kHtMaxSplit, HT_WARPS / ((ncols + nb - 1) / nb))); };
   // first owned column >= r, as a local index
   auto first = [&](int r) { return max(0, (r - (int)blockIdx.x + nb - 1) / nb); };
-  int S_prev;
+  // the owned columns' products from those of their chunks; S > 1: at most HT_WARPS chunks in all
+  auto publish = [&](int S, int r0, double2* yo) {
+    if (S == 1) return;
+    __syncthreads();
+    const int r = blockIdx.x + (first(r0) + tid) * nb;
+    if (tid * S < HT_WARPS && r < m) {
+      double2 acc = part[tid * S];
+      for (int q = 1; q < S; ++q) acc = cadd(acc, part[tid * S + q]);
+      yo[r] = acc;
+    }
+  };
   {
     const int n1 = m - 1;
     const int S = split(max(n1, 1));
@@ -455,67 +484,89 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_res(double2* __restrict__ 
       }
       sx = warp_sum(sx);
       sy = warp_sum(sy);
-      if (lane == 0) y[(long)sidx * m + r] = make_double2(sx, sy);
+      if (lane == 0) (S == 1 ? y[r] : part[g]) = make_double2(sx, sy);
     }
-    S_prev = S;
+    publish(S, 1, y);
   }
   if (!grid_sync(bar, epoch)) return;
   for (int k = 0; k + 1 < m; ++k) {
     const int n1 = m - k - 1;
-    const double2* yk = y + (size_t)(k & 1) * kHtMaxSplit * m;      // step k's partials
-    double2* yn = y + (size_t)((k + 1) & 1) * kHtMaxSplit * m;      // step k+1's
-    // column k+1 as the previous sweep left it (rows k+1 ..), loaded with step k's partials
-    double2 colr[kHtColRegs];
+    const double2* yk = y + (size_t)(k & 1) * m;      // step k's products
+    double2* yn = y + (size_t)((k + 1) & 1) * m;      // step k+1's
+    // column k+1 as the previous sweep left it (rows k+1 ..) and step k's products, a thread's entries at
+    // tid + q HT_THREADS all through the step
+    double2 colr[kHtColRegs], yr[kHtColRegs];
     {
       const double2* col = A + (long)(k + 1) * m + (k + 1);
 #pragma unroll
       for (int q = 0; q < kHtColRegs; ++q) {
         const int i = tid + q * HT_THREADS;
+        yr[q] = i < n1 ? __ldcg(yk + k + 1 + i) : make_double2(0.0, 0.0);
         colr[q] = i < n1 ? __ldcg(col + i) : make_double2(0.0, 0.0);
       }
     }
-    // (1) y = tau A22 v from the partial products; w = y + alpha v, alpha = -tau (y^H v) / 2
+    // (1) y = tau A22 v; w = y + alpha v, alpha = -tau (y^H v) / 2
+    double2 w0;
     {
       double2 p2 = make_double2(0.0, 0.0);
-      for (int i = tid; i < n1; i += HT_THREADS) {
-        double2 acc = make_double2(0.0, 0.0);
-#pragma unroll 8
-        for (int q = 0; q < S_prev; ++q) acc = cadd(acc, __ldcg(yk + (long)q * m + k + 1 + i));
-        const double2 yi = cmul(t, acc), vi = sv[i];
-        sw[i] = yi;
+#pragma unroll
+      for (int q = 0; q < kHtColRegs; ++q) {
+        const int i = tid + q * HT_THREADS;
+        if (i >= n1) break;
+        const double2 yi = cmul(t, yr[q]), vi = sv[i];
+        yr[q] = yi;
         p2.x += yi.x * vi.x + yi.y * vi.y;
         p2.y += yi.x * vi.y - yi.y * vi.x;
       }
-      const double2 sdot = block_sum2(p2, red);
+      if (tid == 0) s_y0 = yr[0];
+      const double2 sdot = block_sum2(p2, red[0]);
       const double2 al = cscale(cmul(t, sdot), -0.5);
-      for (int i = tid; i < n1; i += HT_THREADS) sw[i] = cadd(sw[i], cmul(al, sv[i]));
+#pragma unroll
+      for (int q = 0; q < kHtColRegs; ++q) {
+        const int i = tid + q * HT_THREADS;
+        if (i >= n1) break;
+        yr[q] = cadd(yr[q], cmul(al, sv[i]));
+        sw[i] = yr[q];
+      }
+      w0 = cadd(s_y0, al);  // v_0 = 1
       if (blockIdx.x == 0) {
         // column k now holds its reflector (no block reads column k any more)
         double2* cw = A + (long)k * m + (k + 1);
         for (int i = tid; i < n1; i += HT_THREADS) cw[i] = i == 0 ? make_double2(beta, 0.0) : sv[i];
       }
-      __syncthreads();
     }
     // (2) column k+1 after step k's update (rows k+1 .. m-1), its diagonal, and reflector k+1
     const bool next = k + 2 < m;  // a reflector k+1 exists
     double2 tn = make_double2(0.0, 0.0);
     double betan = 0.0;
     {
-      const double2 w0c = cconj(sw[0]);  // v_0 = 1
+      const double2 w0c = cconj(w0);
+      double ss = 0.0;
 #pragma unroll
       for (int q = 0; q < kHtColRegs; ++q) {
         const int i = tid + q * HT_THREADS;
         if (i >= n1) break;
-        const double2 x = csub(colr[q], cadd(cmul(sv[i], w0c), sw[i]));
+        const double2 x = csub(colr[q], cadd(cmul(sv[i], w0c), yr[q]));
+        colr[q] = x;
         if (i == 0) {
           if (blockIdx.x == 0) dd[k + 1] = x.x;
+        } else if (i == 1) {
+          s_alpha = x;
         } else {
-          sn[i - 1] = x;
+          ss += x.x * x.x + x.y * x.y;
         }
       }
-      __syncthreads();
       if (next) {
-        block_reflector(sn, n1 - 1, red, tn, betan);
+        double2 sc;
+        const double xnorm2 = block_sum1(ss, red[1]);
+        reflector_scalars(s_alpha, xnorm2, tn, betan, sc);
+#pragma unroll
+        for (int q = 0; q < kHtColRegs; ++q) {
+          const int i = tid + q * HT_THREADS;
+          if (i >= n1) break;
+          if (i > 0) sn[i - 1] = i == 1 ? make_double2(1.0, 0.0) : cmul(colr[q], sc);
+        }
+        __syncthreads();
         if (blockIdx.x == 0 && tid == 0) {
           ee[k + 1] = betan;
           tau[k + 1] = tn;
@@ -550,9 +601,9 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_res(double2* __restrict__ 
         }
         sx = warp_sum(sx);
         sy = warp_sum(sy);
-        if (lane == 0) yn[(long)sidx * m + r] = make_double2(sx, sy);
+        if (lane == 0) (S == 1 ? yn[r] : part[g]) = make_double2(sx, sy);
       }
-      S_prev = S;
+      publish(S, k + 2, yn);
     }
     if (!grid_sync(bar, epoch)) return;
     double2* tmp = sv;
