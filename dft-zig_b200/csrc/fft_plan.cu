@@ -196,7 +196,9 @@ __global__ void k_fft_axis(double2* __restrict__ data, Fft1d p, int es, int ninn
 
 // The same pass for the lengths with a four-step split (fft_reg.cuh): a tile of 16 pencils crosses shared
 // memory once, between the two register sub-transforms, which read and write global memory themselves.
-// 75^3: 3.3 us a pass against 13 with the staged kernel above, whose x pass had 16 threads per block.
+// Bound by the latency of its two exchanges with global memory.  75^3: 10 us a pass from a cold cache against
+// 13 with the staged kernel above, whose x pass had 16 threads per block; the PBE potential build, 27 such
+// passes, 392 us against 495.
 // ROWS: the pencils are contiguous rows (the x axis), lanes run along them; else lanes run over
 // neighbouring pencils.  Pencil l of a tile starts at outer * os + inner0 + l (ROWS: (tile + l) * N).
 constexpr int kAxisLines = 16;

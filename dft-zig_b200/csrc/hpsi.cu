@@ -1223,7 +1223,7 @@ extern "C" int dftcuda_accumulate_density(dftcuda_kctx* c, const double* vectors
   const bool dv = is_device_pointer(vectors), dr = is_device_pointer(rho);
   // Aligned vectors on this device whose kept bands are consecutive (the occupied bands usually are) are
   // read where they are; otherwise the kept bands are packed into the staging buffer, one copy per run of consecutive
-  // bands (448 bands of 1 MB: the packing took 1.6 of 10.4 ms, one copy per band, a third of it the issue).
+  // bands (448 bands of 1 MB: packing them, one copy per band, took 1.8 of 10.4 ms).
   const double2* vecs = (const double2*)vectors + keep[0] * n;
   cudaPointerAttributes at{};
   const bool here = dv && ((uintptr_t)vectors & 15) == 0 && cudaPointerGetAttributes(&at, vectors) == cudaSuccess && at.device == c->device;

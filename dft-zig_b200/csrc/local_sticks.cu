@@ -226,8 +226,10 @@ __device__ __forceinline__ void plane_y_inverse(const cplx<T>* Srow, const int* 
 // Per (z plane, column): inverse y, then per y line inverse x, x V(r), forward x, then forward y.  The
 // plane's sticks are read by the first step and written by the last one; the x lines exchange through a
 // per-warp buffer in which a lane's rows stay its own from the inverse step B to the forward step A, so that
-// one row at a time is in registers and the lines can take the split that keeps the lanes busy (XSplit).  The four-step twiddles sit in shared memory in the order the lanes
-// read them.  Bound by shared memory / L1 wavefronts and the FP64 pipe, about equally.
+// one row at a time is in registers and the lines can take the split that keeps the lanes busy (XSplit).  The
+// four-step twiddles sit in shared memory in the order the lanes read them.  Bound by shared memory / L1
+// wavefronts (68 % busy) at 12 warps per SM.  108^3, 452 columns: 9.65 ms with the exchange out of place, all of
+// a lane's rows in registers and the sticks scattered and gathered in passes of their own; 7.2 ms now.
 template <typename T, int N>
 __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>* __restrict__ S, int n_st, const int* __restrict__ st_of,
                                                                      int n_act, const int* __restrict__ slot_of_x,
@@ -348,7 +350,8 @@ __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>
 }
 
 // The density pass holds all rows of its middle step while the parts of the exchange pass one after the other:
-// the split with fewer of them.
+// the split with fewer of them.  Bound by L1 wavefronts (70 % busy); 12 warps: 16 take 7.76 ms against 6.37 for
+// 448 columns at 108^3, whose registers then spill.
 template <int N> using DensityGeom = PlaneXGeom<N, Split<N>>;
 
 // Doubles reserved for the density kernel's N x N plane: rounded up to an even count, so the complex
@@ -482,9 +485,10 @@ static int plane_warps_rt(size_t cs, int n, int n_act) {
 }
 
 // Layout choice at context creation: DFTCUDA_LOCAL=planes or =sticks forces one; by default the
-// stick layout serves boxes from 96 points along x on (Si216, 108^3: 12.0 against 14.2 ms per
-// 452-column FP64 block) and the plane layout smaller ones (Si64, 75^3: the stick z-plane pass took
-// 18.1 against 11.3 ms per step).  The autotuner times both either way.
+// stick layout serves boxes from 96 points along x on (Si216, 108^3: measured before the passes of either took
+// their present form, 12.0 against 14.2 ms per 452-column FP64 block) and the plane layout smaller ones
+// (Si64, 75^3, 164 columns of H|psi>: 1,775 us on sticks, 1,781 on planes before and 1,570 after that layout's
+// x lines went in place).  The autotuner times both either way.
 static int local_layout_env() {
   const char* e = std::getenv("DFTCUDA_LOCAL");
   if (e && std::string(e) == "planes") return 1;

@@ -45,7 +45,8 @@ extern "C" {
  *  TF32    FFT passes in FP32 and the projector GEMMs on the tensor cores (tcgen05 kind::tf32, FP32
  *          accumulation in TMEM); relative error ~1e-3;
  *  TF32X3  as TF32 with every operand split into two TF32 parts (hi + lo, three MMAs per real
- *          product): FP32-class accuracy (~1e-6) on the tensor cores.
+ *          product): FP32-class accuracy (~1e-6) on the tensor cores.  Projector GEMMs that the
+ *          FP64 form serves in less time (its exact int8 products) take that form.
  * Wavefunctions are FP64 at the boundary in every mode.  In TF32 and TF32X3 contexts every
  * eigensolver subspace product (V^H W, V C, W C, the orthonormalisation's projections and block
  * overlaps) uses the same tensor-core GEMM (split form); the Cholesky factorisations, the subspace
@@ -454,9 +455,10 @@ int dftcuda_projector_phi(int l, size_t nq, double gmax, const double* table, si
  *   out(r, c) = alpha * sum_k opA(A(r, k)) * opB(B(c, k)) + beta * out(r, c),   r < M, c < N, k < K
  * A(r, k) is A[r*lda + k] when a_kc != 0 (K contiguous), else A[k*lda + r]; the same for B; opX
  * conjugates when conj_x != 0.  out(r, c) is out[r*ldo_r + c*ldo_c].  All pointers are device
- * pointers to interleaved complex128.  precision: DFTCUDA_PRECISION_FP64 (FP64 FMA kernel),
+ * pointers to interleaved complex128.  precision: DFTCUDA_PRECISION_FP64 (exact int8
+ * tensor-core products above a size, FP64 tensor cores below),
  * DFTCUDA_PRECISION_TF32 or DFTCUDA_PRECISION_TF32X3 (tcgen05 tensor-core kernels); FP32 is not
- * accepted.  The call allocates its split-K workspace, runs on a private stream and returns after
+ * accepted.  The call allocates its workspace, runs on a private stream and returns after
  * the product is complete.
  * ------------------------------------------------------------------------------------------ */
 int dftcuda_complex_gemm(int precision, size_t M, size_t N, size_t K, const double* a, long lda, int a_kc, int conj_a,
