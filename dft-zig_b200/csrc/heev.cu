@@ -623,8 +623,8 @@ constexpr size_t kHtResSmem = 226 * 1024;
 // k_hetrd1; warp 0 forms w, the next column and its reflector with warp reductions alone (at most
 // three entries per lane) between the two block barriers of a column, and all warps then update the
 // trailing columns and take their products with the new reflector.  Bound by the latency of those
-// reductions (119 us on average over m = 20-88).  The cyclic Jacobi sweeps that used to serve these sizes took 2.9 ms at
-// m = 40-88.
+// reductions and of the update's chains: 36, 83 and 225 us at m = 24, 48 and 88 (37, 95 and 260 with a warp per
+// column and guarded loads).  The cyclic Jacobi sweeps that used to serve these sizes took 2.9 ms at m = 40-88.
 // status: 1 when the tridiagonal form is not finite.
 constexpr int kHtSmallM = 95;
 
@@ -699,16 +699,16 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
     const bool next = k + 2 < m;
     if (warp == 0) {
       // y = tau A22 v, w = y + alpha v, alpha = -tau (y^H v) / 2; column k takes its reflector
-      double2 y[Q], x[Q];
+      double2 y[Q], x[Q], vq[Q];
       double px = 0.0, pz = 0.0;
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const int i = lane + 32 * q;
-        y[q] = make_double2(0.0, 0.0);
-        if (i >= n1) continue;
-        y[q] = cmul(t, sy[k + 1 + i]);
-        px += y[q].x * v[i].x + y[q].y * v[i].y;
-        pz += y[q].x * v[i].y - y[q].y * v[i].x;
+        const bool in = i < n1;
+        vq[q] = v[in ? i : 0];
+        y[q] = cmul(t, sy[k + 1 + (in ? i : 0)]);
+        px += in ? y[q].x * vq[q].x + y[q].y * vq[q].y : 0.0;
+        pz += in ? y[q].x * vq[q].y - y[q].y * vq[q].x : 0.0;
       }
       px = warp_sum(px);
       pz = warp_sum(pz);
@@ -716,10 +716,11 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const int i = lane + 32 * q;
-        if (i >= n1) continue;
-        y[q] = cadd(y[q], cmul(al, v[i]));
-        sw[i] = y[q];
-        a[k * m + k + 1 + i] = i == 0 ? make_double2(beta, 0.0) : v[i];
+        y[q] = cadd(y[q], cmul(al, vq[q]));
+        if (i < n1) {
+          sw[i] = y[q];
+          a[k * m + k + 1 + i] = i == 0 ? make_double2(beta, 0.0) : vq[q];
+        }
       }
       const double2 w0c = make_double2(__shfl_sync(0xffffffffu, y[0].x, 0), -__shfl_sync(0xffffffffu, y[0].y, 0));
       // column k + 1 after the update: its diagonal, and the entries below it shifted up by one
@@ -727,7 +728,8 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const int i = lane + 32 * q;
-        c[q] = i < n1 ? csub(a[(k + 1) * m + k + 1 + i], cadd(cmul(v[i], w0c), y[q])) : make_double2(0.0, 0.0);
+        const double2 e = csub(a[(k + 1) * m + k + 1 + (i < n1 ? i : 0)], cadd(cmul(vq[q], w0c), y[q]));
+        c[q] = i < n1 ? e : make_double2(0.0, 0.0);
       }
       if (lane == 0) dd[k + 1] = c[0].x;
       finite = finite && isfinite(__shfl_sync(0xffffffffu, c[0].x, 0));
@@ -749,25 +751,38 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
     }
     __syncthreads();
     if (!next) break;
-    // rank-2 update of columns k + 2 .. (rows k + 2 ..) and their products with the new reflector (a warp's
-    // columns unrolled side by side measured 10-30 % slower)
-    for (int c = 1 + warp; c < n1; c += HT_WARPS) {
+    // rank-2 update of columns k + 2 .. (rows k + 2 ..) and their products with the new reflector: eight lanes
+    // per column, 64 columns at a time, four entries per lane in flight.  Indexes are clamped instead of
+    // guarded, so that the loads and chains of the four overlap.
+    for (int cb = 1 + 4 * warp; cb < n1; cb += 4 * HT_WARPS) {
+      const int c = min(cb + (lane >> 3), n1 - 1);
+      const bool on = cb + (lane >> 3) < n1;
       const double2 wr = cconj(sw[c]), vr = cconj(v[c]);
       double2* col = a + (k + 1 + c) * m + k + 1;
       double sx = 0.0, sz = 0.0;
+      for (int i0 = lane & 7; i0 < n1; i0 += 32) {
+        double2 e[4], u[4];
 #pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        const int i = lane + 32 * q;
-        if (i < 1 || i >= n1) continue;
-        const double2 e = csub(col[i], cadd(cmul(v[i], wr), cmul(sw[i], vr)));
-        col[i] = e;
-        const double2 u = vn[i - 1];
-        sx += e.x * u.x + e.y * u.y;
-        sz += e.x * u.y - e.y * u.x;
+        for (int q = 0; q < 4; ++q) {
+          const int i = min(max(i0 + 8 * q, 1), n1 - 1);
+          e[q] = csub(col[i], cadd(cmul(v[i], wr), cmul(sw[i], vr)));
+          u[q] = vn[i - 1];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int i = i0 + 8 * q;
+          const bool in = on && i >= 1 && i < n1;
+          if (in) col[i] = e[q];
+          sx += in ? e[q].x * u[q].x + e[q].y * u[q].y : 0.0;
+          sz += in ? e[q].x * u[q].y - e[q].y * u[q].x : 0.0;
+        }
       }
-      sx = warp_sum(sx);
-      sz = warp_sum(sz);
-      if (lane == 0) sy[k + 1 + c] = make_double2(sx, sz);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        sx += __shfl_xor_sync(0xffffffffu, sx, o);
+        sz += __shfl_xor_sync(0xffffffffu, sz, o);
+      }
+      if (on && (lane & 7) == 0) sy[k + 1 + c] = make_double2(sx, sz);
     }
     __syncthreads();
   }
