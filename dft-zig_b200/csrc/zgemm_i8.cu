@@ -7,9 +7,10 @@
 // Each row of either operand is scaled by a power of two, so that its 2-norm is at most 2^58, and
 // rounded to (Gaussian) integers a' and b'.  By Cauchy-Schwarz |sum a' b'| <= 2^116 < P / 2 for the
 // product P = 2^117.7 of 16 pairwise coprime moduli below 256, so the integer result is determined by
-// its residues.  The only rounding is that of the entries, half a unit of 2^-58 times the row's norm: an
+// its residues.  The rounding is that of the entries, half a unit of 2^-58 times the row's norm: an
 // error of about 2^-59 |a||b| per output whatever K is, against 2^-55 |a||b| for a 64-bit accumulation of
-// the same products.
+// the same products where the rows' entries are of even size.  The reconstruction's coefficients are cut at
+// 76 bits and multiply numbers below 2 p of each modulus p: at most 2^-59 |a||b| more.
 //
 // Every prime factor of the moduli is 1 mod 4, so -1 has a square root w modulo each, and
 // x + iy -> (x + wy, x - wy) maps complex products modulo p onto two independent real ones: a complex
@@ -519,7 +520,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant
 }
 
 // ---- reconstruction -----------------------------------------------------------------------------
-// With s and d the sum and difference of the two planes' residues (summed over the splits),
+// With s and d the sum and difference of the two planes' residues (summed over the splits, then reduced),
 //   Re = P frac(sum_i s_i inv(2) inv_i / p_i),  Im = P frac(sum_i d_i inv(2 w_i) inv_i / p_i),
 // inv_i the inverse of P / p_i modulo p_i; the coefficients held to 76 bits, the fractions taken in
 // [-1/2, 1/2).
@@ -573,8 +574,8 @@ struct I8Sum {
     h[1] += im.hi * d;
     l[1] += im.lo * d;
   }
-  // less: what the moduli added to each split's differences put into the imaginary part (so that a sum of
-  // zeros is exactly zero)
+  // less: what the moduli added to the differences put into the imaginary part (so that a sum of zeros is exactly
+  // zero; nothing where the sums were reduced)
   __device__ __forceinline__ double2 value(int ea, int eb, double scale, I8Less less) const {
     double v[2];
 #pragma unroll
@@ -589,17 +590,22 @@ struct I8Sum {
 };
 
 // Moduli I, I + 1, ... of four neighbouring columns: w holds each plane's four residues, summed over the
-// splits, as 16-bit pairs (columns 0 and 2, then 1 and 3).
-template <int I, int I0, int I1>
+// splits, as 16-bit pairs (columns 0 and 2, then 1 and 3).  Sums over several splits are reduced again, so that what
+// the cut coefficients leave out does not grow with the splits.
+template <int I, int I0, int I1, bool ONE>
 __device__ __forceinline__ void i8_group(I8Sum (&x)[4], const uint2* w, unsigned splits) {
   if constexpr (I < I1) {
-    const unsigned p = (unsigned)std::integral_constant<int, kI8P[I]>::value * splits;
+    constexpr unsigned p = (unsigned)std::integral_constant<int, kI8P[I]>::value;
     const uint2 u = w[2 * (I - I0)], v = w[2 * (I - I0) + 1];
-    x[0].template add<I>((u.x & 0xffffu) + (v.x & 0xffffu), (u.x & 0xffffu) + p - (v.x & 0xffffu));
-    x[1].template add<I>((u.y & 0xffffu) + (v.y & 0xffffu), (u.y & 0xffffu) + p - (v.y & 0xffffu));
-    x[2].template add<I>((u.x >> 16) + (v.x >> 16), (u.x >> 16) + p - (v.x >> 16));
-    x[3].template add<I>((u.y >> 16) + (v.y >> 16), (u.y >> 16) + p - (v.y >> 16));
-    i8_group<I + 1, I0, I1>(x, w, splits);
+    auto take = [&](I8Sum& to, unsigned a, unsigned b) {
+      const unsigned s = a + b, d = a + (ONE ? p : p * splits) - b;
+      to.template add<I>(ONE ? s : s % p, ONE ? d : d % p);
+    };
+    take(x[0], u.x & 0xffffu, v.x & 0xffffu);
+    take(x[1], u.y & 0xffffu, v.y & 0xffffu);
+    take(x[2], u.x >> 16, v.x >> 16);
+    take(x[3], u.y >> 16, v.y >> 16);
+    i8_group<I + 1, I0, I1, ONE>(x, w, splits);
   }
 }
 // In groups of eight moduli: all of a group's loads of one split are in flight together.
@@ -621,7 +627,7 @@ __device__ __forceinline__ void i8_sums(I8Sum (&x)[4], const unsigned char* q, s
         w[i].y += (r[i] >> 8) & 0x00ff00ffu;
       }
     }
-    i8_group<I, I, I + G>(x, w, ONE ? 1u : (unsigned)splits);
+    i8_group<I, I, I + G, ONE>(x, w, ONE ? 1u : (unsigned)splits);
     i8_sums<I + G, ONE>(x, q + 2 * G * plane, plane, splits);
   }
 }
@@ -919,7 +925,7 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
       const bool tr = g.ldo_r < g.ldo_c;
       const dim3 grid = tr ? dim3(ceil_div(rn, 32), ceil_div(rm, 32)) : dim3(ceil_div(rn, 128), ceil_div(rm, 8));
       auto* kernel = tr ? (z == 1 ? k_i8_out<true, true> : k_i8_out<true, false>) : (z == 1 ? k_i8_out<false, true> : k_i8_out<false, false>);
-      kernel<<<grid, 256, 0, s>>>(base + o_res, rm, rn, a.Npad, z, oa.ex + m0, ob.ex + n0, o, g.ldo_r, g.ldo_c, g.alpha, g.beta, i8_scale(), I8Less{kI8Less.hi * (unsigned long long)z, kI8Less.lo * z});
+      kernel<<<grid, 256, 0, s>>>(base + o_res, rm, rn, a.Npad, z, oa.ex + m0, ob.ex + n0, o, g.ldo_r, g.ldo_c, g.alpha, g.beta, i8_scale(), z == 1 ? kI8Less : I8Less{0, 0});
       count_launch();
     }
   }

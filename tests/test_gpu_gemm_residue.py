@@ -114,3 +114,15 @@ def test_not_less_exact_than_the_dmma_kernel(dz):
         plain = dz.complex_gemm(torch.from_numpy(a[:, :]).cuda(), torch.from_numpy(b[:8]).cuda()).cpu().numpy()  # 8 columns: the DMMA kernel
         err, err0 = (np.linalg.norm((x - want).astype(complex)) for x in (out, plain))
         assert err <= 1.05 * err0, (err, err0)
+
+
+def test_many_k_splits(dz):
+    """A product cut into 36 K splits, rows just above a power of two in norm (where the reconstruction's cut is largest
+    against |a||b|).  Its coefficients lose less than 2^-76 each and multiply residues below p of 16 moduli of sum 2736:
+    2^(11.5 - 76) P in either part, 2^-60.3 |a||b| for norms of at least 2^57 each, plus the roundings of the result."""
+    gen = torch.Generator().manual_seed(14)
+    a, b = (torch.view_as_complex(torch.randint(-728, 729, (160, 200000, 2), generator=gen).double()).cuda() for _ in range(2))
+    ref = a @ b.T
+    out = dz.complex_gemm(a, b)
+    na, nb = torch.linalg.vector_norm(a, dim=1), torch.linalg.vector_norm(b, dim=1)
+    assert bool(((out - ref).abs() <= 2.0 ** -60 * na[:, None] * nb[None, :] + 2.0 ** -51 * ref.abs()).all())
