@@ -38,15 +38,17 @@ struct GemmArgs {
   TcScratch* i8 = nullptr;
   int* err = nullptr;
   double a_share = 1.0, b_share = 1.0;  // the part of an operand's conversion this product pays for
+  bool guard = false;  // operands of any kind: rows of uneven size keep 64-bit sums (zgemm_i8.cu)
 };
 int zgemm(const GemmArgs& g, cudaStream_t s, double2* workspace, size_t workspace_elems);
 size_t zgemm_workspace_elems(int M, int N, int K);
 // The FP64 product by residues on the int8 tensor cores (zgemm_i8.cu).  *done = false, with status OK, when
-// its buffers could not be allocated: nothing was launched on the output.
+// its buffers could not be allocated: nothing was launched on the output.  *uneven (guarded products, else null): a
+// device flag, not zero where the product was left to the other kernel.
 bool zgemm_i8_worthwhile(int M, int N, int K, double share_m = 1.0, double share_n = 1.0);
 bool zgemm_i8_beats_split_tf32(int M, int N, int K, double share_m, double share_n);
 size_t zgemm_i8_cache_bytes(int R, int K);  // one operand's kept tiles (a_cache, b_cache)
-int zgemm_i8(const GemmArgs& g, cudaStream_t s, TcScratch* scratch, int* err, bool* done);
+int zgemm_i8(const GemmArgs& g, cudaStream_t s, TcScratch* scratch, int* err, bool* done, const int** uneven);
 // The same contraction on the tensor cores (tc_gemm.cu): TF32 inputs, FP32 accumulation.  err_dev
 // receives 1 if a bounded wait gave up.
 // split = true: 3xTF32 (hi + lo operand parts), FP32-class accuracy.  scratch (may be null): where the

@@ -249,6 +249,7 @@ extern "C" int dftcuda_complex_gemm(int precision, size_t M, size_t N, size_t K,
   en->tiles.valid = false;  // operands differ from call to call
   g.i8 = &en->tiles;
   g.err = en->err;
+  g.guard = true;
   int rc = tc ? cgemm_tf32(g, en->s, en->ws, en->ws_cap, en->err, precision == DFTCUDA_PRECISION_TF32X3, &en->tiles)
               : zgemm(g, en->s, en->ws, en->ws_cap);
   int herr = 0;

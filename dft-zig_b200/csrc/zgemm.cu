@@ -325,7 +325,8 @@ template <bool AKC, bool BKC, bool CJA, bool CJB, int ST>
 __global__ void __launch_bounds__(256, ST == 2 ? 2 : 1) k_zgemm_dmma3m(int M, int N, int K, const double2* __restrict__ A, long lda,
                                                          const double2* __restrict__ B, long ldb, double2* __restrict__ O,
                                                          long ldo_r, long ldo_c, double alpha, double beta, int kps,
-                                                         double2* __restrict__ part) {
+                                                         double2* __restrict__ part, const int* __restrict__ gate) {
+  if (gate && !*gate) return;
   extern __shared__ __align__(16) unsigned char zsm[];
   double2(*As)[BK][BM + kZmPad] = reinterpret_cast<double2(*)[BK][BM + kZmPad]>(zsm);
   double2(*Bs)[BK][BN + kZmPad] = reinterpret_cast<double2(*)[BK][BN + kZmPad]>(zsm + ST * sizeof(double2) * BK * (BM + kZmPad));
@@ -423,9 +424,9 @@ __global__ void __launch_bounds__(256, ST == 2 ? 2 : 1) k_zgemm_dmma3m(int M, in
 }
 
 __global__ void k_zgemm_reduce(int M, int N, int splits, const double2* __restrict__ part, double2* __restrict__ O,
-                               long ldo_r, long ldo_c, double alpha, double beta) {
+                               long ldo_r, long ldo_c, double alpha, double beta, const int* __restrict__ gate) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= (long)M * N) return;
+  if (i >= (long)M * N || (gate && !*gate)) return;
   const int r = (int)(i / N), c = (int)(i - (long)r * N);
   double2 s = make_double2(0.0, 0.0);
   for (int z = 0; z < splits; ++z) {
@@ -482,14 +483,14 @@ static int zgemm_kind() {
 }
 
 template <bool AKC, bool BKC, bool CJA, bool CJB>
-static void launch(const GemmArgs& g, dim3 grid, int kps, double2* part, cudaStream_t s) {
+static void launch(const GemmArgs& g, dim3 grid, int kps, double2* part, const int* gate, cudaStream_t s) {
   if (zgemm_kind() == 3) {
     const bool few = (long)grid.x * grid.y * grid.z <= 148;
     const size_t smem = few ? 2 * kZgemmDmmaSmem : kZgemmDmmaSmem;
     auto* kernel = few ? k_zgemm_dmma3m<AKC, BKC, CJA, CJB, 4> : k_zgemm_dmma3m<AKC, BKC, CJA, CJB, 2>;
     ensure_max_dynamic_smem((const void*)kernel, (int)smem);
     kernel<<<grid, 256, smem, s>>>(g.M, g.N, g.K, g.A, g.lda, g.B, g.ldb, g.O, g.ldo_r,
-                                                                        g.ldo_c, g.alpha, g.beta, kps, part);
+                                                                        g.ldo_c, g.alpha, g.beta, kps, part, gate);
     count_launch();
     return;
   }
@@ -512,16 +513,26 @@ static void launch(const GemmArgs& g, dim3 grid, int kps, double2* part, cudaStr
                                                    g.beta, kps, part); count_launch();
 }
 
-int zgemm(const GemmArgs& g, cudaStream_t s, double2* ws, size_t ws_elems) {
+int zgemm(const GemmArgs& g0, cudaStream_t s, double2* ws, size_t ws_elems) {
+  GemmArgs g = g0;
   if (g.M <= 0 || g.N <= 0) return DFTCUDA_OK;
   if (g.K <= 0) {
     // out = beta * out
     return fail(DFTCUDA_ERR_INVALID_ARGUMENT, "zgemm: K must be positive");
   }
+  const int* gate = nullptr;
   if (g.i8 && g.err && zgemm_i8_worthwhile(g.M, g.N, g.K, g.a_share, g.b_share)) {
     bool done = false;
-    DFT_TRY(zgemm_i8(g, s, g.i8, g.err, &done));
-    if (done) return DFTCUDA_OK;
+    DFT_TRY(zgemm_i8(g, s, g.i8, g.err, &done, &gate));
+    if (done && !gate) return DFTCUDA_OK;
+  }
+  if (ceil_div(g.M, BM) > 65535 && g.N < g.M) {  // the grid's y is the shorter side
+    std::swap(g.M, g.N);
+    std::swap(g.A, g.B);
+    std::swap(g.lda, g.ldb);
+    std::swap(g.a_kc, g.b_kc);
+    std::swap(g.conj_a, g.conj_b);
+    std::swap(g.ldo_r, g.ldo_c);
   }
   int splits = g.splits > 0 ? std::min(g.splits, std::max(1, g.K / 32)) : pick_splits(g.M, g.N, g.K);
   if (splits > 1) splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ws_elems / ((size_t)g.M * g.N)));  // what fits the workspace
@@ -532,26 +543,26 @@ int zgemm(const GemmArgs& g, cudaStream_t s, double2* ws, size_t ws_elems) {
   double2* part = splits > 1 ? ws : nullptr;
   const int key = (g.a_kc ? 8 : 0) | (g.b_kc ? 4 : 0) | (g.conj_a ? 2 : 0) | (g.conj_b ? 1 : 0);
   switch (key) {
-    case 0: launch<false, false, false, false>(g, grid, kps, part, s); break;
-    case 1: launch<false, false, false, true>(g, grid, kps, part, s); break;
-    case 2: launch<false, false, true, false>(g, grid, kps, part, s); break;
-    case 3: launch<false, false, true, true>(g, grid, kps, part, s); break;
-    case 4: launch<false, true, false, false>(g, grid, kps, part, s); break;
-    case 5: launch<false, true, false, true>(g, grid, kps, part, s); break;
-    case 6: launch<false, true, true, false>(g, grid, kps, part, s); break;
-    case 7: launch<false, true, true, true>(g, grid, kps, part, s); break;
-    case 8: launch<true, false, false, false>(g, grid, kps, part, s); break;
-    case 9: launch<true, false, false, true>(g, grid, kps, part, s); break;
-    case 10: launch<true, false, true, false>(g, grid, kps, part, s); break;
-    case 11: launch<true, false, true, true>(g, grid, kps, part, s); break;
-    case 12: launch<true, true, false, false>(g, grid, kps, part, s); break;
-    case 13: launch<true, true, false, true>(g, grid, kps, part, s); break;
-    case 14: launch<true, true, true, false>(g, grid, kps, part, s); break;
-    default: launch<true, true, true, true>(g, grid, kps, part, s); break;
+    case 0: launch<false, false, false, false>(g, grid, kps, part, gate, s); break;
+    case 1: launch<false, false, false, true>(g, grid, kps, part, gate, s); break;
+    case 2: launch<false, false, true, false>(g, grid, kps, part, gate, s); break;
+    case 3: launch<false, false, true, true>(g, grid, kps, part, gate, s); break;
+    case 4: launch<false, true, false, false>(g, grid, kps, part, gate, s); break;
+    case 5: launch<false, true, false, true>(g, grid, kps, part, gate, s); break;
+    case 6: launch<false, true, true, false>(g, grid, kps, part, gate, s); break;
+    case 7: launch<false, true, true, true>(g, grid, kps, part, gate, s); break;
+    case 8: launch<true, false, false, false>(g, grid, kps, part, gate, s); break;
+    case 9: launch<true, false, false, true>(g, grid, kps, part, gate, s); break;
+    case 10: launch<true, false, true, false>(g, grid, kps, part, gate, s); break;
+    case 11: launch<true, false, true, true>(g, grid, kps, part, gate, s); break;
+    case 12: launch<true, true, false, false>(g, grid, kps, part, gate, s); break;
+    case 13: launch<true, true, false, true>(g, grid, kps, part, gate, s); break;
+    case 14: launch<true, true, true, false>(g, grid, kps, part, gate, s); break;
+    default: launch<true, true, true, true>(g, grid, kps, part, gate, s); break;
   }
   if (part) {
     const long tot = (long)g.M * g.N;
-    k_zgemm_reduce<<<ceil_div(tot, 256), 256, 0, s>>>(g.M, g.N, splits, part, g.O, g.ldo_r, g.ldo_c, g.alpha, g.beta); count_launch();
+    k_zgemm_reduce<<<ceil_div(tot, 256), 256, 0, s>>>(g.M, g.N, splits, part, g.O, g.ldo_r, g.ldo_c, g.alpha, g.beta, gate); count_launch();
   }
   DFT_CUDA_TRY(cudaGetLastError());
   return DFTCUDA_OK;

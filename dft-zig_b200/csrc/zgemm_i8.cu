@@ -23,8 +23,16 @@
 //   k_i8_gemm               the residue products, 32 real GEMMs in one persistent launch;
 //   k_i8_out                the sum from its residues (Chinese remainder theorem), scaled.
 //
-// A row that holds an infinity or a NaN gives NaN in its whole output row (or column), and in no other.
+// That error is relative to the rows' norms.  Where entries of very different size meet (a large entry of one row
+// beside zeros or small ones of the other), sum |a_k||b_k| is far below |a||b| and 64-bit sums are closer.  A caller
+// whose operands can be anything sets GemmArgs::guard: the norm pass then also checks on the device that every
+// row's entries are of even size (k_i8_scale), and where one is not, or holds an infinity or a NaN, the
+// kernels here return at once and the FP64 tensor-core kernel, launched behind them, takes the product; else that one
+// returns at once.
+// Without the guard a row that holds an infinity or a NaN gives NaN in its whole output row (or column), and in no
+// other.
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <cmath>
 #include <cstdlib>
@@ -106,8 +114,93 @@ __global__ void __launch_bounds__(256) k_i8_norm(const double2* __restrict__ X, 
   }
 }
 
-// Exponent e of every row: the entries times 2^e have norm <= 2^58.
-__global__ void k_i8_scale(const double2* __restrict__ part, int R, int chunks, int K, int* __restrict__ ex) {
+// What the guarded form asks of a row besides (one chunk of it): entries of at least a quarter of their neighbours'
+// root mean square, and the smallest mean square of any neighbourhood.
+struct I8Even {
+  double good, low;
+};
+// k_i8_norm with the evenness of the rows, the entries in registers.  KC: a warp takes 256 consecutive entries as a
+// neighbourhood (fewer than 32 at the end count as not good); else a thread takes 16 of its row (and what remains of
+// its chunk below 16 counts as not good).
+template <bool KC>
+__global__ void __launch_bounds__(256) k_i8_norm_even(const double2* __restrict__ X, long ld, int R, int K, int kchunk,
+                                                      double2* __restrict__ part, I8Even* __restrict__ even) {
+  const int k0 = blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
+  double mx = 0.0, ss = 0.0;
+  I8Even ev{0.0, DBL_MAX};
+  auto square = [&](double2 v) {
+    mx = fmax(mx, fmax(fabs(v.x), fabs(v.y)));
+    return fma(v.x, v.x, v.y * v.y);
+  };
+  if (KC) {
+    const int r = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const double2* x = X + (long)r * ld;
+    int n = 0;
+    for (int k = k0 + w * 256; k < k1; k += 8 * 256) {
+      double q[8], sub = 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) q[j] = k + lane + 32 * j < k1 ? square(x[k + lane + 32 * j]) : 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sub += q[j];
+      for (int o = 16; o > 0; o >>= 1) sub += __shfl_xor_sync(0xffffffffu, sub, o);
+      const int len = min(256, k1 - k);
+      const double mean = sub / len;
+      ss += sub;
+      if (len >= 32) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) n += 16.0 * q[j] >= mean ? 1 : 0;  // all of them at mean 0, which fails by low
+        ev.low = fmin(ev.low, mean);
+      }
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    __shared__ double2 red[8];
+    __shared__ I8Even er[8];
+    if (lane == 0) {
+      red[w] = make_double2(mx, ss);
+      er[w] = I8Even{(double)n, ev.low};
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      ev = er[0];
+      for (int i = 1; i < 8; ++i) {
+        mx = fmax(mx, red[i].x);
+        ss += red[i].y;
+        ev.good += er[i].good;
+        ev.low = fmin(ev.low, er[i].low);
+      }
+      part[(long)blockIdx.y * R + r] = make_double2(mx, ss);
+      even[(long)blockIdx.y * R + r] = ev;
+    }
+  } else {
+    const int r = blockIdx.x * 256 + threadIdx.x;
+    if (r >= R) return;
+    int k = k0;
+    for (; k + 16 <= k1; k += 16) {
+      double q[16], sub = 0.0;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) q[j] = square(X[(long)(k + j) * ld + r]);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) sub += q[j];
+      int n = 0;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) n += 256.0 * q[j] >= sub ? 1 : 0;
+      ss += sub;
+      ev.good += n;
+      ev.low = fmin(ev.low, sub / 16.0);
+    }
+    for (; k < k1; ++k) ss += square(X[(long)k * ld + r]);
+    part[(long)blockIdx.y * R + r] = make_double2(mx, ss);
+    even[(long)blockIdx.y * R + r] = ev;
+  }
+}
+
+// Exponent e of every row: the entries times 2^e have norm <= 2^58.  even (may be null): *uneven becomes 1 when a
+// row is not of even size: three quarters of its entries at least a quarter of their neighbourhood's root mean square, and every
+// neighbourhood's mean square at least an eighth of the row's.  Of two such rows, half of the products a_k b_k are then at
+// least |a||b| / (128 K) each: sum |a_k||b_k| >= 2^-8 |a||b| whatever the rows hold.
+__global__ void k_i8_scale(const double2* __restrict__ part, const I8Even* __restrict__ even, int R, int chunks, int K,
+                           int* __restrict__ ex, int* __restrict__ uneven) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= R) return;
   double mx = 0.0, ss = 0.0;
@@ -117,11 +210,12 @@ __global__ void k_i8_scale(const double2* __restrict__ part, int R, int chunks, 
     ss += v.y;
   }
   int e;
+  const bool in_range = ss > 1e-280 && ss < 1e300;
   if (isnan(ss) || isinf(mx)) {
     e = I8_BAD;
   } else if (mx == 0.0) {
     e = 0;
-  } else if (ss > 1e-280 && ss < 1e300) {
+  } else if (in_range) {
     frexp(sqrt(ss) * (1.0 + 1e-12), &e);  // norm < 2^e (1e-12: the rounding of the sum of squares)
     e = I8_NORM_EXP - e;
   } else {  // the squares over- or underflow: norm <= sqrt(2 K) max
@@ -131,6 +225,15 @@ __global__ void k_i8_scale(const double2* __restrict__ part, int R, int chunks, 
     e = I8_NORM_EXP - em - ek;
   }
   ex[r] = e;
+  if (even && !(ss == 0.0 && mx == 0.0)) {
+    double good = 0.0, low = DBL_MAX;
+    for (int c = 0; c < chunks; ++c) {
+      const I8Even v = even[(long)c * R + r];
+      good += v.good;
+      low = fmin(low, v.low);
+    }
+    if (!(in_range && good >= 0.75 * K && 8.0 * low * K >= ss)) *uneven = 1;
+  }
 }
 
 // ---- residue tiles ------------------------------------------------------------------------------
@@ -195,7 +298,9 @@ __device__ __forceinline__ void i8_store(const unsigned (&lo)[8], const unsigned
 // 16 bytes read and 32 written per entry: 110e6 entries in 1.18 ms, 4.5 TB/s, with the integer pipes at
 // three quarters of their rate (about 13 instructions per entry and modulus).
 __global__ void __launch_bounds__(256) k_i8_tiles(const double2* __restrict__ X, long ld, bool kc, bool conj, int r0, int rows,
-                                                  int k0, int kn, const int* __restrict__ ex, I8Tiles out) {
+                                                  int k0, int kn, const int* __restrict__ ex, I8Tiles out,
+                                                  const int* __restrict__ skip) {
+  if (skip && *skip) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kcm = blockIdx.y * 8 + warp;  // core matrix along K
   if (kcm >= (kn + I8_KB - 1) / I8_KB * (I8_KB / 16)) return;
@@ -252,6 +357,7 @@ struct I8Gemm {
   int rga, rgb;                                      // row groups of A and B
   unsigned char* out;                                // [split][mod][plane][M][Npad]
   int* err;
+  const int* skip;  // not null and not zero there: nothing to do (the other kernel takes the product)
   I8Mod mod;
 };
 
@@ -331,6 +437,7 @@ __device__ __forceinline__ unsigned i8_mod4(const uint32_t* x, unsigned p, unsig
 }
 
 __global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant__ I8Gemm g) {
+  if (g.skip && *g.skip) return;
   extern __shared__ __align__(1024) unsigned char ism[];
   __shared__ __align__(8) uint64_t bars[3 * I8_STAGES + 5];
   __shared__ uint32_t tmem_slot;
@@ -648,7 +755,9 @@ __device__ __forceinline__ void i8_put(double2* o, double2 s, double alpha, doub
 template <bool TR, bool ONE>
 __global__ void __launch_bounds__(256, 2) k_i8_out(const unsigned char* __restrict__ res, int M, int N, int Npad, int splits,
                                                 const int* __restrict__ exa, const int* __restrict__ exb, double2* __restrict__ O,
-                                                long ldo_r, long ldo_c, double alpha, double beta, double scale, I8Less less) {
+                                                long ldo_r, long ldo_c, double alpha, double beta, double scale, I8Less less,
+                                                const int* __restrict__ skip) {
+  if (skip && *skip) return;
   constexpr int COLS = TR ? 32 : 128, ROWS = 1024 / COLS;
   __shared__ double2 tile[ROWS][TR ? COLS + 1 : COLS];
   const int cl = threadIdx.x % (COLS / 4) * 4;
@@ -764,8 +873,9 @@ constexpr long kI8ChunkOut = 1L << 26;             // outputs whose residues are
 
 size_t zgemm_i8_cache_bytes(int R, int K) { return ((size_t)R * 4 + 255) / 256 * 256 + i8_tile_bytes(R, K); }
 
-int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, bool* done) {
+int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, bool* done, const int** uneven) {
   *done = false;
+  *uneven = nullptr;
   GemmArgs g = g0;
   // The MMA's M side pads to 256 rows, its N side to 32 per tile: the orientation with less padding, or, within
   // a tenth, the one whose N side is contiguous in the output.
@@ -808,7 +918,9 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
   size_t off = 0;
   auto take = [&](size_t b) { const size_t o = off; off += up(b); return o; };
   const size_t o_exa = take(4 * (size_t)g.M), o_exb = take(4 * (size_t)g.N);
-  const size_t o_part = take(sizeof(double2) * std::max((size_t)norm_chunks(g.a_kc, g.M) * g.M, (size_t)norm_chunks(g.b_kc, g.N) * g.N));
+  const size_t parts_max = std::max((size_t)norm_chunks(g.a_kc, g.M) * g.M, (size_t)norm_chunks(g.b_kc, g.N) * g.N);
+  const size_t o_part = take(sizeof(double2) * parts_max), o_even = take(g.guard ? sizeof(I8Even) * parts_max : 0);
+  const size_t o_flag = take(g.guard ? sizeof(int) : 0);
   const size_t o_a = take(g.a_cache ? 0 : i8_tile_bytes(Mc, Kc));
   const size_t o_b = take(g.b_cache ? 0 : i8_tile_bytes(Nc, Kc));
   const size_t o_res = take((size_t)total_splits * I8_MODS * 2 * Mc * ((Nc + 255) / 256 * tile_n(Nc)));
@@ -829,14 +941,21 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
     I8Tiles t;        // of the whole operand (cache) or of the current chunk
     long at_r, at_k;  // chunk held (no cache)
   };
+  int* flag = g.guard ? reinterpret_cast<int*>(base + o_flag) : nullptr;
+  if (flag) DFT_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), s));
   Op oa{g.A, g.lda, g.a_kc, g.conj_a, g.M, g.a_cache, (int*)(base + o_exa), {base + o_a, 0, 0}, -1, -1};
   Op ob{g.B, g.ldb, g.b_kc, g.conj_b, g.N, g.b_cache, (int*)(base + o_exb), {base + o_b, 0, 0}, -1, -1};
   auto exponents = [&](const Op& o) {
     double2* part = reinterpret_cast<double2*>(base + o_part);
-    const int nch = norm_chunks(o.kc, o.R), kchunk = (g.K + nch - 1) / nch;
-    if (o.kc) k_i8_norm<true><<<dim3(o.R, nch), 256, 0, s>>>(o.X, o.ld, o.R, g.K, kchunk, part);
-    else k_i8_norm<false><<<dim3(ceil_div(o.R, 256), nch), 256, 0, s>>>(o.X, o.ld, o.R, g.K, kchunk, part);
-    k_i8_scale<<<ceil_div(o.R, 256), 256, 0, s>>>(part, o.R, nch, g.K, o.ex);
+    I8Even* even = g.guard ? reinterpret_cast<I8Even*>(base + o_even) : nullptr;
+    const int nch = norm_chunks(o.kc, o.R), unit = g.guard ? (o.kc ? 256 : 16) : 1;
+    const int kchunk = (int)((((long)g.K + nch - 1) / nch + unit - 1) / unit * unit);
+    const dim3 grid(o.kc ? (unsigned)o.R : ceil_div(o.R, 256), ceil_div(g.K, kchunk));
+    if (even && o.kc) k_i8_norm_even<true><<<grid, 256, 0, s>>>(o.X, o.ld, o.R, g.K, kchunk, part, even);
+    else if (even) k_i8_norm_even<false><<<grid, 256, 0, s>>>(o.X, o.ld, o.R, g.K, kchunk, part, even);
+    else if (o.kc) k_i8_norm<true><<<grid, 256, 0, s>>>(o.X, o.ld, o.R, g.K, kchunk, part);
+    else k_i8_norm<false><<<grid, 256, 0, s>>>(o.X, o.ld, o.R, g.K, kchunk, part);
+    k_i8_scale<<<ceil_div(o.R, 256), 256, 0, s>>>(part, even, o.R, (int)grid.y, g.K, o.ex, flag);
     count_launch(2);
   };
   auto convert = [&](Op& o, long r0, int rows, long k0, int kn) {
@@ -844,7 +963,7 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
     o.t.kb = i8_groups(rows) * 8 * I8_KB;
     o.t.plane = o.t.kb * kbs;
     k_i8_tiles<<<dim3((unsigned)i8_groups(rows), ceil_div(kbs * (I8_KB / 16), 8)), 256, 0, s>>>(o.X, o.ld, o.kc, o.cj, (int)r0, rows,
-                                                                                             (int)k0, kn, o.ex, o.t);
+                                                                                             (int)k0, kn, o.ex, o.t, flag);
     count_launch();
     o.at_r = r0;
     o.at_k = k0;
@@ -887,6 +1006,7 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
       a.Npad = a.nt * a.tn;
       a.kps = kps;
       a.err = err;
+      a.skip = flag;
       a.mod = i8_mods();
       int z = 0;
       for (int k = 0; k < nk; ++k) {
@@ -925,12 +1045,13 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
       const bool tr = g.ldo_r < g.ldo_c;
       const dim3 grid = tr ? dim3(ceil_div(rn, 32), ceil_div(rm, 32)) : dim3(ceil_div(rn, 128), ceil_div(rm, 8));
       auto* kernel = tr ? (z == 1 ? k_i8_out<true, true> : k_i8_out<true, false>) : (z == 1 ? k_i8_out<false, true> : k_i8_out<false, false>);
-      kernel<<<grid, 256, 0, s>>>(base + o_res, rm, rn, a.Npad, z, oa.ex + m0, ob.ex + n0, o, g.ldo_r, g.ldo_c, g.alpha, g.beta, i8_scale(), z == 1 ? kI8Less : I8Less{0, 0});
+      kernel<<<grid, 256, 0, s>>>(base + o_res, rm, rn, a.Npad, z, oa.ex + m0, ob.ex + n0, o, g.ldo_r, g.ldo_c, g.alpha, g.beta, i8_scale(), z == 1 ? kI8Less : I8Less{0, 0}, flag);
       count_launch();
     }
   }
   DFT_CUDA_TRY(cudaGetLastError());
   *done = true;
+  *uneven = flag;
   return DFTCUDA_OK;
 }
 

@@ -455,8 +455,9 @@ int dftcuda_projector_phi(int l, size_t nq, double gmax, const double* table, si
  *   out(r, c) = alpha * sum_k opA(A(r, k)) * opB(B(c, k)) + beta * out(r, c),   r < M, c < N, k < K
  * A(r, k) is A[r*lda + k] when a_kc != 0 (K contiguous), else A[k*lda + r]; the same for B; opX
  * conjugates when conj_x != 0.  out(r, c) is out[r*ldo_r + c*ldo_c].  All pointers are device
- * pointers to interleaved complex128.  precision: DFTCUDA_PRECISION_FP64 (exact int8
- * tensor-core products above a size, FP64 tensor cores below),
+ * pointers to interleaved complex128.  precision: DFTCUDA_PRECISION_FP64 (64-bit sums on the FP64
+ * tensor cores; above a size, where the entries of every row of A and B are finite and of even size, products of
+ * 2^-58 fixed point on the int8 tensor cores, whose error of about 2^-59 |a||b| is below that of the sums),
  * DFTCUDA_PRECISION_TF32 or DFTCUDA_PRECISION_TF32X3 (tcgen05 tensor-core kernels); FP32 is not
  * accepted.  The call allocates its workspace, runs on a private stream and returns after
  * the product is complete.
