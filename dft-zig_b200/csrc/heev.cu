@@ -128,9 +128,15 @@ __device__ __forceinline__ void reflector_scalars(double2 alpha, double xnorm2, 
   if (xnorm2 == 0.0 && alpha.y == 0.0) return;
   beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xnorm2), alpha.x);
   const double2 den = make_double2(alpha.x - beta, alpha.y);  // v = x / (alpha - beta)
-  const double ib = 1.0 / beta, id = 1.0 / (den.x * den.x + den.y * den.y);
-  t = make_double2(-den.x * ib, -den.y * ib);
-  sc = make_double2(den.x * id, -den.y * id);
+  const double dn2 = den.x * den.x + den.y * den.y;
+  if (dn2 > 1e-290) {
+    const double ib = 1.0 / beta, id = 1.0 / dn2;
+    t = make_double2(-den.x * ib, -den.y * ib);
+    sc = make_double2(den.x * id, -den.y * id);
+  } else {  // reciprocals that may overflow (a column of about 1e-154), or a NaN
+    t = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
+    sc = make_double2(den.x / dn2, -den.y / dn2);
+  }
 }
 
 // Step 1.  A: m x m Hermitian, column-major, both triangles.  Column k of the result holds the
@@ -650,16 +656,8 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
     }
     ss = warp_sum(ss);
     const double2 alpha = make_double2(__shfl_sync(0xffffffffu, x[0].x, 0), __shfl_sync(0xffffffffu, x[0].y, 0));
-    t = make_double2(0.0, 0.0);
-    beta = alpha.x;
-    double2 sc = make_double2(0.0, 0.0);
-    if (!(ss == 0.0 && alpha.y == 0.0)) {
-      beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + ss), alpha.x);
-      const double2 den = make_double2(alpha.x - beta, alpha.y);
-      const double dn2 = den.x * den.x + den.y * den.y, ib = 1.0 / beta, id = 1.0 / dn2;
-      t = make_double2(-den.x * ib, -den.y * ib);
-      sc = make_double2(den.x * id, -den.y * id);
-    }
+    double2 sc;
+    reflector_scalars(alpha, ss, t, beta, sc);
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       const int i = lane + 32 * q;

@@ -125,3 +125,16 @@ def test_incremental_gram_matches_full_rebuild(dz):
             os.environ.pop("DFTCUDA_GRAM", None)
     assert out["full"].converged and out["incremental"].converged
     assert np.abs(out["full"].values - out["incremental"].values).max() < 1e-9
+
+
+@pytest.mark.parametrize("m", [24, 60, 95, 96, 200, 1300])
+def test_columns_whose_squares_are_subnormal(dz, m):
+    """Couplings of 1e-155 between levels of order one: the squared length of a reflector's column (4e-310) is below the
+    smallest normal number, and its reciprocal beyond the largest.  The squares, in units of 5e-324, leave the reflectors
+    unitary to a few 1e-13."""
+    rng = np.random.default_rng(m)
+    e = rng.normal(size=(m, m)) + 1j * rng.normal(size=(m, m))
+    d = np.sort(rng.uniform(1.0, 2.0, m))
+    r = dz.hermitian_eigen_decomp(np.diag(d) + 1e-155 / m ** 0.5 * (e + e.conj().T), 8)
+    assert np.abs(r.values - d[:8]).max() < 4e-12
+    assert np.isfinite(r.vectors).all()
