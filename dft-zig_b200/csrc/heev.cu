@@ -932,7 +932,7 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(const double* __restrict__
         for (int c = 0; c < kIvChunk; ++c) {
           if (c < n) {
             const int i = i0 + c;
-            if (fabs(a) >= fabs(sb[c])) {
+            if (fabs(a) >= fabs(sb[c]) || fabs(sb[c]) < tiny) {  // no pivot below tiny, whichever row it is in
               const double piv = fabs(a) < tiny ? (a < 0.0 ? -tiny : tiny) : a;
               const double l = sb[c] / piv;
               rp[i] = 1.0 / piv; u1[i] = b; u2[i] = 0.0; lm[i] = l; swp[i] = 0;

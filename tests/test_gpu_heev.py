@@ -138,3 +138,16 @@ def test_columns_whose_squares_are_subnormal(dz, m):
     r = dz.hermitian_eigen_decomp(np.diag(d) + 1e-155 / m ** 0.5 * (e + e.conj().T), 8)
     assert np.abs(r.values - d[:8]).max() < 4e-12
     assert np.isfinite(r.vectors).all()
+
+
+@pytest.mark.parametrize("m", [24, 60, 96, 200])
+@pytest.mark.parametrize("coupling", [1e-155, 1e-140, 1e-100, 1e-40])
+def test_levels_almost_decoupled(dz, m, coupling):
+    """An eigenvalue that equals a diagonal entry leaves the coupling as the pivot of the inverse iteration: the vectors
+    stay unit and orthogonal."""
+    rng = np.random.default_rng(m)
+    e = rng.normal(size=(m, m)) + 1j * rng.normal(size=(m, m))
+    d = np.sort(rng.uniform(1.0, 2.0, m))
+    r = dz.hermitian_eigen_decomp(np.diag(d) + coupling / m ** 0.5 * (e + e.conj().T), 8)
+    assert np.abs(r.values - d[:8]).max() < 4e-12
+    assert np.abs(r.vectors.conj() @ r.vectors.T - np.eye(8)).max() < 1e-10
