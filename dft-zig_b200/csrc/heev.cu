@@ -1059,7 +1059,8 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(const double* __restrict__
 
 // Step 4.  E[:, j] = H_0 H_1 ... H_{m-2} Z[:, j] (applied right to left), one warp per column.  SMALL
 // (m <= kHtSmallM): the block first copies the reflectors to shared memory, so that a step's time is not the
-// latency of its global loads (0.75 us a reflector).
+// latency of its global loads (0.75 us a reflector), and the vectors of T, which are made orthogonal to rounding
+// (the cyclic Jacobi sweeps that used to serve these sizes gave them so).
 template <bool SMALL>
 __global__ void __launch_bounds__(BT_WARPS * 32) k_hetrd_back(const double2* __restrict__ A, const double2* __restrict__ tau,
                                                               int m, int nev, const double* __restrict__ Z,
@@ -1069,10 +1070,12 @@ __global__ void __launch_bounds__(BT_WARPS * 32) k_hetrd_back(const double2* __r
   const int j = blockIdx.x * BT_WARPS + wid;
   const double2* refl = A;
   const double2* tk = tau;
+  double2* const s = esm + (size_t)BT_WARPS * m;
+  double* const zs = reinterpret_cast<double*>(s + m * m + m);
   if (SMALL) {
-    double2* s = esm + (size_t)BT_WARPS * m;
     for (int i = threadIdx.x; i < m * m; i += blockDim.x) s[i] = A[i];
     for (int i = threadIdx.x; i < m; i += blockDim.x) s[m * m + i] = tau[i];
+    for (int i = threadIdx.x; i < m * nev; i += blockDim.x) zs[i] = Z[i];
     __syncthreads();
     refl = s;
     tk = s + m * m;
@@ -1080,7 +1083,33 @@ __global__ void __launch_bounds__(BT_WARPS * 32) k_hetrd_back(const double2* __r
   if (j >= nev) return;
   double2* ev = esm + (size_t)wid * m;
   const double* zj = Z + (size_t)j * m;
-  for (int i = lane; i < m; i += 32) ev[i] = make_double2(zj[i], 0.0);
+  if (SMALL) {
+    // z_j (3 - Z^T Z) / 2 in place of z_j: what the vectors of different groups overlap by, up to eps ||T|| / 1e-5
+    // ||T||, is squared away
+    constexpr int Q = (kHtSmallM + 31) / 32;
+    double g[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const double* zi = zs + (size_t)min(lane + 32 * q, nev - 1) * m;
+      g[q] = 0.0;
+      for (int k = 0; k < m; ++k) g[q] = fma(zi[k], zs[(size_t)j * m + k], g[q]);
+    }
+    double x[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) x[q] = lane + 32 * q < m ? 3.0 * zs[(size_t)j * m + lane + 32 * q] : 0.0;
+#pragma unroll
+    for (int p = 0; p < Q; ++p)
+      for (int i = 32 * p; i < min(nev, 32 * p + 32); ++i) {
+        const double gi = __shfl_sync(0xffffffffu, g[p], i & 31);
+#pragma unroll
+        for (int q = 0; q < Q; ++q) x[q] = fma(-gi, zs[(size_t)i * m + min(lane + 32 * q, m - 1)], x[q]);
+      }
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (lane + 32 * q < m) ev[lane + 32 * q] = make_double2(0.5 * x[q], 0.0);
+  } else {
+    for (int i = lane; i < m; i += 32) ev[i] = make_double2(zj[i], 0.0);
+  }
   __syncwarp();
   for (int k = m - 2; k >= 0; --k) {
     const double2 t = tk[k];
@@ -1394,8 +1423,8 @@ int heev_lowest(double2* A, int m, int nev, double* evals, double2* E, long lde,
   if (m >= 192 && nev >= 32) {
     DFT_TRY(heev_back_blocked(A, w.tau, m, nev, w.z, E, lde, w, s));
   } else if (m <= kHtSmallM) {
-    const size_t smem = sizeof(double2) * ((size_t)BT_WARPS * m + (size_t)m * m + m);
-    DFT_TRY(ensure_max_dynamic_smem((const void*)k_hetrd_back<true>, (int)(sizeof(double2) * (kHtSmallM + BT_WARPS + 1) * kHtSmallM)));
+    const size_t smem = sizeof(double2) * ((size_t)BT_WARPS * m + (size_t)m * m + m) + sizeof(double) * m * nev;
+    DFT_TRY(ensure_max_dynamic_smem((const void*)k_hetrd_back<true>, (int)((sizeof(double2) * (kHtSmallM + BT_WARPS + 1) + sizeof(double) * kHtSmallM) * kHtSmallM)));
     k_hetrd_back<true><<<ceil_div(nev, BT_WARPS), BT_WARPS * 32, smem, s>>>(A, w.tau, m, nev, w.z, E, lde);
     count_launch();
   } else {

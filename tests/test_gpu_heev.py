@@ -151,3 +151,20 @@ def test_levels_almost_decoupled(dz, m, coupling):
     r = dz.hermitian_eigen_decomp(np.diag(d) + coupling / m ** 0.5 * (e + e.conj().T), 8)
     assert np.abs(r.values - d[:8]).max() < 4e-12
     assert np.abs(r.vectors.conj() @ r.vectors.T - np.eye(8)).max() < 1e-10
+
+
+def _spectrum(d, seed):
+    rng = np.random.default_rng(seed)
+    q, _ = np.linalg.qr(rng.normal(size=(len(d), len(d))) + 1j * rng.normal(size=(len(d), len(d))))
+    a = (q * d) @ q.conj().T
+    return (a + a.conj().T) / 2
+
+
+@pytest.mark.parametrize("m,nev", [(2, 2), (33, 12), (64, 40), (95, 95)])
+def test_small_vectors_are_orthogonal_to_rounding(dz, m, nev):
+    """Levels 1.5e-5 ||T|| apart, just beyond what the inverse iteration orthogonalises as one group.  The vectors of T are
+    made orthogonal to rounding and m reflectors applied, each good to a few eps: 8 m eps."""
+    a = _spectrum(np.concatenate([[1.0], 0.5 + 1.5e-5 * np.arange(m - 1)]), m)
+    r = dz.hermitian_eigen_decomp(a, nev)
+    _check(a, r, nev)
+    assert np.abs(r.vectors.conj() @ r.vectors.T - np.eye(nev)).max() < 8 * m * np.finfo(float).eps
