@@ -631,11 +631,10 @@ constexpr size_t kHtResSmem = 226 * 1024;
 // trailing columns and take their products with the new reflector.  Bound by the latency of those
 // reductions and of the update's chains: 36, 83 and 225 us at m = 24, 48 and 88 (37, 95 and 260 with a warp per
 // column and guarded loads).  The cyclic Jacobi sweeps that used to serve these sizes took 2.9 ms at m = 40-88.
-// status: 1 when the tridiagonal form is not finite.
 constexpr int kHtSmallM = 95;
 
 __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict__ A, int m, double* __restrict__ dd,
-                                                            double* __restrict__ ee, double2* __restrict__ tau, int* __restrict__ status) {
+                                                            double* __restrict__ ee, double2* __restrict__ tau) {
   extern __shared__ double2 hsm[];
   double2* const a = hsm;  // column-major, leading dimension m
   __shared__ double2 sv[2][kHtSmallM + 1], sw[kHtSmallM + 1], sy[kHtSmallM + 1];
@@ -645,7 +644,6 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
   constexpr int Q = (kHtSmallM + 31) / 32;
   double2 t = make_double2(0.0, 0.0);  // warp 0: tau and beta of the current reflector
   double beta = 0.0;
-  bool finite = true;
   // warp 0: the reflector of x[0 .. n) (lane holds entries lane + 32 q), v to out; as block_reflector
   auto reflector = [&](double2 (&x)[Q], int n, double2* out) {
     double ss = 0.0;
@@ -663,7 +661,6 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
       const int i = lane + 32 * q;
       if (i < n) out[i] = i == 0 ? make_double2(1.0, 0.0) : cmul(x[q], sc);
     }
-    finite = finite && isfinite(beta);
   };
   if (warp == 0) {
     double2 x[Q];
@@ -675,7 +672,6 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
       ee[0] = beta;
       tau[0] = t;
     }
-    finite = finite && isfinite(a[0].x);
   }
   __syncthreads();
   for (int r = 1 + warp; r < m; r += HT_WARPS) {  // products of step 0: conj(a) v
@@ -730,7 +726,6 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
         c[q] = i < n1 ? e : make_double2(0.0, 0.0);
       }
       if (lane == 0) dd[k + 1] = c[0].x;
-      finite = finite && isfinite(__shfl_sync(0xffffffffu, c[0].x, 0));
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         x[q].x = __shfl_down_sync(0xffffffffu, c[q].x, 1);
@@ -786,7 +781,6 @@ __global__ void __launch_bounds__(HT_THREADS) k_hetrd_small(double2* __restrict_
   }
   // the reflectors, for the back-transformation
   for (int i = tid; i < m * m; i += HT_THREADS) A[i] = a[i];
-  if (warp == 0 && lane == 0 && !finite) *status = 1;
 }
 
 // Number of eigenvalues of T below x (Sturm sequence of the LDL^T pivots).
@@ -803,10 +797,11 @@ __device__ __forceinline__ int sturm_count(const double* d, const double* e2, in
 }
 
 // Step 2.  w[j], j < nev: the j-th smallest eigenvalue of T.  Block 0 also writes ||T|| (the
-// Gershgorin radius bound) to *tnorm_out for step 3.
+// Gershgorin radius bound) to *tnorm_out for step 3, and 1 to *status where T is not finite (a NaN or an infinity of
+// the matrix reaches T through the reflectors) unless a timeout stands there.
 __global__ void __launch_bounds__(BS_WARPS * 32) k_tridiag_bisect(const double* __restrict__ dd, const double* __restrict__ ee,
                                                                   int m, int nev, double* __restrict__ w,
-                                                                  double* __restrict__ tnorm_out) {
+                                                                  double* __restrict__ tnorm_out, int* __restrict__ status) {
   extern __shared__ double bsm[];
   double* d = bsm;
   double* e2 = bsm + m;
@@ -816,6 +811,7 @@ __global__ void __launch_bounds__(BS_WARPS * 32) k_tridiag_bisect(const double* 
   for (int i = tid; i < m; i += blockDim.x) {
     const double di = dd[i];
     const double el = i > 0 ? fabs(ee[i - 1]) : 0.0, er = i + 1 < m ? fabs(ee[i]) : 0.0;
+    if (blockIdx.x == 0 && !(isfinite(di) && isfinite(er))) atomicCAS(status, 0, 1);
     d[i] = di;
     if (i + 1 < m) e2[i] = ee[i] * ee[i];
     lo = fmin(lo, di - el - er);
@@ -1372,7 +1368,7 @@ int heev_lowest(double2* A, int m, int nev, double* evals, double2* E, long lde,
   DFT_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
   if (m > 1 && m <= kHtSmallM && !two_barrier) {
     DFT_TRY(ensure_max_dynamic_smem((const void*)k_hetrd_small, (int)(sizeof(double2) * kHtSmallM * kHtSmallM)));
-    k_hetrd_small<<<1, HT_THREADS, sizeof(double2) * m * m, s>>>(A, m, w.d, w.e, w.tau, status);
+    k_hetrd_small<<<1, HT_THREADS, sizeof(double2) * m * m, s>>>(A, m, w.d, w.e, w.tau);
     count_launch();
   } else if (m > 1) {
     GridBarrier bar{w.bar, status, 0};
@@ -1416,7 +1412,7 @@ int heev_lowest(double2* A, int m, int nev, double* evals, double2* E, long lde,
   // rate, still sets the time
   int bw = BS_WARPS;
   while (bw > 1 && bw * nev > 4 * 4 * n_sm) bw /= 2;
-  k_tridiag_bisect<<<nev, bw * 32, sizeof(double) * 2 * m, s>>>(w.d, w.e, m, nev, evals, w.tnorm);
+  k_tridiag_bisect<<<nev, bw * 32, sizeof(double) * 2 * m, s>>>(w.d, w.e, m, nev, evals, w.tnorm, status);
   count_launch();
   k_tridiag_invit<<<nev, 32, invit_smem(m), s>>>(w.d, w.e, m, nev, evals, w.tnorm, w.z);
   count_launch();
@@ -1487,5 +1483,6 @@ extern "C" int dftcuda_hermitian_eigen_decomp(size_t n, const double* a, size_t 
                                is_device_pointer(vectors) ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s));
   DFT_CUDA_TRY(cudaStreamSynchronize(s));
   if (h_status == kBarrierTimeoutFlag) return fail(DFTCUDA_ERR_TIMEOUT, "hermitian_eigen_decomp: grid barrier timed out");
+  if (h_status != 0) return fail(DFTCUDA_ERR_EIGENSOLVER_FAILURE, "hermitian_eigen_decomp: the matrix is not finite");
   return DFTCUDA_OK;
 }

@@ -253,7 +253,8 @@ int dftcuda_fno_train(size_t nsamples, const int* dims, const size_t* offs, cons
  * zheev 'V','U' in hermitian_eigen_decomp_lapack) and lobpcg/common.zig:440-508, restricted to the
  * nev lowest eigenpairs (nev = n gives the full decomposition).  a: n x n column-major complex, the
  * upper triangle is read.  values[nev] ascending, vectors[n x nev]; host or device pointers.
- * n <= 2048.  The Davidson loop above uses the same kernels for subspaces of 96 and more. */
+ * n <= 2048.  A matrix that is not finite gives DFTCUDA_ERR_EIGENSOLVER_FAILURE.  The Davidson loop above uses
+ * the same kernels for its subspaces. */
 int dftcuda_hermitian_eigen_decomp(size_t n, const double* a, size_t nev, double* values, double* vectors);
 
 /* ------------------------------------------------------------------------------------------

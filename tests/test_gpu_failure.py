@@ -95,3 +95,33 @@ def test_allocation_failure_reports_and_recovers(dz, fail_alloc, after):
     x2 = random_block(kp.ctx.n, 3, 5)
     assert rel_err(kc.apply_hamiltonian_batched(x2), kp.ctx.apply_batch(x2)) < 1e-11
     kc.close()
+
+
+@pytest.mark.parametrize("m", [1, 2, 40, 95, 96, 200, 1300])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_matrix_that_is_not_finite_is_refused(dz, m, value):
+    """One bad entry at a size of each reduction: an error instead of eigenpairs, and the next matrix is solved."""
+    a = _hermitian(m, 3)
+    bad = a.copy()
+    bad[m // 3, m - 1 - m // 4] = value
+    if m > 1:
+        bad[m - 1 - m // 4, m // 3] = value
+    with pytest.raises(dz.LapackFailure):
+        dz.hermitian_eigen_decomp(bad, min(m, 5))
+    assert np.abs(dz.hermitian_eigen_decomp(a, 1).values - np.linalg.eigvalsh(a)[:1]).max() < 1e-11 * max(1.0, np.abs(a).sum(0).max())
+
+
+@pytest.mark.parametrize("nbands", [20, 100])
+def test_solve_with_nan_potential_is_refused(dz, nbands):
+    """Subspaces of 24 and of 104 rows: LapackFailure, and the context solves again with the potential set anew."""
+    kp = kproblem("si8", 20.0, (0.25, 0.0, 0.0))
+    kc = make_context(dz, kp)
+    v = kp.ctx.local_r.copy()
+    v[5] = np.nan
+    kc.set_vloc(v)
+    with pytest.raises(dz.LapackFailure):
+        kc.hermitian_eigen_decomp_iterative(kp.ctx.basis.kinetic, nbands, dz.Options(max_iter=3, tol=1e-6))
+    kc.set_vloc(kp.ctx.local_r)
+    r = kc.hermitian_eigen_decomp_iterative(kp.ctx.basis.kinetic, nbands, dz.Options(max_iter=3, tol=1e-6))
+    assert np.isfinite(r.values).all() and np.isfinite(r.max_residual)
+    kc.close()
