@@ -823,8 +823,9 @@ def _radial_meshes(meshes):
 
 def debug_set_wait_limits(polls: int = 0, unreachable: bool = False):
     """Failure injection for the bounded device waits (dftcuda_debug_set_wait_limits): polls > 0 sets
-    the subspace eigensolver's grid-barrier poll budget, unreachable makes every barrier wait run it
-    out (the call then raises Timeout).  debug_set_wait_limits() restores the defaults."""
+    the poll budget of the subspace eigensolver's grid barrier and of the int8 products' pipeline,
+    unreachable makes their waits run it out (the call then raises Timeout).  debug_set_wait_limits()
+    restores the defaults."""
     _check(load_library().dftcuda_debug_set_wait_limits(int(polls), 1 if unreachable else 0))
 
 

@@ -91,7 +91,8 @@ bool is_device_pointer(const void* p);
 int ensure_max_dynamic_smem(const void* kernel, int bytes);
 
 // Failure injection for the bounded device waits (dftcuda_debug_set_wait_limits): polls > 0 replaces
-// the grid barrier's poll budget; unreachable raises every barrier target by one arrival no block makes.
+// the poll budget of the grid barrier and of the int8 products' waits; unreachable makes them wait for one arrival that
+// no block makes.
 struct WaitLimits {
   long polls;
   bool unreachable;

@@ -344,7 +344,7 @@ constexpr int I8_SLOT = 4 * I8_HALF;  // A, then B, of two K blocks
 constexpr int I8_SMEM = I8_STAGES * I8_SLOT;
 constexpr int I8_EPI = 8, I8_THREADS = 32 * (I8_EPI + 2);
 constexpr int I8_MAX_K = 65536;  // of one split: K 121^2 < 2^30 in the int32 accumulators
-constexpr long long I8_WAIT_CYCLES = 1LL << 33;  // about four seconds
+constexpr long long I8_WAIT_CYCLES = 1LL << 33;  // about four seconds, unless polls are set
 constexpr int I8_PAIRS = 74;
 
 struct I8Mod {
@@ -357,6 +357,8 @@ struct I8Gemm {
   int rga, rgb;                                      // row groups of A and B
   unsigned char* out;                                // [split][mod][plane][M][Npad]
   int* err;
+  long polls;     // limit of a wait, 0: I8_WAIT_CYCLES
+  bool withhold;  // failure injection: the second CTA never reports its copies, so that the waits run out
   const int* skip;  // not null and not zero there: nothing to do (the other kernel takes the product)
   I8Mod mod;
 };
@@ -372,16 +374,15 @@ __device__ __forceinline__ bool i8_try(uint32_t mbar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-__device__ __noinline__ bool i8_wait_long(uint32_t mbar, uint32_t parity) {
+__device__ __noinline__ bool i8_wait_long(uint32_t mbar, uint32_t parity, long polls) {
   const long long t0 = clock64();
-  do {
+  for (long n = 0; polls > 0 ? n < polls : clock64() - t0 < I8_WAIT_CYCLES; ++n)
     if (i8_try(mbar, parity)) return true;
-  } while (clock64() - t0 < I8_WAIT_CYCLES);
   return false;
 }
 // Bounded wait for the phase with the given parity; all lanes of the warp.
-__device__ __forceinline__ bool i8_wait(uint32_t mbar, uint32_t parity) {
-  return __all_sync(0xffffffffu, i8_try(mbar, parity) || i8_try(mbar, parity) || i8_wait_long(mbar, parity));
+__device__ __forceinline__ bool i8_wait(uint32_t mbar, uint32_t parity, long polls) {
+  return __all_sync(0xffffffffu, i8_try(mbar, parity) || i8_try(mbar, parity) || i8_wait_long(mbar, parity, polls));
 }
 __device__ __forceinline__ bool i8_elect() {
   uint32_t p;
@@ -491,7 +492,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant
     for (int it = pair; it < items; it += pairs, ++j) {
       const Item w = item_of(it);
       const int buf = j & 1;
-      if (!i8_wait(acc_full + 8 * buf, (uint32_t)((j >> 1) & 1))) {
+      if (!i8_wait(acc_full + 8 * buf, (uint32_t)((j >> 1) & 1), g.polls)) {
         late();
         break;
       }
@@ -533,7 +534,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant
       const unsigned char* b = g.B + (size_t)w.plane * g.b_plane + (size_t)w.kb0 * g.b_kb + (size_t)rb * (8 * I8_KB);
       for (int k = 0; k < w.kbs; k += 2, ++t) {
         const int q = t % I8_STAGES;
-        if (t >= I8_STAGES && !i8_wait(empty + 8 * q, (uint32_t)((t / I8_STAGES - 1) & 1))) {
+        if (t >= I8_STAGES && !i8_wait(empty + 8 * q, (uint32_t)((t / I8_STAGES - 1) & 1), g.polls)) {
           late();
           ok = false;
           break;
@@ -554,10 +555,15 @@ __global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant
         b += 2 * g.b_kb;
       }
     }
-    // no copy may be in flight when the CTA exits, nor a commit on its way to this CTA's barriers
-    const uint32_t last = ok ? empty : full;
-    for (int u = max(0, t - I8_STAGES); u < t; ++u)
-      if (!i8_wait(last + 8 * (u % I8_STAGES), (uint32_t)((u / I8_STAGES) & 1))) late();
+    // no copy may be in flight when the CTA exits (whatever the limit of the waits), nor a commit on its way to this
+    // CTA's barriers
+    for (int u = max(0, t - I8_STAGES); u < t; ++u) {
+      const uint32_t q = u % I8_STAGES, par = (uint32_t)((u / I8_STAGES) & 1);
+      if (ok && i8_wait(empty + 8 * q, par, g.polls)) continue;
+      if (ok) late();
+      ok = false;
+      if (!i8_wait(full + 8 * q, par, 0)) late();
+    }
   } else if (rank == 1) {
     // ---- the second CTA tells the leader that its copies have landed ----
     int t = 0;
@@ -566,12 +572,12 @@ __global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant
       const int kbs = item_of(it).kbs;
       for (int k = 0; k < kbs; k += 2, ++t) {
         const int q = t % I8_STAGES;
-        if (!i8_wait(full + 8 * q, (uint32_t)((t / I8_STAGES) & 1))) {
+        if (!i8_wait(full + 8 * q, (uint32_t)((t / I8_STAGES) & 1), g.polls)) {
           late();
           ok = false;
           break;
         }
-        if (i8_elect()) i8_arrive_leader(peer + 8 * q);
+        if (!g.withhold && i8_elect()) i8_arrive_leader(peer + 8 * q);
         __syncwarp();
       }
     }
@@ -584,7 +590,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant
     const uint64_t desc0 = i8_desc(ring);
     for (int it = pair; it < items && ok; it += pairs, ++j) {
       const int kbs = item_of(it).kbs, buf = j & 1;
-      if (j >= 2 && !i8_wait(acc_empty + 8 * buf, (uint32_t)((j / 2 - 1) & 1))) {
+      if (j >= 2 && !i8_wait(acc_empty + 8 * buf, (uint32_t)((j / 2 - 1) & 1), g.polls)) {
         late();
         break;
       }
@@ -593,7 +599,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant
       for (int k = 0; k < kbs; k += 2, ++t) {
         const int q = t % I8_STAGES;
         const uint32_t par = (uint32_t)((t / I8_STAGES) & 1);
-        if (!i8_wait(full + 8 * q, par) || !i8_wait(peer + 8 * q, par)) {
+        if (!i8_wait(full + 8 * q, par, g.polls) || !i8_wait(peer + 8 * q, par, g.polls)) {
           late();
           ok = false;
           break;
@@ -617,7 +623,7 @@ __global__ void __launch_bounds__(I8_THREADS, 1) k_i8_gemm(const __grid_constant
     if (i8_elect())
       asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(fin) : "memory");
     __syncwarp();
-    if (!i8_wait(fin, 0u)) late();
+    if (!i8_wait(fin, 0u, 0)) late();
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
@@ -996,6 +1002,7 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
     }
   }
   DFT_TRY(ensure_max_dynamic_smem((const void*)k_i8_gemm, I8_SMEM));
+  const WaitLimits limits = wait_limits();
   for (long n0 = 0; n0 < g.N; n0 += Nc) {
     for (long m0 = 0; m0 < g.M; m0 += Mc) {
       const int rm = (int)std::min<long>(Mc, g.M - m0), rn = (int)std::min<long>(Nc, g.N - n0);
@@ -1007,6 +1014,8 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
       a.kps = kps;
       a.err = err;
       a.skip = flag;
+      a.polls = limits.polls;
+      a.withhold = limits.unreachable;
       a.mod = i8_mods();
       int z = 0;
       for (int k = 0; k < nk; ++k) {

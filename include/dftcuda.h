@@ -67,11 +67,11 @@ const char* dftcuda_last_error_message(void);
 int dftcuda_device_count(void);
 
 /* Failure injection for tests of the timeout path (no reference counterpart).  Every device-side wait
- * in the library is bounded: the subspace eigensolver's grid barrier polls about a second, then sets
- * an error flag, its blocks return, and the call reports DFTCUDA_ERR_TIMEOUT with the context still
- * usable.  polls > 0 sets that barrier's poll budget (0 restores the default); unreachable != 0 raises
- * every barrier's target by one arrival that no block makes, so each wait runs out its budget.
- * Process-wide; applies to launches made after the call. */
+ * in the library is bounded: the subspace eigensolver's grid barrier polls about a second, the int8 products'
+ * pipeline waits about four, then they set an error flag, their blocks return, and the call reports
+ * DFTCUDA_ERR_TIMEOUT with the context still usable.  polls > 0 sets the poll budget of both (0 restores the
+ * defaults; the TF32 pipelines keep theirs); unreachable != 0 makes both wait for one arrival that no block
+ * makes, so each wait runs out its budget.  Process-wide; applies to launches made after the call. */
 int dftcuda_debug_set_wait_limits(long polls, int unreachable);
 
 /* Failure injection for tests of the out-of-memory path (no reference counterpart): after >= 0 makes

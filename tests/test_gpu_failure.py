@@ -3,7 +3,8 @@
 Every device-side wait in the library is bounded.  dftcuda_debug_set_wait_limits makes the subspace
 eigensolver's grid barrier wait for an arrival that no block makes, with a short poll budget, so the
 wait runs out: the blocks set the error flag and return, the call reports DFTCUDA_ERR_TIMEOUT, and a
-normal call afterwards (on the same context) must succeed.  A NaN injected on the host into one
+normal call afterwards (on the same context) must succeed.  The same for the int8 products' pipeline,
+whose second CTA then never reports its copies.  A NaN injected on the host into one
 column of psi must come back as a clean status with the NaN confined to that column.
 dftcuda_debug_fail_alloc makes one device allocation fail as cudaMalloc does on a full device: the
 call reports DFTCUDA_ERR_OUT_OF_MEMORY and the context stays usable.
@@ -124,4 +125,40 @@ def test_solve_with_nan_potential_is_refused(dz, nbands):
     kc.set_vloc(kp.ctx.local_r)
     r = kc.hermitian_eigen_decomp_iterative(kp.ctx.basis.kinetic, nbands, dz.Options(max_iter=3, tol=1e-6))
     assert np.isfinite(r.values).all() and np.isfinite(r.max_residual)
+    kc.close()
+
+
+def test_residue_pipeline_timeout_reports_and_recovers(dz, limits):
+    """Every role of the pipeline gives up by itself: one item per pair and several, one CTA pair and all of them."""
+    import torch
+
+    gen = torch.Generator().manual_seed(1)
+    for M, N, K in ((300, 400, 4000), (700, 500, 9000)):
+        a, b = (torch.randn(n, K, dtype=torch.complex128, generator=gen).cuda() for n in (M, N))
+        limits(64, True)
+        with pytest.raises(dz.Timeout):
+            dz.complex_gemm(a, b)
+        limits()
+        ref = a @ b.T
+        assert float((dz.complex_gemm(a, b) - ref).abs().max()) < 1e-13 * float(ref.abs().max()) * K ** 0.5
+
+
+def test_projector_product_timeout_leaves_context_usable(dz, limits):
+    """An H|psi> large enough for the residue form on the projectors."""
+    import torch
+
+    kp = kproblem("si8", 25.0, (0.25, 0.0, 0.0))
+    kc = make_context(dz, kp)
+    n = kp.ctx.n
+    pos = np.random.default_rng(2).uniform(0, 10.0, (64, 3))
+    phi = np.random.default_rng(3).normal(size=(5, n))
+    kc.set_projectors([dz.SpeciesProjectors([0, 0, 1], np.eye(3), phi)], np.zeros(64, dtype=np.int32), pos)
+    x = torch.from_numpy(random_block(n, 400, 7)).cuda()
+    good = kc.apply_hamiltonian_batched(x, torch.empty_like(x)).clone()
+    limits(64, True)
+    with pytest.raises(dz.Timeout):
+        kc.apply_hamiltonian_batched(x, torch.empty_like(x))
+    limits()
+    again = kc.apply_hamiltonian_batched(x, torch.empty_like(x))
+    assert float((again - good).abs().max()) <= 1e-13 * float(good.abs().max())
     kc.close()
