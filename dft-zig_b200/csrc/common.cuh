@@ -75,12 +75,20 @@ void count_launch(int n = 1);
 // the k-th following one fail once, as cudaMalloc does when the device is out of memory, so that
 // tests can check that each entry point reports DFTCUDA_ERR_OUT_OF_MEMORY and keeps its context usable.
 bool alloc_should_fail();
+// Frees the operand tiles and product workspaces of the current device that no call is using; false when there are none.
+bool reclaim_tiles();
+// Where the device is full, kept tiles give way before an allocation fails.
 template <typename T> inline cudaError_t dev_malloc(T** p, size_t bytes) {
-  if (alloc_should_fail()) {
-    *p = nullptr;
-    return cudaErrorMemoryAllocation;
+  *p = nullptr;
+  if (alloc_should_fail()) return cudaErrorMemoryAllocation;
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  if (reclaim_tiles()) {
+    e = cudaMalloc(reinterpret_cast<void**>(p), bytes);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
   }
-  return cudaMalloc(reinterpret_cast<void**>(p), bytes);
+  return e;
 }
 
 // True when p is device (or managed) memory, false for host memory (pageable or pinned).

@@ -703,8 +703,8 @@ static int small_eig(KCtxImpl* e, int m, int nev, cudaStream_t s) {
 
 // V's leading columns were rewritten: the tiles cached from them are stale.
 static void v_changed(KCtxImpl* e) {
-  e->vt_gram.valid = false;
-  e->vt_comb.valid = false;
+  e->vt_gram.invalidate();
+  e->vt_comb.invalidate();
 }
 
 // orthonormalize_all (common.zig:298-312) for V[0:m]: block Gram-Schmidt; columns that drop are
@@ -810,14 +810,11 @@ static int run_init(EigRun& r, const double* diag, const double* init_vecs, size
       bc = std::max(bc, zgemm_i8_cache_bytes((int)n, (int)e->max_sub));
     }
     // kept tiles only save conversions: they leave the memory to workspaces where it is scarce
-    size_t free_b = 0, total_b = 0;
-    const bool room = !i8 || (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && 4 * (bg + bc) <= free_b);
-    if (room && bg + bc <= kVTileCacheBytes && e->vt_gram.ensure(bg) == DFTCUDA_OK && e->vt_comb.ensure(bc) == DFTCUDA_OK) {
+    if (bg + bc <= kVTileCacheBytes && e->vt_gram.ensure(bg, i8) == DFTCUDA_OK && e->vt_comb.ensure(bc, i8) == DFTCUDA_OK) {
       e->v_cache = true;
     } else {
       e->vt_gram.release();
       e->vt_comb.release();
-      cudaGetLastError();
     }
   }
   e->tc_min_flops = c->tc_min_flops;

@@ -370,10 +370,11 @@ int kctx_project(dftcuda_kctx* c, const double2* x, size_t ncols, cudaStream_t s
   g.O = c->d_coef; g.ldo_r = (long)ncols; g.ldo_c = 1;
   g.alpha = 1.0; g.beta = 0.0;
   g.splits = c->split_proj;
-  g.a_cache = &c->tc_ptiles_proj;
   g.a_share = 0.0;
   g.i8 = &c->tc_scratch; g.err = c->d_err;
-  if (projectors_on_tf32(c, g))
+  const bool tf32 = projectors_on_tf32(c, g);
+  g.a_cache = tf32 ? &c->tc_ptiles_proj : &c->i8_ptiles_proj;
+  if (tf32)
     return cgemm_tf32(g, s, c->d_gemm_ws, c->gemm_ws_elems, c->d_err, c->precision == DFTCUDA_PRECISION_TF32X3, &c->tc_scratch);
   return zgemm(g, s, c->d_gemm_ws, c->gemm_ws_elems);
 }
@@ -398,10 +399,11 @@ static int nonlocal_block(dftcuda_kctx* c, const double2* x, double2* y, size_t 
   g.O = y; g.ldo_r = (long)c->npw; g.ldo_c = 1;
   g.alpha = 1.0 / c->volume; g.beta = 1.0;
   g.splits = c->split_back;
-  g.b_cache = &c->tc_ptiles_back;
   g.b_share = 0.0;
   g.i8 = &c->tc_scratch; g.err = c->d_err;
-  if (projectors_on_tf32(c, g))
+  const bool tf32 = projectors_on_tf32(c, g);
+  g.b_cache = tf32 ? &c->tc_ptiles_back : &c->i8_ptiles_back;
+  if (tf32)
     return cgemm_tf32(g, s, c->d_gemm_ws, c->gemm_ws_elems, c->d_err, c->precision == DFTCUDA_PRECISION_TF32X3, &c->tc_scratch);
   return zgemm(g, s, c->d_gemm_ws, c->gemm_ws_elems);
 }
@@ -554,8 +556,7 @@ extern "C" int dftcuda_kctx_destroy(dftcuda_kctx* c) {
     if (p) cudaFree(p);
   c->fx.destroy(); c->fy.destroy(); c->fz.destroy();
   c->tc_scratch.release();
-  c->tc_ptiles_proj.release();
-  c->tc_ptiles_back.release();
+  for (TcScratch* t : {&c->tc_ptiles_proj, &c->tc_ptiles_back, &c->i8_ptiles_proj, &c->i8_ptiles_back}) t->release();
   if (c->ev_order) cudaEventDestroy(c->ev_order);
   for (int i = 0; i < kPipeChunks; ++i) {
     if (c->ev_in[i]) cudaEventDestroy(c->ev_in[i]);
@@ -698,8 +699,8 @@ extern "C" int dftcuda_set_projectors(dftcuda_kctx* c, size_t n_species, const d
   DFT_TRY(dg.status);
   cudaStreamSynchronize(c->stream);
   free_nonlocal(c);
-  c->tc_ptiles_proj.release();  // the split copies of the old projector matrix
-  c->tc_ptiles_back.release();
+  // the converted copies of the old projector matrix
+  for (TcScratch* t : {&c->tc_ptiles_proj, &c->tc_ptiles_back, &c->i8_ptiles_proj, &c->i8_ptiles_back}) t->release();
   c->natoms = 0;
   c->atom_row.clear();
   c->atom_mt.clear();

@@ -7,16 +7,38 @@
 
 namespace dftcuda {
 
-// Device buffer of the tensor-core GEMM's pre-split operands (grown on demand, owned by a context).
-// As the cache of a constant operand (the projector matrix) it also records what it holds: valid
-// and the key of the layout it was split for.
+// Device buffer of the tensor-core GEMMs: converted operands, or as a cache one constant operand (the projector
+// matrix) with what it holds (valid, and the key of the layout it was converted for).  Grown on demand, owned by a
+// context, and given back when another allocation of the library finds the device full: a call that uses the
+// buffer holds a TilePins on it while it enqueues its kernels, and whoever frees it synchronises the device first.
 struct TcScratch {
   void* p = nullptr;
   size_t bytes = 0;
   bool valid = false;
   unsigned long long key = 0;
-  int ensure(size_t need);
+  TcScratch() = default;
+  TcScratch(const TcScratch&) = delete;
+  TcScratch& operator=(const TcScratch&) = delete;
+  // spare: for a product that has another kernel to run on.  It gets at most a quarter of the memory then free (what the
+  // buffer has counting as free); a request beyond that fails and leaves the buffer as it is, and the next ones that
+  // need it grown fail unseen (eight of them).
+  int ensure(size_t need, bool spare = false);
   void release();
+  void trim(size_t most);  // release where it holds more
+  void invalidate();
+  bool holds(unsigned long long k, size_t need);
+
+ private:
+  friend struct TilePins;
+  friend bool reclaim_tiles();
+  int pins = 0, device = -1, unseen = 0;
+};
+struct TilePins {
+  TcScratch* s[3];
+  TilePins(TcScratch* a, TcScratch* b, TcScratch* c);
+  ~TilePins();
+  TilePins(const TilePins&) = delete;
+  TilePins& operator=(const TilePins&) = delete;
 };
 
 // Complex GEMM over strided operands (zgemm.cu):
@@ -30,7 +52,7 @@ struct GemmArgs {
   double2* O; long ldo_r; long ldo_c;
   double alpha, beta;
   int splits = 0;  // split-K count; 0 = the kernel's wave-filling heuristic
-  // Constant operands whose TF32 split the tensor-core GEMM may keep between calls (null: split per call).
+  // Constant operands whose converted form the tensor-core GEMMs may keep between calls (null: converted per call).
   TcScratch* a_cache = nullptr;
   TcScratch* b_cache = nullptr;
   // FP64 products large enough for the int8 residue form (zgemm_i8.cu) run there when the caller gives
@@ -166,8 +188,9 @@ struct dftcuda_kctx {
   size_t box_bytes = 0;
 
   dftcuda::NonlocalDev nl;
-  dftcuda::TcScratch tc_scratch;  // pre-split tensor-core GEMM operands (TF32 and TF32X3 contexts)
-  dftcuda::TcScratch tc_ptiles_proj, tc_ptiles_back;  // the projector matrix split for the two projector GEMMs
+  dftcuda::TcScratch tc_scratch;  // workspace of the tensor-core GEMMs: the operands of one product, its residues
+  // the projector matrix converted for the two projector GEMMs: TF32 splits (TF32 and TF32X3 contexts), int8 residues
+  dftcuda::TcScratch tc_ptiles_proj, tc_ptiles_back, i8_ptiles_proj, i8_ptiles_back;
   int natoms = 0;                   // atoms given to set_projectors
   std::vector<int> atom_row, atom_mt;  // per atom (set_projectors order): first projector row, row count
   std::vector<int> atom_species;       // per atom: species index

@@ -4,6 +4,7 @@
 #include <map>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include "kctx.cuh"
 
@@ -94,6 +95,113 @@ bool alloc_should_fail() {
     if (g_fail_alloc.compare_exchange_weak(v, v - 1)) return v == 0;
   }
   return false;
+}
+
+// Every TcScratch that holds memory.  One lock for the list and the fields that reclaim_tiles() reads or changes; a
+// pinned buffer is its owner's alone.
+static std::mutex g_tiles_mu;
+static std::vector<TcScratch*> g_tiles;
+
+TilePins::TilePins(TcScratch* a, TcScratch* b, TcScratch* c) : s{a, b, c} {
+  std::lock_guard<std::mutex> lock(g_tiles_mu);
+  for (TcScratch* t : s)
+    if (t) ++t->pins;
+}
+TilePins::~TilePins() {
+  std::lock_guard<std::mutex> lock(g_tiles_mu);
+  for (TcScratch* t : s)
+    if (t) --t->pins;
+}
+
+bool reclaim_tiles() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> lock(g_tiles_mu);
+  bool any = false;
+  for (size_t i = 0; i < g_tiles.size();) {
+    TcScratch* t = g_tiles[i];
+    if (t->pins > 0 || t->device != dev) {
+      ++i;
+      continue;
+    }
+    if (!any && cudaDeviceSynchronize() != cudaSuccess) return false;  // kernels that read the tiles are done
+    any = true;
+    cudaFree(t->p);
+    t->p = nullptr;
+    t->bytes = 0;
+    t->valid = false;
+    g_tiles[i] = g_tiles.back();
+    g_tiles.pop_back();
+  }
+  return any;
+}
+
+int TcScratch::ensure(size_t need, bool spare) {
+  {
+    std::lock_guard<std::mutex> lock(g_tiles_mu);
+    if (need <= bytes) return DFTCUDA_OK;
+  }
+  if (spare) {
+    if (unseen > 0) {
+      --unseen;
+      return DFTCUDA_ERR_OUT_OF_MEMORY;
+    }
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || 4 * need > free_b + bytes) {
+      cudaGetLastError();
+      unseen = 8;
+      return DFTCUDA_ERR_OUT_OF_MEMORY;
+    }
+  }
+  release();
+  void* q = nullptr;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev_malloc(&q, need) != cudaSuccess) {
+    unseen = spare ? 8 : 0;
+    return fail(DFTCUDA_ERR_OUT_OF_MEMORY, "tensor-core operand tiles");
+  }
+  std::lock_guard<std::mutex> lock(g_tiles_mu);
+  p = q;
+  bytes = need;
+  device = dev;
+  g_tiles.push_back(this);
+  return DFTCUDA_OK;
+}
+
+void TcScratch::release() {
+  void* q = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(g_tiles_mu);
+    q = p;
+    p = nullptr;
+    bytes = 0;
+    valid = false;
+    for (size_t i = 0; i < g_tiles.size(); ++i)
+      if (g_tiles[i] == this) {
+        g_tiles[i] = g_tiles.back();
+        g_tiles.pop_back();
+        break;
+      }
+  }
+  if (q) cudaFree(q);
+}
+
+void TcScratch::trim(size_t most) {
+  {
+    std::lock_guard<std::mutex> lock(g_tiles_mu);
+    if (bytes <= most) return;
+  }
+  release();
+}
+
+void TcScratch::invalidate() {
+  std::lock_guard<std::mutex> lock(g_tiles_mu);
+  valid = false;
+}
+
+bool TcScratch::holds(unsigned long long k, size_t need) {
+  std::lock_guard<std::mutex> lock(g_tiles_mu);
+  return valid && key == k && bytes >= need;
 }
 
 DeviceGuard::DeviceGuard(int dev) {
@@ -221,6 +329,7 @@ extern "C" int dftcuda_complex_gemm(int precision, size_t M, size_t N, size_t K,
     TcScratch tiles;
     std::mutex mu;
   };
+  constexpr size_t kEngineTileBytes = (size_t)2 << 30;  // tiles kept from call to call
   static std::mutex map_mu;
   static std::map<int, Engine*> engines;
   Engine* en = nullptr;
@@ -246,7 +355,6 @@ extern "C" int dftcuda_complex_gemm(int precision, size_t M, size_t N, size_t K,
     en->ws_cap = ws_elems;
   }
   DFT_CUDA_TRY(cudaMemsetAsync(en->err, 0, sizeof(int), en->s));
-  en->tiles.valid = false;  // operands differ from call to call
   g.i8 = &en->tiles;
   g.err = en->err;
   g.guard = true;
@@ -255,6 +363,7 @@ extern "C" int dftcuda_complex_gemm(int precision, size_t M, size_t N, size_t K,
   int herr = 0;
   const cudaError_t e = rc == DFTCUDA_OK ? cudaMemcpyAsync(&herr, en->err, sizeof(int), cudaMemcpyDeviceToHost, en->s) : cudaSuccess;
   const cudaError_t e2 = cudaStreamSynchronize(en->s);
+  en->tiles.trim(kEngineTileBytes);
   if (rc == DFTCUDA_OK) {
     if (e != cudaSuccess || e2 != cudaSuccess) rc = fail(DFTCUDA_ERR_CUDA, std::string("complex_gemm: ") + cudaGetErrorString(e2));
     else if (herr) rc = fail(DFTCUDA_ERR_TIMEOUT, "complex_gemm: a tensor-core pipeline wait timed out");

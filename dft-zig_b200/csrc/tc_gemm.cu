@@ -1344,20 +1344,20 @@ static int tc4_run(const GemmArgs& g, cudaStream_t s, double2* ws, size_t ws_ele
       h = h * 1000003ULL ^ v;
     return h;
   };
-  DFT_TRY(scratch->ensure((g.a_cache ? 0 : a_bytes) + (g.b_cache ? 0 : b_bytes)));
+  const TilePins pins(scratch, g.a_cache, g.b_cache);
+  // an operand whose cache finds no room is split into the scratch
+  TcScratch* const a_cache = g.a_cache && g.a_cache->ensure(a_bytes) == DFTCUDA_OK ? g.a_cache : nullptr;
+  TcScratch* const b_cache = g.b_cache && g.b_cache->ensure(b_bytes) == DFTCUDA_OK ? g.b_cache : nullptr;
+  DFT_TRY(scratch->ensure((a_cache ? 0 : a_bytes) + (b_cache ? 0 : b_bytes)));
   unsigned char* sp = static_cast<unsigned char*>(scratch->p);
   auto place = [&](TcScratch* cache, size_t bytes, const double2* X, long ld, bool kc, bool cj, int R, int RG,
-                   float** out) -> int {
+                   float** out) {
     bool convert = true;
     if (cache) {
       const unsigned long long key = key_of(X, ld, kc, cj, R);
-      if (cache->valid && cache->key == key && cache->bytes >= bytes) convert = false;
-      else {
-        cache->valid = false;
-        DFT_TRY(cache->ensure(bytes));
-        cache->key = key;
-        cache->valid = true;
-      }
+      convert = !(cache->valid && cache->key == key);
+      cache->key = key;
+      cache->valid = true;
       *out = reinterpret_cast<float*>(cache->p);
     } else {
       *out = reinterpret_cast<float*>(sp);
@@ -1369,11 +1369,10 @@ static int tc4_run(const GemmArgs& g, cudaStream_t s, double2* ws, size_t ws_ele
       else k_tf32_tiles<false><<<ceil_div(units, 256), 256, 0, s>>>(X, ld, kc, cj, R, g.K, RG, KS, *out);
       count_launch();
     }
-    return DFTCUDA_OK;
   };
   float *At = nullptr, *Bt = nullptr;
-  DFT_TRY(place(g.a_cache, a_bytes, g.A, g.lda, g.a_kc, g.conj_a, g.M, RGA, &At));
-  DFT_TRY(place(g.b_cache, b_bytes, g.B, g.ldb, g.b_kc, g.conj_b, g.N, RGB, &Bt));
+  place(a_cache, a_bytes, g.A, g.lda, g.a_kc, g.conj_a, g.M, RGA, &At);
+  place(b_cache, b_bytes, g.B, g.ldb, g.b_kc, g.conj_b, g.N, RGB, &Bt);
   int splits = g.splits > 0 ? std::min(g.splits, std::max(1, KS / 4)) : t3_splits(g.M, g.N, g.K);
   if (splits > 1) splits = (int)std::max<size_t>(1, std::min<size_t>(splits, ws_elems / ((size_t)g.M * g.N)));
   const int kps = (KS + splits - 1) / splits;  // K steps per split
@@ -1397,24 +1396,6 @@ static int tc4_run(const GemmArgs& g, cudaStream_t s, double2* ws, size_t ws_ele
   }
   DFT_CUDA_TRY(cudaGetLastError());
   return DFTCUDA_OK;
-}
-
-int TcScratch::ensure(size_t need) {
-  if (need <= bytes) return DFTCUDA_OK;
-  if (p) cudaFree(p);
-  p = nullptr;
-  bytes = 0;
-  valid = false;
-  if (dev_malloc(&p, need) != cudaSuccess) return fail(DFTCUDA_ERR_OUT_OF_MEMORY, "tensor-core operand tiles");
-  bytes = need;
-  return DFTCUDA_OK;
-}
-
-void TcScratch::release() {
-  if (p) cudaFree(p);
-  p = nullptr;
-  bytes = 0;
-  valid = false;
 }
 
 int cgemm_tf32(const GemmArgs& g0, cudaStream_t s, double2* ws, size_t ws_elems, int* err_dev, bool split, TcScratch* scratch) {

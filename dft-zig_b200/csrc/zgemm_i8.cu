@@ -874,8 +874,10 @@ bool zgemm_i8_beats_split_tf32(int M, int N, int K, double share_m, double share
   return zgemm_i8_worthwhile(M, N, K, share_m, share_n) && i8_seconds(M, N, K, share_m, share_n) < 8.0 * M * (double)N * K / 105e12 + 10e-6;
 }
 
-constexpr size_t kI8ChunkElems = (size_t)1 << 25;  // entries of one operand whose tiles are held at a time
-constexpr long kI8ChunkOut = 1L << 26;             // outputs whose residues are held at a time
+constexpr size_t kI8ChunkElems = (size_t)1 << 25;  // entries of one operand whose tiles are held at a time (1 GB)
+constexpr long kI8ChunkOut = 1L << 26;             // outputs whose residues are held at a time,
+constexpr size_t kI8ResBytes = (size_t)2 << 30;    // over all splits in no more than this
+constexpr size_t kI8KeptBytes = (size_t)4 << 30;   // kept tiles of one operand
 
 size_t zgemm_i8_cache_bytes(int R, int K) { return ((size_t)R * 4 + 255) / 256 * 256 + i8_tile_bytes(R, K); }
 
@@ -898,6 +900,14 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
     std::swap(g.ldo_r, g.ldo_c);
     std::swap(g.a_cache, g.b_cache);
   }
+  const TilePins pins(scratch, g.a_cache, g.b_cache);
+  // an operand whose kept tiles find no room is converted into the scratch
+  auto room = [&](TcScratch*& cache, int R) {
+    const size_t need = zgemm_i8_cache_bytes(R, g.K);
+    if (cache && (need > kI8KeptBytes || cache->ensure(need, true) != DFTCUDA_OK)) cache = nullptr;
+  };
+  room(g.a_cache, g.M);
+  room(g.b_cache, g.N);
   // chunks: equal parts of K, then of the rows, so that the tiles held are bounded
   auto parts = [](long n, long most, long unit) {  // size of the equal parts of n, a multiple of unit
     const long c = (n + most - 1) / most;
@@ -905,14 +915,22 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
   };
   const long Kc = parts(g.K, std::max<long>(8192, std::min<long>(I8_MAX_K, (long)(kI8ChunkElems / std::max(g.M, g.N)))), I8_KB);
   const long rmax = std::max<long>(256, (long)(kI8ChunkElems / Kc));
-  const long Mc = parts(g.M, rmax, 256), Nc = parts(g.N, std::min(rmax, std::max<long>(256, kI8ChunkOut / Mc)), 256);
+  long Mc = parts(g.M, rmax, 256), Nc = parts(g.N, std::min(rmax, std::max<long>(256, kI8ChunkOut / Mc)), 256);
   const int nk = (int)((g.K + Kc - 1) / Kc), KBc = (int)((Kc + I8_KB - 1) / I8_KB), KB = (g.K + I8_KB - 1) / I8_KB;
-  const int splits = i8_splits(Mc, Nc, KBc);
-  const int kps = (KBc + splits - 1) / splits;
-  int total_splits = 0;
-  for (int k = 0; k < nk; ++k) {
-    const int kb = (int)((std::min<long>(Kc, g.K - k * Kc) + I8_KB - 1) / I8_KB);
-    total_splits += (kb + kps - 1) / kps;
+  int kps = 0, total_splits = 0;
+  size_t res_bytes = 0;
+  for (;;) {
+    const int splits = i8_splits(Mc, Nc, KBc);
+    kps = (KBc + splits - 1) / splits;
+    total_splits = 0;
+    for (int k = 0; k < nk; ++k) {
+      const int kb = (int)((std::min<long>(Kc, g.K - k * Kc) + I8_KB - 1) / I8_KB);
+      total_splits += (kb + kps - 1) / kps;
+    }
+    res_bytes = (size_t)total_splits * I8_MODS * 2 * Mc * ((Nc + 255) / 256 * tile_n(Nc));
+    if (res_bytes <= kI8ResBytes || (Mc <= 256 && Nc <= 256)) break;
+    long& longer = Mc >= Nc ? Mc : Nc;
+    longer = (longer / 2 + 255) / 256 * 256;
   }
   if (total_splits > I8_MAX_SPLITS) return DFTCUDA_OK;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
@@ -929,12 +947,8 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
   const size_t o_flag = take(g.guard ? sizeof(int) : 0);
   const size_t o_a = take(g.a_cache ? 0 : i8_tile_bytes(Mc, Kc));
   const size_t o_b = take(g.b_cache ? 0 : i8_tile_bytes(Nc, Kc));
-  const size_t o_res = take((size_t)total_splits * I8_MODS * 2 * Mc * ((Nc + 255) / 256 * tile_n(Nc)));
-  auto no_room = [] {  // not done: the caller's other kernel runs, and must not meet this failure
-    cudaGetLastError();
-    return DFTCUDA_OK;
-  };
-  if (scratch->ensure(off) != DFTCUDA_OK) return no_room();
+  const size_t o_res = take(res_bytes);
+  if (scratch->ensure(off, true) != DFTCUDA_OK) return DFTCUDA_OK;  // not done: the caller's other kernel runs
   unsigned char* base = static_cast<unsigned char*>(scratch->p);
 
   struct Op {
@@ -984,12 +998,8 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
     for (unsigned long long v : {(unsigned long long)(uintptr_t)o->X, (unsigned long long)o->ld, (unsigned long long)o->kc,
                                  (unsigned long long)o->cj, (unsigned long long)o->R, (unsigned long long)g.K})
       key = key * 1000003ULL ^ v;
-    const size_t head = up((size_t)o->R * 4), need = zgemm_i8_cache_bytes(o->R, g.K);
-    const bool have = o->cache->valid && o->cache->key == key && o->cache->bytes >= need;
-    if (!have) {
-      o->cache->valid = false;
-      if (o->cache->ensure(need) != DFTCUDA_OK) return no_room();
-    }
+    const size_t head = up((size_t)o->R * 4);
+    const bool have = o->cache->valid && o->cache->key == key;
     o->ex = static_cast<int*>(o->cache->p);
     o->t.p = static_cast<unsigned char*>(o->cache->p) + head;
     o->t.kb = i8_groups(o->R) * 8 * I8_KB;

@@ -1,0 +1,72 @@
+"""Memory of the tensor-core products: the converted operands that contexts keep, and the workspaces."""
+import numpy as np
+import pytest
+import torch
+
+from tests.helpers import kproblem, make_context, random_block
+
+pytestmark = pytest.mark.gpu
+MB = 1 << 20
+
+
+def _free():
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.cuda.mem_get_info()[0]
+
+
+def _with_projectors(dz, natoms, precision=0, seed=3):
+    """An 8-atom box whose projector matrix has 5 natoms rows: products of the residue form's size."""
+    kp = kproblem("si8", 25.0, (0.25, 0.0, 0.0))
+    kc = make_context(dz, kp, precision)
+    rng = np.random.default_rng(seed)
+    decay = np.exp(-0.1 * kp.ctx.basis.kinetic)
+    kc.set_projectors([dz.SpeciesProjectors([0, 0, 1], 0.1 * np.eye(3), rng.normal(size=(5, kp.ctx.n)) * decay)],
+                      np.zeros(natoms, dtype=np.int32), rng.uniform(0, 10.0, (natoms, 3)))
+    return kp, kc
+
+
+def test_kept_tiles_give_way_on_a_full_device(dz):
+    """One context keeps its projectors' tiles and its workspace; another one's solve needs more than what is left, but less
+    than with the tiles freed: it runs, and the first context's results stay."""
+    kp, kc = _with_projectors(dz, 512)
+    x = torch.from_numpy(random_block(kp.ctx.n, 500, 7)).cuda()
+    empty = _free()
+    for _ in range(8):
+        want = kc.apply_hamiltonian_batched(x, torch.empty_like(x)).clone()
+    kept = empty - _free()
+    kp2 = kproblem("si8", 20.0, (0.25, 0.0, 0.0))
+    opts = dz.Options(max_iter=3, tol=1e-6)
+    kin = kp2.ctx.basis.kinetic
+    trial, late = make_context(dz, kp2), make_context(dz, kp2)
+    before = _free()
+    ref = trial.hermitian_eigen_decomp_iterative(kin, 60, opts)
+    need = before - _free()
+    trial.close()
+    assert kept > 250 * MB and 30 * MB < need < kept
+    filler = torch.empty(_free() - need // 2, dtype=torch.uint8, device="cuda")
+    try:
+        got = late.hermitian_eigen_decomp_iterative(kin, 60, opts)
+    finally:
+        del filler
+        _free()
+    assert np.abs(got.values - ref.values).max() < 1e-9
+    again = kc.apply_hamiltonian_batched(x, torch.empty_like(x))
+    assert float((again - want).abs().max()) <= 1e-13 * float(want.abs().max())
+    late.close()
+    kc.close()
+
+
+def test_product_workspace_is_bounded(dz):
+    """The residues of 4096 x 4096 outputs over 13 K chunks would take 7 GB: the outputs go in parts, and no more than 2 GB
+    stay with the library after the call."""
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    a, b = (torch.randn(4096, 100000, dtype=torch.complex128, device="cuda", generator=gen) for _ in range(2))
+    small = torch.randn(64, 64, dtype=torch.complex128, device="cuda")
+    dz.complex_gemm(small, small)
+    before = _free()
+    out = dz.complex_gemm(a, b)
+    ref = torch.cat([a @ b[i : i + 512].T for i in range(0, 4096, 512)], 1)
+    assert float(torch.linalg.vector_norm(out - ref)) < 1e-13 * float(torch.linalg.vector_norm(ref))
+    del out, ref
+    assert before - _free() <= 2100 * MB
