@@ -322,15 +322,15 @@ int kctx_ensure_err(dftcuda_kctx* c) {
 
 int kctx_ensure_coef(dftcuda_kctx* c, size_t cols) {
   if (c->nl.nproj == 0) return DFTCUDA_OK;
-  if (cols > c->coef_cols) {
+  const size_t elems = (size_t)c->nl.nproj * cols;  // the projectors may have changed since the last call
+  if (elems > c->coef_elems) {
     if (c->d_coef) cudaFree(c->d_coef);
     if (c->d_coef2) cudaFree(c->d_coef2);
     c->d_coef = c->d_coef2 = nullptr;
-    c->coef_cols = 0;
-    const size_t b = sizeof(double2) * (size_t)c->nl.nproj * cols;
-    if (dev_malloc(&c->d_coef, b) != cudaSuccess || dev_malloc(&c->d_coef2, b) != cudaSuccess)
+    c->coef_elems = 0;
+    if (dev_malloc(&c->d_coef, sizeof(double2) * elems) != cudaSuccess || dev_malloc(&c->d_coef2, sizeof(double2) * elems) != cudaSuccess)
       return fail(DFTCUDA_ERR_OUT_OF_MEMORY, "projector coefficients");
-    c->coef_cols = cols;
+    c->coef_elems = elems;
   }
   size_t need = std::max(zgemm_workspace_elems(c->nl.nproj, (int)cols, (int)c->npw),
                          zgemm_workspace_elems((int)cols, (int)c->npw, c->nl.nproj));

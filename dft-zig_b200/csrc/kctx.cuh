@@ -198,7 +198,7 @@ struct dftcuda_kctx {
   std::vector<size_t> species_mt;      // per species: m_total
   double2* d_coef = nullptr;   // [nproj][cols] projector coefficients
   double2* d_coef2 = nullptr;
-  size_t coef_cols = 0;
+  size_t coef_elems = 0;
   double2* d_gemm_ws = nullptr;
   size_t gemm_ws_elems = 0;
   int* d_err = nullptr;  // device error flag of the bounded waits (TF32 tensor-core GEMMs)

@@ -15,14 +15,18 @@ def _free():
     return torch.cuda.mem_get_info()[0]
 
 
-def _with_projectors(dz, natoms, precision=0, seed=3):
-    """An 8-atom box whose projector matrix has 5 natoms rows: products of the residue form's size."""
-    kp = kproblem("si8", 25.0, (0.25, 0.0, 0.0))
-    kc = make_context(dz, kp, precision)
+def _set_projectors(dz, kp, kc, natoms, seed):
     rng = np.random.default_rng(seed)
     decay = np.exp(-0.1 * kp.ctx.basis.kinetic)
     kc.set_projectors([dz.SpeciesProjectors([0, 0, 1], 0.1 * np.eye(3), rng.normal(size=(5, kp.ctx.n)) * decay)],
                       np.zeros(natoms, dtype=np.int32), rng.uniform(0, 10.0, (natoms, 3)))
+
+
+def _with_projectors(dz, natoms, precision=0, seed=3):
+    """An 8-atom box whose projector matrix has 5 natoms rows: products of the residue form's size."""
+    kp = kproblem("si8", 25.0, (0.25, 0.0, 0.0))
+    kc = make_context(dz, kp, precision)
+    _set_projectors(dz, kp, kc, natoms, seed)
     return kp, kc
 
 
@@ -70,3 +74,24 @@ def test_product_workspace_is_bounded(dz):
     assert float(torch.linalg.vector_norm(out - ref)) < 1e-13 * float(torch.linalg.vector_norm(ref))
     del out, ref
     assert before - _free() <= 2100 * MB
+
+
+@pytest.mark.parametrize("precision", [0, 1, 2, 3])
+@pytest.mark.parametrize("sizes", [(2, 40), (300, 512), (512, 300), (512, 512)])
+def test_projectors_set_anew_on_a_used_context(dz, precision, sizes):
+    """More, fewer or as many projectors as before: every buffer follows, and what was kept of the old ones is not read."""
+    cols = 500 if sizes[0] > 2 else 9
+    kp, kc = _with_projectors(dz, sizes[0], precision)
+    x = torch.from_numpy(random_block(kp.ctx.n, cols, 7)).cuda()
+    y = torch.empty_like(x)
+    for _ in range(12):
+        kc.apply_hamiltonian_batched(x, y)
+    _, fresh = _with_projectors(dz, sizes[1], precision, 4)
+    _set_projectors(dz, kp, kc, sizes[1], 4)
+    want = fresh.apply_hamiltonian_batched(x, torch.empty_like(x))
+    tol = (1e-13, 5e-6, 5e-2, 2e-4)[precision]
+    for _ in range(12):
+        got = kc.apply_hamiltonian_batched(x, y)
+        assert float((got - want).abs().max()) <= tol * float(want.abs().max())
+    fresh.close()
+    kc.close()
