@@ -464,7 +464,8 @@ struct KCtxImpl {
   HeevWork hw;
   bool rr_tc = false;  // Rayleigh-Ritz products on the tensor cores (3xTF32), TF32/TF32X3 contexts
   int* err = nullptr;  // the context's tensor-core error flag
-  TcScratch* tcs = nullptr;  // the context's pre-split operand buffer
+  TcScratch* tcs = nullptr;  // the context's tensor-core GEMM workspace
+  bool i8_on = false;        // this run's FP64 products may take the residue form
   // Pre-split tiles of V[0:m] in its two roles (the Gram operand V^H, and the combination V C), kept
   // while V[0:m] is unchanged: the Rayleigh-Ritz products and both orthonormalisation passes of an
   // iteration read the same V[0:m], so each role is split once per iteration instead of three times.
@@ -560,8 +561,10 @@ static int eig_alloc(dftcuda_kctx* c, size_t n, size_t max_sub, size_t nb) {
 // form (FP32-class accuracy); the Cholesky factorisations, the subspace eigensolver and the residual
 // norms stay FP64.  FP64 and FP32 contexts use the FP64 GEMM throughout.
 static int gemm_dispatch(KCtxImpl* e, GemmArgs& g, bool /*rr*/, cudaStream_t s) {
-  g.i8 = e->tcs;
-  g.err = e->err;
+  if (e->i8_on) {
+    g.i8 = e->tcs;
+    g.err = e->err;
+  }
   if (e->rr_tc && tc_worthwhile(g.M, g.N, g.K, e->tc_min_flops)) return cgemm_tf32(g, s, e->ws, e->ws_elems, e->err, true, e->tcs);
   return zgemm(g, s, e->ws, e->ws_elems);
 }
@@ -797,20 +800,29 @@ static int run_init(EigRun& r, const double* diag, const double* init_vecs, size
   DFT_TRY(eig_alloc(c, n, r.max_sub, r.nbands));
   KCtxImpl* e = r.e = c->eig;
   e->rr_tc = precision_uses_tc(c->precision);
-  if (e->rr_tc || zgemm_i8_worthwhile((int)r.max_sub, (int)r.max_sub, (int)n, 1.0 / 3.0, 1.0 / 3.0)) DFT_TRY(kctx_ensure_err(c));
   e->err = c->d_err;
   e->tcs = &c->tc_scratch;
   v_changed(e);
-  const bool i8 = !e->rr_tc && zgemm_i8_worthwhile((int)r.max_sub, (int)r.nbands, (int)n, 1.0 / 3.0, 1.0);
-  if ((e->rr_tc || i8) && !e->v_cache) {
+  // FP64 products on residues where the run gains more than the buffers cost that it would allocate: a sweep makes three
+  // products with V^H and three with V, on average with half the largest subspace
+  e->i8_on = false;
+  if (!e->rr_tc) {
+    const int mh = (int)r.max_sub / 2, nb = (int)r.nbands;
+    const double sweep = 3.0 * (std::max(0.0, zgemm_i8_gain(mh, nb, (int)n, 1.0 / 3.0, 1.0)) + std::max(0.0, zgemm_i8_gain(nb, (int)n, mh, 1.0, 1.0 / 3.0)));
+    const double buffers = e->v_cache ? 0.0 : alloc_seconds(zgemm_i8_cache_bytes((int)e->max_sub, (int)n)) + alloc_seconds(zgemm_i8_cache_bytes((int)n, (int)e->max_sub));
+    e->i8_on = sweep * std::min<double>((double)opts.max_iter, 8.0) > buffers + alloc_seconds(0);
+  }
+  c->err_used = c->err_used || e->rr_tc || e->i8_on;
+  for (int& products : c->p_products) products += (int)std::min<size_t>(opts.max_iter, 8);  // this solve's, ahead of them
+  if ((e->rr_tc || e->i8_on) && !e->v_cache) {
     size_t bg = e->rr_tc ? tc4_operand_bytes((int)e->max_sub, (int)n, true) : 0;
     size_t bc = e->rr_tc ? tc4_operand_bytes((int)n, (int)e->max_sub, true) : 0;
-    if (i8) {
+    if (e->i8_on) {
       bg = std::max(bg, zgemm_i8_cache_bytes((int)e->max_sub, (int)n));
       bc = std::max(bc, zgemm_i8_cache_bytes((int)n, (int)e->max_sub));
     }
     // kept tiles only save conversions: they leave the memory to workspaces where it is scarce
-    if (bg + bc <= kVTileCacheBytes && e->vt_gram.ensure(bg, i8) == DFTCUDA_OK && e->vt_comb.ensure(bc, i8) == DFTCUDA_OK) {
+    if (bg + bc <= kVTileCacheBytes && e->vt_gram.ensure(bg, e->i8_on) == DFTCUDA_OK && e->vt_comb.ensure(bc, e->i8_on) == DFTCUDA_OK) {
       e->v_cache = true;
     } else {
       e->vt_gram.release();

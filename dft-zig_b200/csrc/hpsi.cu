@@ -312,35 +312,27 @@ static int local_block(dftcuda_kctx* c, const double2* x, double2* y, size_t nco
   return DFTCUDA_OK;
 }
 
-int kctx_ensure_err(dftcuda_kctx* c) {
-  if (c->d_err) return DFTCUDA_OK;
-  if (dev_malloc(&c->d_err, sizeof(int)) != cudaSuccess) return fail(DFTCUDA_ERR_OUT_OF_MEMORY, "error flag");
-  DFT_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-  DFT_CUDA_TRY(cudaStreamSynchronize(c->stream));
-  return DFTCUDA_OK;
-}
-
 int kctx_ensure_coef(dftcuda_kctx* c, size_t cols) {
   if (c->nl.nproj == 0) return DFTCUDA_OK;
   const size_t elems = (size_t)c->nl.nproj * cols;  // the projectors may have changed since the last call
   if (elems > c->coef_elems) {
     if (c->d_coef) cudaFree(c->d_coef);
-    if (c->d_coef2) cudaFree(c->d_coef2);
     c->d_coef = c->d_coef2 = nullptr;
     c->coef_elems = 0;
-    if (dev_malloc(&c->d_coef, sizeof(double2) * elems) != cudaSuccess || dev_malloc(&c->d_coef2, sizeof(double2) * elems) != cudaSuccess)
-      return fail(DFTCUDA_ERR_OUT_OF_MEMORY, "projector coefficients");
+    if (dev_malloc(&c->d_coef, sizeof(double2) * 2 * elems) != cudaSuccess) return fail(DFTCUDA_ERR_OUT_OF_MEMORY, "projector coefficients");
+    c->d_coef2 = c->d_coef + elems;
     c->coef_elems = elems;
   }
+  return DFTCUDA_OK;
+}
+
+int kctx_ensure_gemm_ws(dftcuda_kctx* c, size_t cols) {
   size_t need = std::max(zgemm_workspace_elems(c->nl.nproj, (int)cols, (int)c->npw),
                          zgemm_workspace_elems((int)cols, (int)c->npw, c->nl.nproj));
   if (precision_uses_tc(c->precision)) {
     need = std::max(need, cgemm_tf32_workspace_elems(c->nl.nproj, (int)cols, (int)c->npw));
     need = std::max(need, cgemm_tf32_workspace_elems((int)cols, (int)c->npw, c->nl.nproj));
   }
-  if (precision_uses_tc(c->precision) || zgemm_i8_worthwhile(c->nl.nproj, (int)cols, (int)c->npw, 0.0, 1.0) ||
-      zgemm_i8_worthwhile((int)cols, (int)c->npw, c->nl.nproj, 1.0, 0.0))
-    DFT_TRY(kctx_ensure_err(c));
   // forced split counts (autotuner) need their partial sums
   need = std::max(need, (size_t)std::max(c->split_proj, 0) * c->nl.nproj * cols);
   need = std::max(need, (size_t)std::min(std::max(c->split_back, 0), std::max(1, c->nl.nproj / 32)) * cols * c->npw);
@@ -361,8 +353,7 @@ static bool projectors_on_tf32(const dftcuda_kctx* c, const GemmArgs& g) {
   return c->precision == DFTCUDA_PRECISION_TF32 || !zgemm_i8_beats_split_tf32(g.M, g.N, g.K, g.a_share, g.b_share);
 }
 
-// d_coef[p][c] = sum_g P[p][g] x[c][g]   (batch_project_coeffs, apply.zig:1143-1183)
-int kctx_project(dftcuda_kctx* c, const double2* x, size_t ncols, cudaStream_t s) {
+static GemmArgs projection(const dftcuda_kctx* c, const double2* x, size_t ncols) {
   GemmArgs g{};
   g.M = c->nl.nproj; g.N = (int)ncols; g.K = (int)c->npw;
   g.A = c->nl.P; g.lda = (long)c->npw; g.a_kc = true; g.conj_a = false;
@@ -370,13 +361,58 @@ int kctx_project(dftcuda_kctx* c, const double2* x, size_t ncols, cudaStream_t s
   g.O = c->d_coef; g.ldo_r = (long)ncols; g.ldo_c = 1;
   g.alpha = 1.0; g.beta = 0.0;
   g.splits = c->split_proj;
-  g.a_share = 0.0;
-  g.i8 = &c->tc_scratch; g.err = c->d_err;
-  const bool tf32 = projectors_on_tf32(c, g);
-  g.a_cache = tf32 ? &c->tc_ptiles_proj : &c->i8_ptiles_proj;
-  if (tf32)
+  return g;
+}
+static GemmArgs back_projection(const dftcuda_kctx* c, double2* y, size_t ncols) {
+  GemmArgs g{};
+  g.M = (int)ncols; g.N = (int)c->npw; g.K = c->nl.nproj;
+  g.A = c->d_coef2; g.lda = (long)ncols; g.a_kc = false; g.conj_a = false;
+  g.B = c->nl.P; g.ldb = (long)c->npw; g.b_kc = false; g.conj_b = true;
+  g.O = y; g.ldo_r = (long)c->npw; g.ldo_c = 1;
+  g.alpha = 1.0 / c->volume; g.beta = 1.0;
+  g.splits = c->split_back;
+  return g;
+}
+
+// One of the two projector products.  A context's first products pay no more than they gain: the residue form's workspace takes
+// the place of the other kernel's (which is allocated where that one runs), sized for both products at once, and the
+// projectors' tiles are kept only when the conversions seen have cost what their buffer does (zgemm_i8_keep; the
+// back-projection's one product later, so that no call allocates both).  64 atoms at 30 Ry, 164 columns, us a call
+// on a fresh context: FP64 tensor cores alone 2,640 then 2,160; with all buffers allocated and converted by the first
+// call 4,540 then 1,585; now 2,330,
+// then 1,830, from the eighth call on 1,585 (a cudaMalloc of 0.4 ms hides behind the local passes).
+// TF32X3 contexts keep tiles from the first product on, whichever form serves it, so that its accuracy does not depend on
+// the call.
+static int projector_product(dftcuda_kctx* c, GemmArgs& g, bool back, size_t ncols, cudaStream_t s) {
+  TcScratch& tiles = back ? c->i8_ptiles_back : c->i8_ptiles_proj;
+  const int seen = c->p_products[back]++;
+  const bool full = tiles.full(), tc = precision_uses_tc(c->precision);
+  const bool keep = tc || full || zgemm_i8_keep(back ? g.N : g.M, g.K, seen - (back ? 1 : 0), tiles.size());
+  (back ? g.b_share : g.a_share) = tc || full ? 0.0 : keep ? 1.0 / (1.0 + seen) : 1.0;
+  if (projectors_on_tf32(c, g)) {
+    (back ? g.b_cache : g.a_cache) = back ? &c->tc_ptiles_back : &c->tc_ptiles_proj;
+    DFT_TRY(kctx_ensure_gemm_ws(c, ncols));
+    c->err_used = true;
     return cgemm_tf32(g, s, c->d_gemm_ws, c->gemm_ws_elems, c->d_err, c->precision == DFTCUDA_PRECISION_TF32X3, &c->tc_scratch);
+  }
+  if (zgemm_i8_worthwhile(g.M, g.N, g.K, g.a_share, g.b_share)) {
+    if (keep) (back ? g.b_cache : g.a_cache) = &tiles;
+    if (c->tc_scratch.size() == 0)
+      c->tc_scratch.ensure(std::max(zgemm_i8_scratch_bytes(g), zgemm_i8_scratch_bytes(back ? projection(c, nullptr, ncols) : back_projection(c, nullptr, ncols))), true);
+    bool done = false;
+    const int* uneven = nullptr;
+    c->err_used = true;
+    DFT_TRY(zgemm_i8(g, s, &c->tc_scratch, c->d_err, &done, &uneven));
+    if (done) return DFTCUDA_OK;
+  }
+  DFT_TRY(kctx_ensure_gemm_ws(c, ncols));
   return zgemm(g, s, c->d_gemm_ws, c->gemm_ws_elems);
+}
+
+// d_coef[p][c] = sum_g P[p][g] x[c][g]   (batch_project_coeffs, apply.zig:1143-1183)
+int kctx_project(dftcuda_kctx* c, const double2* x, size_t ncols, cudaStream_t s) {
+  GemmArgs g = projection(c, x, ncols);
+  return projector_product(c, g, false, ncols, s);
 }
 
 static int nonlocal_block(dftcuda_kctx* c, const double2* x, double2* y, size_t ncols, cudaStream_t s) {
@@ -392,20 +428,8 @@ static int nonlocal_block(dftcuda_kctx* c, const double2* x, double2* y, size_t 
   }
   // y[c][g] += (1/Omega) sum_p coef2[p][c] conj(P[p][g])   (apply.zig:1278-1336)
   ProfScope ps(c, P_NL_BACK, s);
-  GemmArgs g{};
-  g.M = (int)ncols; g.N = (int)c->npw; g.K = c->nl.nproj;
-  g.A = c->d_coef2; g.lda = (long)ncols; g.a_kc = false; g.conj_a = false;
-  g.B = c->nl.P; g.ldb = (long)c->npw; g.b_kc = false; g.conj_b = true;
-  g.O = y; g.ldo_r = (long)c->npw; g.ldo_c = 1;
-  g.alpha = 1.0 / c->volume; g.beta = 1.0;
-  g.splits = c->split_back;
-  g.b_share = 0.0;
-  g.i8 = &c->tc_scratch; g.err = c->d_err;
-  const bool tf32 = projectors_on_tf32(c, g);
-  g.b_cache = tf32 ? &c->tc_ptiles_back : &c->i8_ptiles_back;
-  if (tf32)
-    return cgemm_tf32(g, s, c->d_gemm_ws, c->gemm_ws_elems, c->d_err, c->precision == DFTCUDA_PRECISION_TF32X3, &c->tc_scratch);
-  return zgemm(g, s, c->d_gemm_ws, c->gemm_ws_elems);
+  GemmArgs g = back_projection(c, y, ncols);
+  return projector_product(c, g, true, ncols, s);
 }
 
 int kctx_apply_h_dev(dftcuda_kctx* c, const double2* x, double2* y, size_t ncols, cudaStream_t s) {
@@ -499,10 +523,11 @@ int kctx_density_dev(dftcuda_kctx* c, const double2* vecs, size_t nbands, const 
 
 // Turns the device error flag of the bounded waits into DFTCUDA_ERR_TIMEOUT (and clears it).
 int kctx_check_error(dftcuda_kctx* c) {
-  if (!c->d_err) return DFTCUDA_OK;
+  if (!c->err_used) return DFTCUDA_OK;
   int h = 0;
   DFT_CUDA_TRY(cudaMemcpyAsync(&h, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   DFT_CUDA_TRY(cudaStreamSynchronize(c->stream));
+  c->err_used = false;
   if (h == 0) return DFTCUDA_OK;
   DFT_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
   DFT_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -548,9 +573,9 @@ extern "C" int dftcuda_kctx_destroy(dftcuda_kctx* c) {
   c->prof.destroy();
   free_nonlocal(c);
   void* ptrs[] = {c->d_plane_off, c->d_pw_idx, c->d_pw_spos, c->d_slot_xpos, c->d_kinetic, c->d_gcart, c->d_vt,
-                  c->d_vt32, c->d_box, c->d_coef, c->d_coef2, c->d_gemm_ws, c->d_x, c->d_y, c->d_rho, c->d_w,
+                  c->d_vt32, c->d_box, c->d_coef, c->d_gemm_ws, c->d_x, c->d_y, c->d_rho, c->d_w,
                   c->d_pwmap, c->d_stick_off, c->d_stick_y, c->d_slot_of_x, c->d_tw4x64, c->d_tw4x32,
-                  c->d_tw4p64, c->d_tw4p32, c->d_err, c->d_mlp, c->d_vstage, c->d_st_of, c->d_st_map, c->d_st_sox,
+                  c->d_tw4p64, c->d_tw4p32, c->d_mlp, c->d_vstage, c->d_st_of, c->d_st_map, c->d_st_sox,
                   c->d_twz64, c->d_twz32, c->d_twx64, c->d_twx32, c->d_vn, c->d_vn32};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -636,7 +661,7 @@ extern "C" int dftcuda_kctx_create(dftcuda_kctx** out, int nx, int ny, int nz, d
   bool ok = dev_malloc(&c->d_plane_off, sizeof(int) * (c->n_act + 1)) == cudaSuccess &&
             dev_malloc(&c->d_pw_idx, sizeof(int) * n_pw) == cudaSuccess &&
             dev_malloc(&c->d_pw_spos, sizeof(int) * n_pw) == cudaSuccess &&
-            dev_malloc(&c->d_slot_xpos, sizeof(int) * c->n_act) == cudaSuccess &&
+            dev_malloc(&c->d_slot_xpos, sizeof(int) * (c->n_act + 1)) == cudaSuccess &&
             dev_malloc(&c->d_kinetic, sizeof(double) * n_pw) == cudaSuccess &&
             dev_malloc(&c->d_gcart, sizeof(double) * 3 * n_pw) == cudaSuccess &&
             dev_malloc(&c->d_vt, sizeof(double) * c->N) == cudaSuccess &&
@@ -652,6 +677,8 @@ extern "C" int dftcuda_kctx_create(dftcuda_kctx** out, int nx, int ny, int nz, d
   cudaMemcpyAsync(c->d_pw_idx, pw_idx.data(), sizeof(int) * n_pw, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(c->d_pw_spos, pw_spos.data(), sizeof(int) * n_pw, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(c->d_slot_xpos, slot_xpos.data(), sizeof(int) * c->n_act, cudaMemcpyHostToDevice, st);
+  c->d_err = c->d_slot_xpos + c->n_act;
+  cudaMemsetAsync(c->d_err, 0, sizeof(int), st);
   cudaMemcpyAsync(c->d_kinetic, kinetic, sizeof(double) * n_pw, cudaMemcpyHostToDevice, st);
   cudaMemcpyAsync(c->d_gcart, gcart, sizeof(double) * 3 * n_pw, cudaMemcpyHostToDevice, st);
   if (cudaStreamSynchronize(st) != cudaSuccess) {
@@ -699,8 +726,12 @@ extern "C" int dftcuda_set_projectors(dftcuda_kctx* c, size_t n_species, const d
   DFT_TRY(dg.status);
   cudaStreamSynchronize(c->stream);
   free_nonlocal(c);
-  // the converted copies of the old projector matrix
-  for (TcScratch* t : {&c->tc_ptiles_proj, &c->tc_ptiles_back, &c->i8_ptiles_proj, &c->i8_ptiles_back}) t->release();
+  // the converted copies of the old projector matrix; their buffers serve the next one
+  for (TcScratch* t : {&c->tc_ptiles_proj, &c->tc_ptiles_back, &c->i8_ptiles_proj, &c->i8_ptiles_back}) {
+    t->invalidate();
+    if (n_species == 0 || n_atoms == 0) t->release();
+  }
+  c->p_products[0] = c->p_products[1] = 0;
   c->natoms = 0;
   c->atom_row.clear();
   c->atom_mt.clear();
@@ -1115,6 +1146,7 @@ extern "C" int dftcuda_nonlocal_stress(dftcuda_kctx* c, const double* kpg, size_
   const size_t nch = std::min<size_t>(nbands, 256);
   DFT_TRY(kctx_stage(c, nch));
   DFT_TRY(kctx_ensure_coef(c, nch));
+  DFT_TRY(kctx_ensure_gemm_ws(c, nch));
   // derivative projectors of all atoms, per direction a: DP_a[(atom, m)][G] = dphi_m,a(G) e^{i G . tau}
   double2* DP = nullptr;
   double* d_tab = nullptr;
@@ -1177,6 +1209,7 @@ extern "C" int dftcuda_nonlocal_stress(dftcuda_kctx* c, const double* kpg, size_
           g.O = d_u; g.ldo_r = (long)nc; g.ldo_c = 1;
           g.alpha = 1.0; g.beta = 0.0;
           g.i8 = &c->tc_scratch; g.err = c->d_err;
+          c->err_used = true;
           DFT_TRY(zgemm(g, s, c->d_gemm_ws, c->gemm_ws_elems));
           k_stress_reduce<<<rb, 256, 0, s>>>(c->d_coef2, d_u, nullptr, d_w + c0, nproj, (long)nc,
                                              -2.0 / (c->volume * c->volume), d_acc + packed(a, b), nullptr);

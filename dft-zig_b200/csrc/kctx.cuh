@@ -26,7 +26,8 @@ struct TcScratch {
   void release();
   void trim(size_t most);  // release where it holds more
   void invalidate();
-  bool holds(unsigned long long k, size_t need);
+  bool full();  // holds a converted operand
+  size_t size();
 
  private:
   friend struct TilePins;
@@ -69,7 +70,12 @@ size_t zgemm_workspace_elems(int M, int N, int K);
 // device flag, not zero where the product was left to the other kernel.
 bool zgemm_i8_worthwhile(int M, int N, int K, double share_m = 1.0, double share_n = 1.0);
 bool zgemm_i8_beats_split_tf32(int M, int N, int K, double share_m, double share_n);
+double zgemm_i8_gain(int M, int N, int K, double share_m, double share_n);  // seconds saved, estimated
 size_t zgemm_i8_cache_bytes(int R, int K);  // one operand's kept tiles (a_cache, b_cache)
+size_t zgemm_i8_scratch_bytes(const GemmArgs& g);
+double alloc_seconds(size_t bytes);  // of one device allocation
+// Tiles of an operand are worth keeping once the conversions seen, one per product, have cost what their buffer does.
+bool zgemm_i8_keep(int R, int K, int products, size_t have);
 int zgemm_i8(const GemmArgs& g, cudaStream_t s, TcScratch* scratch, int* err, bool* done, const int** uneven);
 // The same contraction on the tensor cores (tc_gemm.cu): TF32 inputs, FP32 accumulation.  err_dev
 // receives 1 if a bounded wait gave up.
@@ -191,6 +197,7 @@ struct dftcuda_kctx {
   dftcuda::TcScratch tc_scratch;  // workspace of the tensor-core GEMMs: the operands of one product, its residues
   // the projector matrix converted for the two projector GEMMs: TF32 splits (TF32 and TF32X3 contexts), int8 residues
   dftcuda::TcScratch tc_ptiles_proj, tc_ptiles_back, i8_ptiles_proj, i8_ptiles_back;
+  int p_products[2] = {0, 0};  // projections and back-projections made with the present projectors
   int natoms = 0;                   // atoms given to set_projectors
   std::vector<int> atom_row, atom_mt;  // per atom (set_projectors order): first projector row, row count
   std::vector<int> atom_species;       // per atom: species index
@@ -201,7 +208,8 @@ struct dftcuda_kctx {
   size_t coef_elems = 0;
   double2* d_gemm_ws = nullptr;
   size_t gemm_ws_elems = 0;
-  int* d_err = nullptr;  // device error flag of the bounded waits (TF32 tensor-core GEMMs)
+  int* d_err = nullptr;   // device error flag of the tensor-core GEMMs' bounded waits (at the end of d_slot_xpos),
+  bool err_used = false;  // to be read where one of them may have run
 
   // Staging for host pointers.
   double2* d_x = nullptr;
@@ -223,7 +231,7 @@ namespace dftcuda {
 int kctx_apply_h_dev(dftcuda_kctx* c, const double2* x, double2* y, size_t ncols, cudaStream_t s);
 int kctx_project(dftcuda_kctx* c, const double2* x, size_t ncols, cudaStream_t s);  // d_coef = P x
 int kctx_ensure_coef(dftcuda_kctx* c, size_t cols);
-int kctx_ensure_err(dftcuda_kctx* c);  // d_err, the bounded waits' error flag
+int kctx_ensure_gemm_ws(dftcuda_kctx* c, size_t cols);  // split-K workspace of the projector products
 int kctx_stage(dftcuda_kctx* c, size_t cols);
 int kctx_check_error(dftcuda_kctx* c);
 int kctx_density_dev(dftcuda_kctx* c, const double2* vecs, size_t nbands, const double* w_dev, double* rho_dev,

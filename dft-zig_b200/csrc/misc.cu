@@ -1,4 +1,5 @@
 // Status strings, per-thread last-error message, pointer classification.
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 #include <map>
@@ -153,6 +154,7 @@ int TcScratch::ensure(size_t need, bool spare) {
       return DFTCUDA_ERR_OUT_OF_MEMORY;
     }
   }
+  if (spare && bytes > 0) need = std::max(need, bytes + bytes / 4);  // a growing workspace does not grow every time
   release();
   void* q = nullptr;
   int dev = 0;
@@ -199,9 +201,14 @@ void TcScratch::invalidate() {
   valid = false;
 }
 
-bool TcScratch::holds(unsigned long long k, size_t need) {
+bool TcScratch::full() {
   std::lock_guard<std::mutex> lock(g_tiles_mu);
-  return valid && key == k && bytes >= need;
+  return valid;
+}
+
+size_t TcScratch::size() {
+  std::lock_guard<std::mutex> lock(g_tiles_mu);
+  return bytes;
 }
 
 DeviceGuard::DeviceGuard(int dev) {

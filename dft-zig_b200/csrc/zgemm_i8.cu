@@ -863,11 +863,12 @@ static double i8_seconds(double M, double N, double K, double share_m, double sh
   return 64.0 * K * (M * share_m + N * share_n) / 4.5e12 + 64.0 * padded * K / 3.1e15 + 64.0 * M * N / 2e12 + 50e-6;
 }
 
-bool zgemm_i8_worthwhile(int M, int N, int K, double share_m, double share_n) {
-  if (!i8_enabled() || M <= 0 || N <= 0 || K < 64) return false;
+double zgemm_i8_gain(int M, int N, int K, double share_m, double share_n) {
+  if (!i8_enabled() || M <= 0 || N <= 0 || K < 64) return -1.0;
   const double dmma = 8.0 * ((M + 63) / 64 * 64.0) * ((N + 63) / 64 * 64.0) * K / 31e12 + 12e-6;
-  return i8_seconds(M, N, K, share_m, share_n) < dmma;
+  return dmma - i8_seconds(M, N, K, share_m, share_n);
 }
+bool zgemm_i8_worthwhile(int M, int N, int K, double share_m, double share_n) { return zgemm_i8_gain(M, N, K, share_m, share_n) > 0.0; }
 
 // The same against the split TF32 form (105 TFLOP/s with its own conversions), for the projector products.
 bool zgemm_i8_beats_split_tf32(int M, int N, int K, double share_m, double share_n) {
@@ -879,16 +880,27 @@ constexpr long kI8ChunkOut = 1L << 26;             // outputs whose residues are
 constexpr size_t kI8ResBytes = (size_t)2 << 30;    // over all splits in no more than this
 constexpr size_t kI8KeptBytes = (size_t)4 << 30;   // kept tiles of one operand
 
+// cudaMalloc and later cudaFree, measured: 0.4 ms to 256 MB, 0.85 at 1 GB, 1.5 at 4 GB.
+double alloc_seconds(size_t bytes) { return 0.4e-3 + 0.3e-12 * (double)bytes; }
+
+bool zgemm_i8_keep(int R, int K, int products, size_t have) {
+  const size_t need = zgemm_i8_cache_bytes(R, K);
+  return have >= need || products * 64.0 * (double)R * K / 4.5e12 >= alloc_seconds(need);
+}
+
 size_t zgemm_i8_cache_bytes(int R, int K) { return ((size_t)R * 4 + 255) / 256 * 256 + i8_tile_bytes(R, K); }
 
-int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, bool* done, const int** uneven) {
-  *done = false;
-  *uneven = nullptr;
+// How a product is cut up, and where its parts lie in the workspace.
+static size_t i8_up(size_t b) { return (b + 255) / 256 * 256; }
+static long i8_tile_n(long n) {
+  const long nt = (n + 255) / 256;
+  return (n + 32 * nt - 1) / (32 * nt) * 32;
+}
+// The MMA's M side pads to 256 rows, its N side to 32 per tile: the orientation with less padding, or, within
+// a tenth, the one whose N side is contiguous in the output.
+static GemmArgs i8_oriented(const GemmArgs& g0) {
   GemmArgs g = g0;
-  // The MMA's M side pads to 256 rows, its N side to 32 per tile: the orientation with less padding, or, within
-  // a tenth, the one whose N side is contiguous in the output.
-  auto tile_n = [](long n) { const long nt = (n + 255) / 256; return (n + 32 * nt - 1) / (32 * nt) * 32; };
-  auto padded = [&](long m, long n) { return (double)((m + 255) / 256 * 256) * ((n + tile_n(n) - 1) / tile_n(n) * tile_n(n)); };
+  auto padded = [](long m, long n) { return (double)((m + 255) / 256 * 256) * ((n + i8_tile_n(n) - 1) / i8_tile_n(n) * i8_tile_n(n)); };
   const double keep = padded(g0.M, g0.N) * (g0.ldo_c <= g0.ldo_r ? 1.0 : 1.1);
   const double turn = padded(g0.N, g0.M) * (g0.ldo_r <= g0.ldo_c ? 1.0 : 1.1);
   if (turn < keep) {
@@ -900,6 +912,67 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
     std::swap(g.ldo_r, g.ldo_c);
     std::swap(g.a_cache, g.b_cache);
   }
+  return g;
+}
+
+struct I8Plan {
+  long Kc, Mc, Nc;  // chunks: equal parts of K, then of the rows, so that the tiles held are bounded
+  int nk, kps, total_splits;
+  size_t o_exa, o_exb, o_part, o_even, o_flag, o_a, o_b, o_res, bytes;
+};
+// norm chunks: enough blocks to cover the latency of their loads
+static int i8_norm_chunks(bool kc, long R, long K) {
+  const long blocks = kc ? R : (R + 255) / 256, least = kc ? 2048 : 32;
+  return (int)std::max<long>(1, std::min<long>({64, K / least, (1184 + blocks - 1) / blocks}));
+}
+static I8Plan i8_plan(const GemmArgs& g) {
+  I8Plan p;
+  auto parts = [](long n, long most, long unit) {  // size of the equal parts of n, a multiple of unit
+    const long c = (n + most - 1) / most;
+    return std::min(n, ((n + c - 1) / c + unit - 1) / unit * unit);
+  };
+  p.Kc = parts(g.K, std::max<long>(8192, std::min<long>(I8_MAX_K, (long)(kI8ChunkElems / std::max(g.M, g.N)))), I8_KB);
+  // (65535 * 8 rows: the reconstruction's grid)
+  const long rmax = std::min<long>(65535L * 8 / 256 * 256, std::max<long>(256, (long)(kI8ChunkElems / p.Kc)));
+  p.Mc = parts(g.M, rmax, 256);
+  p.Nc = parts(g.N, std::min(rmax, std::max<long>(256, kI8ChunkOut / p.Mc)), 256);
+  p.nk = (int)((g.K + p.Kc - 1) / p.Kc);
+  const int KBc = (int)((p.Kc + I8_KB - 1) / I8_KB);
+  size_t res_bytes = 0;
+  for (;;) {
+    const int splits = i8_splits(p.Mc, p.Nc, KBc);
+    p.kps = (KBc + splits - 1) / splits;
+    p.total_splits = 0;
+    for (int k = 0; k < p.nk; ++k) {
+      const int kb = (int)((std::min<long>(p.Kc, g.K - k * p.Kc) + I8_KB - 1) / I8_KB);
+      p.total_splits += (kb + p.kps - 1) / p.kps;
+    }
+    res_bytes = (size_t)p.total_splits * I8_MODS * 2 * p.Mc * ((p.Nc + 255) / 256 * i8_tile_n(p.Nc));
+    if (res_bytes <= kI8ResBytes || (p.Mc <= 256 && p.Nc <= 256)) break;
+    long& longer = p.Mc >= p.Nc ? p.Mc : p.Nc;
+    longer = (longer / 2 + 255) / 256 * 256;
+  }
+  size_t off = 0;
+  auto take = [&](size_t b) { const size_t o = off; off += i8_up(b); return o; };
+  p.o_exa = take(4 * (size_t)g.M);
+  p.o_exb = take(4 * (size_t)g.N);
+  const size_t parts_max = std::max((size_t)i8_norm_chunks(g.a_kc, g.M, g.K) * g.M, (size_t)i8_norm_chunks(g.b_kc, g.N, g.K) * g.N);
+  p.o_part = take(sizeof(double2) * parts_max);
+  p.o_even = take(g.guard ? sizeof(I8Even) * parts_max : 0);
+  p.o_flag = take(g.guard ? sizeof(int) : 0);
+  p.o_a = take(g.a_cache ? 0 : i8_tile_bytes(p.Mc, p.Kc));
+  p.o_b = take(g.b_cache ? 0 : i8_tile_bytes(p.Nc, p.Kc));
+  p.o_res = take(res_bytes);
+  p.bytes = off;
+  return p;
+}
+
+size_t zgemm_i8_scratch_bytes(const GemmArgs& g) { return i8_plan(i8_oriented(g)).bytes; }
+
+int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, bool* done, const int** uneven) {
+  *done = false;
+  *uneven = nullptr;
+  GemmArgs g = i8_oriented(g0);
   const TilePins pins(scratch, g.a_cache, g.b_cache);
   // an operand whose kept tiles find no room is converted into the scratch
   auto room = [&](TcScratch*& cache, int R) {
@@ -908,48 +981,12 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
   };
   room(g.a_cache, g.M);
   room(g.b_cache, g.N);
-  // chunks: equal parts of K, then of the rows, so that the tiles held are bounded
-  auto parts = [](long n, long most, long unit) {  // size of the equal parts of n, a multiple of unit
-    const long c = (n + most - 1) / most;
-    return std::min(n, ((n + c - 1) / c + unit - 1) / unit * unit);
-  };
-  const long Kc = parts(g.K, std::max<long>(8192, std::min<long>(I8_MAX_K, (long)(kI8ChunkElems / std::max(g.M, g.N)))), I8_KB);
-  const long rmax = std::max<long>(256, (long)(kI8ChunkElems / Kc));
-  long Mc = parts(g.M, rmax, 256), Nc = parts(g.N, std::min(rmax, std::max<long>(256, kI8ChunkOut / Mc)), 256);
-  const int nk = (int)((g.K + Kc - 1) / Kc), KBc = (int)((Kc + I8_KB - 1) / I8_KB), KB = (g.K + I8_KB - 1) / I8_KB;
-  int kps = 0, total_splits = 0;
-  size_t res_bytes = 0;
-  for (;;) {
-    const int splits = i8_splits(Mc, Nc, KBc);
-    kps = (KBc + splits - 1) / splits;
-    total_splits = 0;
-    for (int k = 0; k < nk; ++k) {
-      const int kb = (int)((std::min<long>(Kc, g.K - k * Kc) + I8_KB - 1) / I8_KB);
-      total_splits += (kb + kps - 1) / kps;
-    }
-    res_bytes = (size_t)total_splits * I8_MODS * 2 * Mc * ((Nc + 255) / 256 * tile_n(Nc));
-    if (res_bytes <= kI8ResBytes || (Mc <= 256 && Nc <= 256)) break;
-    long& longer = Mc >= Nc ? Mc : Nc;
-    longer = (longer / 2 + 255) / 256 * 256;
-  }
-  if (total_splits > I8_MAX_SPLITS) return DFTCUDA_OK;
-  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  // norm chunks: enough blocks to cover the latency of their loads
-  auto norm_chunks = [&](bool kc, long R) {
-    const long blocks = kc ? R : (R + 255) / 256, least = kc ? 2048 : 32;
-    return (int)std::max<long>(1, std::min<long>({64, g.K / least, (1184 + blocks - 1) / blocks}));
-  };
-  size_t off = 0;
-  auto take = [&](size_t b) { const size_t o = off; off += up(b); return o; };
-  const size_t o_exa = take(4 * (size_t)g.M), o_exb = take(4 * (size_t)g.N);
-  const size_t parts_max = std::max((size_t)norm_chunks(g.a_kc, g.M) * g.M, (size_t)norm_chunks(g.b_kc, g.N) * g.N);
-  const size_t o_part = take(sizeof(double2) * parts_max), o_even = take(g.guard ? sizeof(I8Even) * parts_max : 0);
-  const size_t o_flag = take(g.guard ? sizeof(int) : 0);
-  const size_t o_a = take(g.a_cache ? 0 : i8_tile_bytes(Mc, Kc));
-  const size_t o_b = take(g.b_cache ? 0 : i8_tile_bytes(Nc, Kc));
-  const size_t o_res = take(res_bytes);
-  if (scratch->ensure(off, true) != DFTCUDA_OK) return DFTCUDA_OK;  // not done: the caller's other kernel runs
+  const I8Plan p = i8_plan(g);
+  if (p.total_splits > I8_MAX_SPLITS) return DFTCUDA_OK;
+  if (scratch->ensure(p.bytes, true) != DFTCUDA_OK) return DFTCUDA_OK;  // not done: the caller's other kernel runs
   unsigned char* base = static_cast<unsigned char*>(scratch->p);
+  const long Kc = p.Kc, Mc = p.Mc, Nc = p.Nc;
+  const int nk = p.nk, kps = p.kps, KB = (g.K + I8_KB - 1) / I8_KB;
 
   struct Op {
     const double2* X;
@@ -961,14 +998,14 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
     I8Tiles t;        // of the whole operand (cache) or of the current chunk
     long at_r, at_k;  // chunk held (no cache)
   };
-  int* flag = g.guard ? reinterpret_cast<int*>(base + o_flag) : nullptr;
+  int* flag = g.guard ? reinterpret_cast<int*>(base + p.o_flag) : nullptr;
   if (flag) DFT_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), s));
-  Op oa{g.A, g.lda, g.a_kc, g.conj_a, g.M, g.a_cache, (int*)(base + o_exa), {base + o_a, 0, 0}, -1, -1};
-  Op ob{g.B, g.ldb, g.b_kc, g.conj_b, g.N, g.b_cache, (int*)(base + o_exb), {base + o_b, 0, 0}, -1, -1};
+  Op oa{g.A, g.lda, g.a_kc, g.conj_a, g.M, g.a_cache, (int*)(base + p.o_exa), {base + p.o_a, 0, 0}, -1, -1};
+  Op ob{g.B, g.ldb, g.b_kc, g.conj_b, g.N, g.b_cache, (int*)(base + p.o_exb), {base + p.o_b, 0, 0}, -1, -1};
   auto exponents = [&](const Op& o) {
-    double2* part = reinterpret_cast<double2*>(base + o_part);
-    I8Even* even = g.guard ? reinterpret_cast<I8Even*>(base + o_even) : nullptr;
-    const int nch = norm_chunks(o.kc, o.R), unit = g.guard ? (o.kc ? 256 : 16) : 1;
+    double2* part = reinterpret_cast<double2*>(base + p.o_part);
+    I8Even* even = g.guard ? reinterpret_cast<I8Even*>(base + p.o_even) : nullptr;
+    const int nch = i8_norm_chunks(o.kc, o.R, g.K), unit = g.guard ? (o.kc ? 256 : 16) : 1;
     const int kchunk = (int)((((long)g.K + nch - 1) / nch + unit - 1) / unit * unit);
     const dim3 grid(o.kc ? (unsigned)o.R : ceil_div(o.R, 256), ceil_div(g.K, kchunk));
     if (even && o.kc) k_i8_norm_even<true><<<grid, 256, 0, s>>>(o.X, o.ld, o.R, g.K, kchunk, part, even);
@@ -998,7 +1035,7 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
     for (unsigned long long v : {(unsigned long long)(uintptr_t)o->X, (unsigned long long)o->ld, (unsigned long long)o->kc,
                                  (unsigned long long)o->cj, (unsigned long long)o->R, (unsigned long long)g.K})
       key = key * 1000003ULL ^ v;
-    const size_t head = up((size_t)o->R * 4);
+    const size_t head = i8_up((size_t)o->R * 4);
     const bool have = o->cache->valid && o->cache->key == key;
     o->ex = static_cast<int*>(o->cache->p);
     o->t.p = static_cast<unsigned char*>(o->cache->p) + head;
@@ -1019,7 +1056,7 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
       I8Gemm a{};
       a.M = rm; a.N = rn;
       a.mt = (rm + 255) / 256; a.nt = (rn + 255) / 256;
-      a.tn = (int)tile_n(rn);
+      a.tn = (int)i8_tile_n(rn);
       a.Npad = a.nt * a.tn;
       a.kps = kps;
       a.err = err;
@@ -1043,7 +1080,7 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
         }
         a.kblocks = (kn + I8_KB - 1) / I8_KB;
         a.splits = (a.kblocks + kps - 1) / kps;
-        a.out = base + o_res + (size_t)z * I8_MODS * 2 * rm * a.Npad;
+        a.out = base + p.o_res + (size_t)z * I8_MODS * 2 * rm * a.Npad;
         const int items = a.mt * a.nt * a.splits * I8_MODS * 2;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(2 * std::min(items, I8_PAIRS));
@@ -1064,7 +1101,7 @@ int zgemm_i8(const GemmArgs& g0, cudaStream_t s, TcScratch* scratch, int* err, b
       const bool tr = g.ldo_r < g.ldo_c;
       const dim3 grid = tr ? dim3(ceil_div(rn, 32), ceil_div(rm, 32)) : dim3(ceil_div(rn, 128), ceil_div(rm, 8));
       auto* kernel = tr ? (z == 1 ? k_i8_out<true, true> : k_i8_out<true, false>) : (z == 1 ? k_i8_out<false, true> : k_i8_out<false, false>);
-      kernel<<<grid, 256, 0, s>>>(base + o_res, rm, rn, a.Npad, z, oa.ex + m0, ob.ex + n0, o, g.ldo_r, g.ldo_c, g.alpha, g.beta, i8_scale(), z == 1 ? kI8Less : I8Less{0, 0}, flag);
+      kernel<<<grid, 256, 0, s>>>(base + p.o_res, rm, rn, a.Npad, z, oa.ex + m0, ob.ex + n0, o, g.ldo_r, g.ldo_c, g.alpha, g.beta, i8_scale(), z == 1 ? kI8Less : I8Less{0, 0}, flag);
       count_launch();
     }
   }

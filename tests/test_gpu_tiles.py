@@ -95,3 +95,20 @@ def test_projectors_set_anew_on_a_used_context(dz, precision, sizes):
         assert float((got - want).abs().max()) <= tol * float(want.abs().max())
     fresh.close()
     kc.close()
+
+
+def test_first_products_keep_no_tiles(dz):
+    """A context's first products convert the projectors in the workspace; the tiles of either product are kept, at different
+    calls, once the conversions seen have cost what their buffers do.  Results do not depend on which it was."""
+    kp, kc = _with_projectors(dz, 512)
+    x = torch.from_numpy(random_block(kp.ctx.n, 500, 7)).cuda()
+    y = torch.empty_like(x)
+    want = kc.apply_hamiltonian_batched(x, y).clone()
+    used = [-_free()]
+    for _ in range(24):
+        assert float((kc.apply_hamiltonian_batched(x, y) - want).abs().max()) <= 1e-13 * float(want.abs().max())
+        used.append(-_free())
+    tiles = 512 * 5 * kp.ctx.n * 32  # of one product
+    grown = [b - a for a, b in zip(used, used[1:])]
+    assert sum(g > tiles // 2 for g in grown) == 2 and not any(g > 1.5 * tiles for g in grown) and grown[0] < tiles // 2
+    kc.close()
