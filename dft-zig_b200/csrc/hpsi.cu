@@ -389,6 +389,7 @@ static int projector_product(dftcuda_kctx* c, GemmArgs& g, bool back, size_t nco
   const bool full = tiles.full(), tc = precision_uses_tc(c->precision);
   const bool keep = tc || full || zgemm_i8_keep(back ? g.N : g.M, g.K, seen - (back ? 1 : 0), tiles.size());
   (back ? g.b_share : g.a_share) = tc || full ? 0.0 : keep ? 1.0 / (1.0 + seen) : 1.0;
+  c->p_i8[back] = false;
   if (projectors_on_tf32(c, g)) {
     (back ? g.b_cache : g.a_cache) = back ? &c->tc_ptiles_back : &c->tc_ptiles_proj;
     DFT_TRY(kctx_ensure_gemm_ws(c, ncols));
@@ -403,6 +404,7 @@ static int projector_product(dftcuda_kctx* c, GemmArgs& g, bool back, size_t nco
     const int* uneven = nullptr;
     c->err_used = true;
     DFT_TRY(zgemm_i8(g, s, &c->tc_scratch, c->d_err, &done, &uneven));
+    c->p_i8[back] = done;
     if (done) return DFTCUDA_OK;
   }
   DFT_TRY(kctx_ensure_gemm_ws(c, ncols));

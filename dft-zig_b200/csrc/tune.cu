@@ -4,7 +4,8 @@
 //   1. FFT passes: four-step register kernels (local4.cu) or the generic shared-memory passes;
 //   2. the box workspace budget that sets how many columns one chunk of FFT passes carries
 //      (L2 residency of the active-plane workspace against launch count);
-//   3. split-K of the projection GEMM; 4. split-K of the back-projection GEMM.
+//   3. split-K of the projection GEMM; 4. split-K of the back-projection GEMM (either only where the
+//   product does not run on residues, which take their own split).
 // The reference sizes its FFT plans and BLAS calls once and never measures; here the shapes of
 // every cell and k-point differ (uneven n_pw, box sizes 20^3 ... 108^3), so they are measured.
 #include <algorithm>
@@ -75,6 +76,8 @@ extern "C" int dftcuda_kctx_autotune(dftcuda_kctx* c, size_t ncols, dftcuda_tune
     ++evaluated;
     return DFTCUDA_OK;
   };
+  // dozens of products follow: whatever the context keeps of its projectors is kept from the first warm-up on
+  for (int& products : c->p_products) products += 64;
   double best = 0.0;
   st = measure(&best);
   const double default_ms = best;
@@ -122,6 +125,10 @@ extern "C" int dftcuda_kctx_autotune(dftcuda_kctx* c, size_t ncols, dftcuda_tune
   if (st == DFTCUDA_OK && c->nl.nproj > 0) {
     for (int which = 0; which < 2 && st == DFTCUDA_OK; ++which) {
       int& knob = which == 0 ? c->split_proj : c->split_back;
+      if (c->p_i8[which]) {
+        knob = 0;
+        continue;
+      }
       const int keep = knob;
       int pick = keep;
       // the back-projection (M = columns, N = n_pw) already fills the GPU with output tiles: only

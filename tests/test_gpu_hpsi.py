@@ -219,6 +219,19 @@ def test_autotune_keeps_results(dz):
     kc.close()
 
 
+def test_autotune_leaves_out_splits_that_no_kernel_reads(dz):
+    """Projector products on residues choose their own split: no candidates for them, and none reported."""
+    kp = kproblem("si8", 25.0, (0.25, 0.0, 0.0))
+    kc = make_context(dz, kp)
+    few = kc.autotune(8)  # both products on the FP64 kernel: eight candidates more
+    rng = np.random.default_rng(3)
+    phi = rng.normal(size=(5, kp.ctx.n)) * np.exp(-0.1 * kp.ctx.basis.kinetic)
+    kc.set_projectors([dz.SpeciesProjectors([0, 0, 1], 0.1 * np.eye(3), phi)], np.zeros(512, dtype=np.int32), rng.uniform(0, 10.0, (512, 3)))
+    many = kc.autotune(500)
+    assert many["candidates"] == few["candidates"] - 8 and many["proj_splits"] == many["back_splits"] == 0
+    kc.close()
+
+
 @pytest.mark.parametrize("name,ecut,k", [("si8", 15.0, (0.25, 0.0, 0.125)), ("al4", 15.0, (0.1, 0.2, 0.3))])
 def test_hamiltonian_is_hermitian(dz, name, ecut, k):
     """The reference's Hamiltonian Hermiticity test (src/tests.zig:765-831) on the device operator:
