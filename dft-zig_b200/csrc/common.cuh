@@ -67,8 +67,9 @@ inline int fail(int status, const std::string& msg) {
 
 inline unsigned ceil_div(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }
 
-// Count of kernels this library has launched (all contexts); every launch site calls count_launch().
-uint64_t launches_total();
+// Count of kernels this library has launched from the calling thread (runs of a batch are issued by several); every
+// launch site calls count_launch().
+uint64_t launches_here();
 void count_launch(int n = 1);
 
 // Every device allocation of the library goes through dev_malloc.  dftcuda_debug_fail_alloc(k) makes

@@ -294,14 +294,14 @@ struct ProfScope {
     if (!c->prof.on) return;
     a = c->prof.take();
     cudaEventRecord(a, s);
-    l0 = launches_total();
+    l0 = launches_here();
   }
   void stop() {
     if (!a) return;
     cudaEvent_t b = c->prof.take();
     cudaEventRecord(b, s);
     c->prof.pending.push_back({cat, a, b});
-    c->prof.launches[cat] += launches_total() - l0;
+    c->prof.launches[cat] += launches_here() - l0;
     a = nullptr;
   }
   ~ProfScope() { stop(); }

@@ -11,9 +11,9 @@
 
 namespace dftcuda {
 
-static std::atomic<uint64_t> g_launches{0};
-uint64_t launches_total() { return g_launches.load(std::memory_order_relaxed); }
-void count_launch(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
+static thread_local uint64_t t_launches = 0;
+uint64_t launches_here() { return t_launches; }
+void count_launch(int n) { t_launches += (uint64_t)n; }
 
 cudaEvent_t Profiler::take() {
   if (!pool.empty()) {

@@ -134,6 +134,25 @@ def test_batch_matches_independent_solves(dz):
         assert np.abs(b.values - dense).max() < 1e-7
 
 
+def test_profile_of_a_batch_counts_each_run_alone(dz):
+    """A batch's runs are issued by several host threads: each context's profile counts its own launches."""
+    kps = [kproblem("si8", 12.0, (0.1 * i, 0.25, 0.0)) for i in range(6)]
+    opts = dz.Options(max_iter=5, tol=1e-12)
+
+    def launches(batches):
+        ctxs = [make_context(dz, kp) for kp in kps]
+        for kc in ctxs:
+            kc.set_profiling()
+        for at in batches:
+            dz.hermitian_eigen_decomp_iterative_batch([ctxs[i] for i in at], [kps[i].ctx.basis.kinetic for i in at], 16, opts)
+        got = [kc.profile()["kernel_launches"] for kc in ctxs]
+        for kc in ctxs:
+            kc.close()
+        return got
+
+    assert launches([range(6)]) == launches([[i] for i in range(6)])
+
+
 def test_large_block_uses_panel_cholesky(dz):
     """100 bands: 104-column Davidson blocks go through the panel Cholesky (GEMM trailing updates);
     eigenvalues against dense diagonalisation."""
