@@ -26,6 +26,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <system_error>
 #include <vector>
 
 #include "kctx.cuh"
@@ -1031,9 +1032,17 @@ static int issue_threads(size_t nruns) {
 // fn(run) for every run, on up to issue_threads() host threads (dynamic assignment).
 template <typename F>
 static void for_each_run(std::vector<EigRun>& runs, F&& fn) {
+  // no exception may leave a worker thread, or the C entry point
+  auto guarded = [&](EigRun& r) {
+    try {
+      fn(r);
+    } catch (const std::exception& e) {
+      r.status = fail(DFTCUDA_ERR_OUT_OF_MEMORY, std::string("eig_solve: ") + e.what());
+    }
+  };
   const int nt = issue_threads(runs.size());
   if (nt <= 1) {
-    for (EigRun& r : runs) fn(r);
+    for (EigRun& r : runs) guarded(r);
     return;
   }
   int dev = 0;
@@ -1044,13 +1053,16 @@ static void for_each_run(std::vector<EigRun>& runs, F&& fn) {
     for (size_t i; (i = next.fetch_add(1)) < runs.size();) {
       EigRun& r = runs[i];
       const int before = r.status;
-      fn(r);
+      guarded(r);
       if (before == DFTCUDA_OK && r.status != DFTCUDA_OK) r.err_msg = dftcuda_last_error_message();
     }
   };
   std::vector<std::thread> th;
   th.reserve(nt - 1);
-  for (int t = 1; t < nt; ++t) th.emplace_back(work);
+  try {
+    for (int t = 1; t < nt; ++t) th.emplace_back(work);
+  } catch (const std::system_error&) {  // no more threads to be had: those that started and this one do it
+  }
   work();
   for (std::thread& t : th) t.join();
 }

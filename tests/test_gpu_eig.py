@@ -134,6 +134,38 @@ def test_batch_matches_independent_solves(dz):
         assert np.abs(b.values - dense).max() < 1e-7
 
 
+NO_THREADS = """
+import ctypes, sys
+sys.path.insert(0, {root!r})
+import dftzig_loader
+from tests.helpers import kproblem, make_context
+dz = dftzig_loader.load()
+kps = [kproblem("si2", 10.0, (0.1 * i, 0.25, 0.0)) for i in range(4)]
+ctxs = [make_context(dz, kp) for kp in kps]
+kin = [kp.ctx.basis.kinetic for kp in kps]
+first = dz.hermitian_eigen_decomp_iterative_batch(ctxs, kin, 4)
+libc = ctypes.CDLL(None)
+attr = ctypes.create_string_buffer(256)
+libc.pthread_attr_init(attr)
+libc.pthread_attr_setstacksize(attr, ctypes.c_size_t(1 << 46))  # more than there is address space for
+assert libc.pthread_setattr_default_np(attr) == 0
+again = dz.hermitian_eigen_decomp_iterative_batch(ctxs, kin, 4)
+assert max(abs(a.values - b.values).max() for a, b in zip(first, again)) < 1e-9
+"""
+
+
+def test_batch_without_threads_to_start():
+    """Where the host has no thread to give, the batch is issued with those it has (in a process of its own: the default
+    stack size that keeps threads from starting is the process's)."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", NO_THREADS.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_profile_of_a_batch_counts_each_run_alone(dz):
     """A batch's runs are issued by several host threads: each context's profile counts its own launches."""
     kps = [kproblem("si8", 12.0, (0.1 * i, 0.25, 0.0)) for i in range(6)]
