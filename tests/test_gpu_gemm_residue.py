@@ -1,9 +1,9 @@
 """The FP64 complex GEMM's residue form (csrc/zgemm_i8.cu) at the edges of its tiles.
 
 Entries are integers of at most 11 bits, so torch's complex128 product is exact and every difference is
-the residue form's own.  Its entries are then exact too, which leaves the reconstruction (32 coefficients
-cut at 76 bits times residue sums below 2^9 P, P = 2^117.7: 2^54.6 against scaled norms of at least 2^57
-each, so 2^-59 |a||b|) and four roundings of the result: 2^-58 |a||b| + 2^-51 |c| bounds both.  Where the
+the residue form's own.  Its entries are then exact too, which leaves the reconstruction (16 coefficients
+cut at 76 bits for either part, times numbers below 2 p of moduli of sum 2736: 2^(12.5 - 76) P, P = 2^117.7, so 2^54.2
+against scaled norms of at least 2^57 each: 2^-59 |a||b|) and four roundings of the result: 2^-58 |a||b| + 2^-51 |c| bounds both.  Where the
 squares of a row leave the range its norm is bounded by sqrt(2 K) times the largest entry, up to 2^3.4
 above the norm here: 2^-54 |a||b|."""
 import numpy as np
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _ints(rows, k, kc, gen):
-    x = torch.randint(-1024, 1025, (rows, k, 2), generator=gen).double()
+    x = torch.randint(-1024, 1025, (rows, k, 2), generator=gen, device=gen.device).double()
     x = torch.view_as_complex(x).cuda()
     return x if kc else x.T.contiguous().T
 
@@ -24,18 +24,34 @@ def _bound(a, b, ref, bits=58):
     return 2.0 ** -bits * na[:, None] * nb[None, :] + 2.0 ** -51 * ref.abs()
 
 
-# rows around the 128- and 256-row tiles and the 8-row groups, columns around 32 and 256, K around the
-# 64-deep blocks, the 128-deep slots and the K chunks
-SHAPES = [(256, 256, 3008), (257, 255, 3009), (129, 1025, 2047), (32, 4000, 1500), (513, 33, 16385), (700, 320, 1087), (2000, 96, 1056),
-          (40, 140, 40000), (131200, 33, 264)]
+def _assert_on_residues(dz, M, N, K, akc, bkc):
+    """That products of this size run in the residue form: on random rows its error (2^-59 |a||b|) is below that of
+    FP64 sums, which a corner of the same product takes, cut into up to 64 short sums (0.1 to 0.65 of it; the sums of the
+    whole product are longer)."""
+    rng = np.random.default_rng(M + N + K)
+    a, b = (torch.randn((n, K) if kc else (K, n), dtype=torch.complex128, device="cuda", generator=torch.Generator("cuda").manual_seed(int(rng.integers(1 << 30))))
+            for n, kc in ((M, akc), (N, bkc)))
+    a, b = a if akc else a.T, b if bkc else b.T
+    out, plain = dz.complex_gemm(a, b)[:32, :32].cpu().numpy(), dz.complex_gemm(a[:32], b[:32]).cpu().numpy()
+    want = a[:32].cpu().numpy().astype(np.clongdouble) @ b[:32].cpu().numpy().astype(np.clongdouble).T
+    err, err0 = (np.linalg.norm((x - want).astype(complex)) for x in (out, plain))
+    assert err < 0.8 * err0, (err, err0)
+
+
+# above the line of the size rule: rows around the 128- and 256-row tiles and the 8-row groups, columns around 32 and
+# 256, K around the 64-deep blocks and the 128-deep slots; several K chunks, row chunks and output chunks
+SHAPES = [(256, 256, 6016), (257, 255, 6017), (257, 513, 6001), (129, 1025, 2047), (1000, 97, 20000), (4000, 130, 1500), (513, 320, 16385),
+          (700, 640, 1087), (2000, 224, 1056), (136, 300, 40000), (385, 289, 3073), (5000, 130, 8190), (600, 513, 60001), (1025, 1030, 33001),
+          (131200, 520, 264)]
 
 
 @pytest.mark.parametrize("M,N,K", SHAPES)
 @pytest.mark.parametrize("akc,bkc,cja,cjb", [(1, 1, 1, 0), (1, 0, 0, 0), (0, 0, 0, 1), (0, 1, 1, 1)])
 def test_exact_on_integers(dz, M, N, K, akc, bkc, cja, cjb):
-    gen = torch.Generator().manual_seed(M + 3 * N + 7 * K)
+    _assert_on_residues(dz, M, N, K, akc, bkc)
+    gen = torch.Generator("cuda").manual_seed(M + 3 * N + 7 * K)
     a, b = _ints(M, K, akc, gen), _ints(N, K, bkc, gen)
-    o0 = torch.randint(-8, 9, (M, N), generator=gen).to(torch.complex128).cuda()
+    o0 = torch.randint(-8, 9, (M, N), generator=gen, device="cuda").to(torch.complex128)
     ref = 2.0 * ((a.conj() if cja else a) @ (b.conj() if cjb else b).T) - o0
     for rowmajor in (True, False):
         out = o0.clone() if rowmajor else o0.T.contiguous().T
@@ -44,9 +60,10 @@ def test_exact_on_integers(dz, M, N, K, akc, bkc, cja, cjb):
 
 
 def test_padded_strides(dz):
+    _assert_on_residues(dz, 330, 300, 6000, 1, 0)
     gen = torch.Generator().manual_seed(5)
-    a = _ints(330, 2100, True, gen)[:, 17:2017]
-    b = _ints(2100, 310, False, gen)[50:2050].T[:300]
+    a = _ints(330, 6100, True, gen)[:, 17:6017]
+    b = _ints(6100, 310, False, gen)[50:6050].T[:300]
     out = torch.zeros(330, 640, dtype=torch.complex128, device="cuda")[:, 5:605:2]
     dz.complex_gemm(a, b, out)
     ref = a @ b.T
@@ -103,18 +120,48 @@ def test_without_room_for_the_tiles(dz):
 
 
 def test_not_less_exact_than_the_dmma_kernel(dz):
-    """Against a double-double product, on band-like columns and on random ones: no further off than the
-    FP64 tensor-core sums of the same product."""
+    """Against a double-double product: random columns (residues) are no further off than the FP64 tensor-core sums of eight
+    columns of the product; band-like ones (uneven rows) keep FP64 sums, a few 2^-53 sqrt(K) of sum |a_k||b_k|."""
     rng = np.random.default_rng(3)
     K = 20000
-    for envelope in (np.ones(K), 1.0 / (1.0 + np.linspace(0, 25, K)) ** 1.5):
-        a = (rng.normal(size=(64, K)) + 1j * rng.normal(size=(64, K))) * envelope
-        b = (rng.normal(size=(160, K)) + 1j * rng.normal(size=(160, K))) * envelope
-        want = a.astype(np.clongdouble) @ b[:8].astype(np.clongdouble).T
+    _assert_on_residues(dz, 160, 200, K, 1, 1)
+    for envelope in (None, 1.0 / (1.0 + np.linspace(0, 25, K)) ** 1.5):
+        a, b = (rng.normal(size=(n, K)) + 1j * rng.normal(size=(n, K)) for n in (160, 200))
+        if envelope is not None:
+            a, b = a * envelope, b * envelope
+        want = (a.astype(np.clongdouble) @ b[:8].astype(np.clongdouble).T).astype(complex)
         out = dz.complex_gemm(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()).cpu().numpy()[:, :8]
-        plain = dz.complex_gemm(torch.from_numpy(a[:, :]).cuda(), torch.from_numpy(b[:8]).cuda()).cpu().numpy()  # 8 columns: the DMMA kernel
-        err, err0 = (np.linalg.norm((x - want).astype(complex)) for x in (out, plain))
-        assert err <= 1.05 * err0, (err, err0)
+        if envelope is None:
+            plain = dz.complex_gemm(torch.from_numpy(a).cuda(), torch.from_numpy(b[:8]).cuda()).cpu().numpy()
+            assert np.linalg.norm(out - want) <= 1.05 * np.linalg.norm(plain - want)
+        else:
+            assert (np.abs(out - want) <= 4 * K ** 0.5 * 2.0 ** -53 * (np.abs(a) @ np.abs(b[:8]).T)).all()
+
+
+def test_projector_products_on_band_like_columns(dz):
+    """A context's projector products take the residue form with whatever rows they have.  Its energies of 500 bands against
+    those of 8 at a time (FP64 sums): the coefficients may differ by 2^-54 |P||x| of each, so E = 0.1 sum |c|^2 / Omega by
+    2 * 2^-54 sqrt(rows) |P||x| |c| of 0.1 / Omega, with the largest row's |P|."""
+    from tests.helpers import kproblem, make_context
+
+    kp = kproblem("si8", 25.0, (0.25, 0.0, 0.0))
+    kc = make_context(dz, kp)
+    rng = np.random.default_rng(5)
+    kin, n, rows = kp.ctx.basis.kinetic, kp.ctx.n, 5 * 512
+    phi = rng.normal(size=(5, n)) * np.exp(-0.1 * kin)
+    kc.set_projectors([dz.SpeciesProjectors([0, 0, 1], 0.1 * np.eye(3), phi)], np.zeros(512, dtype=np.int32), rng.uniform(0, 10.0, (512, 3)))
+    size = np.linalg.norm(phi, axis=1).max()
+    plain = (rng.normal(size=(500, n)) + 1j * rng.normal(size=(500, n)))
+    steep = plain * np.exp(-0.4 * kin)
+    spike = plain / (1.0 + kin) ** 1.5
+    spike[:, np.argmax(kin)] *= 1e6
+    for x in (plain, plain / (1.0 + kin) ** 1.5, steep, spike):
+        got = kc.nonlocal_energies(x)
+        want = np.concatenate([kc.nonlocal_energies(x[i : i + 8]) for i in range(0, 500, 8)])
+        c = np.sqrt(want * kp.grid.volume / 0.1)
+        bound = 0.1 / kp.grid.volume * 2 * 2.0 ** -54 * rows ** 0.5 * size * np.linalg.norm(x, axis=1) * c + 1e-14 * want
+        assert (np.abs(got - want) <= bound).all(), (np.abs(got - want) / bound).max()
+    kc.close()
 
 
 def test_many_k_splits(dz):
@@ -164,17 +211,3 @@ def test_uneven_rows_keep_64_bit_sums(dz, kind, akc, bkc):
     want = (a[:20].astype(np.clongdouble) @ b[::50].astype(np.clongdouble).T).astype(complex)
     size = np.abs(a[:20]) @ np.abs(b[::50]).T
     assert (np.abs(out[at] - want) <= 4 * 4000 ** 0.5 * 2.0 ** -53 * size).all()
-
-
-@pytest.mark.parametrize("akc,bkc", [(1, 1), (0, 0)])
-@pytest.mark.parametrize("M,N,K", [(300, 400, 4000), (129, 1025, 2047), (330, 300, 6007)])
-def test_even_rows_run_on_residues(dz, M, N, K, akc, bkc):
-    """Random rows stay in the residue form, whose error (2^-59 |a||b|) is far below the FP64 sums'."""
-    rng = np.random.default_rng(22)
-    a, b = (rng.normal(size=(n, K)) + 1j * rng.normal(size=(n, K)) for n in (M, N))
-    da, db = _layout(a, akc), _layout(b, bkc)
-    out = dz.complex_gemm(da, db).cpu().numpy()[:, :8]
-    plain = dz.complex_gemm(da, db[:8]).cpu().numpy()  # too few columns: the FP64 kernel
-    want = a.astype(np.clongdouble) @ b[:8].astype(np.clongdouble).T
-    err, err0 = (np.linalg.norm((x - want).astype(complex)) for x in (out, plain))
-    assert err < 0.5 * err0, (err, err0)
