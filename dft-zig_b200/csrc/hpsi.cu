@@ -379,8 +379,7 @@ static GemmArgs back_projection(const dftcuda_kctx* c, double2* y, size_t ncols)
 // projectors' tiles are kept only when the conversions seen have cost what their buffer does (zgemm_i8_keep; the
 // back-projection's one product later, so that no call allocates both).  64 atoms at 30 Ry, 164 columns, us a call
 // on a fresh context: FP64 tensor cores alone 2,640 then 2,160; with all buffers allocated and converted by the first
-// call 4,540 then 1,585; now 2,330,
-// then 1,830, from the eighth call on 1,585 (a cudaMalloc of 0.4 ms hides behind the local passes).
+// call 4,540 then 1,585; now 2,340 1,840 1,850 1,730 1,585 (a cudaMalloc of 0.4 ms hides behind the local passes).
 // TF32X3 contexts keep tiles from the first product on, whichever form serves it, so that its accuracy does not depend on
 // the call.
 static int projector_product(dftcuda_kctx* c, GemmArgs& g, bool back, size_t ncols, cudaStream_t s) {
