@@ -229,7 +229,7 @@ __device__ __forceinline__ void plane_y_inverse(const cplx<T>* Srow, const int* 
 // one row at a time is in registers and the lines can take the split that keeps the lanes busy (XSplit).  The
 // four-step twiddles sit in shared memory in the order the lanes read them.  Bound by shared memory / L1
 // wavefronts (68 % busy) at 12 warps per SM.  108^3, 452 columns: 9.65 ms with the exchange out of place, all of
-// a lane's rows in registers and the sticks scattered and gathered in passes of their own; 7.2 ms now.
+// a lane's rows in registers and the sticks scattered and gathered in passes of their own; 6.95 ms now.
 template <typename T, int N>
 __global__ void __launch_bounds__(plane_max_warps<T>() * 32, 1) k_zplane(cplx<T>* __restrict__ S, int n_st, const int* __restrict__ st_of,
                                                                      int n_act, const int* __restrict__ slot_of_x,
@@ -485,10 +485,15 @@ static int plane_warps_rt(size_t cs, int n, int n_act) {
 }
 
 // Layout choice at context creation: DFTCUDA_LOCAL=planes or =sticks forces one; by default the
-// stick layout serves boxes from 96 points along x on (Si216, 108^3: measured before the passes of either took
-// their present form, 12.0 against 14.2 ms per 452-column FP64 block) and the plane layout smaller ones
-// (Si64, 75^3, 164 columns of H|psi>: 1,775 us on sticks, 1,781 on planes before and 1,570 after that layout's
-// x lines went in place).  The autotuner times both either way.
+// stick layout serves boxes from 96 points along x on and the plane layout smaller ones.  H|psi> without projectors, cubic
+// boxes with a sphere of a quarter of their width, 160 columns, us, planes / sticks in FP64 and in FP32:
+//   60  619 /  765   393 /  391     90  2192 / 2256  1184 / 1090
+//   64  749 /  574   399 /  341     96  2690 / 2335  1381 / 1288
+//   72 1018 / 1120   631 /  545    100  3520 / 2773  1978 / 1585
+//   75 1200 / 1531   683 /  768    108  4058 / 4009  2187 / 2138
+//   80 1997 / 1700   885 /  849    120  5943 / 4878  3160 / 2540
+// Below 96 the splits of the lengths decide (64 and 80 do better on sticks, the autotuner finds them).  The density of the same
+// blocks is the faster on planes at 100 and 108 (1646 / 2027, 2047 / 2277 in FP64).
 static int local_layout_env() {
   const char* e = std::getenv("DFTCUDA_LOCAL");
   if (e && std::string(e) == "planes") return 1;

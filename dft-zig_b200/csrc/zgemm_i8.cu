@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(256) k_i8_tiles(const double2* __restrict__ X,
 // single-CTA 128 x 256 tile would.  Bound by the tensor pipe (88 % busy at 864 x 452 x 30784, L2 at 56 %).  TMEM holds two accumulators: eight
 // warps reduce a finished one to residues while the next item's MMAs run.  The producing and issuing warps run
 // their loops with all lanes and elect one for the copies and MMAs: from inside a divergent branch the same
-// loop took three times as long.  1344 x 448 x 61565 (a sixth of its tiles padding): 0.88 ms, 2.7e15 useful
+// loop took three times as long.  1344 x 448 x 61565 (an eighth of its work padding): 0.88 ms, 2.7e15 useful
 // operations/s of 4.5e15 nominal; the single-CTA form with four products per complex one took 2.0 ms.
 constexpr int I8_STAGES = 6;
 constexpr int I8_HALF = 128 * I8_KB;  // bytes of 128 rows of a K block

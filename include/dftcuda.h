@@ -40,13 +40,16 @@ extern "C" {
 #define DFTCUDA_ERR_TIMEOUT (-8)             /* a bounded device wait gave up (no reference counterpart) */
 
 /* Arithmetic of one k-point context's H|psi>:
- *  FP64    every pass in FP64;
+ *  FP64    every pass in FP64.  Large products with the projectors and of the eigensolver's blocks hold their rows in
+ *          fixed point at 2^-58 of their norm and multiply exactly on the int8 tensor cores: an error of about
+ *          2^-59 |a||b| per output, below that of 64-bit sums for such rows.  A row with an infinity or a NaN gives
+ *          NaN in all of its output row or column, and in no other;
  *  FP32    local-potential FFT passes in FP32, projector GEMMs in FP64;
  *  TF32    FFT passes in FP32 and the projector GEMMs on the tensor cores (tcgen05 kind::tf32, FP32
  *          accumulation in TMEM); relative error ~1e-3;
  *  TF32X3  as TF32 with every operand split into two TF32 parts (hi + lo, three MMAs per real
  *          product): FP32-class accuracy (~1e-6) on the tensor cores.  Projector GEMMs that the
- *          FP64 form serves in less time (its exact int8 products) take that form.
+ *          FP64 form's int8 products serve in less time take those.
  * Wavefunctions are FP64 at the boundary in every mode.  In TF32 and TF32X3 contexts every
  * eigensolver subspace product (V^H W, V C, W C, the orthonormalisation's projections and block
  * overlaps) uses the same tensor-core GEMM (split form); the Cholesky factorisations, the subspace
