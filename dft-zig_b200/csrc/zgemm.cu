@@ -520,7 +520,8 @@ int zgemm(const GemmArgs& g0, cudaStream_t s, double2* ws, size_t ws_elems) {
     // out = beta * out
     return fail(DFTCUDA_ERR_INVALID_ARGUMENT, "zgemm: K must be positive");
   }
-  const int* gate = nullptr;
+  const int* gate = nullptr;  // in the residue form's workspace, which stays until the gated kernels are enqueued
+  const TilePins pins(g.i8, nullptr, nullptr);
   if (g.i8 && g.err && zgemm_i8_worthwhile(g.M, g.N, g.K, g.a_share, g.b_share)) {
     bool done = false;
     DFT_TRY(zgemm_i8(g, s, g.i8, g.err, &done, &gate));
