@@ -878,7 +878,7 @@ bool zgemm_i8_beats_split_tf32(int M, int N, int K, double share_m, double share
 constexpr size_t kI8ChunkElems = (size_t)1 << 25;  // entries of one operand whose tiles are held at a time (1 GB)
 constexpr long kI8ChunkOut = 1L << 26;             // outputs whose residues are held at a time,
 constexpr size_t kI8ResBytes = (size_t)2 << 30;    // over all splits in no more than this
-constexpr size_t kI8KeptBytes = (size_t)4 << 30;   // kept tiles of one operand
+constexpr size_t kI8KeptBytes = (size_t)16 << 30;  // kept tiles of one operand (512 atoms at 25 Ry: 12 GB a role)
 
 // cudaMalloc and later cudaFree, measured: 0.4 ms to 256 MB, 0.85 at 1 GB, 1.5 at 4 GB.
 double alloc_seconds(size_t bytes) { return 0.4e-3 + 0.3e-12 * (double)bytes; }
