@@ -895,11 +895,17 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(const double* __restrict__
   extern __shared__ double ism[];
   const int j = blockIdx.x, lane = threadIdx.x;
   if (j >= nev) return;
-  const double tnorm = fmax(*tnorm_p, DBL_MIN);
+  // T and its eigenvalues times a power of two that brings ||T|| near one, so that neither the reciprocal of the pivot
+  // threshold nor the vectors' squares leave the range; ||T|| = 0: every pivot is the threshold
+  double tnorm = *tnorm_p;
+  int ex = 0;
+  if (tnorm > 0.0) frexp(tnorm, &ex);
+  const double sc = scalbn(1.0, -max(ex, -1000));
+  tnorm = tnorm > 0.0 ? tnorm * sc : 1.0;
   const double gtol = kGroupTol * tnorm;
-  if (j > 0 && !(w[j] - w[j - 1] > gtol)) return;
+  if (j > 0 && !((w[j] - w[j - 1]) * sc > gtol)) return;
   int jend = j + 1;
-  while (jend < nev && !(w[jend] - w[jend - 1] > gtol)) ++jend;
+  while (jend < nev && !((w[jend] - w[jend - 1]) * sc > gtol)) ++jend;
   double* const rp = ism;      // 1 / U's diagonal
   double* const u1 = rp + m;   // U's first superdiagonal
   double* const u2 = u1 + m;   // U's second superdiagonal (nonzero after a row swap)
@@ -911,7 +917,7 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(const double* __restrict__
     const double lam = w[p];
     if (lane == 0) {
       // Row-pivoted elimination of T - lam I.  (a, b): the running row at columns (i, i+1).
-      double a = dd[0] - lam, b = m > 1 ? ee[0] : 0.0;
+      double a = (dd[0] - lam) * sc, b = m > 1 ? ee[0] * sc : 0.0;
       for (int i0 = 0; i0 + 1 < m; i0 += kIvChunk) {
         const int n = min(kIvChunk, m - 1 - i0);
         double sb[kIvChunk], dn[kIvChunk], up[kIvChunk];
@@ -919,9 +925,9 @@ __global__ void __launch_bounds__(32) k_tridiag_invit(const double* __restrict__
         for (int c = 0; c < kIvChunk; ++c) {
           if (c < n) {
             const int i = i0 + c;
-            sb[c] = __ldg(ee + i);
-            dn[c] = __ldg(dd + i + 1) - lam;
-            up[c] = i + 2 < m ? __ldg(ee + i + 1) : 0.0;
+            sb[c] = __ldg(ee + i) * sc;
+            dn[c] = (__ldg(dd + i + 1) - lam) * sc;
+            up[c] = i + 2 < m ? __ldg(ee + i + 1) * sc : 0.0;
           }
         }
 #pragma unroll

@@ -32,6 +32,16 @@ def test_lobpcg_diagonal_kats(dz, case):
     kc.close()
 
 
+@pytest.mark.parametrize("diag,nbands", [([0.0], 1), ([0.0] * 4, 2), ([0.0, 0.0, 1.0], 3)])
+def test_operator_with_zero_levels(dz, diag, nbands):
+    """One plane wave at Gamma, and subspaces whose matrix is zero: unit, orthogonal vectors all the same."""
+    kc = _diag_context(dz, diag)
+    r = kc.hermitian_eigen_decomp_iterative(np.array(diag), nbands, dz.Options(max_iter=20, tol=1e-9))
+    assert np.abs(r.values - np.sort(diag)[:nbands]).max() < 1e-12
+    assert np.abs(r.vectors.conj() @ r.vectors.T - np.eye(nbands)).max() < 1e-10
+    kc.close()
+
+
 @pytest.mark.parametrize("k", [(0.0, 0.0, 0.0), (0.25, 0.125, 0.0), (0.5, 0.25, 0.75)])
 def test_si2_eigenvalues_match_oracle(dz, k):
     kp = kproblem("si2", 20.0, k)

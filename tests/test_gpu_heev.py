@@ -4,6 +4,7 @@ one-CTA Jacobi path.
 
 Bars: eigenvalues within 1e-12 ||A||, residual ||A v - lambda v|| within 1e-12 ||A||, eigenvectors
 orthonormal to 1e-10 (the Rayleigh-Ritz step only needs the spanned subspace, so phases are free)."""
+import dataclasses
 import os
 
 import numpy as np
@@ -168,3 +169,12 @@ def test_small_vectors_are_orthogonal_to_rounding(dz, m, nev):
     r = dz.hermitian_eigen_decomp(a, nev)
     _check(a, r, nev)
     assert np.abs(r.vectors.conj() @ r.vectors.T - np.eye(nev)).max() < 8 * m * np.finfo(float).eps
+
+
+@pytest.mark.parametrize("m", [1, 2, 31, 95, 96, 200])
+@pytest.mark.parametrize("scale", [0.0, 1e-140, 1e140])
+def test_zero_and_extreme_matrices(dz, m, scale):
+    """The vectors stay unit and orthogonal where ||T|| is zero or far from one."""
+    a = _rand_herm(m, seed=m)
+    r = dz.hermitian_eigen_decomp(scale * a, min(m, 40))
+    _check(a * (scale > 0), dataclasses.replace(r, values=r.values / (scale or 1.0)), min(m, 40))
