@@ -404,9 +404,13 @@ static int projector_product(dftcuda_kctx* c, GemmArgs& g, bool back, size_t nco
     c->err_used = true;
     DFT_TRY(zgemm_i8(g, s, &c->tc_scratch, c->d_err, &done, &uneven));
     c->p_i8[back] = done;
+    c->i8_ran = c->i8_ran || done;
     if (done) return DFTCUDA_OK;
   }
-  DFT_TRY(kctx_ensure_gemm_ws(c, ncols));
+  // A context whose residue workspace had to give way on a full device may not get this one either: it then does without
+  // (one K split).
+  const int ws = kctx_ensure_gemm_ws(c, ncols);
+  if (ws != DFTCUDA_OK && (ws != DFTCUDA_ERR_OUT_OF_MEMORY || !c->i8_ran)) return ws;
   return zgemm(g, s, c->d_gemm_ws, c->gemm_ws_elems);
 }
 

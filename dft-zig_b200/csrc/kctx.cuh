@@ -198,7 +198,8 @@ struct dftcuda_kctx {
   // the projector matrix converted for the two projector GEMMs: TF32 splits (TF32 and TF32X3 contexts), int8 residues
   dftcuda::TcScratch tc_ptiles_proj, tc_ptiles_back, i8_ptiles_proj, i8_ptiles_back;
   int p_products[2] = {0, 0};  // projections and back-projections made with the present projectors
-  bool p_i8[2] = {false, false};  // the last one of each ran on residues
+  bool p_i8[2] = {false, false};  // the last one of each ran on residues,
+  bool i8_ran = false;            // and any of this context's
   int natoms = 0;                   // atoms given to set_projectors
   std::vector<int> atom_row, atom_mt;  // per atom (set_projectors order): first projector row, row count
   std::vector<int> atom_species;       // per atom: species index

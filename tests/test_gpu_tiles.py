@@ -112,3 +112,55 @@ def test_first_products_keep_no_tiles(dz):
     grown = [b - a for a, b in zip(used, used[1:])]
     assert sum(g > tiles // 2 for g in grown) == 2 and not any(g > 1.5 * tiles for g in grown) and grown[0] < tiles // 2
     kc.close()
+
+
+def test_contexts_of_several_threads_on_a_full_device(dz):
+    """Two threads apply contexts that keep tiles while a third solves, again and again, on a context that needs what they
+    keep: tiles go and come back under the running calls, and every result is as before."""
+    import threading
+
+    held = [_with_projectors(dz, 512, seed=s) for s in (3, 4)]
+    n = held[0][0].ctx.n
+    x = torch.from_numpy(random_block(n, 500, 7)).cuda()
+    want = []
+    for _, kc in held:
+        for _ in range(8):
+            y = kc.apply_hamiltonian_batched(x, torch.empty_like(x))
+        want.append(y)
+    kp = kproblem("si8", 20.0, (0.25, 0.0, 0.0))
+    opts = dz.Options(max_iter=3, tol=1e-6)
+    kcs = [make_context(dz, kp) for _ in range(6)]
+    before = _free()
+    ref = kcs[0].hermitian_eigen_decomp_iterative(kp.ctx.basis.kinetic, 60, opts).values
+    need = before - _free()
+    out = [torch.empty_like(x) for _ in held]
+    filler = torch.empty(_free() - need // 2, dtype=torch.uint8, device="cuda")
+    errors = []
+
+    def guarded(work, *args):
+        try:
+            work(*args)
+        except Exception as e:  # noqa: BLE001 (reported by the main thread)
+            errors.append(repr(e))
+
+    def apply(i):
+        for _ in range(60):
+            held[i][1].apply_hamiltonian_batched(x, out[i])
+            bad = float((out[i] - want[i]).abs().max())
+            assert bad <= 1e-13 * float(want[i].abs().max()), bad
+
+    def solve():
+        for kc in kcs[1:]:
+            got = kc.hermitian_eigen_decomp_iterative(kp.ctx.basis.kinetic, 60, opts)
+            assert np.abs(got.values - ref).max() < 1e-9
+            kc.close()
+
+    threads = [threading.Thread(target=guarded, args=a) for a in ((apply, 0), (apply, 1), (solve,))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    del filler
+    for kc in [kcs[0]] + [h[1] for h in held]:
+        kc.close()
+    assert not errors, errors
