@@ -122,6 +122,8 @@ struct I8Even {
 // k_i8_norm with the evenness of the rows, the entries in registers.  KC: a warp takes 256 consecutive entries as a
 // neighbourhood (fewer than 32 at the end count as not good); else a thread takes 16 of its row (and what remains of
 // its chunk below 16 counts as not good).
+// Bound by its read: 1344 rows of 61565 entries in 216 us, 6.1 TB/s (a block per 2,048 entries with two block barriers
+// made the 1344 x 448 product 0.05 ms slower).
 template <bool KC>
 __global__ void __launch_bounds__(256) k_i8_norm_even(const double2* __restrict__ X, long ld, int R, int K, int kchunk,
                                                       double2* __restrict__ part, I8Even* __restrict__ even) {
